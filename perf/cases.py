@@ -21,10 +21,10 @@ from molds_gb300 import workloads as W
 # DIIS alone, as the batched water benchmark runs it (those clusters converge so) ...
 DIIS = dict(max_iter=500, rms_density=1e-8, damping_thresh=1.0, damping_weight=0.0, diis_start_error=0.1,
             diis_end_error=0.0)
-# ... and with the densities mixed first and the default DIIS start: what a user sets for
+# ... and with the densities mixed first (default weight and DIIS start): what a user sets for
 # larger clusters and branched alkanes, where DIIS alone can cycle; tight enough that the
 # forces do not carry what is left of the convergence
-DAMPED = dict(DIIS, damping_thresh=3e-3, damping_weight=0.7, diis_start_error=1e-2, rms_density=1e-10)
+DAMPED = dict(DIIS, damping_thresh=3e-3, damping_weight=0.8, diis_start_error=1e-2, rms_density=1e-10)
 # the mixed path to a tighter threshold, so that its result does not carry FP32 noise
 MIXED = dict(DAMPED, precision="mixed", rms_density=1e-11)
 SCF = {"diis": DIIS, "damped": DAMPED, "mixed": MIXED}
@@ -77,7 +77,7 @@ def draw(rng):
     if kind == "single":
         if rng.random() < 0.4:
             return {"kind": kind, "system": "alkane", "size": rng.randint(3, 16), "theory": "pm3", "scf": "damped",
-                    "epc": rng.choice([0, 0, _log_int(rng, 10, 2000)]), "forces": rng.random() < 0.6}
+                    "epc": rng.choice([0, 0, 3 * _log_int(rng, 4, 700)]), "forces": rng.random() < 0.6}
         k = _log_int(rng, 2, 120)
         return {"kind": kind, "system": "water", "size": k, "theory": theory,
                 "scf": "diis" if k <= 6 else "damped", "epc": 0, "forces": k < 100 and rng.random() < 0.4}
@@ -106,16 +106,16 @@ def _single(case, seed):
     else:
         mol = W.water_cluster_k(case["size"], seed)
     if case["epc"]:
-        # point charges of three-site waters (-0.834, 0.417, 0.417 e) in a shell around the molecule
+        # solvent around the molecule: three-site waters as point charges (-0.834, 0.417, 0.417 e)
         rng = np.random.default_rng(seed + 1)
-        n = case["epc"]
+        n = case["epc"] // 3
         c = mol.xyz.mean(axis=0)
-        inner = np.linalg.norm(mol.xyz - c, axis=1).max() + 5.0
-        d = rng.normal(size=(n, 3))
-        d /= np.linalg.norm(d, axis=1)[:, None]
+        inner = np.linalg.norm(mol.xyz - c, axis=1).max() + 6.0
+        d, h1, h2 = (v / np.linalg.norm(v, axis=1)[:, None] for v in rng.normal(size=(3, n, 3)))
         r = (inner ** 3 + rng.uniform(0.0, 1.0, n) * ((inner + 15.0) ** 3 - inner ** 3)) ** (1.0 / 3.0)
-        q = np.where(np.arange(n) % 3 == 0, -0.834, 0.417)
-        mol = M.Molecule(mol.Z, mol.xyz, np.column_stack([c + d * r[:, None], q]))
+        o = c + d * r[:, None]
+        pos = np.concatenate([o, o + 0.96 * M.ANG2AU * h1, o + 0.96 * M.ANG2AU * h2])
+        mol = M.Molecule(mol.Z, mol.xyz, np.column_stack([pos, np.repeat([-0.834, 0.417, 0.417], n)]))
     return mol
 
 
@@ -252,7 +252,7 @@ def work(case):
         k = case["size"]
         blk = 100 * k * (k - 1) / 2 + 10 * k * 2 * k + k * (2 * k - 1)
         return {"bytes": 8 * blk + 8 * (6 * k) ** 2 + 24 * 3 * k, "flops": 3000 * k * (k - 1) / 2}
-    its = {"diis": 14, "damped": 34, "mixed": 36}[case["scf"]]
+    its = {"diis": 14, "damped": 38, "mixed": 40}[case["scf"]]
     if kind in ("uneven", "server"):
         sizes = []
         for i, a in enumerate(np.exp(np.linspace(math.log(case["smallest"]), math.log(case["largest"]),
