@@ -71,20 +71,23 @@ __global__ void init_state_kernel(const DevMol* __restrict__ mols, const int* __
     }
 }
 
+// out[0] = molecules still active, out[1] = those of them that wait for the eigensolver
 __global__ void count_active_kernel(const int* __restrict__ list, int n, const MolState* __restrict__ st,
                                     int* __restrict__ out, char* __restrict__ active) {
-  __shared__ int cnt;
-  if (threadIdx.x == 0) cnt = 0;
+  __shared__ int cnt[2];
+  if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
   __syncthreads();
-  int c = 0;
+  int c = 0, w = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int a = (st[list[i]].status == kActive);
     active[list[i]] = (char)a;
     c += a;
+    w += a && (st[list[i]].flags & kNeedEigen);
   }
-  atomicAdd(&cnt, c);
+  atomicAdd(&cnt[0], c);
+  atomicAdd(&cnt[1], w);
   __syncthreads();
-  if (threadIdx.x == 0) *out = cnt;
+  if (threadIdx.x < 2) out[threadIdx.x] = cnt[threadIdx.x];
 }
 
 // ---------------------------------------------------------------------------
@@ -342,6 +345,12 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_td = dalloc<double>(3 * (size_t)vec, &bytes_);
   d_hh_small_ = dalloc<int>(nm, &bytes_);
   d_hh_large_ = dalloc<int>(nm, &bytes_);
+  for (int k = 0; k < 3; ++k) d_pur_list_[k] = dalloc<int>(nm, &bytes_);
+  d_pur_ = dalloc<PurState>(nm, &bytes_);
+  // 129 basis functions have four tiles; larger bases have fewer per element
+  pur_tile_cap_ = cap.max_n > kPurSmallMaxN ? (size_t)(mat / 4096) + 16 : 1;
+  d_pur_tiles_ = dalloc<int4>(pur_tile_cap_, &bytes_);
+  cuda_check(cudaHostAlloc(&h_pur_tiles_, sizeof(int4) * pur_tile_cap_, cudaHostAllocDefault), "cudaHostAlloc");
   grid_ctas_ = hh_grid_ctas();
   d_gridmap_ = dalloc<int>(3 * ((size_t)nm + grid_ctas_), &bytes_);
   cuda_check(cudaHostAlloc(&h_gridmap_, sizeof(int) * 3 * ((size_t)nm + grid_ctas_), cudaHostAllocDefault),
@@ -350,7 +359,7 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_state = dalloc<MolState>(nm, &bytes_);
   d_charges = dalloc<double>(cap.atoms, &bytes_);
   d_sweeps = dalloc<int>(nm, &bytes_);
-  d_count = dalloc<int>(1, &bytes_);
+  d_count = dalloc<int>(2, &bytes_);
   d_tc_err = dalloc<int>(1, &bytes_);
   {
     const size_t b = diis_scratch_bytes(nm);
@@ -388,7 +397,7 @@ void Batch::allocate(const BatchCapacity& cap) {
     bytes_ += b;
   }
   cuda_check(cudaHostAlloc(&h_bj_pending, sizeof(int), cudaHostAllocDefault), "cudaHostAlloc");
-  cuda_check(cudaHostAlloc(&h_block_count_, 2 * sizeof(int), cudaHostAllocDefault), "cudaHostAlloc");
+  cuda_check(cudaHostAlloc(&h_block_count_, 4 * sizeof(int), cudaHostAllocDefault), "cudaHostAlloc");
   cuda_check(cudaHostAlloc(&h_block_active_, 2 * (size_t)nm, cudaHostAllocDefault), "cudaHostAlloc");
   for (int k = 0; k < 2; ++k)
     cuda_check(cudaEventCreateWithFlags(&block_ev_[k], cudaEventDisableTiming), "cudaEventCreate");
@@ -398,7 +407,7 @@ void Batch::allocate(const BatchCapacity& cap) {
   JobSet* all[] = {&j_trans1_, &j_trans2_, &j_dens_, &j_w_, &j_kt_, &j_yt_, &j_m_, &j_d2_, &j_z_, &j_p_, &j_ns1_, &j_ns2_, &j_ov_, &j_hh_};
   for (JobSet* j : all) { j->d = dalloc<GemmJob>(job_cap_, &bytes_); j->cap = job_cap_; }
   cuda_check(cudaHostAlloc(&h_jobs_, sizeof(GemmJob) * (size_t)job_cap_ * 14, cudaHostAllocDefault), "cudaHostAlloc jobs");
-  cuda_check(cudaHostAlloc(&h_lists_, sizeof(int) * (size_t)nm * (kJacobiBuckets + 3), cudaHostAllocDefault),
+  cuda_check(cudaHostAlloc(&h_lists_, sizeof(int) * (size_t)nm * (kJacobiBuckets + 6), cudaHostAllocDefault),
              "cudaHostAlloc lists");
   for (int b = 0; b < kJacobiBuckets; ++b) d_bucket_lists_.push_back(dalloc<int>(nm, &bytes_));
   cuda_check(cudaStreamSynchronize(stream_), "allocate");
@@ -487,7 +496,7 @@ void Batch::release(int slot) {
 }
 
 Batch::~Batch() {
-  if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
+  for (cudaGraphExec_t g : graph_exec_) if (g) cudaGraphExecDestroy(g);
   for (cudaEvent_t e : block_ev_) if (e) cudaEventDestroy(e);
   if (h_block_count_) cudaFreeHost(h_block_count_);
   if (h_block_active_) cudaFreeHost(h_block_active_);
@@ -505,7 +514,8 @@ Batch::~Batch() {
   for (void* p : ptrs) if (p) cudaFree(p);
   for (int i = 0; i < 6; ++i) if (d_S[i]) cudaFree(d_S[i]);
   if (d_td) cudaFree(d_td);
-  void* hh[] = {d_hh_small_, d_hh_large_, d_gridmap_, d_gridbar_, d_pgrad_, d_forces_};
+  if (h_pur_tiles_) cudaFreeHost(h_pur_tiles_);
+  void* hh[] = {d_pur_list_[0], d_pur_list_[1], d_pur_list_[2], d_pur_, d_pur_tiles_, d_hh_small_, d_hh_large_, d_gridmap_, d_gridbar_, d_pgrad_, d_forces_};
   for (void* p : hh) if (p) cudaFree(p);
   if (h_gridmap_) cudaFreeHost(h_gridmap_);
 }
@@ -617,6 +627,20 @@ void Batch::build_jobs(const std::vector<int>& which) {
       hh_large_max_k_ = std::max(hh_large_max_k_, kd);
     }
   }
+  // purification lists and tiles
+  for (int k = 0; k < 3; ++k) { pur_list_[k].clear(); pur_max_n_[k] = 0; }
+  pur_tiles_.clear();
+  for (int m : which) {
+    const int n = h_mols[m].nao, k = n <= 64 ? 0 : (n <= kPurSmallMaxN ? 1 : 2);
+    pur_list_[k].push_back(m);
+    pur_max_n_[k] = std::max(pur_max_n_[k], n);
+    if (k == 2) {
+      const size_t t = pur_tiles_.size();
+      pur_tiles_.resize(t + purify_tiles(m, n, nullptr));
+      purify_tiles(m, n, pur_tiles_.data() + t);
+    }
+  }
+  if (pur_tiles_.size() > pur_tile_cap_) throw std::logic_error("purification tile table overflow");
   // chunks of at most grid_ctas_ molecules and their CTA maps
   grid_chunks_.clear();
   int off = 0;
@@ -657,6 +681,18 @@ void Batch::upload_list(const std::vector<int>& which) {
     int* stage = h_lists_ + (size_t)(kJacobiBuckets + 1) * nm;
     std::copy(hh_small_.begin(), hh_small_.end(), stage);
     std::copy(hh_large_.begin(), hh_large_.end(), stage + nm);
+    for (int k = 0; k < 3; ++k) {
+      int* ps = stage + (size_t)(2 + k) * nm;
+      std::copy(pur_list_[k].begin(), pur_list_[k].end(), ps);
+      if (!pur_list_[k].empty())
+        cuda_check(cudaMemcpyAsync(d_pur_list_[k], ps, pur_list_[k].size() * sizeof(int), cudaMemcpyHostToDevice, stream_),
+                   "upload list");
+    }
+    if (!pur_tiles_.empty()) {
+      std::copy(pur_tiles_.begin(), pur_tiles_.end(), h_pur_tiles_);
+      cuda_check(cudaMemcpyAsync(d_pur_tiles_, h_pur_tiles_, pur_tiles_.size() * sizeof(int4), cudaMemcpyHostToDevice,
+                                 stream_), "upload tiles");
+    }
     if (!hh_small_.empty())
       cuda_check(cudaMemcpyAsync(d_hh_small_, stage, hh_small_.size() * sizeof(int), cudaMemcpyHostToDevice, stream_),
                  "upload list");
@@ -714,7 +750,7 @@ const char* kernel_class_name(int k) {
   static const char* names[kKNumClasses] = {"pair_integrals", "core_hamiltonian", "fock_build", "basis_orthonormalise",
                                             "warm_start_transform", "jacobi_eigensolver", "density", "fp64_refinement",
                                             "diis", "energy", "dipole", "tridiagonalisation",
-                                            "tridiagonal_eigenvectors"};
+                                            "tridiagonal_eigenvectors", "purification"};
   return (k >= 0 && k < kKNumClasses) ? names[k] : "?";
 }
 
@@ -795,6 +831,8 @@ double Batch::active_work_estimate(int cls) const {
       case kKTridiag: w += 4.0 / 3.0 * n * n * n; break;
       // back-transformation of the k = min(o, v) density vectors (2 N^2 k flops)
       case kKEigvec: w += 2.0 * n * n * std::min(o, v); break;
+      // P from F: the same count as the eigensolve and density it stands in for
+      case kKPurify: w += 4.0 / 3.0 * n * n * n + 3.0 * n * n * std::min(o, v); break;
       case kKTransform: w += 4.0 * n * n * n; break;
       case kKOrtho: w += 4.0 * n * n * n; break;
       case kKDensity: w += 2.0 * n * n * o; break;
@@ -1021,26 +1059,49 @@ void Batch::hh_vectors(const ScfSettings& s, int final_pass, int require_active)
   }
 }
 
-void Batch::eigen_step(const ScfSettings& s) {
+// FP64 Householder tridiagonalisation (one launch per size bucket, each with
+// its own shared-memory footprint)
+void Batch::hh_reduce(int require) {
+  for (size_t b = 0; b < buckets_.size(); ++b) {
+    if (bucket_hh_max_n_[b] == 0) continue;
+    launches_ += 1;
+    launch_hh_tridiag(d_mols, bucket_dev_[b], (int)buckets_[b].size(), bucket_hh_max_n_[b], d_state, require, d_F, d_G64,
+                      d_td, vec_total_, d_S[4], hh_served_max_n_, stream_);
+  }
+  // the whole-GPU path: each chunk's molecules share one cooperative launch
+  for (const GridChunk& c : grid_chunks_) {
+    launches_ += 1;
+    launch_hh_grid_tridiag(d_mols, d_hh_large_ + c.first, d_gridmap_ + c.map_off, c.nctas, c.count, d_state, require,
+                           d_F, d_G64, d_td, vec_total_, d_S[4], d_S[5], d_gridbar_, stream_);
+  }
+}
+
+bool Batch::purified(const ScfSettings& s) const { return s.eigensolver == 0 && householder(s); }
+
+void Batch::eigen_step(const ScfSettings& s, bool eigen) {
   if (householder(s)) {
-    // FP64 Householder tridiagonalisation (one launch per size bucket, each
-    // with its own shared-memory footprint), then the density's eigenpairs
-    int h = prof_begin(kKTridiag, active_work_estimate(kKTridiag));
-    for (size_t b = 0; b < buckets_.size(); ++b) {
-      if (bucket_hh_max_n_[b] == 0) continue;
-      launches_ += 1;
-      launch_hh_tridiag(d_mols, bucket_dev_[b], (int)buckets_[b].size(), bucket_hh_max_n_[b], d_state, 1, d_F, d_G64,
-                        d_td, vec_total_, d_S[4], hh_served_max_n_, stream_);
+    // the purification gives the density itself; the eigenpairs then only
+    // serve the molecules it could not treat (eigen: launch them as well)
+    const int require = purified(s) ? 2 : 1;
+    if (purified(s)) {
+      const int h = prof_begin(kKPurify, active_work_estimate(kKPurify));
+      for (int k = 0; k < 2; ++k) {
+        launches_ += !pur_list_[k].empty();
+        launch_purify_small(d_mols, d_pur_list_[k], (int)pur_list_[k].size(), pur_max_n_[k], d_state, d_F, d_P,
+                            d_tc_err, stream_);
+      }
+      const PurScratch ws{{d_T64, d_S[0], d_S[1], d_S[2], d_S[3], d_S[4], d_S[5]}};
+      launches_ += launch_purify_big(d_mols, d_pur_list_[2], (int)pur_list_[2].size(), pur_max_n_[2], d_pur_tiles_,
+                                     (int)pur_tiles_.size(), d_state, d_F, d_P, d_pur_, ws, kPurBigSteps, d_tc_err,
+                                     stream_);
+      prof_end(h);
+      if (!eigen) return;
     }
-    // the whole-GPU path: each chunk's molecules share one cooperative launch
-    for (const GridChunk& c : grid_chunks_) {
-      launches_ += 1;
-      launch_hh_grid_tridiag(d_mols, d_hh_large_ + c.first, d_gridmap_ + c.map_off, c.nctas, c.count, d_state, 1,
-                             d_F, d_G64, d_td, vec_total_, d_S[4], d_S[5], d_gridbar_, stream_);
-    }
+    int h = prof_begin(kKTridiag, purified(s) ? 0.0 : active_work_estimate(kKTridiag));
+    hh_reduce(require);
     prof_end(h);
-    h = prof_begin(kKEigvec, active_work_estimate(kKEigvec));
-    hh_vectors(s, 0, 1);
+    h = prof_begin(kKEigvec, purified(s) ? 0.0 : active_work_estimate(kKEigvec));
+    hh_vectors(s, 0, require);
     prof_end(h);
   } else if (s.precision == 0) {
     // size buckets on the cluster Jacobi (a few molecules) form G = C F C^T
@@ -1111,12 +1172,15 @@ void Batch::density_step(const ScfSettings& s) {
     // on the CUDA cores; in the FP32 phase of the mixed path from the FP32
     // rows on the tensor cores (3xTF32, FP32 accumulation)
     const bool mixed = s.precision == 1;
-    int h = prof_begin(kKDensity, active_work_estimate(kKDensity));
+    const int require = purified(s) ? 2 : 1;
+    int h = prof_begin(kKDensity, purified(s) ? 0.0 : active_work_estimate(kKDensity));
     launches_ += 1;
-    launch_gemm(j_hh_.d, j_hh_.n, j_hh_.tiles, d_C, d_C, d_P, true, false, 0.0, d_state, 1, mixed ? 1 : -1, stream_);
+    launch_gemm(j_hh_.d, j_hh_.n, j_hh_.tiles, d_C, d_C, d_P, true, false, 0.0, d_state, require, mixed ? 1 : -1,
+                stream_);
     if (mixed) {
       launches_ += 1;
-      launch_tc_gemm(j_hh_.d, j_hh_.n, j_hh_.tc_tiles, d_Cf, d_Cf, d_P, true, false, d_state, 1, 0, d_tc_err, stream_);
+      launch_tc_gemm(j_hh_.d, j_hh_.n, j_hh_.tc_tiles, d_Cf, d_Cf, d_P, true, false, d_state, require, 0, d_tc_err,
+                     stream_);
     }
     prof_end(h);
   } else if (s.precision == 0) {
@@ -1160,7 +1224,7 @@ void Batch::density_step(const ScfSettings& s) {
   cuda_check(cudaGetLastError(), "density step");
 }
 
-void Batch::iterate(const ScfSettings& s, const std::vector<int>& which) {
+void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, bool eigen) {
   upload_list(which);
   const int nl = (int)which.size();
   launches_ += 4;   // fock + three DIIS kernels
@@ -1169,10 +1233,12 @@ void Batch::iterate(const ScfSettings& s, const std::vector<int>& which) {
                      1, 1, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "fock_kernel");
-  eigen_step(s);
-  density_step(s);
+  eigen_step(s, eigen);
+  if (eigen || !purified(s)) density_step(s);
   h = prof_begin(kKDiis, active_work_estimate(kKDiis));
-  launch_diis(d_mols, d_list, nl, d_state, to_dev(s), d_P, d_Pold, d_hist_dens, d_hist_err, mat_total_,
+  ScfParamsDev prm = to_dev(s);
+  prm.eigen_ran = eigen || !purified(s);
+  launch_diis(d_mols, d_list, nl, d_state, prm, d_P, d_Pold, d_hist_dens, d_hist_err, mat_total_,
               s.keep_trace ? d_trace : nullptr, max_iter_alloc_, d_diis_ws, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "diis_kernel");
@@ -1190,39 +1256,45 @@ bool same_launches(const ScfSettings& a, const ScfSettings& b) {
 // settings, and every kernel reads the per-molecule state from device memory,
 // so an iteration captured once can be replayed: one graph launch instead of
 // a dozen kernel launches.  Not while profiling (per-launch events), nor on the
-// block Jacobi, which reads a host flag between its sweeps, nor for lists with
-// a molecule on the whole-GPU eigensolver (its cooperative launches run long
-// enough that a launch costs nothing, and are not captured).
-void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which) {
+// block Jacobi, which reads a host flag between its sweeps, nor for an iteration
+// with a molecule on the whole-GPU eigensolver (its cooperative launches run long
+// enough that a launch costs nothing, and are not captured).  The iterations
+// with and without the eigensolver launches are two graphs.
+void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which, bool eigen) {
   upload_list(which);   // outside any capture: may synchronise when the list changes
-  if (!s.graphs || prof_on_ || !householder(s) || !hh_large_.empty()) {
-    iterate(s, which);
+  if (!s.graphs || prof_on_ || !householder(s) || ((eigen || !purified(s)) && !hh_large_.empty())) {
+    iterate(s, which, eigen);
     return;
   }
-  if (!graph_exec_ || !same_launches(graph_settings_, s) || graph_layout_ != layout_version_) {
-    if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
+  if (!same_launches(graph_settings_, s) || graph_layout_ != layout_version_) {
+    for (cudaGraphExec_t& g : graph_exec_)
+      if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    graph_settings_ = s;
+    graph_layout_ = layout_version_;
+  }
+  cudaGraphExec_t& exec = graph_exec_[eigen];
+  if (!exec) {
     hh_prepare();
+    purify_prepare();
     const long long before = launches_;
     cudaGraph_t g = nullptr;
     cuda_check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
-      iterate(s, which);
+      iterate(s, which, eigen);
     } catch (...) {
       cudaStreamEndCapture(stream_, &g);
       if (g) cudaGraphDestroy(g);
       throw;
     }
     cuda_check(cudaStreamEndCapture(stream_, &g), "end capture");
-    const cudaError_t e = cudaGraphInstantiate(&graph_exec_, g, 0);
+    const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     cuda_check(e, "graph instantiate");
-    graph_kernels_ = launches_ - before;
+    graph_kernels_[eigen] = launches_ - before;
     launches_ = before;
-    graph_settings_ = s;
-    graph_layout_ = layout_version_;
   }
-  cuda_check(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
-  launches_ += graph_kernels_;
+  cuda_check(cudaGraphLaunch(exec, stream_), "graph launch");
+  launches_ += graph_kernels_[eigen];
   ++graph_launches_;
 }
 
@@ -1245,7 +1317,7 @@ void Batch::count_active_async(const std::vector<int>& which, int* h_count, char
   upload_list(which);
   launches_ += 1;
   count_active_kernel<<<1, 256, 0, stream_>>>(d_list, (int)which.size(), d_state, d_count, d_active);
-  cuda_check(cudaMemcpyAsync(h_count, d_count, sizeof(int), cudaMemcpyDeviceToHost, stream_), "count copy");
+  cuda_check(cudaMemcpyAsync(h_count, d_count, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "count copy");
   cuda_check(cudaMemcpyAsync(h_active, d_active, h_mols.size(), cudaMemcpyDeviceToHost, stream_), "active copy");
   cuda_check(cudaEventRecord(done, stream_), "count event");
 }
@@ -1265,6 +1337,7 @@ void Batch::finish(const ScfSettings& s, const std::vector<int>& which) {
   const int max_atoms = list_max_atoms();
   // every eigenpair of the last diagonalised Fock matrix: MO energies and
   // eigenvector rows, as Dsyevd leaves them after the last iteration
+  if (purified(s)) hh_reduce(0);   // the SCF itself needed no tridiagonalisation
   if (householder(s)) hh_vectors(s, 1, 0);
   launches_ += 2;
   int h = prof_begin(kKEnergy, 0.0);
@@ -1296,20 +1369,30 @@ void Batch::scf(const ScfSettings& s, bool requires_guess) {
   // so the device never waits for the host.  Every kernel of an iteration
   // skips molecules that are no longer active, so the iterations enqueued past
   // convergence change nothing (and cost only their empty launches).
+  // A molecule that the purification cannot treat waits without advancing until
+  // the host has read that count too and enqueues an iteration with the
+  // eigensolver; from the second such wait on every iteration has it.
   const int block = all.size() == 1 ? 3 : tuned_check_block();
-  int it = 0, nblock = 0;
-  while (it < s.max_iter) {
-    for (int b = 0; b < block && it < s.max_iter; ++b, ++it) iterate_graph(s, all);
+  const bool pur = purified(s);
+  int it = 0, nblock = 0, waits = 0;
+  bool eigen = false;
+  for (;;) {
+    // past max_iter only molecules that waited are still active
+    for (int b = 0; b < block && (b == 0 || it < s.max_iter); ++b, ++it) iterate_graph(s, all, eigen && (b == 0 || waits > 1));
+    const bool last = it >= s.max_iter;
     const int slot = nblock & 1;
-    count_active_async(all, h_block_count_ + slot, h_block_active_ + (size_t)slot * cap_.slots, block_ev_[slot]);
+    count_active_async(all, h_block_count_ + 2 * slot, h_block_active_ + (size_t)slot * cap_.slots, block_ev_[slot]);
     ++nblock;
-    if (nblock >= 2) {
-      const int prev = (nblock - 2) & 1;
-      cuda_check(cudaEventSynchronize(block_ev_[prev]), "block count");
-      if (prof_on_) std::copy(h_block_active_ + (size_t)prev * cap_.slots,
-                              h_block_active_ + (size_t)prev * cap_.slots + h_mols.size(), active_host_.begin());
-      if (h_block_count_[prev] == 0) break;
-    }
+    if (last && !pur) break;
+    if (nblock < 2 && !last) continue;
+    const int seen = last ? slot : slot ^ 1;
+    cuda_check(cudaEventSynchronize(block_ev_[seen]), "block count");
+    if (prof_on_) std::copy(h_block_active_ + (size_t)seen * cap_.slots,
+                            h_block_active_ + (size_t)seen * cap_.slots + h_mols.size(), active_host_.begin());
+    if (h_block_count_[2 * seen] == 0) break;
+    const bool waiting = h_block_count_[2 * seen + 1] > 0;
+    waits += waiting && !eigen;
+    eigen = waiting || waits > 1;
   }
   finish(s, all);
   int tc_err = 0;

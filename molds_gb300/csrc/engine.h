@@ -47,7 +47,7 @@ bool same_launches(const ScfSettings& a, const ScfSettings& b);
 // kernel classes timed by the optional per-launch CUDA-event profiler
 enum KernelClass {
   kKPair = 0, kKHcore, kKFock, kKOrtho, kKTransform, kKJacobi, kKDensity, kKRefine, kKDiis, kKEnergy, kKDipole,
-  kKTridiag, kKEigvec, kKNumClasses
+  kKTridiag, kKEigvec, kKPurify, kKNumClasses
 };
 const char* kernel_class_name(int k);
 
@@ -107,8 +107,8 @@ class Batch {
   static size_t bytes_per_mat_element(int diis_m);
   // pair integrals, H and core-core energy of the listed molecules
   void integrals(const std::vector<int>& which);
-  // count_active without a host wait: the count and per-slot active flags land
-  // in pinned host memory, and `done` is recorded after the copies
+  // count_active without a host wait: the counts (active, waiting for the
+  // eigensolver) and per-slot active flags land in pinned host memory, and `done` is recorded after the copies
   void count_active_async(const std::vector<int>& which, int* h_count, char* h_active, cudaEvent_t done);
   // asynchronous copies into pinned host memory (complete at the next stream sync)
   void copy_states_async(MolState* host);
@@ -124,15 +124,16 @@ class Batch {
   void scf(const ScfSettings& s, bool requires_guess);
   // Initialise the SCF state of the listed molecules (serving: admission).
   void begin(const ScfSettings& s, const std::vector<int>& which, bool requires_guess);
-  // One SCF iteration over the listed (active) molecules.
-  void iterate(const ScfSettings& s, const std::vector<int>& which);
+  // One SCF iteration over the listed (active) molecules; eigen: the eigensolver
+  // serves the molecules whose density the purification cannot give
+  void iterate(const ScfSettings& s, const std::vector<int>& which, bool eigen = false);
   // Energies / charges of the listed molecules after convergence.
   void finish(const ScfSettings& s, const std::vector<int>& which);
   // Number of still-active molecules among `which` (synchronises).
   int count_active(const std::vector<int>& which);
   // One SCF iteration, replayed from a captured CUDA graph when the settings
   // allow it (iterate() otherwise)
-  void iterate_graph(const ScfSettings& s, const std::vector<int>& which);
+  void iterate_graph(const ScfSettings& s, const std::vector<int>& which, bool eigen = false);
   long long graph_launches() const { return graph_launches_; }
 
   // results (synchronise and copy out)
@@ -170,7 +171,11 @@ class Batch {
   int list_max_atoms() const;   // largest molecule (atoms) of the current list
   void build_jobs(const std::vector<int>& which);
   void upload_list(const std::vector<int>& which);
-  void eigen_step(const ScfSettings& s);
+  void eigen_step(const ScfSettings& s, bool eigen);
+  // the current list's Householder tridiagonalisations of F (require: see mol_skipped)
+  void hh_reduce(int require);
+  // density by purification, the eigensolver only for molecules it leaves over
+  bool purified(const ScfSettings& s) const;
   void density_step(const ScfSettings& s);
   // FP64 Householder path (tridiag.cu): used for this list and these settings
   bool householder(const ScfSettings& s) const;
@@ -223,6 +228,16 @@ class Batch {
   int* d_hh_large_ = nullptr;
   int hh_small_max_n_ = 0, hh_small_max_k_ = 0;
   int hh_large_max_n_ = 0, hh_large_max_k_ = 0;
+  // purification: molecules on the one-CTA kernel (up to 64, up to kPurSmallMaxN
+  // basis functions) and on the tile kernel, with the latter's tiles
+  std::vector<int> pur_list_[3];
+  int* d_pur_list_[3] = {};
+  int pur_max_n_[3] = {};
+  std::vector<int4> pur_tiles_;
+  int4* d_pur_tiles_ = nullptr;
+  int4* h_pur_tiles_ = nullptr;          // pinned staging of d_pur_tiles_
+  size_t pur_tile_cap_ = 0;
+  PurState* d_pur_ = nullptr;
   std::vector<int> bucket_hh_max_n_;     // per size bucket: largest basis on the per-molecule kernels
   int hh_served_max_n_ = 0;              // the per-molecule kernels serve bases up to this; larger: whole-GPU kernels
   // whole-GPU path: the large molecules in chunks of at most one per SM, each
@@ -269,11 +284,11 @@ class Batch {
   void make_jobset(JobSet* js, const std::vector<GemmJob>& jobs);
 
   // captured SCF iteration
-  cudaGraphExec_t graph_exec_ = nullptr;
+  cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};   // without and with the eigensolver launches
   ScfSettings graph_settings_;
   long long graph_layout_ = -1;           // layout_version_ the graph was captured for
   long long layout_version_ = 0;          // bumped whenever the job tables and size buckets are rebuilt
-  long long graph_kernels_ = 0;           // kernels in one replay
+  long long graph_kernels_[2] = {0, 0};   // kernels in one replay
   long long graph_launches_ = 0;          // replays so far
   // pipelined convergence checks: pinned counts and their events (two blocks in flight)
   int* h_block_count_ = nullptr;

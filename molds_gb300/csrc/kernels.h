@@ -128,6 +128,24 @@ void launch_jacobi_f64(const DevMol* mols, const int* mol_list, int nlist, int m
 // tridiag.cu: FP64 Householder tridiagonalisation + bisection + inverse
 // iteration + back-transformation.  td holds d, e, tau of every molecule at
 // vec0, vec0 + vstride, vec0 + 2 vstride; W (N x N arena) the reflectors.
+// Purification (purify.cu): P = 2 (projector on the nocc lowest eigenvectors of
+// F) of the listed active molecules; sets or clears kNeedEigen in their state.
+constexpr int kPurSmallMaxN = 128;   // one CTA per molecule up to here, tiles of every step above
+constexpr int kPurBigSteps = 56;     // steps launched above kPurSmallMaxN: HOMO-LUMO gaps down to ~3e-4 of the interval
+struct PurState {
+  unsigned long long lo, hi;         // Gershgorin interval, order-preserving keys
+  long long trace[kPurBigSteps + 1]; // tr X_k
+};
+struct PurScratch { double* m[7]; }; // N x N scratch matrices holding two digit buffers of seven digits each
+void purify_prepare();               // one-time kernel attributes (before any stream capture)
+int purify_tiles(int mol, int n, int4* out);   // tiles of one molecule (out may be null); returns their number
+void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
+                         double* P, int* err, cudaStream_t s);
+// returns the number of kernels launched
+int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
+                      MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
+                      int* err, cudaStream_t s);
+
 int hh_smem_max_n();     // largest basis whose packed matrix fits one CTA's shared memory
 int hh_back_max_n();     // largest basis the back-transformation kernel serves
 void hh_prepare();       // one-time kernel attributes and device limits (before any stream capture)

@@ -42,6 +42,10 @@ struct DevMol {
 // SCF state machine of one molecule (MolDS Cndo2::DoSCF, src/cndo/Cndo2.cpp:585-729)
 enum MolStatus { kActive = 0, kConverged = 1, kNotConverged = 2, kFailed = 3 };
 
+// MolState::flags: the purification gave no density.  The molecule then waits,
+// its state untouched, for an iteration that runs the eigensolver as well.
+constexpr int kNeedEigen = 1;
+
 struct MolState {
   int iter;           // iteration about to run / running
   int status;
@@ -59,6 +63,12 @@ struct MolState {
   double ecore_epc;   // Coulomb energy of the cores in the point charges' field
 };
 
+// Which molecules a launch serves: require 0 all, 1 the active ones, 2 the
+// active ones the purification left to the eigensolver.
+__device__ __forceinline__ bool mol_skipped(const MolState& s, int require) {
+  return require && (s.status != kActive || (require == 2 && !(s.flags & kNeedEigen)));
+}
+
 struct TraceEntry {
   double rms, diis_err;
   int diis_on, damp_on;
@@ -70,7 +80,7 @@ struct ScfParamsDev {
   double rms_density, damping_thresh, damping_weight, diis_start, diis_end;
   double switch_error;      // mixed precision: FP64 phase once the DIIS error is below this
   int precision;            // 0 = FP64 throughout, 1 = mixed
-  int pad;
+  int eigen_ran;            // the eigensolver served the molecules flagged kNeedEigen this iteration
 };
 
 __host__ __device__ inline long long pair_index(int a, int b, int natoms) {

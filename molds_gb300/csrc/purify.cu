@@ -1,0 +1,720 @@
+// Density matrix by spectral purification on the tensor cores.
+//
+// The SCF needs P = 2 (projector on the nocc lowest eigenvectors of F).  The
+// SP2 iteration (A. M. N. Niklasson, Phys. Rev. B 66, 155115 (2002)) reaches
+// the projector from X_0 = (hi - F) / (hi - lo), [lo, hi] a Gershgorin
+// interval of F, by X <- X^2 when tr X > nocc and X <- 2 X - X^2 otherwise:
+// one symmetric matrix product per step, 18 to 24 steps for the HOMO-LUMO gaps
+// of converging molecules.
+//
+// Why: GB300 issues two FP64 FMAs per clock and SM but 4096 FP16 ones on its
+// tensor cores.  X has its spectrum in [0, 1], so |X_ij| <= 1 and it can be
+// held in fixed point: 64-bit integers with 55 fraction bits.  Each is split
+// into seven signed 8-bit digits, X = sum_i d_i 2^(-7-8i), which FP16 holds
+// exactly.  A product of two digits has 14 bits, a sum of up to K of them stays
+// an integer that FP32 holds exactly, so tcgen05 MMAs with FP32 accumulators
+// multiply the digit matrices without any rounding (the error-free splitting of
+// Ozaki, Ogita, Oishi & Rump, Numer. Algorithms 59, 95 (2012)).  Level l sums
+// the digit products with i + j = l, levels 0 to 7 are kept (34 products) and
+// recombined in 64-bit integers.  What is dropped is below 2^-70 times the
+// number of terms, and each step's result is rounded once, at 2^-56 absolute:
+// finer than FP64's rounding of entries of order one.  Integer sums do not
+// depend on their order, so X stays exactly symmetric and a molecule's result
+// does not depend on its batch.
+//
+// The error of the last step is known from the traces: tr X_{k+1} - tr X_k is
+// +- tr(X_k - X_k^2), the sum of lambda (1 - lambda).  Once that is below 2^-30
+// one step of each kind squares what is left on both sides (4e-18).  A molecule
+// that does not get there, or to the wrong rank (a vanishing gap, a non-finite
+// F), is flagged and waits for an iteration with the Householder eigensolver
+// (tridiag.cu).
+//
+// MolDS's counterpart: Dsyevd and CalcOrbitalElectronPopulation
+// (src/cndo/Cndo2.cpp:652-656, 1702-1719).
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <algorithm>
+#include <mutex>
+#include "nddo_batch.cuh"
+#include "kernels.h"
+
+namespace nddo {
+
+constexpr int kDigits = 7, kLevels = 8;
+constexpr int kPurSmallThreads = 512;
+constexpr int kPurSmallSteps = 100;                // the one-CTA kernel stops by itself; its steps are cheap
+constexpr long long kPurWaitCycles = 2000000000LL; // ~1 s: a copy or an MMA that has not completed by then never will
+constexpr int kTraceShift = 12;                    // traces are summed in units of 2^-43
+constexpr long long kTraceOne = 1LL << (55 - kTraceShift);
+constexpr long long kTraceTol = kTraceOne >> 30;   // tr(X - X^2) that two more steps square away
+
+__device__ __forceinline__ uint32_t pu_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Operand descriptors: K-major, no swizzle; core matrices of 8 rows x 16 bytes,
+// K-adjacent ones 128 bytes apart, 8-row groups sbo apart.  Only the low word
+// depends on the address: the issuing thread adds to it and nothing else, since
+// its instruction stream has to keep up with one MMA per few dozen clocks.
+__device__ __forceinline__ uint32_t pu_desc_lo(uint32_t addr) { return (addr >> 4) | (128u >> 4) << 16; }
+__device__ __forceinline__ uint32_t pu_desc_hi(uint32_t sbo) { return (sbo >> 4) | 1u << 14; }
+
+__device__ __forceinline__ void pu_mma(uint32_t tmem, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n mov.b64 da, {%1, %3};\n"
+               " mov.b64 db, {%2, %3};\n tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}"
+               :: "r"(tmem), "r"(a), "r"(b), "r"(hi), "r"(idesc), "r"(acc) : "memory");
+}
+
+// kind::f16: D = F32, A = B = F16, both K-major, M = 128
+__device__ __forceinline__ uint32_t pu_idesc(int ncols) {
+  return (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+
+__device__ __forceinline__ bool pu_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done = 0;
+  const long long t0 = clock64();
+  while (!done && clock64() - t0 < kPurWaitCycles)
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+
+__device__ __forceinline__ void pu_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void pu_ld8(uint32_t addr, float* v) {
+  uint32_t u[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+               : "r"(addr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(u[i]);
+}
+
+__device__ __forceinline__ long long pu_mad(int a, int b, long long c) {
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+
+// the eight levels of eight columns, recombined: units of 2^-55, level l weighs 2^(41 - 8 l)
+__device__ __forceinline__ void pu_gather8(uint32_t addr, int stride, long long* s) {
+  float v[4][8];
+#pragma unroll
+  for (int l = 0; l < 4; ++l) pu_ld8(addr + l * stride, v[l]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    s[i] = pu_mad(__float2int_rn(v[0][i]), 1 << 24,
+                  pu_mad(__float2int_rn(v[1][i]), 1 << 16,
+                         pu_mad(__float2int_rn(v[2][i]), 1 << 8, (long long)__float2int_rn(v[3][i])))) << 17;
+#pragma unroll
+  for (int l = 0; l < 4; ++l) pu_ld8(addr + (l + 4) * stride, v[l]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int t = (__float2int_rn(v[2][i]) + (__float2int_rn(v[3][i]) >> 8) + 64) >> 7;
+    s[i] = pu_mad(__float2int_rn(v[0][i]), 1 << 9, pu_mad(__float2int_rn(v[1][i]), 2, s[i] + t));
+  }
+}
+
+// Balanced base-256 digits of eight values as FP16, most significant slice
+// first.  With 128 added to every digit they are the bytes of one 64-bit word
+// (the top one up to 256), and 0x6400 | byte is the FP16 number 1024 + byte.
+__device__ __forceinline__ void pu_split8(const long long* x, uint4* out) {
+  uint32_t w[kDigits][4];
+  constexpr uint32_t kBias = 0x64806480u;   // two times 1024 + 128
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const unsigned long long a = (unsigned long long)x[2 * p] + 0x0080808080808080ull;
+    const unsigned long long b = (unsigned long long)x[2 * p + 1] + 0x0080808080808080ull;
+    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+#pragma unroll
+    for (int d = 0; d < kDigits; ++d) {
+      const int byte = 6 - d;
+      uint32_t v;
+      if (d == 0) v = (ah >> 16) | (bh & 0xFFFF0000u);   // 0 .. 256: nine bits
+      else if (byte >= 4) v = __byte_perm(ah, bh, (byte - 4) | (byte << 8)) & 0x00FF00FFu;
+      else v = __byte_perm(al, bl, byte | ((byte + 4) << 8)) & 0x00FF00FFu;
+      v += 0x64006400u;
+      asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(w[d][p]) : "r"(v), "r"(kBias));
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < kDigits; ++d) out[d] = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+}
+
+// eight values back from their digits
+__device__ __forceinline__ void pu_join8(const uint4* in, long long* x) {
+  constexpr uint32_t kBias = 0x64806480u;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    uint32_t b[kDigits];   // digit + 128 of both values in the halves
+#pragma unroll
+    for (int d = 0; d < kDigits; ++d) {
+      const uint32_t u = p == 0 ? in[d].x : p == 1 ? in[d].y : p == 2 ? in[d].z : in[d].w;
+      asm("add.rn.f16x2 %0, %1, %2;" : "=r"(b[d]) : "r"(u), "r"(kBias));
+    }
+    // low halves, then high halves; the top digit keeps nine bits
+    const uint32_t lo0 = __byte_perm(__byte_perm(b[6], b[5], 0x0040), __byte_perm(b[4], b[3], 0x0040), 0x5410);
+    const uint32_t hi0 = (__byte_perm(b[2], b[1], 0x0040) & 0xFFFFu) | ((b[0] - 0x6400u) << 16);
+    const uint32_t lo1 = __byte_perm(__byte_perm(b[6], b[5], 0x0062), __byte_perm(b[4], b[3], 0x0062), 0x5410);
+    const uint32_t hi1 = (__byte_perm(b[2], b[1], 0x0062) & 0xFFFFu) | (((b[0] >> 16) - 0x6400u) << 16);
+    x[2 * p] = (long long)((unsigned long long)hi0 << 32 | lo0) - 0x0080808080808080LL;
+    x[2 * p + 1] = (long long)((unsigned long long)hi1 << 32 | lo1) - 0x0080808080808080LL;
+  }
+}
+
+__device__ __forceinline__ long long pu_fixed(double v) { return __double2ll_rn(v * 36028797018963968.0); }   // 2^55
+__device__ __forceinline__ double pu_density(long long x) { return (double)x * 5.5511151231257827e-17; }       // 2 * 2^-55
+
+// Where the iteration stands after the traces T_0 .. T_k: the step to take from
+// X_k (1: X^2, 0: 2 X - X^2), or -1 when X_k is the projector.  first = the
+// first step j whose tr(X_j - X_j^2) was below the tolerance (-1: none yet).
+__device__ __forceinline__ int pu_step(const long long* T, int k, int first, long long occ) {
+  if (first >= 0 && k >= first + 3) return -1;
+  if (first >= 0 && k == first + 2) return T[k - 1] > occ ? 0 : 1;   // the other kind than step k - 1
+  return T[k] > occ ? 1 : 0;
+}
+__device__ __forceinline__ bool pu_traced(long long a, long long b) {
+  const long long d = a > b ? a - b : b - a;
+  return d < kTraceTol;
+}
+
+// the projector has rank nocc (a level that is degenerate across the gap moves
+// to 0 or 1 as a whole)
+__device__ __forceinline__ bool pu_counted(long long t, long long occ) {
+  const long long d = t > occ ? t - occ : occ - t;
+  return d < kTraceOne / 2;
+}
+
+// ---------------------------------------------------------------------------
+// N <= 128: one CTA per molecule, everything on the SM.  The seven digit
+// matrices (K-major core-matrix tiles, the same copy serves as A and as B
+// because X is symmetric: 224 KB at N = 128) in shared memory, X itself in
+// registers: thread (row r, columns 16 g ..) with r its TMEM lane.  A step is 34
+// digit products into eight TMEM accumulators (512 columns: 64 columns of X at
+// a time), then the recombination in registers.
+// ---------------------------------------------------------------------------
+template <int H>
+__global__ void __launch_bounds__(kPurSmallThreads, 1)
+purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, MolState* __restrict__ st,
+                    const double* __restrict__ F, double* __restrict__ P, int np_max, int* __restrict__ err) {
+  extern __shared__ __align__(1024) unsigned char pu_sm[];
+  const int mi = list[blockIdx.x];
+  if (st[mi].status != kActive) return;
+  const DevMol mol = mols[mi];
+  const int n = mol.nao, np = (n + 15) & ~15;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = warp & 3, g = warp >> 2;
+  const int r = q * 32 + lane;
+  // behind the digits (the last one padded to the MMA's 128 rows)
+  unsigned char* tail = pu_sm + (size_t)(kDigits - 1) * 2 * np_max * np_max + (size_t)256 * np_max;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(tail);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 8);
+  double* red = reinterpret_cast<double*>(tail + 16);                      // 2 x 16
+  long long* T = reinterpret_cast<long long*>(tail + 16 + 32 * 8);         // traces, kPurSmallSteps + 1
+  const double* Fm = F + mol.mat0;
+
+  // Gershgorin interval
+  double lo = 1e300, hi = -1e300, bad = 0.0;
+  for (int i = warp; i < n; i += kPurSmallThreads / 32) {
+    double s = 0.0;
+    for (int j = lane; j < n; j += 32)
+      if (j != i) s += fabs(Fm[(long long)i * n + j]);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const double d = Fm[(long long)i * n + i];
+    if (!(s + fabs(d) < 1e290)) bad = 1.0;
+    lo = fmin(lo, d - s);
+    hi = fmax(hi, d + s);
+  }
+  if (lane == 0) { red[warp] = bad > 0.0 ? -1e300 : lo; red[16 + warp] = hi; }
+  for (int i = tid; i <= kPurSmallSteps; i += kPurSmallThreads) T[i] = 0;
+  int ncols = 32;
+  while (ncols < kLevels * (H == 2 ? 64 : np)) ncols <<= 1;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(pu_smem(tmem_slot)), "r"(ncols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(pu_smem(mbar)));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+  for (int w = 0; w < 16; ++w) { lo = fmin(lo, red[w]); hi = fmax(hi, red[16 + w]); }
+  const bool usable = lo > -1e299 && hi > lo;
+  const double scale = usable ? 1.0 / (hi - lo) : 0.0;
+
+  long long x[H][16];
+#pragma unroll
+  for (int h = 0; h < H; ++h)
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      const int col = 64 * h + 16 * g + c;
+      long long v = 0;
+      if (r < n && col < n) {
+        const double f = Fm[(long long)max(r, col) * n + min(r, col)];
+        v = pu_fixed(((r == col ? hi : 0.0) - f) * scale);
+      }
+      x[h][c] = v;
+    }
+
+  const long long occ = (long long)mol.nocc * kTraceOne;
+  const uint32_t slice = 2u * np * np, sbo = 16u * np;
+  uint32_t parity = 0;
+  bool ok = true, done = false;
+  int first = -1;
+  for (int k = 0; usable; ++k) {
+    // digits of X_k into shared memory, its trace
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int c0 = 64 * h + 16 * g;
+      if (r < np && c0 < np) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          uint4 dg[kDigits];
+          pu_split8(&x[h][8 * s], dg);
+          unsigned char* to = pu_sm + (r >> 3) * sbo + ((c0 >> 3) + s) * 128 + (r & 7) * 16;
+#pragma unroll
+          for (int d = 0; d < kDigits; ++d) *reinterpret_cast<uint4*>(to + d * slice) = dg[d];
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+          if (c0 + c == r && r < n)
+            atomicAdd(reinterpret_cast<unsigned long long*>(T + k), (unsigned long long)(x[h][c] >> kTraceShift));
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (first < 0 && k > 0 && pu_traced(T[k], T[k - 1])) first = k - 1;
+    const int op = pu_step(T, k, first, occ);
+    if (op < 0) { done = pu_counted(T[k], occ); break; }
+    if (k == kPurSmallSteps) break;
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int cols = H == 2 ? min(64, np - 64 * h) : np, lstride = H == 2 ? 64 : np;
+      if (tid == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t idesc = pu_idesc(cols), dhi = pu_desc_hi(sbo);
+        uint32_t a[kDigits], b[kDigits];
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d) {
+          a[d] = pu_desc_lo(pu_smem(pu_sm) + d * slice);
+          b[d] = a[d] + (((uint32_t)(64 * h >> 3) * sbo) >> 4);
+        }
+        for (int s = 0; s < np / 16; ++s) {
+#pragma unroll
+          for (int l = 0; l < kLevels; ++l)
+#pragma unroll
+            for (int i = 0; i < kDigits; ++i)
+              if (i <= l && l - i < kDigits)
+                pu_mma(tmem + l * lstride, a[i] + s * (256 >> 4), b[l - i] + s * (256 >> 4), dhi, idesc,
+                       (s > 0 || i > (l < kDigits ? 0 : l - kDigits + 1)) ? 1u : 0u);
+        }
+        pu_commit(pu_smem(mbar));
+      }
+      ok = pu_wait(pu_smem(mbar), parity) && ok;
+      parity ^= 1;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int c0 = 16 * g;
+      if (c0 < cols && q * 32 < n) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          long long v[8];
+          pu_gather8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + 8 * s), lstride, v);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) x[h][8 * s + c] = op ? v[c] : 2 * x[h][8 * s + c] - v[c];
+        }
+        // rows past the basis came from whatever lies behind the digits
+        if (r >= n) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c) x[h][c] = 0;
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      if (H == 2 && h == 0) __syncthreads();   // TMEM is reused for the second half
+    }
+    if (!__syncthreads_and(ok)) { ok = false; break; }
+  }
+  if (ok && done) {
+    double* Pm = P + mol.mat0;
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const int col = 64 * h + 16 * g + c;
+        if (r < n && col < n) Pm[(long long)r * n + col] = pu_density(x[h][c]);
+      }
+  }
+  if (tid == 0) {
+    if (!ok) atomicExch(err, 1);
+    st[mi].flags = (ok && done) ? 0 : kNeedEigen;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols));
+}
+
+// ---------------------------------------------------------------------------
+// N > 128: one launch per step over the 128 x 64 tiles of every molecule's
+// upper triangle.  The digit matrices live in global memory (L2) in the layout
+// of the MMA operands, [K chunk of 32][8-row group][4 k-blocks][8 rows][8 k], so a
+// tile's rows of one K chunk are one contiguous bulk copy per digit; two
+// buffers alternate between steps.  They share the eigensolver's scratch
+// matrices: two digits per N x N doubles (Np = N rounded up to 32 has
+// Np^2 <= 2 N^2 from N = 79 on).
+// ---------------------------------------------------------------------------
+constexpr int kPurTileThreads = 256;
+constexpr int kTileM = 128, kTileN = 64, kChunkK = 32, kStages = 2;
+constexpr uint32_t kStageA = kTileM * kChunkK * 2, kStageB = kTileN * kChunkK * 2;   // bytes per digit
+constexpr uint32_t kStageBytes = kDigits * (kStageA + kStageB);
+constexpr int kSegChunks = 32;                            // K = 1024: sums of two digits' products reach 2^24 at most
+constexpr int kXPitch = kTileM + 1;                       // transposed tile, 8-byte elements: no bank conflicts either way
+constexpr size_t kPurTileSmem = kStages * kStageBytes + 256;
+
+__device__ __forceinline__ unsigned char* pu_plane(const PurScratch& ws, const DevMol& mol, int buf, int d) {
+  const int s = buf * kDigits + d;
+  const long long n2 = ((long long)mol.nao * mol.nao + 31) / 32 * 32;
+  return reinterpret_cast<unsigned char*>(ws.m[s >> 1] + mol.mat0) + (s & 1) * (n2 * 4);
+}
+__device__ __forceinline__ int pu_np(int n) { return (n + 31) & ~31; }
+// byte offset of (row r, k-block k / 8) in a plane; k a multiple of 8
+__device__ __forceinline__ size_t pu_at(int np, int r, int k) {
+  return (size_t)(k >> 5) * (64 * (size_t)np) + (size_t)(r >> 3) * 512 + ((k >> 3) & 3) * 128 + (r & 7) * 16;
+}
+
+__device__ __forceinline__ unsigned long long pu_key(double v) {   // order-preserving
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return (b >> 63) ? ~b : b | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double pu_unkey(unsigned long long k) {
+  return __longlong_as_double((long long)((k >> 63) ? k & 0x7fffffffffffffffull : ~k));
+}
+
+// Gershgorin interval of every molecule: a warp per row
+__global__ void __launch_bounds__(256)
+purify_bounds_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, const MolState* __restrict__ st,
+                     const double* __restrict__ F, PurState* __restrict__ pur) {
+  const int mi = list[blockIdx.y];
+  if (st[mi].status != kActive) return;
+  const DevMol mol = mols[mi];
+  const int n = mol.nao, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= n) return;
+  const double* row = F + mol.mat0 + (long long)i * n;
+  double s = 0.0;
+  for (int j = lane; j < n; j += 32)
+    if (j != i) s += fabs(row[j]);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) {
+    const double d = row[i];
+    const bool bad = !(s + fabs(d) < 1e290);
+    atomicMin(&pur[mi].lo, pu_key(bad ? -1e300 : d - s));
+    if (!bad) atomicMax(&pur[mi].hi, pu_key(d + s));
+  }
+}
+
+__device__ __forceinline__ bool pu_interval(const PurState& s, double* lo, double* hi) {
+  *lo = pu_unkey(s.lo);
+  *hi = pu_unkey(s.hi);
+  return *lo > -1e299 && *hi > *lo;
+}
+
+// X_0 and its digits: a thread per row and eight columns
+__global__ void __launch_bounds__(256)
+purify_init_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, const MolState* __restrict__ st,
+                   const double* __restrict__ F, PurState* __restrict__ pur, PurScratch ws) {
+  const int mi = list[blockIdx.y];
+  if (st[mi].status != kActive) return;
+  const DevMol mol = mols[mi];
+  const int n = mol.nao, np = pu_np(n), kb = np >> 3;
+  double lo, hi;
+  if (!pu_interval(pur[mi], &lo, &hi)) return;
+  const double scale = 1.0 / (hi - lo);
+  const double* Fm = F + mol.mat0;
+  // eight consecutive rows (the rows of a core matrix) by consecutive threads
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < (long long)np * kb; e += (long long)gridDim.x * 256) {
+    const int r = (int)(e / (8 * kb)) * 8 + (int)(e & 7), c0 = (int)((e >> 3) % kb) * 8;
+    long long x[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int col = c0 + c;
+      x[c] = 0;
+      if (r < n && col < n) {
+        const double f = Fm[(long long)max(r, col) * n + min(r, col)];
+        x[c] = pu_fixed(((r == col ? hi : 0.0) - f) * scale);
+        if (r == col)
+          atomicAdd(reinterpret_cast<unsigned long long*>(&pur[mi].trace[0]),
+                    (unsigned long long)(x[c] >> kTraceShift));
+      }
+    }
+    uint4 dg[kDigits];
+    pu_split8(x, dg);
+    const size_t at = pu_at(np, r, c0);
+#pragma unroll
+    for (int d = 0; d < kDigits; ++d) *reinterpret_cast<uint4*>(pu_plane(ws, mol, 0, d) + at) = dg[d];
+  }
+}
+
+// first step whose tr(X - X^2) was below the tolerance, from T_0 .. T_k (k < 64)
+__device__ __forceinline__ int pu_first(const long long* T, int k) {
+  const int lane = threadIdx.x & 31;
+  const unsigned a = __ballot_sync(0xffffffffu, lane < k && pu_traced(T[lane + 1], T[lane]));
+  const unsigned b = __ballot_sync(0xffffffffu, lane + 32 < k && pu_traced(T[lane + 33], T[lane + 32]));
+  return a ? __ffs(a) - 1 : (b ? __ffs(b) + 31 : -1);
+}
+
+// One step of the molecules that still need one.  tiles: (molecule, row block,
+// column block, 0).  Warp 0 copies, warp 1 issues the MMAs, all eight
+// recombine.
+__global__ void __launch_bounds__(kPurTileThreads, 1)
+purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ tiles, const MolState* __restrict__ st,
+                   PurState* __restrict__ pur, PurScratch ws, int k, int* __restrict__ err) {
+  extern __shared__ __align__(1024) unsigned char pu_sm[];
+  const int4 tile = tiles[blockIdx.x];
+  const int mi = tile.x;
+  if (st[mi].status != kActive) return;
+  const DevMol mol = mols[mi];
+  const int n = mol.nao, np = pu_np(n);
+  const long long occ = (long long)mol.nocc * kTraceOne;
+  double lo, hi;
+  if (!pu_interval(pur[mi], &lo, &hi)) return;
+  const int op = pu_step(pur[mi].trace, k, pu_first(pur[mi].trace, k), occ);   // the same in every CTA of the molecule
+  if (op < 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r0 = tile.y * kTileM, c0 = tile.z * kTileN;
+  const int rows = min(kTileM, np - r0), cols = min(kTileN, np - c0);
+  const int chunks = np / kChunkK;
+  unsigned char* tail = pu_sm + kStages * kStageBytes;
+  const uint32_t full = pu_smem(tail), empty = full + 8 * kStages, last = empty + 8 * kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 64);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(pu_smem(tmem_slot)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(full + 8 * s));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(empty + 8 * s));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(last));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t sm = pu_smem(pu_sm);
+  const int buf = k & 1;
+  const int q = warp & 3, r = r0 + q * 32 + lane;
+  const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((warp >> 2) * 32);
+  const int groups = q * 32 < rows ? max(0, min(4, (cols - (warp >> 2) * 32) >> 3)) : 0;   // of eight columns
+  long long v[4][8];
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[s][i] = 0;
+  bool ok = true;
+  // K in segments whose digit sums stay integers below 2^24
+  for (int seg = 0, cb = 0; cb < chunks && ok; ++seg, cb += kSegChunks) {
+    const int ce = min(chunks, cb + kSegChunks);
+    if (warp == 0 && lane == 0) {
+      const uint32_t ba = (uint32_t)rows * kChunkK * 2, bb = (uint32_t)cols * kChunkK * 2;
+      for (int c = cb; c < ce; ++c) {
+        const int s = c % kStages;
+        if (c >= kStages && !pu_wait(empty + 8 * s, ((c / kStages) - 1) & 1)) { ok = false; break; }
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     :: "r"(full + 8 * s), "r"((ba + bb) * kDigits) : "memory");
+        for (int d = 0; d < kDigits; ++d) {
+          const unsigned char* p = pu_plane(ws, mol, buf, d) + (size_t)c * (64 * (size_t)np);
+          const uint32_t to = sm + s * kStageBytes + d * (kStageA + kStageB);
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                       :: "r"(to), "l"(p + (size_t)r0 * 64), "r"(ba), "r"(full + 8 * s) : "memory");
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                       :: "r"(to + kStageA), "l"(p + (size_t)c0 * 64), "r"(bb), "r"(full + 8 * s) : "memory");
+        }
+      }
+    } else if (warp == 1 && lane == 0) {
+      const uint32_t idesc = pu_idesc(cols);
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      for (int c = cb; c < ce; ++c) {
+        const int s = c % kStages;
+        if (!pu_wait(full + 8 * s, (c / kStages) & 1)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t base = pu_desc_lo(sm + s * kStageBytes), dhi = pu_desc_hi(512), later = c > cb;
+#pragma unroll
+        for (int l = 0; l < kLevels; ++l)
+#pragma unroll
+          for (int i = 0; i < kDigits; ++i)
+            if (i <= l && l - i < kDigits) {
+#pragma unroll
+              for (int t = 0; t < kChunkK / 16; ++t)
+                pu_mma(tmem + l * kTileN, base + ((i * (kStageA + kStageB) + t * 256) >> 4),
+                       base + (((l - i) * (kStageA + kStageB) + kStageA + t * 256) >> 4), dhi, idesc,
+                       (t > 0 || i > (l < kDigits ? 0 : l - kDigits + 1)) ? 1u : later);
+            }
+        pu_commit(empty + 8 * s);
+      }
+      if (ok) pu_commit(last);
+    }
+    __syncwarp();
+    ok = pu_wait(last, seg & 1) && ok;
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    ok = __syncthreads_and(ok);
+    if (ok) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+        if (s < groups) {
+          long long t[8];
+          pu_gather8(taddr + 8 * s, kTileN, t);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[s][i] += t[i];
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+  }
+  if (!ok) {
+    if (tid == 0) atomicExch(err, 1);
+  } else {
+    // X_{k+1}: row r, the digits of eight columns at a time
+    const bool mirror = tile.z >= 2 * tile.y + 2;   // the transposed block is no tile of its own
+    long long* xt = reinterpret_cast<long long*>(pu_sm);   // the operand stages are free now
+    long long tr = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      if (s >= groups) continue;
+      const int cl = (warp >> 2) * 32 + 8 * s, c = c0 + cl;
+      const size_t at = pu_at(np, r, c);
+      uint4 dg[kDigits];
+      if (!op) {
+        long long x[8];
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d) dg[d] = *reinterpret_cast<const uint4*>(pu_plane(ws, mol, buf, d) + at);
+        pu_join8(dg, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[s][i] = 2 * x[i] - v[s][i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (c + i == r) tr += v[s][i] >> kTraceShift;
+        if (mirror) xt[(cl + i) * kXPitch + q * 32 + lane] = v[s][i];
+      }
+      pu_split8(v[s], dg);
+#pragma unroll
+      for (int d = 0; d < kDigits; ++d) *reinterpret_cast<uint4*>(pu_plane(ws, mol, buf ^ 1, d) + at) = dg[d];
+    }
+    if (tr != 0) atomicAdd(reinterpret_cast<unsigned long long*>(&pur[mi].trace[k + 1]), (unsigned long long)tr);
+    if (mirror) {
+      __syncthreads();
+      // rows c0 + j, columns r0 + 8 t ..: eight consecutive rows by consecutive threads
+      for (int e = tid; e < cols * (rows >> 3); e += kPurTileThreads) {
+        const int t = e / cols, j = e - t * cols;
+        uint4 dg[kDigits];
+        long long x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = xt[j * kXPitch + 8 * t + i];
+        pu_split8(x, dg);
+        const size_t at = pu_at(np, c0 + j, r0 + 8 * t);
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d) *reinterpret_cast<uint4*>(pu_plane(ws, mol, buf ^ 1, d) + at) = dg[d];
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512));
+}
+
+// P = 2 X of the molecules whose iteration ended; the others are flagged
+__global__ void __launch_bounds__(256)
+purify_store_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, MolState* __restrict__ st,
+                    const PurState* __restrict__ pur, PurScratch ws, int steps, double* __restrict__ P) {
+  const int mi = list[blockIdx.y];
+  if (st[mi].status != kActive) return;
+  const DevMol mol = mols[mi];
+  const int n = mol.nao, np = pu_np(n), kb = np >> 3;
+  double lo, hi;
+  const int first = pu_first(pur[mi].trace, steps);
+  const bool done = pu_interval(pur[mi], &lo, &hi) && first >= 0 && first + 3 <= steps &&
+                    pu_counted(pur[mi].trace[first + 3], (long long)mol.nocc * kTraceOne);
+  if (blockIdx.x == 0 && threadIdx.x == 0) st[mi].flags = done ? 0 : kNeedEigen;
+  if (!done) return;
+  const int buf = (first + 3) & 1;
+  double* Pm = P + mol.mat0;
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < (long long)n * kb; e += (long long)gridDim.x * 256) {
+    const int r = (int)(e / kb), c0 = (int)(e % kb) * 8;
+    uint4 dg[kDigits];
+    const size_t at = pu_at(np, r, c0);
+#pragma unroll
+    for (int d = 0; d < kDigits; ++d) dg[d] = *reinterpret_cast<const uint4*>(pu_plane(ws, mol, buf, d) + at);
+    long long x[8];
+    pu_join8(dg, x);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (c0 + c < n) Pm[(long long)r * n + c0 + c] = pu_density(x[c]);
+  }
+}
+
+// traces and bounds of the next call
+__global__ void purify_reset_kernel(const int* __restrict__ list, PurState* __restrict__ pur) {
+  PurState& s = pur[list[blockIdx.x]];
+  for (int i = threadIdx.x; i <= kPurBigSteps; i += blockDim.x) s.trace[i] = 0;
+  if (threadIdx.x == 0) { s.lo = ~0ull; s.hi = 0ull; }
+}
+
+// ---------------------------------------------------------------------------
+static size_t small_smem(int np) {
+  return (size_t)(kDigits - 1) * 2 * np * np + (size_t)256 * np + 16 + 32 * 8 + (kPurSmallSteps + 1) * 8;
+}
+
+void purify_prepare() {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaFuncSetAttribute(purify_small_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(64));
+    cudaFuncSetAttribute(purify_small_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(128));
+    cudaFuncSetAttribute(purify_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPurTileSmem);
+  });
+}
+
+int purify_tiles(int mol, int n, int4* out) {
+  const int np = (n + 31) / 32 * 32, nr = (np + kTileM - 1) / kTileM, nc = (np + kTileN - 1) / kTileN;
+  int t = 0;
+  for (int i = 0; i < nr; ++i)
+    for (int j = 2 * i; j < nc; ++j, ++t)
+      if (out) out[t] = make_int4(mol, i, j, 0);
+  return t;
+}
+
+void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
+                         double* P, int* err, cudaStream_t s) {
+  if (nlist <= 0) return;
+  purify_prepare();
+  const int np = (max_n + 15) / 16 * 16;
+  if (np <= 64)
+    purify_small_kernel<1><<<nlist, kPurSmallThreads, small_smem(np), s>>>(mols, list, st, F, P, np, err);
+  else
+    purify_small_kernel<2><<<nlist, kPurSmallThreads, small_smem(np), s>>>(mols, list, st, F, P, np, err);
+}
+
+int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
+                      MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
+                      int* err, cudaStream_t s) {
+  if (nlist <= 0) return 0;
+  purify_prepare();
+  const int np = (max_n + 31) / 32 * 32;
+  const int blocks = std::max(1, std::min(512, np * (np / 8) / 512));
+  purify_reset_kernel<<<nlist, 64, 0, s>>>(list, pur);
+  purify_bounds_kernel<<<dim3((max_n + 7) / 8, nlist), 256, 0, s>>>(mols, list, st, F, pur);
+  purify_init_kernel<<<dim3(blocks, nlist), 256, 0, s>>>(mols, list, st, F, pur, ws);
+  for (int k = 0; k < steps; ++k)
+    purify_step_kernel<<<ntiles, kPurTileThreads, kPurTileSmem, s>>>(mols, tiles, st, pur, ws, k, err);
+  purify_store_kernel<<<dim3(blocks, nlist), 256, 0, s>>>(mols, list, st, pur, ws, steps, P);
+  return steps + 4;
+}
+
+}  // namespace nddo

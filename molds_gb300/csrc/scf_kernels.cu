@@ -38,7 +38,7 @@ gemm_kernel(const GemmJob* __restrict__ jobs, int njobs, const TA* __restrict__ 
     if (jobs[mid].tile0 <= t) lo = mid; else hi = mid - 1;
   }
   const GemmJob job = jobs[lo];
-  if (require_active && st[job.mol].status != kActive) return;
+  if (mol_skipped(st[job.mol], require_active)) return;
   if (require_phase >= 0 && st[job.mol].phase != require_phase) return;
   const int local = t - job.tile0;
   int tm, tn;
@@ -208,7 +208,7 @@ diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol
   const int li = blockIdx.y;
   const int m = mol_list[li];
   const MolState s = st[m];
-  if (s.status != kActive) return;
+  if (s.status != kActive || ((s.flags & kNeedEigen) && !prm.eigen_ran)) return;
   const DevMol mol = mols[m];
   const long long n2 = (long long)mol.nao * mol.nao;
   const int chunks = diis_chunks(n2);
@@ -265,7 +265,8 @@ __global__ void diis_solve_kernel(const DevMol* __restrict__ mols, const int* __
   out.apply = 0; out.damp = 0; out.active = 0; out.pad = 0;
   const int m = mol_list[li];
   MolState* s = st + m;
-  if (s->status != kActive) { steps[li] = out; return; }
+  if (s->status != kActive || ((s->flags & kNeedEigen) && !prm.eigen_ran)) { steps[li] = out; return; }
+  s->flags &= ~kNeedEigen;
   out.active = 1;
   const DevMol mol = mols[m];
   const long long n2 = (long long)mol.nao * mol.nao;

@@ -77,7 +77,7 @@ Server::Server(Engine* eng, const ScfSettings& s, size_t hbm_budget, int max_bas
     L->slot_ticket.assign(slots, -1);
     L->slot_tsubmit.assign(slots, 0.0);
     L->slot_tadmit.assign(slots, 0.0);
-    cuda_check(cudaHostAlloc(&L->h_count, sizeof(int), cudaHostAllocDefault), "pinned");
+    cuda_check(cudaHostAlloc(&L->h_count, 2 * sizeof(int), cudaHostAllocDefault), "pinned");
     cuda_check(cudaHostAlloc(&L->h_active, slots, cudaHostAllocDefault), "pinned");
     cuda_check(cudaHostAlloc(&L->h_states, slots * sizeof(MolState), cudaHostAllocDefault), "pinned");
     cuda_check(cudaHostAlloc(&L->h_charges, c.atoms * sizeof(double), cudaHostAllocDefault), "pinned");
@@ -277,9 +277,12 @@ bool Server::lane_step(Lane& L) {
   }
   L.n_active = (int)L.active.size();
   if (L.active.empty()) return false;
-  b.iterate(s_, L.active);
+  // a molecule the purification cannot treat waits for an iteration with the
+  // eigensolver; it waited once, so its next iterations have it as well
+  b.iterate(s_, L.active, L.eigen > 0);
   b.count_active_async(L.active, L.h_count, L.h_active, L.ev);
   cuda_check(cudaEventSynchronize(L.ev), "lane iteration");
+  L.eigen = L.h_count[1] > 0 ? 8 : std::max(0, L.eigen - 1);
   std::vector<int> fin, still;
   for (int m : L.active) (L.h_active[m] ? still : fin).push_back(m);
   if (!fin.empty()) {

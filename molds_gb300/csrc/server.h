@@ -69,7 +69,8 @@ class Server {
     std::vector<int> active;
     std::vector<long long> slot_ticket;
     std::vector<double> slot_tsubmit, slot_tadmit;
-    int* h_count = nullptr;
+    int eigen = 0;                            // iterations still to run with the eigensolver launches
+    int* h_count = nullptr;                   // active molecules, those waiting for the eigensolver
     char* h_active = nullptr;
     MolState* h_states = nullptr;
     double* h_charges = nullptr;

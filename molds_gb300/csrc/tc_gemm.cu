@@ -80,7 +80,7 @@ tc_gemm_kernel(const GemmJob* __restrict__ jobs, int njobs, const TA* __restrict
     if (jobs[mid].tc_tile0 <= t) lo = mid; else hi = mid - 1;
   }
   const GemmJob job = jobs[lo];
-  if (require_active && st[job.mol].status != kActive) return;
+  if (mol_skipped(st[job.mol], require_active)) return;
   if (require_phase >= 0 && st[job.mol].phase != require_phase) return;
   const int local = t - job.tc_tile0;
   int tm, tn;

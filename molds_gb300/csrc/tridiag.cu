@@ -83,7 +83,7 @@ hh_tridiag_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list,
                   long long vstride, double* __restrict__ Aws, int max_n_served) {
   extern __shared__ __align__(16) double hsm[];
   const int mi = list[blockIdx.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
   if (n > max_n_served) return;   // served by the whole-GPU kernel (tridiag_grid.cu)
@@ -542,7 +542,7 @@ tri_vectors_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list
                    double* __restrict__ S2, double* __restrict__ S3, int vec_smem, int pairs) {
   extern __shared__ __align__(16) double vsm[];
   const int mi = list[blockIdx.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
   int lo, hi;
@@ -734,7 +734,7 @@ tri_orth_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, c
   __shared__ double red[kOrthThreads / 32];
   __shared__ double onenrm_s;
   const int mi = list[blockIdx.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
   int lo, hi;
@@ -831,7 +831,7 @@ hh_back_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, co
                const double* __restrict__ td, long long vstride, const double* __restrict__ Z, T* __restrict__ C) {
   extern __shared__ __align__(16) double bsm[];
   const int mi = list[blockIdx.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   if (require_phase >= 0 && st[mi].phase != require_phase) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;

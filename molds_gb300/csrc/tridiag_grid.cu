@@ -144,7 +144,7 @@ hh_tridiag_grid_kernel(const DevMol* __restrict__ mols, const int* __restrict__ 
   __shared__ double red[kGridWarps], wred[kGridWarps], hs[4];
   const int3 slot = map[blockIdx.x];   // (list entry, CTA within the molecule's sub-grid, sub-grid size)
   const int mi = list[slot.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -340,7 +340,7 @@ tri_orth_grid_kernel(const DevMol* __restrict__ mols, const int* __restrict__ li
   __shared__ double rs[32];
   const int3 slot = map[blockIdx.x];
   const int mi = list[slot.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
   int lo, hi;
@@ -518,7 +518,7 @@ hh_back_wide_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   extern __shared__ __align__(16) double bwm[];
   constexpr int kSpw = 32 / kCols, kS = kWideWarps * kSpw, kT = kWideWarps * 32;
   const int mi = list[blockIdx.x];
-  if (require_active && st[mi].status != kActive) return;
+  if (mol_skipped(st[mi], require_active)) return;
   if (require_phase >= 0 && st[mi].phase != require_phase) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
