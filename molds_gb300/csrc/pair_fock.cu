@@ -1165,217 +1165,311 @@ void launch_cartesian_matrix(const DevAtom* atoms, const DevPair* pairs, const D
 // with W = T2 L T2^T the rotated (mu nu|la si) block, C_PQ = m_P m_Q P_P P_Q
 // - 1/2 X_PQ (Coulomb and exchange, m = 2 for mu != nu, X summed over both
 // orbital orders) plus the electron-core attractions -Z_B (mu nu|s_B s_B) on
-// the (mu nu, ss) column and -Z_A on the (ss, la si) row.  One thread per
-// pair evaluates E_AB in dual numbers seeded with d (the exact derivatives of
-// the same local integrals, rotation and overlaps the pair kernels use), and
-// writes dE_AB/dd; the gradient of atom i is then
+// the (mu nu, ss) column and -Z_A on the (ss, la si) row.
+//
+// The derivative is taken in the pair's local frame (z along d).  With
+// C' = T2^T C T2 the density factors of that frame, E = sum C'_PQ L_PQ(R):
+//   along z:  sum C'_PQ dL_PQ/dR (each local integral's terms differentiated);
+//   along x:  moving B by delta turns the frame by delta / R about y, so the
+//             columns of T2 change by T2 G with the generator G of that
+//             rotation on orbital products, and dE = (delta / R) sum C'_PQ
+//             (G L + L G^T)_PQ; y alike.
+// Resonance: the same with the 4 x 4 overlap block and w' = Rm^T w Rm; core-core
+// and dispersion depend on R alone.  These are the exact derivatives of the
+// formulas the pair kernels evaluate, for any azimuth of the frame (the local
+// integrals are cylindrically symmetric).  One warp per pair: lane = local
+// integral, then lane = (P, Q).  The gradient of atom i is then
 //   g_i = sum_{a < i} dE_ai/dd - sum_{b > i} dE_ib/dd   (fixed order).
-// The local frame here is z along d and x from the coordinate axis least
-// aligned with it (smooth in d near every axis); the rotated integrals do not
-// depend on the azimuth of the frame (the local integrals are cylindrically
-// symmetric), so they equal the pair kernels' values.
+// What bounds it: latency, a few thousand clocks of dependent FP64 per pair.
+// One thread per pair in three-component dual numbers kept its 10 x 10 matrices
+// in local memory: 1.30 ms for octane's 325 pairs.
 // ---------------------------------------------------------------------------
-namespace {
+constexpr int kGradWarps = 4;
 
-__device__ void smooth_frame(const Dual3& x, const Dual3& y, const Dual3& z, Dual3 Rm[4][4]) {
-  const Dual3 r = sqrt(x * x + y * y + z * z);
-  const Dual3 ez[3] = {x / r, y / r, z / r};
-  int k = 0;
-  for (int i = 1; i < 3; ++i)
-    if (::fabs(ez[i].v) < ::fabs(ez[k].v)) k = i;
-  Dual3 ex[3] = {-ez[k] * ez[0], -ez[k] * ez[1], -ez[k] * ez[2]};
-  ex[k] += 1.0;
-  const Dual3 nx = sqrt(ex[0] * ex[0] + ex[1] * ex[1] + ex[2] * ex[2]);
-  for (int i = 0; i < 3; ++i) ex[i] /= nx;
-  const Dual3 ey[3] = {ez[1] * ex[2] - ez[2] * ex[1], ez[2] * ex[0] - ez[0] * ex[2], ez[0] * ex[1] - ez[1] * ex[0]};
-  for (int i = 0; i < 4; ++i)
-    for (int j = 0; j < 4; ++j) Rm[i][j] = 0.0;
-  Rm[0][0] = 1.0;
-  // rows: space-frame orbitals s, py, pz, px; columns: local s, y, z, x
-  const int comp[4] = {-1, 1, 2, 0};
-  for (int row = 1; row < 4; ++row) {
-    Rm[row][1] = ey[comp[row]];
-    Rm[row][2] = ez[comp[row]];
-    Rm[row][3] = ex[comp[row]];
-  }
+struct GradShared {
+  double T2[100], C[100], M[100];
+  double val[24], dval[24];
+  double ab[4][2][9];      // per exponent combination: A_0..8, B_0..8
+  double Rm[16], w[16], ls[8], dls[8], pA[10], pB[10], pab[16];
+};
+
+// where the generator of a frame rotation takes local orbital i (s, y, z, x):
+// axis 0 turns z towards x, axis 1 turns z towards y; sign 0: nowhere
+__device__ __forceinline__ double turned(int axis, int i, int* k) {
+  const int to = axis == 0 ? 3 : 1;
+  if (i == 2) { *k = to; return 1.0; }
+  if (i == to) { *k = 2; return -1.0; }
+  *k = 0;
+  return 0.0;
 }
 
-}  // namespace
-
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(kGradWarps * 32)
 pair_grad_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, long long pair0,
                  long long npairs, const DevMol* __restrict__ mols, const EriTable* __restrict__ eri,
                  const OverlapTable* __restrict__ ovt, const double* __restrict__ P, VdwParams vdw,
                  double* __restrict__ grad) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ GradShared shared[kGradWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long t = (long long)blockIdx.x * kGradWarps + warp;
   if (t >= npairs) return;
-  const long long p = pair0 + t;
-  const DevPair pr = pairs[p];
+  GradShared& sh = shared[warp];
+  const DevPair pr = pairs[pair0 + t];
   const DevAtom A = atoms[pr.a], B = atoms[pr.b];
   const DevMol mol = mols[pr.mol];
   const nddo_atom_params& pa = c_params[A.pidx];
   const nddo_atom_params& pb = c_params[B.pidx];
   const int nA = A.nao, nB = B.nao, dA = nA == 4 ? 10 : 1, dB = nB == 4 ? 10 : 1;
-  const Dual3 dx(B.x - A.x, 1.0, 0.0, 0.0), dy(B.y - A.y, 0.0, 1.0, 0.0), dz(B.z - A.z, 0.0, 0.0, 1.0);
-  const Dual3 R = sqrt(dx * dx + dy * dy + dz * dz);
+  const double dx = B.x - A.x, dy = B.y - A.y, dz = B.z - A.z;
+  const double R = sqrt(dx * dx + dy * dy + dz * dz);
   const double* Pm = P + mol.mat0;
   const long long ld = mol.nao;
 
-  // local integrals (the slots this pair's orbitals need)
-  Dual3 val[kNumSlots];
-  {
-    const Dual3 dAv[3] = {pa.d[0], pa.d[1], pa.d[2]}, dBv[3] = {pb.d[0], pb.d[1], pb.d[2]};
-    const Dual3 rAv[3] = {pa.rho[0], pa.rho[1], pa.rho[2]}, rBv[3] = {pb.rho[0], pb.rho[1], pb.rho[2]};
-    for (int sl = 0; sl < 21; ++sl) {
-      bool need;
-      if (nA == 4 && nB == 4) need = true;
-      else if (nA == 4) need = (sl == 0 || sl == 3 || sl == 4 || sl == 10);
-      else if (nB == 4) need = (sl == 0 || sl == 1 || sl == 2 || sl == 13);
-      else need = (sl == 0);
-      Dual3 v = 0.0;
-      if (need)
-        for (int k = 0; k < eri->nterms[sl]; ++k) v += eval_term(eri->terms[sl][k], R, dAv, dBv, rAv, rBv);
-      val[sl] = v;
-    }
-    val[21] = (nA == 4 && nB == 4) ? 0.5 * (val[5] - val[6]) : Dual3(0.0);
+  if (lane == 0) {
+    double Rm[4][4];
+    rotation_matrix(dx, dy, dz, Rm);
+    for (int i = 0; i < 16; ++i) sh.Rm[i] = Rm[i >> 2][i & 3];
   }
-  Dual3 Rm[4][4];
-  smooth_frame(dx, dy, dz, Rm);
-
-  // C: the density factors of each (mu nu, la si) integral
-  double C[10][10];
+  // density of both atoms and between them
+  if (lane < 10 && lane < dA) {
+    int m, n;
+    unpack_index(lane, &m, &n);
+    sh.pA[lane] = Pm[(A.ao0 + m) * ld + A.ao0 + n];
+  }
+  if (lane >= 10 && lane - 10 < dB) {
+    int m, n;
+    unpack_index(lane - 10, &m, &n);
+    sh.pB[lane - 10] = Pm[(B.ao0 + m) * ld + B.ao0 + n];
+  }
+  if (lane < 16) {
+    const int mu = lane >> 2, la = lane & 3;
+    sh.pab[lane] = mu < nA && la < nB ? Pm[(A.ao0 + mu) * ld + B.ao0 + la] : 0.0;
+  }
+  // local integrals and their derivatives in R: lane = slot
+  double val = 0.0, dval = 0.0;
+  if (lane < 21) {
+    bool need;
+    if (nA == 4 && nB == 4) need = true;
+    else if (nA == 4) need = (lane == 0 || lane == 3 || lane == 4 || lane == 10);
+    else if (nB == 4) need = (lane == 0 || lane == 1 || lane == 2 || lane == 13);
+    else need = (lane == 0);
+    if (need) {
+      const int nt = eri->nterms[lane];
+      for (int k = 0; k < nt; ++k) {
+        const EriTerm e = eri->terms[lane][k];
+        const double da = sel3(e.la, pa.d[0], pa.d[1], pa.d[2]);
+        const double db = sel3(e.lb, pb.d[0], pb.d[1], pb.d[2]);
+        const double a = sel3(e.la, pa.rho[0], pa.rho[1], pa.rho[2]) + sel3(e.lb, pb.rho[0], pb.rho[1], pb.rho[2]);
+        const double l = R + (double)e.c1 * da + (double)e.c2 * db;
+        const double u = (double)e.c3 * da + (double)e.c4 * db;
+        const double v = (double)e.c5 * da + (double)e.c6 * db;
+        const double r = rsqrt(l * l + u * u + v * v + a * a);
+        const double w = e.coef * r;
+        val += w;
+        dval -= w * l * (r * r);
+      }
+    }
+  }
   {
-    double pA[10], pB[10], mA[10], mB[10];
-    for (int q = 0; q < dA; ++q) {
-      int m, n;
-      unpack_index(q, &m, &n);
-      pA[q] = Pm[(A.ao0 + m) * ld + A.ao0 + n];
-      mA[q] = m == n ? 1.0 : 2.0;
+    const double s5 = __shfl_sync(0xffffffffu, val, 5), s6 = __shfl_sync(0xffffffffu, val, 6);
+    const double d5 = __shfl_sync(0xffffffffu, dval, 5), d6 = __shfl_sync(0xffffffffu, dval, 6);
+    if (lane == 21 && nA == 4 && nB == 4) { val = 0.5 * (s5 - s6); dval = 0.5 * (d5 - d6); }
+  }
+  if (lane < 22) { sh.val[lane] = val; sh.dval[lane] = dval; }
+  // overlap auxiliary integrals (as pair_kernel), one order more for the
+  // derivatives: A_k' = -A_{k+1}, B_k' = -B_{k+1}
+  const int na = pa.principal_n, nb = pb.principal_n;
+  if (lane < 8) {
+    const int zc = lane & 3;
+    const bool need = (zc == 0) || (zc == 1 && nB == 4) || (zc == 2 && nA == 4) || (zc == 3 && nA == 4 && nB == 4);
+    if (need) {
+      const double za = (zc >= 2) ? pa.zeta[1] : pa.zeta[0];
+      const double zb = (zc & 1) ? pb.zeta[1] : pb.zeta[0];
+      double v[9];
+      if (lane < 4) aux_a_all(0.5 * R * (za + zb), 8, v);
+      else aux_b_all(0.5 * R * (za - zb), 8, v, c_inv);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) sh.ab[zc][lane >> 2][k] = v[k];
     }
-    for (int q = 0; q < dB; ++q) {
-      int m, n;
-      unpack_index(q, &m, &n);
-      pB[q] = Pm[(B.ao0 + m) * ld + B.ao0 + n];
-      mB[q] = m == n ? 1.0 : 2.0;
+  }
+  __syncwarp();
+  // rotation of orbital products, density factors of the space-frame integrals
+  for (int e = lane; e < 100; e += 32) {
+    int m, n, i, j;
+    unpack_index(e / 10, &m, &n);
+    unpack_index(e % 10, &i, &j);
+    const double* Rm = sh.Rm;
+    sh.T2[e] = (i == j) ? Rm[m * 4 + i] * Rm[n * 4 + i] : Rm[m * 4 + i] * Rm[n * 4 + j] + Rm[m * 4 + j] * Rm[n * 4 + i];
+  }
+  for (int e = lane; e < dA * dB; e += 32) {
+    const int q = e / dB, r = e % dB;
+    int a, b, c, d;
+    unpack_index(q, &a, &b);
+    unpack_index(r, &c, &d);
+    const double mA = a == b ? 1.0 : 2.0, mB = c == d ? 1.0 : 2.0;
+    // exchange: both orders of (a b) and of (c d)
+    double x = sh.pab[a * 4 + c] * sh.pab[b * 4 + d];
+    if (a != b) x += sh.pab[b * 4 + c] * sh.pab[a * 4 + d];
+    if (c != d) x += sh.pab[a * 4 + d] * sh.pab[b * 4 + c];
+    if (a != b && c != d) x += sh.pab[b * 4 + d] * sh.pab[a * 4 + c];
+    double f = mA * mB * sh.pA[q] * sh.pB[r] - 0.5 * x;
+    if (r == 0) f -= (double)pb.core_charge * mA * sh.pA[q];
+    if (q == 0) f -= (double)pa.core_charge * mB * sh.pB[r];
+    sh.C[q * 10 + r] = f;
+  }
+  // overlaps and their derivatives (ss, s-sigma, sigma-s, sigma-sigma, pi-pi)
+  if (lane < 5) {
+    const int c = lane;
+    const bool need = (c == 0) || (c == 1 && nB == 4) || (c == 2 && nA == 4) || (c >= 3 && nA == 4 && nB == 4);
+    double s = 0.0, ds = 0.0;
+    if (need) {
+      const int zc = (c == 4) ? 3 : c;
+      const double za = (zc >= 2) ? pa.zeta[1] : pa.zeta[0], zb = (zc & 1) ? pb.zeta[1] : pb.zeta[0];
+      const double dp = 0.5 * (za + zb), dq = 0.5 * (za - zb);
+      const double* a = sh.ab[zc][0];
+      const double* b = sh.ab[zc][1];
+      const int nt = ovt->nterms[na - 1][nb - 1][c];
+      for (int k = 0; k < nt; ++k) {
+        const double tc = ovt->tc[na - 1][nb - 1][c][k];
+        const int i = ovt->ti[na - 1][nb - 1][c][k], j = ovt->tj[na - 1][nb - 1][c][k];
+        s += tc * a[i] * b[j];
+        ds -= tc * (dp * a[i + 1] * b[j] + dq * a[i] * b[j + 1]);
+      }
+      const double norm = pa.sto_norm[c >= 2 ? 1 : 0] * pb.sto_norm[(c == 1 || c >= 3) ? 1 : 0] * ovt->ang[c];
+      double rp = 1.0;
+      for (int i = 0; i < na + nb + 1; ++i) rp *= 0.5 * R;
+      ds = norm * rp * (ds + (double)(na + nb + 1) / R * s);
+      s *= norm * rp;
     }
-    for (int q = 0; q < dA; ++q) {
-      int a, b;
-      unpack_index(q, &a, &b);
-      for (int r = 0; r < dB; ++r) {
-        int c, e;
-        unpack_index(r, &c, &e);
-        // exchange: both orders of (a b) and of (c e)
-        double x = 0.0;
-        for (int o1 = 0; o1 < (a == b ? 1 : 2); ++o1) {
-          const int u = o1 ? b : a, w = o1 ? a : b;
-          for (int o2 = 0; o2 < (c == e ? 1 : 2); ++o2) {
-            const int y = o2 ? e : c, z = o2 ? c : e;
-            x += Pm[(A.ao0 + u) * ld + B.ao0 + y] * Pm[(A.ao0 + w) * ld + B.ao0 + z];
-          }
+    sh.ls[c] = s;
+    sh.dls[c] = ds;
+  }
+  // w' = Rm^T w Rm of the resonance energy sum w_mu,la S_mu,la
+  if (lane < 16) {
+    const int i = lane >> 2, j = lane & 3;
+    double s = 0.0;
+    for (int mu = 0; mu < 4; ++mu)
+      for (int la = 0; la < 4; ++la)
+        s += sh.Rm[mu * 4 + i] * sh.pab[mu * 4 + la] * (pa.beta[mu == 0 ? 0 : 1] + pb.beta[la == 0 ? 0 : 1]) *
+             sh.Rm[la * 4 + j];
+    sh.w[lane] = s;
+  }
+  __syncwarp();
+  // C' = T2^T C T2
+  for (int e = lane; e < dA * dB; e += 32) {
+    const int q = e / dB, r = e % dB;
+    double s = 0.0;
+    for (int k = 0; k < dB; ++k) s += sh.C[q * 10 + k] * sh.T2[k * 10 + r];
+    sh.M[q * 10 + r] = s;
+  }
+  __syncwarp();
+  for (int e = lane; e < dA * dB; e += 32) {
+    const int q = e / dB, r = e % dB;
+    double s = 0.0;
+    for (int k = 0; k < dA; ++k) s += sh.T2[k * 10 + q] * sh.M[k * 10 + r];
+    sh.C[q * 10 + r] = s;
+  }
+  __syncwarp();
+  double gr = 0.0, g[2] = {0.0, 0.0};
+  for (int e = lane; e < dA * dB; e += 32) {
+    const int q = e / dB, r = e % dB;
+    const int sl = eri->slot_of[q][r];
+    if (sl < 0) continue;
+    gr += sh.C[q * 10 + r] * sh.dval[sl];
+    const double L = sh.val[sl];
+    int i, j, k;
+#pragma unroll
+    for (int axis = 0; axis < 2; ++axis) {
+      double f = 0.0, sg;
+      if (dA == 10) {
+        unpack_index(q, &i, &j);
+        sg = turned(axis, i, &k);
+        if (sg != 0.0) f += sg * (i != j && k == j ? 2.0 : 1.0) * sh.C[pack_index(k, j) * 10 + r];
+        if (i != j) {
+          sg = turned(axis, j, &k);
+          if (sg != 0.0) f += sg * (k == i ? 2.0 : 1.0) * sh.C[pack_index(k, i) * 10 + r];
         }
-        C[q][r] = mA[q] * mB[r] * pA[q] * pB[r] - 0.5 * x;
       }
-    }
-    for (int q = 0; q < dA; ++q) C[q][0] += -(double)pb.core_charge * mA[q] * pA[q];
-    for (int r = 0; r < dB; ++r) C[0][r] += -(double)pa.core_charge * mB[r] * pB[r];
-  }
-
-  // two-electron and electron-core part: sum_PQ C_PQ (T2 L T2^T)_PQ
-  Dual3 e_pair = 0.0;
-  {
-    Dual3 T2[10][10];
-    for (int q = 0; q < 10; ++q)
-      for (int r = 0; r < 10; ++r) T2[q][r] = (q < dA || q < dB) ? pair_rotation(Rm, q, r) : Dual3(0.0);
-    // M[P][Q'] = sum_Q L[P][Q] T2[Q'][Q]
-    for (int Pl = 0; Pl < dA; ++Pl) {
-      Dual3 Mrow[10];
-      for (int Qp = 0; Qp < dB; ++Qp) {
-        Dual3 acc = 0.0;
-        for (int Q = 0; Q < dB; ++Q) {
-          const int sl = eri->slot_of[Pl][Q];
-          if (sl >= 0) acc += val[sl] * T2[Qp][Q];
+      if (dB == 10) {
+        unpack_index(r, &i, &j);
+        sg = turned(axis, i, &k);
+        if (sg != 0.0) f += sg * (i != j && k == j ? 2.0 : 1.0) * sh.C[q * 10 + pack_index(k, j)];
+        if (i != j) {
+          sg = turned(axis, j, &k);
+          if (sg != 0.0) f += sg * (k == i ? 2.0 : 1.0) * sh.C[q * 10 + pack_index(k, i)];
         }
-        Mrow[Qp] = acc;
       }
-      // W[P'][Q'] = sum_P T2[P'][P] M[P][Q']: accumulate C[P'][Q'] T2[P'][P] M[P][Q']
-      for (int Pp = 0; Pp < dA; ++Pp) {
-        Dual3 cm = 0.0;
-        for (int Qp = 0; Qp < dB; ++Qp) cm += C[Pp][Qp] * Mrow[Qp];
-        e_pair += T2[Pp][Pl] * cm;
+      g[axis] += L * f;
+    }
+  }
+  if (lane < 16) {
+    const int i = lane >> 2, j = lane & 3;
+    const int c = (i == 0 && j == 0) ? 0 : (i == 0 && j == 2) ? 1 : (i == 2 && j == 0) ? 2 : (i == 2 && j == 2) ? 3
+                  : ((i == 1 && j == 1) || (i == 3 && j == 3)) ? 4 : -1;
+    if (c >= 0) {
+      gr += sh.w[lane] * sh.dls[c];
+      int k;
+#pragma unroll
+      for (int axis = 0; axis < 2; ++axis) {
+        double sg = turned(axis, i, &k);
+        if (sg != 0.0) g[axis] += sh.ls[c] * sg * sh.w[k * 4 + j];
+        sg = turned(axis, j, &k);
+        if (sg != 0.0) g[axis] += sh.ls[c] * sg * sh.w[i * 4 + k];
       }
     }
   }
-
-  // resonance: sum P_mu,la (beta_mu + beta_la) S_mu,la
-  {
-    const int na = pa.principal_n, nb = pb.principal_n;
-    Dual3 ov[5];
-    for (int c = 0; c < 5; ++c) {
-      const bool need = (c == 0) || (c == 1 && nB == 4) || (c == 2 && nA == 4) || (c >= 3 && nA == 4 && nB == 4);
-      if (!need) { ov[c] = 0.0; continue; }
-      const double za = c >= 2 ? pa.zeta[1] : pa.zeta[0];
-      const double zb = (c == 1 || c >= 3) ? pb.zeta[1] : pb.zeta[0];
-      const double norm = pa.sto_norm[c >= 2 ? 1 : 0] * pb.sto_norm[(c == 1 || c >= 3) ? 1 : 0];
-      ov[c] = overlap_combo(ovt, na, nb, c, za, zb, norm, R);
-    }
-    Dual3 Ls[4][4];
-    Ls[0][0] = ov[0]; Ls[0][2] = ov[1]; Ls[2][0] = ov[2]; Ls[2][2] = ov[3]; Ls[1][1] = ov[4]; Ls[3][3] = ov[4];
-    for (int mu = 0; mu < nA; ++mu)
-      for (int la = 0; la < nB; ++la) {
-        Dual3 sv = 0.0;
-        for (int i = 0; i < 4; ++i)
-          for (int j = 0; j < 4; ++j)
-            if (i == j || (i == 0 && j == 2) || (i == 2 && j == 0)) sv += Rm[mu][i] * Ls[i][j] * Rm[la][j];
-        const double w = Pm[(A.ao0 + mu) * ld + B.ao0 + la] * (pa.beta[mu == 0 ? 0 : 1] + pb.beta[la == 0 ? 0 : 1]);
-        e_pair += w * sv;
+  if (lane == 31) {
+    // core-core repulsion (with the AM1 / PM3 Gaussians and the PDDG term) and
+    // the empirical dispersion (energy_kernel's pair term): functions of R
+    const Dual3 Rd(R, 1.0, 0.0, 0.0);
+    Dual3 e = core_core(pa, pb, Rd, Dual3(sh.val[0], sh.dval[0], 0.0, 0.0), mol.theory);
+    const bool dtheory = mol.theory == NDDO_AM1D || mol.theory == NDDO_PM3D;
+    if (vdw.on || dtheory) {
+      const double s6 = dtheory ? NDDO_VDW_S6_D : vdw.s6, dd = dtheory ? NDDO_VDW_DAMP_D : vdw.d;
+      const double csum = pa.vdw_c6 + pb.vdw_c6;
+      if (csum > 0.0) {
+        const double c6 = 2.0 * pa.vdw_c6 * pb.vdw_c6 / csum;
+        const Dual3 damp = 1.0 / (1.0 + exp(-1.0 * dd * (Rd / (pa.vdw_r0 + pb.vdw_r0) - 1.0)));
+        const Dual3 R2 = Rd * Rd;
+        e += (-1.0 * s6 * c6) * damp / (R2 * R2 * R2);
       }
-  }
-
-  // core-core repulsion (with the AM1 / PM3 Gaussians and the PDDG term)
-  e_pair += core_core(pa, pb, R, val[0], mol.theory);
-
-  // empirical dispersion (energy_kernel's pair term)
-  const bool dtheory = mol.theory == NDDO_AM1D || mol.theory == NDDO_PM3D;
-  if (vdw.on || dtheory) {
-    const double s6 = dtheory ? NDDO_VDW_S6_D : vdw.s6, dd = dtheory ? NDDO_VDW_DAMP_D : vdw.d;
-    const double csum = pa.vdw_c6 + pb.vdw_c6;
-    if (csum > 0.0) {
-      const double c6 = 2.0 * pa.vdw_c6 * pb.vdw_c6 / csum;
-      const Dual3 damp = 1.0 / (1.0 + exp(-1.0 * dd * (R / (pa.vdw_r0 + pb.vdw_r0) - 1.0)));
-      const Dual3 R2 = R * R;
-      e_pair += (-1.0 * s6 * c6) * damp / (R2 * R2 * R2);
     }
+    gr += e.d[0];
   }
-  grad[3 * t] = e_pair.d[0];
-  grad[3 * t + 1] = e_pair.d[1];
-  grad[3 * t + 2] = e_pair.d[2];
+  gr = warp_sum(gr);
+  g[0] = warp_sum(g[0]) / R;
+  g[1] = warp_sum(g[1]) / R;
+  if (lane < 3) {
+    // rows of Rm: s, py, pz, px; columns: local s, y, z, x
+    const int row = lane == 0 ? 3 : lane;
+    grad[3 * t + lane] = sh.Rm[row * 4 + 2] * gr + sh.Rm[row * 4 + 3] * g[0] + sh.Rm[row * 4 + 1] * g[1];
+  }
 }
 
-// forces F_i = -g_i of one molecule's atoms from its pair gradients
-__global__ void force_reduce_kernel(const DevMol* __restrict__ mols, int m, const double* __restrict__ grad,
-                                    double* __restrict__ forces) {
+// forces F_i = -g_i of one molecule's atoms from its pair gradients: a warp per atom
+__global__ void __launch_bounds__(128)
+force_reduce_kernel(const DevMol* __restrict__ mols, int m, const double* __restrict__ grad,
+                    double* __restrict__ forces) {
   const DevMol mol = mols[m];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= mol.natoms) return;
   double g[3] = {0.0, 0.0, 0.0};
-  for (int a = 0; a < i; ++a) {
-    const long long q = pair_index(a, i, mol.natoms);
-    for (int k = 0; k < 3; ++k) g[k] += grad[3 * q + k];
+  for (int a = lane; a < mol.natoms; a += 32) {
+    if (a == i) continue;
+    const double sg = a < i ? 1.0 : -1.0;
+    const double* q = grad + 3 * (a < i ? pair_index(a, i, mol.natoms) : pair_index(i, a, mol.natoms));
+    for (int k = 0; k < 3; ++k) g[k] += sg * q[k];
   }
-  for (int b = i + 1; b < mol.natoms; ++b) {
-    const long long q = pair_index(i, b, mol.natoms);
-    for (int k = 0; k < 3; ++k) g[k] -= grad[3 * q + k];
-  }
-  for (int k = 0; k < 3; ++k) forces[3 * i + k] = -g[k];
+  for (int k = 0; k < 3; ++k) g[k] = warp_sum(g[k]);
+  if (lane < 3) forces[3 * i + lane] = -(lane == 0 ? g[0] : lane == 1 ? g[1] : g[2]);
 }
 
 void launch_forces(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, int m, long long pair0,
                    long long npairs, int natoms, const EriTable* eri, const OverlapTable* ovt, const double* P,
                    VdwParams vdw, double* grad, double* forces, cudaStream_t s) {
   if (npairs > 0)
-    pair_grad_kernel<<<(unsigned)((npairs + 63) / 64), 64, 0, s>>>(atoms, pairs, pair0, npairs, mols, eri, ovt, P,
-                                                                      vdw, grad);
-  force_reduce_kernel<<<(natoms + 127) / 128, 128, 0, s>>>(mols, m, grad, forces);
+    pair_grad_kernel<<<(unsigned)((npairs + kGradWarps - 1) / kGradWarps), kGradWarps * 32, 0, s>>>(
+        atoms, pairs, pair0, npairs, mols, eri, ovt, P, vdw, grad);
+  force_reduce_kernel<<<(natoms + 3) / 4, 128, 0, s>>>(mols, m, grad, forces);
 }
 
 }  // namespace nddo
