@@ -135,6 +135,7 @@ constexpr int kPurBigSteps = 56;     // steps launched above kPurSmallMaxN: HOMO
 struct PurState {
   unsigned long long lo, hi;         // Gershgorin interval, order-preserving keys
   long long trace[kPurBigSteps + 1]; // tr X_k
+  int bad;                           // a digit sum left the range its recombination covers
 };
 struct PurScratch { double* m[7]; }; // N x N scratch matrices holding two digit buffers of seven digits each
 void purify_prepare();               // one-time kernel attributes (before any stream capture)

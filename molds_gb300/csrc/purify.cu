@@ -41,7 +41,7 @@
 namespace nddo {
 
 constexpr int kDigits = 7, kLevels = 8;
-constexpr int kPurSmallThreads = 512;
+constexpr int kPurSmallThreads = 17 * 32;
 constexpr int kPurSmallSteps = 100;                // the one-CTA kernel stops by itself; its steps are cheap
 constexpr long long kPurWaitCycles = 2000000000LL; // ~1 s: a copy or an MMA that has not completed by then never will
 constexpr int kTraceShift = 12;                    // traces are summed in units of 2^-43
@@ -68,6 +68,39 @@ __device__ __forceinline__ uint32_t pu_idesc(int ncols) {
   return (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
+// The digit products of levels [L0, L1) over `steps` K steps of 16, by one
+// thread.  The digits of B lie behind one another (stride sb, cols rows each) and
+// so do the level accumulators (cols columns each), so one MMA multiplies digit i
+// of A with up to MOST = 256 / cols digits j, j + 1, .. of B into levels i + j,
+// i + j + 1, ..: 12 MMAs of up to 256 columns per K step at 64 columns instead of
+// 34.  Reading A costs an MMA 32 clocks of shared memory whatever its width, so
+// a 64-column one runs at half the tensor rate and a 256-column one at all of it.
+// Unrolled: the issuing thread has about a hundred clocks per MMA.
+template <int MOST, int L0, int L1>
+__device__ __forceinline__ void pu_products(uint32_t tmem, uint32_t a, uint32_t sa, uint32_t b, uint32_t sb, uint32_t hi,
+                                            int cols, int steps, bool fresh) {
+#pragma unroll
+  for (int i = 0; i < kDigits; ++i) {
+    const int j0 = L0 > i ? L0 - i : 0, top = L1 - 1 - i < kDigits - 1 ? L1 - 1 - i : kDigits - 1;
+    // the first product into a level overwrites it: digit 0 of A for levels
+    // 0 .. 6, product (1, 6), by itself, for level 7
+    const int j1 = i == 1 && L1 == kLevels ? top - 1 : top;
+#pragma unroll
+    for (int t = 0; t < kDigits; ++t) {
+      const bool extra = t == kDigits - 1;
+      const int j = extra ? kDigits - 1 : j0 + t * MOST;
+      if (extra ? !(i == 1 && L1 == kLevels) : j > j1) continue;
+      const int w = extra ? 1 : (MOST < j1 - j + 1 ? MOST : j1 - j + 1);
+      const uint32_t d = tmem + (i + j - L0) * cols, idesc = pu_idesc(w * cols);
+      uint32_t ai = a + ((i * sa) >> 4), bj = b + ((j * sb) >> 4), acc = (i == 0 || extra) && fresh ? 0u : 1u;
+      for (int s = 0; s < steps; ++s, ai += 256 >> 4, bj += 256 >> 4) {
+        pu_mma(d, ai, bj, hi, idesc, acc);
+        acc = 1;
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ bool pu_wait(uint32_t bar, uint32_t parity) {
   uint32_t done = 0;
   const long long t0 = clock64();
@@ -81,6 +114,10 @@ __device__ __forceinline__ void pu_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
 
+// Accumulators as integers.  They are integers below 2^22 in magnitude, so
+// adding 1.5 * 2^23 leaves them in the low mantissa bits: a full-rate FP32 add
+// where the conversion instruction runs at a quarter of it (5390 -> 1800 clocks
+// for a 128 x 64 tile).  range collects the bits that would show a larger one.
 __device__ __forceinline__ void pu_ld8(uint32_t addr, float* v) {
   uint32_t u[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -89,6 +126,13 @@ __device__ __forceinline__ void pu_ld8(uint32_t addr, float* v) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(u[i]);
 }
+constexpr int kMagic = 0x4B400000;
+__device__ __forceinline__ int pu_int(float f, uint32_t& range) {
+  const int b = __float_as_int(f + 12582912.0f);
+  range |= (uint32_t)(b ^ kMagic);
+  return b - kMagic;
+}
+__device__ __forceinline__ bool pu_in_range(uint32_t range) { return range < (1u << 23); }
 
 __device__ __forceinline__ long long pu_mad(int a, int b, long long c) {
   long long r;
@@ -96,25 +140,31 @@ __device__ __forceinline__ long long pu_mad(int a, int b, long long c) {
   return r;
 }
 
-// the eight levels of eight columns, recombined: units of 2^-55, level l weighs 2^(41 - 8 l)
-__device__ __forceinline__ void pu_gather8(uint32_t addr, int stride, long long* s) {
-  float v[4][8];
-#pragma unroll
-  for (int l = 0; l < 4; ++l) pu_ld8(addr + l * stride, v[l]);
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    s[i] = pu_mad(__float2int_rn(v[0][i]), 1 << 24,
-                  pu_mad(__float2int_rn(v[1][i]), 1 << 16,
-                         pu_mad(__float2int_rn(v[2][i]), 1 << 8, (long long)__float2int_rn(v[3][i])))) << 17;
-#pragma unroll
-  for (int l = 0; l < 4; ++l) pu_ld8(addr + (l + 4) * stride, v[l]);
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int t = (__float2int_rn(v[2][i]) + (__float2int_rn(v[3][i]) >> 8) + 64) >> 7;
-    s[i] = pu_mad(__float2int_rn(v[0][i]), 1 << 9, pu_mad(__float2int_rn(v[1][i]), 2, s[i] + t));
+// x += sgn * (levels L .. END - 1), units of 2^-55: level l weighs 2^(41 - 8 l);
+// an even level and the next one make one 32-bit number, the last two are rounded
+template <int L, int END, int NL>
+__device__ __forceinline__ void pu_add(const float (&v)[NL][8], int i, int sgn, long long& x, uint32_t& range) {
+  constexpr int w = 41 - 8 * L, at = L - (END - NL);
+  if constexpr (L + 2 == kLevels) {
+    x = pu_mad((pu_int(v[at][i], range) + (pu_int(v[at + 1][i], range) >> 8) + 64) >> 7, sgn, x);
+  } else if constexpr ((L & 1) == 0 && L + 1 < END) {
+    const int t = pu_int(v[at][i], range) * 256 + pu_int(v[at + 1][i], range);
+    if constexpr (L == 0) x += (long long)((unsigned long long)(unsigned)(t * sgn * 2) << 32);
+    else x = pu_mad(t, sgn * (1 << (w - 8)), x);
+    if constexpr (L + 2 < END) pu_add<L + 2, END, NL>(v, i, sgn, x, range);
+  } else {
+    if constexpr (w < 31) x = pu_mad(pu_int(v[at][i], range), sgn * (1 << w), x);
+    if constexpr (L + 1 < END) pu_add<L + 1, END, NL>(v, i, sgn, x, range);
   }
+}
+template <int L0, int NL>
+__device__ __forceinline__ void pu_levels8(uint32_t addr, int stride, int sgn, long long* x, uint32_t& range) {
+  float v[NL][8];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) pu_ld8(addr + l * stride, v[l]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) pu_add<L0, L0 + NL, NL>(v, i, sgn, x[i], range);
 }
 
 // Balanced base-256 digits of eight values as FP16, most significant slice
@@ -167,13 +217,14 @@ __device__ __forceinline__ void pu_join8(const uint4* in, long long* x) {
 __device__ __forceinline__ long long pu_fixed(double v) { return __double2ll_rn(v * 36028797018963968.0); }   // 2^55
 __device__ __forceinline__ double pu_density(long long x) { return (double)x * 5.5511151231257827e-17; }       // 2 * 2^-55
 
-// Where the iteration stands after the traces T_0 .. T_k: the step to take from
-// X_k (1: X^2, 0: 2 X - X^2), or -1 when X_k is the projector.  first = the
-// first step j whose tr(X_j - X_j^2) was below the tolerance (-1: none yet).
-__device__ __forceinline__ int pu_step(const long long* T, int k, int first, long long occ) {
+// Where the iteration stands at X_k, with t0, t1 the traces of X_k and X_{k-1}:
+// the step to take (1: X^2, 0: 2 X - X^2), or -1 when X_k is the projector.
+// first = the first step j whose tr(X_j - X_j^2) was below the tolerance (-1:
+// none yet).
+__device__ __forceinline__ int pu_step(long long t0, long long t1, int k, int first, long long occ) {
   if (first >= 0 && k >= first + 3) return -1;
-  if (first >= 0 && k == first + 2) return T[k - 1] > occ ? 0 : 1;   // the other kind than step k - 1
-  return T[k] > occ ? 1 : 0;
+  if (first >= 0 && k == first + 2) return t1 > occ ? 0 : 1;   // the other kind than step k - 1
+  return t0 > occ ? 1 : 0;
 }
 __device__ __forceinline__ bool pu_traced(long long a, long long b) {
   const long long d = a > b ? a - b : b - a;
@@ -191,32 +242,76 @@ __device__ __forceinline__ bool pu_counted(long long t, long long occ) {
 // N <= 128: one CTA per molecule, everything on the SM.  The seven digit
 // matrices (K-major core-matrix tiles, the same copy serves as A and as B
 // because X is symmetric: 224 KB at N = 128) in shared memory, X itself in
-// registers: thread (row r, columns 16 g ..) with r its TMEM lane.  A step is 34
-// digit products into eight TMEM accumulators (512 columns: 64 columns of X at
-// a time), then the recombination in registers.
+// registers: thread (row r, columns 16 g .. of each 64) with r its TMEM lane.
+// A step is 34 digit products over all N columns (an MMA costs its 4 KB of A
+// whatever its width: 50 clocks, so few wide ones).  The eight accumulators do
+// not fit tensor memory together above N = 64, so the levels go in groups of L
+// through two buffers of it: the issuing warp fills one while the others
+// recombine the other.
+// Measured (clocks a step, N = 50 / 72 / 120): 18000 / 32000 / 50000 with all
+// levels of 64 columns at a time, conversions by instruction and the trace by
+// shared atomics; see the table in the launcher for what it is now.
 // ---------------------------------------------------------------------------
-template <int H>
+constexpr int kPurSmallWarps = 16;   // recombining; one more issues the MMAs
+
+template <int H, int L, int J>
+__device__ __forceinline__ void pu_group(uint32_t taddr, int np, int g, int sgn, long long (&x)[H][16],
+                                         uint32_t& range) {
+  constexpr int L0 = J * L, NL = L0 + L <= kLevels ? L : kLevels - L0;
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    const int c0 = 64 * h + 16 * g;
+    if (c0 < np) {
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+        pu_levels8<L0, NL>(taddr + (J & 1) * L * np + c0 + 8 * s, np, sgn, &x[h][8 * s], range);
+    }
+  }
+}
+
+template <int L, int J>
+__device__ __forceinline__ void pu_level_group(uint32_t to, uint32_t lo, uint32_t slice, uint32_t hi, int np) {
+  constexpr int L0 = J * L, L1 = L0 + L < kLevels ? L0 + L : kLevels;
+  const int k = np / 16;
+  if (L == 2) pu_products<2, L0, L1>(to, lo, slice, lo, slice, hi, np, k, true);
+  else if (L == 3) pu_products<3, L0, L1>(to, lo, slice, lo, slice, hi, np, k, true);
+  else if (np <= 32) pu_products<7, L0, L1>(to, lo, slice, lo, slice, hi, np, k, true);
+  else pu_products<4, L0, L1>(to, lo, slice, lo, slice, hi, np, k, true);
+}
+
+// The recombining warps have read level group j (buffer j of a step's first two
+// groups).  A named barrier per group: a warp that runs ahead reaches the next
+// group's while others are still to arrive at this one.
+__device__ __forceinline__ void pu_drained(int j, bool issuer) {
+  constexpr int kAll = (kPurSmallWarps + 1) * 32;
+  if (issuer) asm volatile("bar.sync %0, %1;" :: "r"(1 + j), "n"(kAll) : "memory");
+  else asm volatile("bar.arrive %0, %1;" :: "r"(1 + j), "n"(kAll) : "memory");
+}
+
+template <int H, int L>
 __global__ void __launch_bounds__(kPurSmallThreads, 1)
 purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, MolState* __restrict__ st,
                     const double* __restrict__ F, double* __restrict__ P, int np_max, int* __restrict__ err) {
+  constexpr int G = (kLevels + L - 1) / L;   // level groups
   extern __shared__ __align__(1024) unsigned char pu_sm[];
   const int mi = list[blockIdx.x];
   if (st[mi].status != kActive) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao, np = (n + 15) & ~15;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = warp & 3, g = warp >> 2;
-  const int r = q * 32 + lane;
+  const bool issuer = warp == kPurSmallWarps;
+  const int r = issuer ? 128 : q * 32 + lane;
   // behind the digits (the last one padded to the MMA's 128 rows)
   unsigned char* tail = pu_sm + (size_t)(kDigits - 1) * 2 * np_max * np_max + (size_t)256 * np_max;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(tail);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 8);
-  double* red = reinterpret_cast<double*>(tail + 16);                      // 2 x 16
-  long long* T = reinterpret_cast<long long*>(tail + 16 + 32 * 8);         // traces, kPurSmallSteps + 1
+  const uint32_t bar = pu_smem(tail);                                      // two, one per buffer
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 16);
+  double* red = reinterpret_cast<double*>(tail + 32);                      // 2 x 17
+  long long* diag = reinterpret_cast<long long*>(tail + 32 + 34 * 8);      // 2 x 128
   const double* Fm = F + mol.mat0;
 
   // Gershgorin interval
   double lo = 1e300, hi = -1e300, bad = 0.0;
-  for (int i = warp; i < n; i += kPurSmallThreads / 32) {
+  for (int i = warp; i < n; i += kPurSmallWarps + 1) {
     double s = 0.0;
     for (int j = lane; j < n; j += 32)
       if (j != i) s += fabs(Fm[(long long)i * n + j]);
@@ -226,24 +321,25 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
     lo = fmin(lo, d - s);
     hi = fmax(hi, d + s);
   }
-  if (lane == 0) { red[warp] = bad > 0.0 ? -1e300 : lo; red[16 + warp] = hi; }
-  for (int i = tid; i <= kPurSmallSteps; i += kPurSmallThreads) T[i] = 0;
+  if (lane == 0) { red[warp] = bad > 0.0 ? -1e300 : lo; red[17 + warp] = hi; }
+  for (int i = tid; i < 256; i += kPurSmallThreads) diag[i] = 0;
   int ncols = 32;
-  while (ncols < kLevels * (H == 2 ? 64 : np)) ncols <<= 1;
+  while (ncols < 2 * L * np) ncols <<= 1;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  :: "r"(pu_smem(tmem_slot)), "r"(ncols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(pu_smem(mbar)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar + 8));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  for (int w = 0; w < 16; ++w) { lo = fmin(lo, red[w]); hi = fmax(hi, red[16 + w]); }
+  for (int w = 0; w < kPurSmallWarps + 1; ++w) { lo = fmin(lo, red[w]); hi = fmax(hi, red[17 + w]); }
   const bool usable = lo > -1e299 && hi > lo;
   const double scale = usable ? 1.0 / (hi - lo) : 0.0;
 
@@ -263,11 +359,14 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
 
   const long long occ = (long long)mol.nocc * kTraceOne;
   const uint32_t slice = 2u * np * np, sbo = 16u * np;
-  uint32_t parity = 0;
+  const uint32_t taddr = tmem + ((uint32_t)((q * 32) & 127) << 16);
+  const bool work = !issuer && q * 32 < n;
+  uint32_t parity[2] = {0, 0}, range = 0;
   bool ok = true, done = false;
   int first = -1;
+  long long t0 = 0, t1 = 0;   // traces of X_k and X_{k-1}
   for (int k = 0; usable; ++k) {
-    // digits of X_k into shared memory, its trace
+    // digits of X_k into shared memory, its diagonal
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const int c0 = 64 * h + 16 * g;
@@ -282,64 +381,71 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
         }
 #pragma unroll
         for (int c = 0; c < 16; ++c)
-          if (c0 + c == r && r < n)
-            atomicAdd(reinterpret_cast<unsigned long long*>(T + k), (unsigned long long)(x[h][c] >> kTraceShift));
+          if (c0 + c == r) diag[(k & 1) * 128 + r] = x[h][c] >> kTraceShift;
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    if (first < 0 && k > 0 && pu_traced(T[k], T[k - 1])) first = k - 1;
-    const int op = pu_step(T, k, first, occ);
-    if (op < 0) { done = pu_counted(T[k], occ); break; }
+    if (!__syncthreads_and(ok)) { ok = false; break; }
+    t1 = t0;
+    t0 = 0;
+    for (int i = lane; i < n; i += 32) t0 += diag[(k & 1) * 128 + i];
+    for (int o = 16; o > 0; o >>= 1) t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+    if (first < 0 && k > 0 && pu_traced(t0, t1)) first = k - 1;
+    const int op = pu_step(t0, t1, k, first, occ);
+    if (op < 0) { done = pu_counted(t0, occ); break; }
     if (k == kPurSmallSteps) break;
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      const int cols = H == 2 ? min(64, np - 64 * h) : np, lstride = H == 2 ? 64 : np;
-      if (tid == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t idesc = pu_idesc(cols), dhi = pu_desc_hi(sbo);
-        uint32_t a[kDigits], b[kDigits];
-#pragma unroll
-        for (int d = 0; d < kDigits; ++d) {
-          a[d] = pu_desc_lo(pu_smem(pu_sm) + d * slice);
-          b[d] = a[d] + (((uint32_t)(64 * h >> 3) * sbo) >> 4);
-        }
-        for (int s = 0; s < np / 16; ++s) {
-#pragma unroll
-          for (int l = 0; l < kLevels; ++l)
-#pragma unroll
-            for (int i = 0; i < kDigits; ++i)
-              if (i <= l && l - i < kDigits)
-                pu_mma(tmem + l * lstride, a[i] + s * (256 >> 4), b[l - i] + s * (256 >> 4), dhi, idesc,
-                       (s > 0 || i > (l < kDigits ? 0 : l - kDigits + 1)) ? 1u : 0u);
-        }
-        pu_commit(pu_smem(mbar));
-      }
-      ok = pu_wait(pu_smem(mbar), parity) && ok;
-      parity ^= 1;
+    if (issuer) {
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const int c0 = 16 * g;
-      if (c0 < cols && q * 32 < n) {
+      const uint32_t lo = pu_desc_lo(pu_smem(pu_sm));
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          long long v[8];
-          pu_gather8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + 8 * s), lstride, v);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) x[h][8 * s + c] = op ? v[c] : 2 * x[h][8 * s + c] - v[c];
+      for (int j = 0; j < G; ++j) {
+        if (j >= 2) {
+          pu_drained(j - 2, true);
+          asm volatile("tcgen05.fence::after_thread_sync;");
         }
-        // rows past the basis came from whatever lies behind the digits
-        if (r >= n) {
+        if (lane == 0) {
+          const uint32_t to = tmem + (j & 1) * L * np, hi = pu_desc_hi(sbo);
+          if (j == 0) pu_level_group<L, 0>(to, lo, slice, hi, np);
+          else if (j == 1) pu_level_group<L, 1>(to, lo, slice, hi, np);
+          else if (j == 2) pu_level_group<L, (G > 2 ? 2 : 0)>(to, lo, slice, hi, np);
+          else pu_level_group<L, (G > 3 ? 3 : 0)>(to, lo, slice, hi, np);
+          pu_commit(bar + 8 * (j & 1));
+        }
+        __syncwarp();
+      }
+    } else {
+      const int sgn = op ? 1 : -1;
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) x[h][c] = op ? 0 : 2 * x[h][c];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        ok = pu_wait(bar + 8 * (j & 1), parity[j & 1]) && ok;
+        parity[j & 1] ^= 1;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (work) {
+          if (j == 0) pu_group<H, L, 0>(taddr, np, g, sgn, x, range);
+          else if (j == 1) pu_group<H, L, 1>(taddr, np, g, sgn, x, range);
+          else if (j == 2) pu_group<H, L, (G > 2 ? 2 : 0)>(taddr, np, g, sgn, x, range);
+          else pu_group<H, L, (G > 3 ? 3 : 0)>(taddr, np, g, sgn, x, range);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        if (j + 2 < G) pu_drained(j, false);
+      }
+      // rows past the basis came from whatever lies behind the digits
+      if (r >= n) {
+        range = 0;
+#pragma unroll
+        for (int h = 0; h < H; ++h)
 #pragma unroll
           for (int c = 0; c < 16; ++c) x[h][c] = 0;
-        }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      if (H == 2 && h == 0) __syncthreads();   // TMEM is reused for the second half
     }
-    if (!__syncthreads_and(ok)) { ok = false; break; }
   }
-  if (ok && done) {
+  done = __syncthreads_and(ok && done && pu_in_range(range));
+  if (done && !issuer) {
     double* Pm = P + mol.mat0;
 #pragma unroll
     for (int h = 0; h < H; ++h)
@@ -351,10 +457,8 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   }
   if (tid == 0) {
     if (!ok) atomicExch(err, 1);
-    st[mi].flags = (ok && done) ? 0 : kNeedEigen;
+    st[mi].flags = done ? 0 : kNeedEigen;
   }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols));
 }
 
@@ -367,11 +471,11 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
 // matrices: two digits per N x N doubles (Np = N rounded up to 32 has
 // Np^2 <= 2 N^2 from N = 79 on).
 // ---------------------------------------------------------------------------
-constexpr int kPurTileThreads = 256;
+constexpr int kPurTileThreads = 512;
 constexpr int kTileM = 128, kTileN = 64, kChunkK = 32, kStages = 2;
 constexpr uint32_t kStageA = kTileM * kChunkK * 2, kStageB = kTileN * kChunkK * 2;   // bytes per digit
 constexpr uint32_t kStageBytes = kDigits * (kStageA + kStageB);
-constexpr int kSegChunks = 32;                            // K = 1024: sums of two digits' products reach 2^24 at most
+constexpr int kSegChunks = 16;                            // K = 512: the largest sums, of a digit's squares, stay near 0.7 * 2^22
 constexpr int kXPitch = kTileM + 1;                       // transposed tile, 8-byte elements: no bank conflicts either way
 constexpr size_t kPurTileSmem = kStages * kStageBytes + 256;
 
@@ -482,7 +586,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   const long long occ = (long long)mol.nocc * kTraceOne;
   double lo, hi;
   if (!pu_interval(pur[mi], &lo, &hi)) return;
-  const int op = pu_step(pur[mi].trace, k, pu_first(pur[mi].trace, k), occ);   // the same in every CTA of the molecule
+  const int op = pu_step(pur[mi].trace[k], pur[mi].trace[k > 0 ? k - 1 : 0], k, pu_first(pur[mi].trace, k), occ);   // the same in every CTA of the molecule
   if (op < 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = tile.y * kTileM, c0 = tile.z * kTileN;
@@ -511,13 +615,15 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   const uint32_t sm = pu_smem(pu_sm);
   const int buf = k & 1;
   const int q = warp & 3, r = r0 + q * 32 + lane;
-  const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((warp >> 2) * 32);
-  const int groups = q * 32 < rows ? max(0, min(4, (cols - (warp >> 2) * 32) >> 3)) : 0;   // of eight columns
-  long long v[4][8];
+  const int cw = (warp >> 2) * 16;   // this warp's columns of the tile: cw .. cw + 15
+  const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cw;
+  const int groups = q * 32 < rows ? max(0, min(2, (cols - cw) >> 3)) : 0;   // of eight columns
+  long long v[2][8];
 #pragma unroll
-  for (int s = 0; s < 4; ++s)
+  for (int s = 0; s < 2; ++s)
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[s][i] = 0;
+  uint32_t range = 0;
   bool ok = true;
   // K in segments whose digit sums stay integers below 2^24
   for (int seg = 0, cb = 0; cb < chunks && ok; ++seg, cb += kSegChunks) {
@@ -531,32 +637,26 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
                      :: "r"(full + 8 * s), "r"((ba + bb) * kDigits) : "memory");
         for (int d = 0; d < kDigits; ++d) {
           const unsigned char* p = pu_plane(ws, mol, buf, d) + (size_t)c * (64 * (size_t)np);
-          const uint32_t to = sm + s * kStageBytes + d * (kStageA + kStageB);
+          const uint32_t to = sm + s * kStageBytes;
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                       :: "r"(to), "l"(p + (size_t)r0 * 64), "r"(ba), "r"(full + 8 * s) : "memory");
+                       :: "r"(to + d * kStageA), "l"(p + (size_t)r0 * 64), "r"(ba), "r"(full + 8 * s) : "memory");
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                       :: "r"(to + kStageA), "l"(p + (size_t)c0 * 64), "r"(bb), "r"(full + 8 * s) : "memory");
+                       :: "r"(to + kDigits * kStageA + d * bb), "l"(p + (size_t)c0 * 64), "r"(bb), "r"(full + 8 * s)
+                       : "memory");
         }
       }
     } else if (warp == 1 && lane == 0) {
-      const uint32_t idesc = pu_idesc(cols);
       asm volatile("tcgen05.fence::after_thread_sync;");
       for (int c = cb; c < ce; ++c) {
         const int s = c % kStages;
         if (!pu_wait(full + 8 * s, (c / kStages) & 1)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t base = pu_desc_lo(sm + s * kStageBytes), dhi = pu_desc_hi(512), later = c > cb;
-#pragma unroll
-        for (int l = 0; l < kLevels; ++l)
-#pragma unroll
-          for (int i = 0; i < kDigits; ++i)
-            if (i <= l && l - i < kDigits) {
-#pragma unroll
-              for (int t = 0; t < kChunkK / 16; ++t)
-                pu_mma(tmem + l * kTileN, base + ((i * (kStageA + kStageB) + t * 256) >> 4),
-                       base + (((l - i) * (kStageA + kStageB) + kStageA + t * 256) >> 4), dhi, idesc,
-                       (t > 0 || i > (l < kDigits ? 0 : l - kDigits + 1)) ? 1u : later);
-            }
+        const uint32_t base = pu_desc_lo(sm + s * kStageBytes);
+        const uint32_t bb = base + (kDigits * kStageA >> 4), sb = (uint32_t)cols * kChunkK * 2;
+        if (cols == kTileN)
+          pu_products<4, 0, kLevels>(tmem, base, kStageA, bb, sb, pu_desc_hi(512), cols, kChunkK / 16, c == cb);
+        else
+          pu_products<7, 0, kLevels>(tmem, base, kStageA, bb, sb, pu_desc_hi(512), cols, kChunkK / 16, c == cb);
         pu_commit(empty + 8 * s);
       }
       if (ok) pu_commit(last);
@@ -567,12 +667,10 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     ok = __syncthreads_and(ok);
     if (ok) {
 #pragma unroll
-      for (int s = 0; s < 4; ++s)
+      for (int s = 0; s < 2; ++s)
         if (s < groups) {
-          long long t[8];
-          pu_gather8(taddr + 8 * s, kTileN, t);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[s][i] += t[i];
+          pu_levels8<0, 4>(taddr + 8 * s, cols, 1, v[s], range);
+          pu_levels8<4, 4>(taddr + 4 * cols + 8 * s, cols, 1, v[s], range);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -584,11 +682,13 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     // X_{k+1}: row r, the digits of eight columns at a time
     const bool mirror = tile.z >= 2 * tile.y + 2;   // the transposed block is no tile of its own
     long long* xt = reinterpret_cast<long long*>(pu_sm);   // the operand stages are free now
+    // rows past the padded basis are whatever the stage held before
+    if (r < np && !pu_in_range(range)) atomicExch(&pur[mi].bad, 1);
     long long tr = 0;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
+    for (int s = 0; s < 2; ++s) {
       if (s >= groups) continue;
-      const int cl = (warp >> 2) * 32 + 8 * s, c = c0 + cl;
+      const int cl = cw + 8 * s, c = c0 + cl;
       const size_t at = pu_at(np, r, c);
       uint4 dg[kDigits];
       if (!op) {
@@ -640,7 +740,7 @@ purify_store_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   const int n = mol.nao, np = pu_np(n), kb = np >> 3;
   double lo, hi;
   const int first = pu_first(pur[mi].trace, steps);
-  const bool done = pu_interval(pur[mi], &lo, &hi) && first >= 0 && first + 3 <= steps &&
+  const bool done = !pur[mi].bad && pu_interval(pur[mi], &lo, &hi) && first >= 0 && first + 3 <= steps &&
                     pu_counted(pur[mi].trace[first + 3], (long long)mol.nocc * kTraceOne);
   if (blockIdx.x == 0 && threadIdx.x == 0) st[mi].flags = done ? 0 : kNeedEigen;
   if (!done) return;
@@ -664,19 +764,20 @@ purify_store_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
 __global__ void purify_reset_kernel(const int* __restrict__ list, PurState* __restrict__ pur) {
   PurState& s = pur[list[blockIdx.x]];
   for (int i = threadIdx.x; i <= kPurBigSteps; i += blockDim.x) s.trace[i] = 0;
-  if (threadIdx.x == 0) { s.lo = ~0ull; s.hi = 0ull; }
+  if (threadIdx.x == 0) { s.lo = ~0ull; s.hi = 0ull; s.bad = 0; }
 }
 
 // ---------------------------------------------------------------------------
 static size_t small_smem(int np) {
-  return (size_t)(kDigits - 1) * 2 * np * np + (size_t)256 * np + 16 + 32 * 8 + (kPurSmallSteps + 1) * 8;
+  return (size_t)(kDigits - 1) * 2 * np * np + (size_t)256 * np + 32 + 34 * 8 + 2 * 128 * 8;
 }
 
 void purify_prepare() {
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncSetAttribute(purify_small_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(64));
-    cudaFuncSetAttribute(purify_small_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(128));
+    cudaFuncSetAttribute(purify_small_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(64));
+    cudaFuncSetAttribute(purify_small_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(80));
+    cudaFuncSetAttribute(purify_small_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(128));
     cudaFuncSetAttribute(purify_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPurTileSmem);
   });
 }
@@ -695,10 +796,11 @@ void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max
   if (nlist <= 0) return;
   purify_prepare();
   const int np = (max_n + 15) / 16 * 16;
-  if (np <= 64)
-    purify_small_kernel<1><<<nlist, kPurSmallThreads, small_smem(np), s>>>(mols, list, st, F, P, np, err);
-  else
-    purify_small_kernel<2><<<nlist, kPurSmallThreads, small_smem(np), s>>>(mols, list, st, F, P, np, err);
+  const size_t sm = small_smem(np);
+  // levels per group: two buffers of L x np of the 512 columns of tensor memory
+  if (np <= 64) purify_small_kernel<1, 4><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
+  else if (np <= 80) purify_small_kernel<2, 3><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
+  else purify_small_kernel<2, 2><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
 }
 
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
