@@ -33,15 +33,17 @@ static T* dalloc(size_t count, size_t* total) {
 }
 
 // ---------------------------------------------------------------------------
-__global__ void init_state_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, int n,
+// grid: (CTAs per molecule, molecules).  The DIIS history needs no reset: its
+// slots are only read once this SCF has pushed them.
+__global__ void init_state_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list,
                                   MolState* __restrict__ st, double* __restrict__ C, double* __restrict__ P,
                                   double* __restrict__ eps, int requires_guess, int reset_density,
-                                  double* __restrict__ hist_dens, double* __restrict__ hist_err, int diis_m,
-                                  long long mat_total, int* __restrict__ sweeps) {
-  const int m = list[blockIdx.x];
+                                  int* __restrict__ sweeps) {
+  const int m = list[blockIdx.y];
   const DevMol mol = mols[m];
   const long long n2 = (long long)mol.nao * mol.nao;
-  if (threadIdx.x == 0) {
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if (first == 0) {
     MolState s;
     memset(&s, 0, sizeof(s));
     s.status = kActive;
@@ -55,20 +57,14 @@ __global__ void init_state_kernel(const DevMol* __restrict__ mols, const int* __
   // previous eigenvectors as the eigensolver's warm-start basis
   // a cold start also forgets the eigenvalues of the last solve, which the
   // FP64 eigensolver would otherwise take as starting points
-  if (reset_density)
-    for (int i = threadIdx.x; i < mol.nao; i += blockDim.x) eps[mol.vec0 + i] = __longlong_as_double(0x7ff8000000000000LL);
-  if (reset_density)
-    for (long long i = threadIdx.x; i < n2; i += blockDim.x) {
+  if (reset_density) {
+    for (long long i = first; i < mol.nao; i += step) eps[mol.vec0 + i] = __longlong_as_double(0x7ff8000000000000LL);
+    for (long long i = first; i < n2; i += step) {
       const long long r = i / mol.nao, c = i % mol.nao;
       C[mol.mat0 + i] = (r == c) ? 1.0 : 0.0;
       P[mol.mat0 + i] = 0.0;
     }
-  // the DIIS window starts zero-filled (as the reference's zero-initialised history)
-  for (int k = 0; k < diis_m; ++k)
-    for (long long i = threadIdx.x; i < n2; i += blockDim.x) {
-      hist_dens[k * mat_total + mol.mat0 + i] = 0.0;
-      hist_err[k * mat_total + mol.mat0 + i] = 0.0;
-    }
+  }
 }
 
 // out[0] = molecules still active, out[1] = those of them that wait for the eigensolver
@@ -364,6 +360,7 @@ void Batch::allocate(const BatchCapacity& cap) {
   {
     const size_t b = diis_scratch_bytes(nm);
     cuda_check(cudaMalloc(&d_diis_ws, b), "cudaMalloc DIIS scratch");
+    cuda_check(cudaMemsetAsync(d_diis_ws, 0, b, stream_), "memset DIIS scratch");
     bytes_ += b;
   }
   d_dip_ws = dalloc<double>((size_t)nm * kDipChunks * 4, &bytes_);
@@ -934,9 +931,9 @@ void Batch::integrals(const std::vector<int>& which) {
   prof_end(h);
   cuda_check(cudaGetLastError(), "pair_kernel");
   h = prof_begin(kKHcore, 0.0);
-  launches_ += 1;
-  launch_hcore_kernel(d_atoms, d_pairs, d_mols, d_list, (int)which.size(), d_blocks, d_ecore_pair, eng_->eri(), d_epc,
-                      d_H, d_state, stream_);
+  launches_ += 2;
+  launch_hcore_kernel(d_atoms, d_pairs, d_mols, d_list, (int)which.size(), list_max_atoms(), d_blocks, d_ecore_pair,
+                      eng_->eri(), d_epc, d_H, d_state, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "hcore_kernel");
   // the pageable index vectors above must outlive their copies
@@ -970,9 +967,10 @@ void Batch::begin(const ScfSettings& s, const std::vector<int>& which, bool requ
   active_host_.resize(h_mols.size(), 0);
   for (int m : which) active_host_[m] = 1;
   launches_ += 1;
-  init_state_kernel<<<(unsigned)which.size(), 256, 0, stream_>>>(d_mols, d_list, (int)which.size(), d_state, d_C,
-                                                                 d_P, d_eps, requires_guess ? 1 : 0, requires_guess ? 1 : 0,
-                                                                 d_hist_dens, d_hist_err, diis_m_, mat_total_, d_sweeps);
+  const int ctas = std::max(1, std::min(64, list_max_n_ * list_max_n_ / 4096));
+  init_state_kernel<<<dim3(ctas, (unsigned)which.size()), 256, 0, stream_>>>(d_mols, d_list, d_state, d_C, d_P, d_eps,
+                                                                             requires_guess ? 1 : 0,
+                                                                             requires_guess ? 1 : 0, d_sweeps);
   cuda_check(cudaGetLastError(), "init_state");
 }
 
@@ -1227,7 +1225,7 @@ void Batch::density_step(const ScfSettings& s) {
 void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, bool eigen) {
   upload_list(which);
   const int nl = (int)which.size();
-  launches_ += 4;   // fock + three DIIS kernels
+  launches_ += 3;   // fock + two DIIS kernels
   int h = prof_begin(kKFock, active_work_estimate(kKFock));
   launch_fock_kernel(d_atoms, d_pairs, d_mols, d_list, nl, list_max_atoms(), d_blocks, d_H, d_P, d_F, d_Pold, d_state, -1,
                      1, 1, stream_);
@@ -1238,8 +1236,8 @@ void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, bool ei
   h = prof_begin(kKDiis, active_work_estimate(kKDiis));
   ScfParamsDev prm = to_dev(s);
   prm.eigen_ran = eigen || !purified(s);
-  launch_diis(d_mols, d_list, nl, d_state, prm, d_P, d_Pold, d_hist_dens, d_hist_err, mat_total_,
-              s.keep_trace ? d_trace : nullptr, max_iter_alloc_, d_diis_ws, stream_);
+  launch_diis(d_mols, d_list, nl, list_max_n_, d_state, prm, d_P, d_Pold, d_hist_dens, d_hist_err, mat_total_,
+              s.keep_trace ? d_trace : nullptr, max_iter_alloc_, d_diis_ws, cap_.slots, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "diis_kernel");
 }
@@ -1339,7 +1337,7 @@ void Batch::finish(const ScfSettings& s, const std::vector<int>& which) {
   // eigenvector rows, as Dsyevd leaves them after the last iteration
   if (purified(s)) hh_reduce(0);   // the SCF itself needed no tridiagonalisation
   if (householder(s)) hh_vectors(s, 1, 0);
-  launches_ += 2;
+  launches_ += 3;
   int h = prof_begin(kKEnergy, 0.0);
   launch_fock_kernel(d_atoms, d_pairs, d_mols, d_list, nl, max_atoms, d_blocks, d_H, d_P, d_F, d_Pold, d_state, 0,
                      0, 0, stream_);
@@ -1347,7 +1345,8 @@ void Batch::finish(const ScfSettings& s, const std::vector<int>& which) {
   vdw.on = s.vdw;
   vdw.s6 = s.vdw_s6;
   vdw.d = s.vdw_d;
-  launch_energy_kernel(d_atoms, d_pairs, d_mols, d_list, nl, d_P, d_F, d_H, d_state, d_charges, vdw, stream_);
+  launch_energy_kernel(d_atoms, d_pairs, d_mols, d_list, nl, list_max_n_, d_P, d_F, d_H, d_dip_ws, d_state, d_charges,
+                       vdw, stream_);
   prof_end(h);
   if (s.dipole) {
     launches_ += 2;

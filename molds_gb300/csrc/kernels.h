@@ -75,7 +75,7 @@ void launch_pair_kernels_split(const DevAtom* atoms, const DevPair* pairs, const
                                const OverlapTable* ovt, double* blocks, double* H, double* ecore_pair,
                                cudaStream_t s);
 void launch_hcore_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
-                         int nlist, const double* blocks, const double* ecore_pair, const EriTable* eri,
+                         int nlist, int max_atoms, const double* blocks, double* ecore_pair, const EriTable* eri,
                          const double* epc, double* H, MolState* st, cudaStream_t s);
 void launch_fock_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
                         int nlist, int max_atoms, const double* blocks, const double* H, const double* P, double* F,
@@ -91,9 +91,10 @@ struct VdwParams {
 void launch_forces(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, int m, long long pair0,
                    long long npairs, int natoms, const EriTable* eri, const OverlapTable* ovt, const double* P,
                    VdwParams vdw, double* grad, double* forces, cudaStream_t s);
+// partial: scratch of nlist x kDipChunks x 2 doubles
 void launch_energy_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
-                          int nlist, const double* P, const double* F, const double* H, MolState* st,
-                          double* charges, VdwParams vdw, cudaStream_t s);
+                          int nlist, int max_n, const double* P, const double* F, const double* H, double* partial,
+                          MolState* st, double* charges, VdwParams vdw, cudaStream_t s);
 // dipole moment of the listed molecules into MolState::dipole; partial holds
 // nlist * kDipChunks * 4 doubles
 constexpr int kDipChunks = 64;
@@ -219,9 +220,9 @@ void launch_gemm(const GemmJob* jobs, int njobs, int ntiles, const float* A, con
 // DIIS in three launches (partial sums, per-molecule solve, apply); scratch
 // holds diis_scratch_bytes(nlist) bytes
 size_t diis_scratch_bytes(int slots);
-void launch_diis(const DevMol* mols, const int* mol_list, int nlist, MolState* st, const ScfParamsDev& prm,
+void launch_diis(const DevMol* mols, const int* mol_list, int nlist, int max_n, MolState* st, const ScfParamsDev& prm,
                  double* P, const double* Pold, double* hist_dens, double* hist_err, long long hist_stride,
-                 TraceEntry* trace, int trace_len, void* scratch, cudaStream_t s);
+                 TraceEntry* trace, int trace_len, void* scratch, int slots, cudaStream_t s);
 
 void launch_newton_scale(const DevMol* mols, const int* mol_list, int nlist, const MolState* st, int require_phase,
                          double* K, const double* O, const double* eps, cudaStream_t s);

@@ -18,6 +18,7 @@
 namespace nddo {
 
 constexpr int kMaxTermsPerSlot = 24;
+constexpr int kMaxFlatTerms = 256; // terms of all slots together
 constexpr int kNumSlots = 22;     // distinct local integrals of an sp-sp pair
 
 // one point-charge term of a local integral
@@ -37,6 +38,11 @@ struct EriTable {
   EriTerm terms[kNumSlots][kMaxTermsPerSlot];
   // local packed 10x10 entry (mu<=nu on A, la<=si on B) -> slot (or -1 = zero)
   signed char slot_of[10][10];
+  // the terms of all slots behind one another, those a pair with a hydrogen can
+  // need first (flat_light of flat_heavy): slot s has nterms[s] from flat_first[s] on
+  int flat_light, flat_heavy;
+  int flat_first[kNumSlots];
+  EriTerm flat[kMaxFlatTerms];
 };
 
 // Overlap polynomial tables: S_local = norm * ang * (R/2)^(na+nb+1) *

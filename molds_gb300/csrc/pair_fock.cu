@@ -90,6 +90,56 @@ __device__ __forceinline__ T core_core(const nddo_atom_params& pa, const nddo_at
   return e;
 }
 
+// core_core by a warp: the up to fourteen exponentials over the lanes, the sums
+// in core_core's order by every lane
+__device__ __forceinline__ double core_core_warp(const nddo_atom_params& pa, const nddo_atom_params& pb, double R,
+                                                 double ssss, int theory, int lane) {
+  // lanes 0-3 and 4-7: the Gaussians of A and B; 8, 9: e^{-alpha R}; 10-13: PDDG
+  double x = 0.0;
+  bool use = false;
+  if (lane < 8) {
+    const nddo_atom_params& p = lane < 4 ? pa : pb;
+    const int i = lane & 3;
+    use = theory != NDDO_MNDO && p.gk[i] != 0.0;
+    const double d = R - p.gm[i];
+    x = -p.gl[i] * (d * d);
+  } else if (lane < 10) {
+    use = true;
+    x = -(lane == 8 ? pa : pb).alpha * R;
+  } else if (lane < 14) {
+    use = theory == NDDO_PM3PDDG;
+    const double d = R - pa.pddg_da[(lane - 10) >> 1] - pb.pddg_da[(lane - 10) & 1];
+    x = -10.0 / (NDDO_ANG2AU * NDDO_ANG2AU) * (d * d);
+  }
+  const double e = use ? exp(x) : 0.0;
+  auto at = [&](int l) { return __shfl_sync(0xffffffffu, e, l); };
+  const double ea = at(8), eb = at(9);
+  const bool a_no = (pa.atomic_number == 7 || pa.atomic_number == 8);
+  const bool b_no = (pb.atomic_number == 7 || pb.atomic_number == 8);
+  double f;
+  if (pa.atomic_number == 1 && b_no) f = 1.0 + (R / NDDO_ANG2AU) * eb + ea;
+  else if (pb.atomic_number == 1 && a_no) f = 1.0 + (R / NDDO_ANG2AU) * ea + eb;
+  else f = 1.0 + ea + eb;
+  double s = (double)(pa.core_charge * pb.core_charge) * ssss * f;
+  if (theory != NDDO_MNDO) {
+    double t = 0.0;
+    for (int i = 0; i < 4; ++i) {
+      const double ga = at(i), gb = at(4 + i);
+      if (pa.gk[i] != 0.0) t += pa.gk[i] * ga;
+      if (pb.gk[i] != 0.0) t += pb.gk[i] * gb;
+    }
+    s += (double)(pa.core_charge * pb.core_charge) * t * NDDO_ANG2AU / R;
+  }
+  if (theory == NDDO_PM3PDDG) {
+    const double na = pa.core_charge, nb = pb.core_charge;
+    double t = 0.0;
+    for (int i = 0; i < 2; ++i)
+      for (int k = 0; k < 2; ++k) t += (na * pa.pddg_pa[i] + nb * pb.pddg_pa[k]) * at(10 + 2 * i + k);
+    s += t / (na + nb);
+  }
+  return s;
+}
+
 // One overlap combination of the pair in the diatomic frame (thread-level):
 // norm * ang * (R/2)^(na+nb+1) * sum_t c_t A_i(p) B_j(q).
 template <typename T>
@@ -142,9 +192,10 @@ pair_light_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__
                   double* __restrict__ blocks, double* __restrict__ H, double* __restrict__ ecore_pair) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  const int p = list[t];
+  const long long p = list ? list[t] : t;
   const DevPair pr = pairs[p];
   const DevAtom A = atoms[pr.a], B = atoms[pr.b];
+  if (A.nao == 4 && B.nao == 4) return;   // no list: pair_kernel's
   const bool swap = (A.nao == 1 && B.nao == 4);
   const DevAtom X = swap ? B : A, Y = swap ? A : B;       // Y is a hydrogen
   const nddo_atom_params& px = c_params[X.pidx];
@@ -201,6 +252,7 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   __shared__ double s_ab[kPairWarps][4][24];
   __shared__ double s_ov[kPairWarps][8];
   __shared__ double s_R[kPairWarps][16];
+  __shared__ double s_term[kPairWarps][kMaxFlatTerms];
   const unsigned full = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long pi = (long long)blockIdx.x * kPairWarps + warp;
@@ -209,6 +261,7 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
 
   const DevPair pr = pairs[p];
   const DevAtom A = atoms[pr.a], B = atoms[pr.b];
+  if (!list && (A.nao == 1 || B.nao == 1)) return;   // no list: pair_light_kernel's
   const DevMol mol = mols[pr.mol];
   const nddo_atom_params& pa = c_params[A.pidx];
   const nddo_atom_params& pb = c_params[B.pidx];
@@ -224,33 +277,39 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
     for (int i = 0; i < 16; ++i) s_R[warp][i] = Rm[i >> 2][i & 3];
   }
 
-  // ---- local two-centre integrals: lane = slot ----------------------------
+  // ---- local two-centre integrals: lane = point-charge term, then lane = slot.
+  // A warp instruction takes the FP64 pipe 64 clocks however few lanes it has:
+  // by slot, 21 lanes walked up to 24 terms each.
+  const bool heavy = nA == 4 && nB == 4;
+  const int nterm = heavy ? eri->flat_heavy : eri->flat_light;
+  for (int t = lane; t < nterm; t += 32) {
+    const EriTerm e = eri->flat[t];
+    const double da = sel3(e.la, pa.d[0], pa.d[1], pa.d[2]);
+    const double db = sel3(e.lb, pb.d[0], pb.d[1], pb.d[2]);
+    const double ra = sel3(e.la, pa.rho[0], pa.rho[1], pa.rho[2]);
+    const double rb = sel3(e.lb, pb.rho[0], pb.rho[1], pb.rho[2]);
+    const double l = R + (double)e.c1 * da + (double)e.c2 * db;
+    const double u = (double)e.c3 * da + (double)e.c4 * db;
+    const double v = (double)e.c5 * da + (double)e.c6 * db;
+    const double a = ra + rb;
+    const double arg = l * l + u * u + v * v + a * a;
+    s_term[warp][t] = e.coef * rsqrt(arg);
+  }
+  __syncwarp();
   double val = 0.0;
   if (lane < 21) {
     bool need;
-    if (nA == 4 && nB == 4) need = true;
+    if (heavy) need = true;
     else if (nA == 4) need = (lane == 0 || lane == 3 || lane == 4 || lane == 10);
     else if (nB == 4) need = (lane == 0 || lane == 1 || lane == 2 || lane == 13);
     else need = (lane == 0);
     if (need) {
-      const int nt = eri->nterms[lane];
-      for (int t = 0; t < nt; ++t) {
-        const EriTerm e = eri->terms[lane][t];
-        const double da = sel3(e.la, pa.d[0], pa.d[1], pa.d[2]);
-        const double db = sel3(e.lb, pb.d[0], pb.d[1], pb.d[2]);
-        const double ra = sel3(e.la, pa.rho[0], pa.rho[1], pa.rho[2]);
-        const double rb = sel3(e.lb, pb.rho[0], pb.rho[1], pb.rho[2]);
-        const double l = R + (double)e.c1 * da + (double)e.c2 * db;
-        const double u = (double)e.c3 * da + (double)e.c4 * db;
-        const double v = (double)e.c5 * da + (double)e.c6 * db;
-        const double a = ra + rb;
-        const double arg = l * l + u * u + v * v + a * a;
-        val += e.coef * rsqrt(arg);
-      }
+      const int first = eri->flat_first[lane], nt = eri->nterms[lane];
+      for (int t = 0; t < nt; ++t) val += s_term[warp][first + t];
     }
   }
   const double s5 = __shfl_sync(full, val, 5), s6 = __shfl_sync(full, val, 6);
-  if (lane == 21) val = (nA == 4 && nB == 4) ? 0.5 * (s5 - s6) : 0.0;
+  if (lane == 21) val = heavy ? 0.5 * (s5 - s6) : 0.0;
   if (lane < 22) s_val[warp][lane] = val;
 
   // ---- overlap auxiliary integrals: lane zc computes A_0..11 of zeta combination
@@ -351,7 +410,8 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   }
 
   // ---- core-core repulsion --------------------------------------------------
-  if (lane == 0) ecore_pair[p] = core_core(pa, pb, R, s_val[warp][0], mol.theory);
+  const double ec = core_core_warp(pa, pb, R, s_val[warp][0], mol.theory, lane);
+  if (lane == 0) ecore_pair[p] = ec;
 }
 
 // warp-wide sum with a fixed tree (bitwise reproducible)
@@ -390,26 +450,35 @@ __device__ __forceinline__ double epc_slot_value(const EriTable* __restrict__ er
 }
 
 // One-centre block of H (U on the diagonal plus the attraction of every other
-// core, -Z_B (mu nu|s_B s_B)) and the molecule's core-core energy.  With
+// core, -Z_B (mu nu|s_B s_B)).  With
 // environmental point charges each adds -q (mu nu|s s) to the block (MolDS
 // Mndo::GetFockDiagElement / GetFockOffDiagElement, src/mndo/Mndo.cpp:474-484,
 // 546-556, present in every non-guess Fock matrix and so in H = F(P = 0) of
 // the energy, src/cndo/Cndo2.cpp:1324-1416), the block rotated from the local
-// values exactly as a pair with a hydrogen (pair_light_kernel), and the
+// values exactly as a pair with a hydrogen (pair_light_kernel); the
 // cores' energy in their field, sum Z_A q / R (Mndo.cpp:329-331,
-// Cndo2.cpp:418-426), goes to ecore_epc.
+// Cndo2.cpp:418-426), is ecore_kernel's.  CTAs over the atoms of every molecule
+// (one CTA per molecule, its pair energies summed by one warp, took 1.7 ms for
+// (H2O)180).
 __global__ void __launch_bounds__(kFockThreads)
 hcore_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, const DevMol* __restrict__ mols,
              const int* __restrict__ mol_list, const double* __restrict__ blocks,
-             const double* __restrict__ ecore_pair, const EriTable* __restrict__ eri,
-             const double* __restrict__ epc, double* __restrict__ H, MolState* __restrict__ st) {
-  __shared__ double s_epc[kFockThreads / 32];
-  const int m = mol_list[blockIdx.x];
+             double* __restrict__ ecore_pair, const EriTable* __restrict__ eri,
+             const double* __restrict__ epc, double* __restrict__ H) {
+  const int m = mol_list[blockIdx.y];
   const DevMol mol = mols[m];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const long long ld = mol.nao;
-  double e_epc = 0.0;   // this lane's share of sum Z_A q / R
-  for (int ia = warp; ia < mol.natoms; ia += nwarps) {
+  // a warp per atom
+  for (int ia = blockIdx.x * nwarps + warp; ia < mol.natoms; ia += gridDim.x * nwarps) {
+    // the row's core-core energies, sum over B > A, in the place of its first one
+    if (ia + 1 < mol.natoms) {
+      double* row = ecore_pair + mol.pair0 + pair_index(ia, ia + 1, mol.natoms);
+      double e = 0.0;
+      for (int k = lane; k < mol.natoms - 1 - ia; k += 32) e += row[k];
+      e = warp_sum(e);
+      if (lane == 0) row[0] = e;
+    }
     const DevAtom A = atoms[mol.atom0 + ia];
     const int dA = A.nao == 4 ? 10 : 1;
     double acc[10];
@@ -433,7 +502,6 @@ hcore_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pair
         const double dx = pc[0] - A.x, dy = pc[1] - A.y, dz = pc[2] - A.z, q = pc[3];
         const double R = sqrt(dx * dx + dy * dy + dz * dz);
         const double iR = 1.0 / R;
-        e_epc += pa.core_charge * q / R;
         acc[0] -= q * epc_slot_value(eri, 0, R, pa);
         if (dA == 10) {
           const double s3 = epc_slot_value(eri, 3, R, pa);
@@ -464,19 +532,34 @@ hcore_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pair
       H[mol.mat0 + c * ld + r] = v;
     }
   }
-  e_epc = warp_sum(e_epc);
-  if (lane == 0) s_epc[warp] = e_epc;
+}
+
+// The molecule's core-core energy from its rows' sums, and the cores' energy
+// in the field of the point charges
+__global__ void __launch_bounds__(kFockThreads)
+ecore_kernel(const DevAtom* __restrict__ atoms, const DevMol* __restrict__ mols, const int* __restrict__ mol_list,
+             const double* __restrict__ ecore_pair, const double* __restrict__ epc, MolState* __restrict__ st) {
+  __shared__ double red[2][kFockThreads / 32];
+  const int m = mol_list[blockIdx.x];
+  const DevMol mol = mols[m];
+  const int tid = threadIdx.x;
+  double e = 0.0, q = 0.0;
+  for (int ia = tid; ia + 1 < mol.natoms; ia += kFockThreads)
+    e += ecore_pair[mol.pair0 + pair_index(ia, ia + 1, mol.natoms)];
+  for (long long t = tid; t < (long long)mol.natoms * mol.nepc; t += kFockThreads) {
+    const DevAtom& A = atoms[mol.atom0 + t / mol.nepc];
+    const double* pc = epc + 4 * (mol.epc0 + t % mol.nepc);
+    const double dx = pc[0] - A.x, dy = pc[1] - A.y, dz = pc[2] - A.z;
+    q += c_params[A.pidx].core_charge * pc[3] / sqrt(dx * dx + dy * dy + dz * dz);
+  }
+  e = warp_sum(e);
+  q = warp_sum(q);
+  if ((tid & 31) == 0) { red[0][tid >> 5] = e; red[1][tid >> 5] = q; }
   __syncthreads();
-  if (warp == 0) {
-    double s = 0.0;
-    for (int k = lane; k < mol.npairs; k += 32) s += ecore_pair[mol.pair0 + k];
-    s = warp_sum(s);
-    if (lane == 0) {
-      st[m].ecore = s;
-      double e = 0.0;
-      for (int w = 0; w < nwarps; ++w) e += s_epc[w];
-      st[m].ecore_epc = e;
-    }
+  if (tid < 2) {
+    double v = 0.0;
+    for (int w = 0; w < kFockThreads / 32; ++w) v += red[tid][w];
+    if (tid == 0) st[m].ecore = v; else st[m].ecore_epc = v;
   }
 }
 
@@ -491,135 +574,184 @@ __device__ __forceinline__ double h_one(const nddo_atom_params& p, int m, int n)
   return p.hpp;
 }
 
-// F = H + G(P) (mode 0), the MolDS guess Fock (mode 1: U on the diagonal,
-// zero one-centre off-diagonal, resonance blocks between atoms), or H itself
-// (mode 2).  P_old <- P is copied on the way when copy_old is set.
-__global__ void __launch_bounds__(kFockThreads)
+// packed index of an orbital pair of one atom as a nibble table: pack_index(m, n)
+__device__ __forceinline__ int pack_lut(int m, int n) {
+  constexpr unsigned long long kTable = 0x9863875265413210ULL;   // [4 m + n]
+  return (int)(kTable >> (16 * m + 4 * n)) & 15;
+}
+
+constexpr int kFockAtomThreads = 128;
+constexpr int kFockStage = 256;   // atoms whose densities are staged at a time (20 KB)
+
+// F = H + G(P) (mode 0) or the MolDS guess Fock (mode 1: U on the diagonal,
+// zero one-centre off-diagonal, resonance blocks between atoms).  P_old <- P
+// is copied on the way when copy_old is set.
+// One CTA per atom A.  Coulomb: a thread per (B, orbital pair of A), its dot
+// product over B's orbital pairs against B's one-centre densities, staged packed
+// in shared memory; the threads of one orbital pair are summed in a fixed order.
+// Exchange with B > A: a thread per element of the A-B block.
+// What bounds it: latency and the number of loads in flight (the blocks of one
+// molecule are L2-resident).  A warp per atom, with a lane walking whole 10 x 10
+// blocks, left a single molecule on natoms / 8 CTAs.
+__global__ void __launch_bounds__(kFockAtomThreads)
 fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, const DevMol* __restrict__ mols,
             const int* __restrict__ mol_list, const double* __restrict__ blocks, const double* __restrict__ H,
             const double* __restrict__ P, double* __restrict__ F, double* __restrict__ Pold,
             const MolState* __restrict__ st, int mode_override, int copy_old, int require_active) {
-  // grid: x = groups of atom rows (a warp per atom row), y = molecule
-  const int m = mol_list[blockIdx.y];
+  __shared__ double s_p[kFockStage * 10];
+  __shared__ double s_red[kFockAtomThreads];
+  __shared__ short s_list[kFockStage];
+  __shared__ int s_n[4];
+  const int m = mol_list[blockIdx.y], ia = blockIdx.x;
   const DevMol mol = mols[m];
-  const MolState s = st[m];
-  if (require_active && s.status != kActive) return;
+  if (ia >= mol.natoms) return;
+  const int status = st[m].status;
+  if (require_active && status != kActive) return;
   int mode = mode_override;
-  if (mode < 0) mode = (s.iter == 0 && s.requires_guess) ? 1 : 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  if (mode < 0) mode = (st[m].iter == 0 && st[m].requires_guess) ? 1 : 0;
+  const int tid = threadIdx.x;
   const long long ld = mol.nao;
   const double* Pm = P + mol.mat0;
   const double* Hm = H + mol.mat0;
   double* Fm = F + mol.mat0;
-  const long long n2 = ld * ld;
-  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, tstep = (long long)gridDim.x * blockDim.x;
+  const DevAtom* am = atoms + mol.atom0;
+  const DevAtom A = am[ia];
+  const nddo_atom_params& pa = c_params[A.pidx];
+  const int nA = A.nao, dA = nA == 4 ? 10 : 1, fa = A.ao0;
   if (copy_old) {
-    double* Po = Pold + mol.mat0;
-    for (long long i = t0; i < n2; i += tstep) Po[i] = Pm[i];
+    const double* from = Pm + fa * ld;
+    double* to = Pold + mol.mat0 + fa * ld;
+    for (long long i = tid; i < nA * ld; i += kFockAtomThreads) to[i] = from[i];
   }
-  if (mode == 2) {
-    for (long long i = t0; i < n2; i += tstep) Fm[i] = Hm[i];
-    return;
-  }
-  for (int ia = blockIdx.x * nwarps + warp; ia < mol.natoms; ia += gridDim.x * nwarps) {
-    const DevAtom A = atoms[mol.atom0 + ia];
-    const nddo_atom_params& pa = c_params[A.pidx];
-    const int nA = A.nao, dA = nA == 4 ? 10 : 1;
-    const int fa = A.ao0;
-    double acc[10];
-#pragma unroll
-    for (int k = 0; k < 10; ++k) acc[k] = 0.0;
-    if (mode == 0) {
-      // Coulomb: sum_B sum_{la si in B} P_la,si (mu nu|la si)
-      for (int ib = lane; ib < mol.natoms; ib += 32) {
+  // threads k + dA j share orbital pair k
+  const int per = kFockAtomThreads / dA, k = tid % dA, j0 = tid / dA;
+  double acc = 0.0;
+  for (int b0 = 0; b0 < mol.natoms; b0 += kFockStage) {
+    const int nb = min(kFockStage, mol.natoms - b0);
+    __syncthreads();
+    // heavy atoms first in the list, hydrogens from its end: a warp then works
+    // on one kind, and the FP64 pipe, which takes 64 clocks a warp instruction,
+    // is not spent on lanes that sit out
+    if (tid < 32) {
+      int h = 0, l = 0, h0 = 0, l0 = 0;
+      for (int base = 0; base < nb; base += 32) {
+        const int i = base + tid;
+        const bool in = i < nb, heavy = in && am[b0 + i].nao == 4;
+        const unsigned mh = __ballot_sync(0xffffffffu, heavy), ml = __ballot_sync(0xffffffffu, in && !heavy);
+        const unsigned below = (1u << tid) - 1u;
+        if (heavy) s_list[h + __popc(mh & below)] = (short)i;
+        else if (in) s_list[kFockStage - 1 - (l + __popc(ml & below))] = (short)i;
+        const unsigned upto = __ballot_sync(0xffffffffu, in && b0 + i <= ia);
+        h0 += __popc(mh & upto);
+        l0 += __popc(ml & upto);
+        h += __popc(mh);
+        l += __popc(ml);
+      }
+      if (tid == 0) { s_n[0] = h; s_n[1] = l; s_n[2] = h0; s_n[3] = l0; }   // counts, those up to atom A
+    }
+    if (mode == 0)
+      for (int e = tid; e < nb * 10; e += kFockAtomThreads) {
+        const DevAtom& B = am[b0 + e / 10];
+        int l, sg;
+        unpack_index(e % 10, &l, &sg);
+        double v = 0.0;
+        if (B.nao == 4 || e % 10 == 0) v = Pm[(B.ao0 + l) * ld + B.ao0 + sg] * (l == sg ? 1.0 : 2.0);
+        s_p[e] = v;
+      }
+    __syncthreads();
+    const int nh = s_n[0], nl = s_n[1], h0 = s_n[2], l0 = s_n[3];
+    if (mode == 0 && j0 < per) {
+      for (int t = j0; t < nh; t += per) {
+        const int i = s_list[t], ib = b0 + i;
         if (ib == ia) continue;
-        const DevAtom Bt = atoms[mol.atom0 + ib];
-        const int nB = Bt.nao, dB = nB == 4 ? 10 : 1, fb = Bt.ao0;
-        double pB[10];
-#pragma unroll
-        for (int q = 0; q < 10; ++q) {
-          pB[q] = 0.0;
-          if (q < dB) {
-            int l, sg;
-            unpack_index(q, &l, &sg);
-            pB[q] = Pm[(fb + l) * ld + fb + sg] * (l == sg ? 1.0 : 2.0);
-          }
-        }
         bool rows;
         const double* blk = partner_block(pairs, blocks, mol, ia, ib, &rows);
-        if (rows) {
+        const double* x = rows ? blk + k * 10 : blk + k;
+        const int step = rows ? 1 : dA;
+        double v = 0.0;
 #pragma unroll
-          for (int k = 0; k < 10; ++k) {
-            if (k >= dA) break;
-            double t = 0.0;
-#pragma unroll
-            for (int q = 0; q < 10; ++q) if (q < dB) t += blk[k * dB + q] * pB[q];
-            acc[k] += t;
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 10; ++k) {
-            if (k >= dA) break;
-            double t = 0.0;
-#pragma unroll
-            for (int q = 0; q < 10; ++q) if (q < dB) t += blk[q * dA + k] * pB[q];
-            acc[k] += t;
-          }
-        }
+        for (int q = 0; q < 10; ++q) v += x[q * step] * s_p[i * 10 + q];
+        acc += v;
       }
-#pragma unroll
-      for (int k = 0; k < 10; ++k) acc[k] = warp_sum(acc[k]);
-    }
-    // one-centre block
-    if (lane < dA) {
-      int mu, nu;
-      unpack_index(lane, &mu, &nu);
-      double v;
-      if (mode == 1) {
-        v = (mu == nu) ? pa.u[mu == 0 ? 0 : 1] : 0.0;
-      } else {
-        double j = 0.0;
-#pragma unroll
-        for (int k = 0; k < 10; ++k) if (k == lane) j = acc[k];
-        v = Hm[(fa + mu) * ld + fa + nu];
-        if (mu == nu) {
-          double t = 0.0;
-          for (int n = 0; n < nA; ++n) t += Pm[(fa + n) * ld + fa + n] * (g_one(pa, mu, n) - 0.5 * h_one(pa, mu, n));
-          v += t;
-        } else {
-          v += (1.5 * h_one(pa, mu, nu) - 0.5 * g_one(pa, mu, nu)) * Pm[(fa + mu) * ld + fa + nu];
-        }
-        v += j;
+      for (int t = j0; t < nl; t += per) {
+        const int i = s_list[kFockStage - 1 - t], ib = b0 + i;
+        if (ib == ia) continue;
+        bool rows;
+        acc += partner_block(pairs, blocks, mol, ia, ib, &rows)[k] * s_p[i * 10];
       }
-      Fm[(fa + mu) * ld + fa + nu] = v;
-      Fm[(fa + nu) * ld + fa + mu] = v;
     }
-    // two-centre blocks (A, B > A): resonance + exchange -1/2 sum P_nu,si (mu nu|la si)
-    for (int ib = ia + 1 + lane; ib < mol.natoms; ib += 32) {
-      const DevAtom Bt = atoms[mol.atom0 + ib];
-      const int nB = Bt.nao, dB = nB == 4 ? 10 : 1, fb = Bt.ao0;
-      const double* blk = blocks + pairs[mol.pair0 + pair_index(ia, ib, mol.natoms)].blk;
-      double pab[4][4];
+    // two-centre blocks (A, B > A): resonance + exchange -1/2 sum P_nu,si (mu nu|la si);
+    // a thread per (B, mu, la)
+    const int sh = nA == 4 ? 4 : 2;
+    for (int t = h0 + (tid >> sh); t < nh; t += kFockAtomThreads >> sh) {
+      const int ib = b0 + s_list[t], fb = am[ib].ao0, mu = (tid >> 2) & (nA - 1), la = tid & 3;
+      double v = Hm[(fa + mu) * ld + fb + la];
       if (mode == 0) {
-        for (int n = 0; n < nA; ++n)
-          for (int sg = 0; sg < nB; ++sg) pab[n][sg] = Pm[(fa + n) * ld + fb + sg];
-      }
-      for (int mu = 0; mu < nA; ++mu)
-        for (int la = 0; la < nB; ++la) {
-          double v = Hm[(fa + mu) * ld + fb + la];
-          if (mode == 0) {
-            double k = 0.0;
-            for (int n = 0; n < nA; ++n)
-              for (int sg = 0; sg < nB; ++sg) k += pab[n][sg] * blk[pack_index(mu, n) * dB + pack_index(la, sg)];
-            v -= 0.5 * k;
+        const double* blk = blocks + pairs[mol.pair0 + pair_index(ia, ib, mol.natoms)].blk;
+        const double* Pab = Pm + fa * ld + fb;
+        double x = 0.0;
+        if (nA == 4) {
+#pragma unroll
+          for (int n = 0; n < 4; ++n) {
+            const double* row = blk + pack_lut(mu, n) * 10;
+#pragma unroll
+            for (int sg = 0; sg < 4; ++sg) x += Pab[n * ld + sg] * row[pack_lut(la, sg)];
           }
-          Fm[(fa + mu) * ld + fb + la] = v;
-          Fm[(fb + la) * ld + fa + mu] = v;
+        } else {
+#pragma unroll
+          for (int sg = 0; sg < 4; ++sg) x += Pab[sg] * blk[pack_lut(la, sg)];
         }
+        v -= 0.5 * x;
+      }
+      Fm[(fa + mu) * ld + fb + la] = v;
+      Fm[(fb + la) * ld + fa + mu] = v;
     }
+    const int sl = nA == 4 ? 2 : 0;
+    for (int t = l0 + (tid >> sl); t < nl; t += kFockAtomThreads >> sl) {
+      const int ib = b0 + s_list[kFockStage - 1 - t], fb = am[ib].ao0, mu = tid & (nA - 1);
+      double v = Hm[(fa + mu) * ld + fb];
+      if (mode == 0) {
+        const double* blk = blocks + pairs[mol.pair0 + pair_index(ia, ib, mol.natoms)].blk;
+        const double* Pab = Pm + fa * ld + fb;
+        double x = 0.0;
+        for (int n = 0; n < nA; ++n) x += Pab[n * ld] * blk[pack_lut(mu, n)];
+        v -= 0.5 * x;
+      }
+      Fm[(fa + mu) * ld + fb] = v;
+      Fm[fb * ld + fa + mu] = v;
+    }
+  }
+  if (mode == 0) {
+    s_red[tid] = j0 < per ? acc : 0.0;
+    __syncthreads();
+  }
+  // one-centre block
+  if (tid < dA) {
+    int mu, nu;
+    unpack_index(tid, &mu, &nu);
+    double v;
+    if (mode == 1) {
+      v = (mu == nu) ? pa.u[mu == 0 ? 0 : 1] : 0.0;
+    } else {
+      double j = 0.0;
+      for (int i = 0; i < per; ++i) j += s_red[i * dA + tid];
+      v = Hm[(fa + mu) * ld + fa + nu];
+      if (mu == nu) {
+        double t = 0.0;
+        for (int n = 0; n < nA; ++n) t += Pm[(fa + n) * ld + fa + n] * (g_one(pa, mu, n) - 0.5 * h_one(pa, mu, n));
+        v += t;
+      } else {
+        v += (1.5 * h_one(pa, mu, nu) - 0.5 * g_one(pa, mu, nu)) * Pm[(fa + mu) * ld + fa + nu];
+      }
+      v += j;
+    }
+    Fm[(fa + mu) * ld + fa + nu] = v;
+    Fm[(fa + nu) * ld + fa + mu] = v;
   }
 }
 
+// All pairs without index lists (each kernel skips the other's): a warp per
+// pair with a hydrogen as well took 1.9 of 3.1 ms for 450 atoms.
 void launch_pair_kernel(const DevAtom* atoms, const DevPair* pairs, long long npairs, const DevMol* mols,
                         const EriTable* eri, const OverlapTable* ovt, double* blocks, double* H,
                         double* ecore_pair, cudaStream_t s) {
@@ -627,6 +759,8 @@ void launch_pair_kernel(const DevAtom* atoms, const DevPair* pairs, long long np
   const long long grid = (npairs + kPairWarps - 1) / kPairWarps;
   pair_kernel<<<(unsigned)grid, kPairWarps * 32, 0, s>>>(atoms, pairs, nullptr, npairs, mols, eri, ovt, blocks, H,
                                                          ecore_pair);
+  pair_light_kernel<<<(unsigned)((npairs + 127) / 128), 128, 0, s>>>(atoms, pairs, nullptr, npairs, mols, eri, ovt,
+                                                                     blocks, H, ecore_pair);
 }
 
 void launch_pair_kernels_split(const DevAtom* atoms, const DevPair* pairs, const int* heavy_list, long long n_heavy,
@@ -646,10 +780,13 @@ void launch_pair_kernels_split(const DevAtom* atoms, const DevPair* pairs, const
 }
 
 void launch_hcore_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
-                         int nlist, const double* blocks, const double* ecore_pair, const EriTable* eri,
+                         int nlist, int max_atoms, const double* blocks, double* ecore_pair, const EriTable* eri,
                          const double* epc, double* H, MolState* st, cudaStream_t s) {
   if (nlist <= 0) return;
-  hcore_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, pairs, mols, mol_list, blocks, ecore_pair, eri, epc, H, st);
+  constexpr int kWarps = kFockThreads / 32;
+  hcore_kernel<<<dim3((max_atoms + kWarps - 1) / kWarps, nlist), kFockThreads, 0, s>>>(
+      atoms, pairs, mols, mol_list, blocks, ecore_pair, eri, epc, H);
+  ecore_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, mols, mol_list, ecore_pair, epc, st);
 }
 
 void launch_fock_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
@@ -657,10 +794,8 @@ void launch_fock_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol
                         double* Pold, const MolState* st, int mode_override, int copy_old, int require_active,
                         cudaStream_t s) {
   if (nlist <= 0) return;
-  const int rows = kFockThreads / 32;
-  dim3 grid((max_atoms + rows - 1) / rows, nlist);
-  fock_kernel<<<grid, kFockThreads, 0, s>>>(atoms, pairs, mols, mol_list, blocks, H, P, F, Pold, st, mode_override,
-                                            copy_old, require_active);
+  fock_kernel<<<dim3(max_atoms, nlist), kFockAtomThreads, 0, s>>>(atoms, pairs, mols, mol_list, blocks, H, P, F, Pold,
+                                                                  st, mode_override, copy_old, require_active);
 }
 
 // E = 1/2 sum P (F + H) + E_core + E_vdW (Cndo2::CalcElecSCFEnergy, src/cndo/Cndo2.cpp:1324-1416),
@@ -669,24 +804,34 @@ void launch_fock_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol
 // E_vdW: the empirical dispersion energy of Cndo2::CalcVdWCorrectionEnergy
 // (Cndo2.cpp:464-513), on when requested or for AM1-D / PM3-D (which fix
 // s6 = 1.40, d = 23).
+// Partial sums over fixed chunks of each molecule's matrix (their number depends
+// on N alone), then one CTA per molecule: a single CTA walking N^2 took 1.26 ms
+// for (H2O)180.
+__host__ __device__ __forceinline__ int energy_chunks(long long n2) {
+  const long long c = (n2 + 2047) / 2048;
+  return (int)(c < 1 ? 1 : (c > kDipChunks ? kDipChunks : c));
+}
+
 __global__ void __launch_bounds__(kFockThreads)
-energy_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, const DevMol* __restrict__ mols,
-              const int* __restrict__ mol_list, const double* __restrict__ P, const double* __restrict__ F,
-              const double* __restrict__ H, MolState* __restrict__ st, double* __restrict__ charges, VdwParams vdw) {
-  __shared__ double red[32], red_v[32];
-  const int m = mol_list[blockIdx.x];
-  const DevMol mol = mols[m];
+energy_partial_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs,
+                      const DevMol* __restrict__ mols, const int* __restrict__ mol_list, const double* __restrict__ P,
+                      const double* __restrict__ F, const double* __restrict__ H, double* __restrict__ partial,
+                      VdwParams vdw) {
+  __shared__ double red[2][kFockThreads / 32];
+  const DevMol mol = mols[mol_list[blockIdx.y]];
   const long long n2 = (long long)mol.nao * mol.nao;
+  const int chunks = energy_chunks(n2);
+  if ((int)blockIdx.x >= chunks) return;
+  const long long step = (long long)chunks * kFockThreads, first = (long long)blockIdx.x * kFockThreads + threadIdx.x;
   double acc = 0.0;
-  for (long long i = threadIdx.x; i < n2; i += blockDim.x)
-    acc += P[mol.mat0 + i] * (F[mol.mat0 + i] + H[mol.mat0 + i]);
+  for (long long i = first; i < n2; i += step) acc += P[mol.mat0 + i] * (F[mol.mat0 + i] + H[mol.mat0 + i]);
   acc = warp_sum(acc);
   const bool dtheory = mol.theory == NDDO_AM1D || mol.theory == NDDO_PM3D;
   const bool vdw_on = vdw.on || dtheory;
   const double s6 = dtheory ? NDDO_VDW_S6_D : vdw.s6, dd = dtheory ? NDDO_VDW_DAMP_D : vdw.d;
   double ev = 0.0;
   if (vdw_on)
-    for (int t = threadIdx.x; t < mol.npairs; t += blockDim.x) {
+    for (long long t = first; t < mol.npairs; t += step) {
       const DevPair pr = pairs[mol.pair0 + t];
       const DevAtom A = atoms[pr.a], B = atoms[pr.b];
       const nddo_atom_params& pa = c_params[A.pidx];
@@ -700,37 +845,60 @@ energy_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pai
       ev += -1.0 * s6 * c6 * damp / (R * R * R * R * R * R);
     }
   ev = warp_sum(ev);
-  if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = acc; red_v[threadIdx.x >> 5] = ev; }
+  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = acc; red[1][threadIdx.x >> 5] = ev; }
   __syncthreads();
-  for (int a = threadIdx.x; a < mol.natoms; a += blockDim.x) {
+  if (threadIdx.x < 2) {
+    double v = 0.0;
+    for (int w = 0; w < kFockThreads / 32; ++w) v += red[threadIdx.x][w];
+    partial[((long long)blockIdx.y * kDipChunks + blockIdx.x) * 2 + threadIdx.x] = v;
+  }
+}
+
+__global__ void __launch_bounds__(kFockThreads)
+energy_kernel(const DevAtom* __restrict__ atoms, const DevMol* __restrict__ mols, const int* __restrict__ mol_list,
+              const double* __restrict__ P, const double* __restrict__ partial, MolState* __restrict__ st,
+              double* __restrict__ charges) {
+  __shared__ double red[3][kFockThreads / 32];
+  const int m = mol_list[blockIdx.x], tid = threadIdx.x;
+  const DevMol mol = mols[m];
+  const int chunks = energy_chunks((long long)mol.nao * mol.nao);
+  double e = 0.0, v = 0.0, f = 0.0;
+  for (int c = tid; c < chunks; c += kFockThreads) {
+    e += partial[((long long)blockIdx.x * kDipChunks + c) * 2];
+    v += partial[((long long)blockIdx.x * kDipChunks + c) * 2 + 1];
+  }
+  for (int a = tid; a < mol.natoms; a += kFockThreads) {
     const DevAtom A = atoms[mol.atom0 + a];
+    const nddo_atom_params& pa = c_params[A.pidx];
     double pop = 0.0;
     for (int k = 0; k < A.nao; ++k) pop += P[mol.mat0 + (long long)(A.ao0 + k) * mol.nao + A.ao0 + k];
-    charges[mol.atom0 + a] = c_params[A.pidx].core_charge - pop;
+    charges[mol.atom0 + a] = pa.core_charge - pop;
+    f += pa.dhf_atom - pa.e_atom;
   }
-  if (threadIdx.x == 0) {
-    double e = 0.0, v = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { e += red[w]; v += red_v[w]; }
+  e = warp_sum(e);
+  v = warp_sum(v);
+  f = warp_sum(f);
+  if ((tid & 31) == 0) { red[0][tid >> 5] = e; red[1][tid >> 5] = v; red[2][tid >> 5] = f; }
+  __syncthreads();
+  if (tid == 0) {
+    e = v = f = 0.0;
+    for (int w = 0; w < kFockThreads / 32; ++w) { e += red[0][w]; v += red[1][w]; f += red[2][w]; }
     e *= 0.5;
     MolState* s = st + m;
     s->energy_electronic = e;
     s->vdw_energy = v;
     s->energy = e + s->ecore + s->ecore_epc + v;
-    double hof = s->energy;
-    for (int a = 0; a < mol.natoms; ++a) {
-      const nddo_atom_params& pa = c_params[atoms[mol.atom0 + a].pidx];
-      hof -= pa.e_atom;
-      hof += pa.dhf_atom;
-    }
-    s->heat_of_formation = hof;
+    s->heat_of_formation = s->energy + f;
   }
 }
 
 void launch_energy_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
-                          int nlist, const double* P, const double* F, const double* H, MolState* st,
-                          double* charges, VdwParams vdw, cudaStream_t s) {
+                          int nlist, int max_n, const double* P, const double* F, const double* H, double* partial,
+                          MolState* st, double* charges, VdwParams vdw, cudaStream_t s) {
   if (nlist <= 0) return;
-  energy_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, pairs, mols, mol_list, P, F, H, st, charges, vdw);
+  energy_partial_kernel<<<dim3(energy_chunks((long long)max_n * max_n), nlist), kFockThreads, 0, s>>>(
+      atoms, pairs, mols, mol_list, P, F, H, partial, vdw);
+  energy_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, mols, mol_list, P, partial, st, charges);
 }
 
 // ---------------------------------------------------------------------------

@@ -9,7 +9,7 @@
 //     parameter: FP32 in the early iterations, FP64 after the switch and on the
 //     plain FP64 path.
 //
-// (e) DIIS -- partial / solve / apply kernels: RMS density change and convergence
+// (e) DIIS -- partial (with the solve) / apply kernels: RMS density change and convergence
 //     test (Cndo2::SatisfyConvergenceCriterion, src/cndo/Cndo2.cpp:1472-1517),
 //     density DIIS with MolDS's exact window/acceptance rules (Cndo2::DoDIIS,
 //     :920-1028) and damping (Cndo2::DoDamp, :1030-1061).  The DIIS history is
@@ -17,6 +17,7 @@
 //     assembled in chronological order so it is the same system.  All
 //     reductions use fixed-order trees.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include "nddo_batch.cuh"
 #include "kernels.h"
 
@@ -139,219 +140,221 @@ GEMM_LAUNCH(float, double, double, float)
 #undef GEMM_LAUNCH
 
 // ---------------------------------------------------------------------------
-// deterministic block reduction helpers (blockDim = 256)
+// One SCF bookkeeping step per molecule, after the new density P is formed, in
+// two launches.  (1) partial sums over fixed chunks of the molecule's matrix
+// (sum e^2, max |e|, the new B row) while the new history entry is written; the
+// molecule's last CTA to finish reduces the chunks in a fixed order and one warp
+// runs the convergence test, the DIIS solve, damping and the phase switch;
+// (2) the extrapolation and damping over the same chunks.  The chunking depends
+// only on N, so a molecule's result does not depend on the rest of the batch.
+// What bounds it: latency for one molecule (a launch, two passes of block
+// reductions and a 6 x 6 solve), HBM for a batch.  A CTA per 4096 elements with
+// a block reduction per sum and the solve on one thread of a launch of its own
+// took 75 us for octane in an iteration of 420.
 // ---------------------------------------------------------------------------
 constexpr int kDiisThreads = 256;
-
-__device__ __forceinline__ double block_sum(double v, double* scratch) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) scratch[w] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r += scratch[i];
-    scratch[32] = r;
-  }
-  __syncthreads();
-  r = scratch[32];
-  __syncthreads();
-  return r;
-}
-
-__device__ __forceinline__ double block_max(double v, double* scratch) {
-  for (int o = 16; o > 0; o >>= 1) { double t = __shfl_xor_sync(0xffffffffu, v, o); v = t > v ? t : v; }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) scratch[w] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r = scratch[i] > r ? scratch[i] : r;
-    scratch[32] = r;
-  }
-  __syncthreads();
-  const double r = scratch[32];
-  __syncthreads();
-  return r;
-}
-
-// One SCF bookkeeping step per molecule, after the new density P is formed,
-// in three launches so that each molecule's N^2 streams are spread over many
-// CTAs: (1) partial sums over fixed chunks of the molecule's matrix (sum e^2,
-// max |e|, the new B row) while the new history entry is written; (2) one
-// thread per molecule reduces the chunks in order and runs the convergence
-// test, the DIIS solve, damping and the phase switch; (3) the extrapolation
-// and damping over the same chunks.  The chunking depends only on N, and the
-// chunk partials are reduced in a fixed order, so a molecule's result does not
-// depend on the rest of the batch.
-constexpr int kDiisChunksMax = 64;
+constexpr int kDiisChunksMax = 128;
 constexpr int kDiisPart = 2 + kMaxDiis;     // sum e^2, max |e|, dots
 
 __device__ __forceinline__ int diis_chunks(long long n2) {
-  const long long c = (n2 + 4095) / 4096;
+  const long long c = (n2 + 2047) / 2048;
   return (int)(c < kDiisChunksMax ? (c < 1 ? 1 : c) : kDiisChunksMax);
 }
 
-struct DiisStep {          // decisions of kernel (2) read by kernel (3)
+struct DiisStep {          // decisions of kernel (1) read by kernel (2)
   double coef[kMaxDiis];
   int apply, damp, active, pad;
 };
 
-__global__ void __launch_bounds__(kDiisThreads)
-diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_list, const MolState* __restrict__ st,
-                    ScfParamsDev prm, const double* __restrict__ P, const double* __restrict__ Pold,
-                    double* __restrict__ hist_dens, double* __restrict__ hist_err, long long hist_stride,
-                    double* __restrict__ part) {
-  __shared__ double scratch[40];
-  const int li = blockIdx.y;
-  const int m = mol_list[li];
-  const MolState s = st[m];
-  if (s.status != kActive || ((s.flags & kNeedEigen) && !prm.eigen_ran)) return;
-  const DevMol mol = mols[m];
-  const long long n2 = (long long)mol.nao * mol.nao;
-  const int chunks = diis_chunks(n2);
-  if ((int)blockIdx.x >= chunks) return;
-  const long long len = (n2 + chunks - 1) / chunks;
-  const long long lo = blockIdx.x * len, hi = (lo + len < n2) ? lo + len : n2;
-  const bool is_guess = (s.iter == 0 && s.requires_guess);
-  const int M = prm.diis_m;
-  const bool do_diis = !is_guess && M > 0;
-  const int slot = do_diis ? (s.diis_count % M) : 0;
-  const int count = do_diis ? min(s.diis_count + 1, M) : 0;
-  const double* Pm = P + mol.mat0;
-  const double* Po = Pold + mol.mat0;
-  double* dslot = hist_dens + slot * hist_stride + mol.mat0;
-  double* eslot = hist_err + slot * hist_stride + mol.mat0;
-  double sq = 0.0, mx = 0.0;
-  double dots[kMaxDiis];
-#pragma unroll
-  for (int k = 0; k < kMaxDiis; ++k) dots[k] = 0.0;
-  for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    const double p = Pm[i];
-    const double e = p - Po[i];
-    sq += e * e;
-    const double ae = fabs(e);
-    mx = ae > mx ? ae : mx;
-    if (do_diis) {
-      dslot[i] = p;
-      eslot[i] = e;
-#pragma unroll
-      for (int k = 0; k < kMaxDiis; ++k)
-        if (k < count) dots[k] += (k == slot ? e : hist_err[k * hist_stride + mol.mat0 + i]) * e;
-    }
-  }
-  const double sumsq = block_sum(sq, scratch);
-  const double maxe = block_max(mx, scratch);
-  double dsum[kMaxDiis];
-#pragma unroll
-  for (int k = 0; k < kMaxDiis; ++k) dsum[k] = (k < count) ? block_sum(dots[k], scratch) : 0.0;
-  if (threadIdx.x == 0) {
-    double* o = part + ((long long)li * kDiisChunksMax + blockIdx.x) * kDiisPart;
-    o[0] = sumsq;
-    o[1] = maxe;
-    for (int k = 0; k < kMaxDiis; ++k) o[2 + k] = dsum[k];
-  }
-}
-
-__global__ void diis_solve_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_list, int nlist,
-                                  MolState* __restrict__ st, ScfParamsDev prm, const double* __restrict__ part,
-                                  DiisStep* __restrict__ steps, TraceEntry* __restrict__ trace, int trace_len) {
-  const int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= nlist) return;
-  DiisStep out;
-  for (int k = 0; k < kMaxDiis; ++k) out.coef[k] = 0.0;
-  out.apply = 0; out.damp = 0; out.active = 0; out.pad = 0;
-  const int m = mol_list[li];
-  MolState* s = st + m;
-  if (s->status != kActive || ((s->flags & kNeedEigen) && !prm.eigen_ran)) { steps[li] = out; return; }
-  s->flags &= ~kNeedEigen;
-  out.active = 1;
-  const DevMol mol = mols[m];
-  const long long n2 = (long long)mol.nao * mol.nao;
-  const int chunks = diis_chunks(n2);
+// The molecule's bookkeeping by one warp, from its summed quantities.
+// a: (kMaxDiis + 1) x (kMaxDiis + 2) doubles, f: kMaxDiis + 1, in shared memory.
+__device__ void diis_decide(MolState* s, const ScfParamsDev& prm, long long n2, const double* sum, TraceEntry* trace,
+                            int trace_len, DiisStep* step, double* a, double* f) {
+  const int lane = threadIdx.x & 31;
   const int iter = s->iter;
   const bool is_guess = (iter == 0 && s->requires_guess);
   const int M = prm.diis_m;
   const bool do_diis = !is_guess && M > 0;
   const int slot = do_diis ? (s->diis_count % M) : 0;
   const int count = do_diis ? min(s->diis_count + 1, M) : 0;
-  double sumsq = 0.0, maxe = 0.0, dsum[kMaxDiis];
-  for (int k = 0; k < kMaxDiis; ++k) dsum[k] = 0.0;
-  for (int c = 0; c < chunks; ++c) {      // fixed order
-    const double* p = part + ((long long)li * kDiisChunksMax + c) * kDiisPart;
-    sumsq += p[0];
-    maxe = p[1] > maxe ? p[1] : maxe;
-    for (int k = 0; k < kMaxDiis; ++k) dsum[k] += p[2 + k];
+  const double rms = sqrt(sum[0] / (double)n2), maxe = sum[1];
+  const bool converged = rms < prm.rms_density;
+  const bool apply = do_diis && !converged && (M <= iter) && (prm.diis_end < maxe) && (maxe < prm.diis_start) &&
+                     (count == M);
+  __syncwarp();
+  if (lane == 0) {
+    s->flags &= ~kNeedEigen;
+    if (trace && iter < trace_len) {
+      TraceEntry te;
+      te.rms = rms; te.diis_err = s->diis_err; te.diis_on = s->diis_on; te.damp_on = s->damp_on;
+      trace[iter] = te;
+    }
+    s->rms = rms;
+    step->apply = step->damp = 0;
+    step->active = converged ? 0 : 1;
+    if (converged) s->status = kConverged;
   }
-  const double rms = sqrt(sumsq / (double)n2);
-  if (trace && iter < trace_len) {
-    TraceEntry te;
-    te.rms = rms; te.diis_err = s->diis_err; te.diis_on = s->diis_on; te.damp_on = s->damp_on;
-    trace[(long long)m * trace_len + iter] = te;
-  }
-  s->rms = rms;
-  if (rms < prm.rms_density) {
-    s->status = kConverged;
-    out.active = 0;
-    steps[li] = out;
-    return;
-  }
-  if (!is_guess) {
-    if (do_diis) {
-      for (int k = 0; k < count; ++k) { s->B[k * kMaxDiis + slot] = dsum[k]; s->B[slot * kMaxDiis + k] = dsum[k]; }
+  if (lane < kMaxDiis) step->coef[lane] = 0.0;
+  if (converged) return;
+  bool solved = false;
+  if (do_diis) {
+    if (lane < count) { s->B[lane * kMaxDiis + slot] = sum[2 + lane]; s->B[slot * kMaxDiis + lane] = sum[2 + lane]; }
+    __syncwarp();
+    if (lane == 0) {
       s->diis_count += 1;
       s->diis_head = slot;
       s->diis_err = maxe;
-      const bool apply = (M <= iter) && (prm.diis_end < maxe) && (maxe < prm.diis_start) && (count == M);
-      if (apply) {
-        // chronological order: oldest ... newest
-        int chron[kMaxDiis];
-        for (int k = 0; k < M; ++k) chron[k] = (slot + 1 + k) % M;
-        double a[(kMaxDiis + 1) * (kMaxDiis + 1)], b[kMaxDiis + 1];
-        const int n = M + 1;
-        for (int i = 0; i < M; ++i)
-          for (int j = 0; j < M; ++j) a[i * n + j] = s->B[chron[i] * kMaxDiis + chron[j]];
-        for (int i = 0; i < M; ++i) { a[i * n + M] = -1.0; a[M * n + i] = -1.0; b[i] = 0.0; }
-        a[M * n + M] = 0.0;
-        b[M] = -1.0;
-        // Gaussian elimination with partial pivoting; an exactly zero pivot
-        // means a singular system, which MolDS answers by skipping the step
-        bool singular = false;
-        for (int c = 0; c < n && !singular; ++c) {
-          int piv = c;
-          for (int r = c + 1; r < n; ++r) if (fabs(a[r * n + c]) > fabs(a[piv * n + c])) piv = r;
-          if (a[piv * n + c] == 0.0) { singular = true; break; }
-          if (piv != c) {
-            for (int j = 0; j < n; ++j) { double t = a[c * n + j]; a[c * n + j] = a[piv * n + j]; a[piv * n + j] = t; }
-            double t = b[c]; b[c] = b[piv]; b[piv] = t;
-          }
-          for (int r = c + 1; r < n; ++r) {
-            const double f = a[r * n + c] / a[c * n + c];
-            for (int j = c; j < n; ++j) a[r * n + j] -= f * a[c * n + j];
-            b[r] -= f * b[c];
-          }
-        }
-        if (!singular) {
-          for (int c = n - 1; c >= 0; --c) {
-            double v = b[c];
-            for (int j = c + 1; j < n; ++j) v -= a[c * n + j] * b[j];
-            b[c] = v / a[c * n + c];
-          }
-          for (int k = 0; k < M; ++k) out.coef[k] = b[k];
-          out.apply = 1;
-        }
-      }
-      s->diis_on = out.apply;
     }
-    out.damp = (prm.damping_weight > 0.0 && prm.damping_thresh < rms) ? 1 : 0;
-    s->damp_on = out.damp;
-    if (prm.precision == 1 && s->phase == 0 && do_diis && maxe < prm.switch_error) s->phase = 1;
+    if (apply) {
+      // augmented matrix in chronological order: oldest ... newest
+      const int n = M + 1, ld = kMaxDiis + 2;
+      for (int e = lane; e < n * (n + 1); e += 32) {
+        const int i = e / (n + 1), j = e % (n + 1);
+        double v;
+        if (j == n) v = i == M ? -1.0 : 0.0;
+        else if (i < M && j < M) v = s->B[((slot + 1 + i) % M) * kMaxDiis + (slot + 1 + j) % M];
+        else v = i == M && j == M ? 0.0 : -1.0;
+        a[i * ld + j] = v;
+      }
+      __syncwarp();
+      // Gaussian elimination with partial pivoting; an exactly zero pivot
+      // means a singular system, which MolDS answers by skipping the step
+      bool singular = false;
+      for (int c = 0; c < n && !singular; ++c) {
+        int piv = c;
+        for (int r = c + 1; r < n; ++r) if (fabs(a[r * ld + c]) > fabs(a[piv * ld + c])) piv = r;
+        if (a[piv * ld + c] == 0.0) { singular = true; break; }
+        __syncwarp();
+        if (piv != c && lane <= n) {
+          const double t = a[c * ld + lane];
+          a[c * ld + lane] = a[piv * ld + lane];
+          a[piv * ld + lane] = t;
+        }
+        __syncwarp();
+        if (lane > c && lane < n) f[lane] = a[lane * ld + c] / a[c * ld + c];
+        __syncwarp();
+        const int w = n + 1 - c;
+        for (int e = lane; e < (n - 1 - c) * w; e += 32) {
+          const int r = c + 1 + e / w, j = c + e % w;
+          a[r * ld + j] -= f[r] * a[c * ld + j];
+        }
+        __syncwarp();
+      }
+      if (!singular) {
+        if (lane == 0) {
+          for (int c = n - 1; c >= 0; --c) {
+            double v = a[c * ld + n];
+            for (int j = c + 1; j < n; ++j) v -= a[c * ld + j] * f[j];
+            f[c] = v / a[c * ld + c];
+          }
+          for (int k = 0; k < M; ++k) step->coef[k] = f[k];
+          step->apply = 1;
+        }
+        solved = true;
+      }
+    }
   }
-  s->iter = iter + 1;
-  if (s->iter >= prm.max_iter) s->status = kNotConverged;
-  steps[li] = out;
+  if (lane == 0) {
+    if (!is_guess) {
+      if (do_diis) s->diis_on = solved ? 1 : 0;
+      const int damp = (prm.damping_weight > 0.0 && prm.damping_thresh < rms) ? 1 : 0;
+      step->damp = damp;
+      s->damp_on = damp;
+      if (prm.precision == 1 && s->phase == 0 && do_diis && maxe < prm.switch_error) s->phase = 1;
+    }
+    s->iter = iter + 1;
+    if (iter + 1 >= prm.max_iter) s->status = kNotConverged;
+  }
+}
+
+__global__ void __launch_bounds__(kDiisThreads)
+diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_list, MolState* __restrict__ st,
+                    ScfParamsDev prm, const double* __restrict__ P, const double* __restrict__ Pold,
+                    double* __restrict__ hist_dens, double* __restrict__ hist_err, long long hist_stride,
+                    double* __restrict__ part, DiisStep* __restrict__ steps, int* __restrict__ ticket,
+                    TraceEntry* __restrict__ trace, int trace_len) {
+  constexpr int kWarps = kDiisThreads / 32;
+  __shared__ double s_red[kWarps][kDiisPart];
+  __shared__ double s_a[(kMaxDiis + 1) * (kMaxDiis + 2)], s_f[kMaxDiis + 1], s_sum[kDiisPart];
+  __shared__ int s_last;
+  const int li = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m = mol_list[li];
+  MolState* s = st + m;
+  if (s->status != kActive || ((s->flags & kNeedEigen) && !prm.eigen_ran)) {
+    if (blockIdx.x == 0 && tid == 0) steps[li].active = 0;
+    return;
+  }
+  const DevMol mol = mols[m];
+  const long long n2 = (long long)mol.nao * mol.nao;
+  const int chunks = diis_chunks(n2);
+  if ((int)blockIdx.x >= chunks) return;
+  const long long len = (n2 + chunks - 1) / chunks;
+  const long long lo = blockIdx.x * len, hi = (lo + len < n2) ? lo + len : n2;
+  const bool is_guess = (s->iter == 0 && s->requires_guess);
+  const int M = prm.diis_m;
+  const bool do_diis = !is_guess && M > 0;
+  const int slot = do_diis ? (s->diis_count % M) : 0;
+  const int count = do_diis ? min(s->diis_count + 1, M) : 0;
+  const double* Pm = P + mol.mat0;
+  const double* Po = Pold + mol.mat0;
+  double* dslot = hist_dens + slot * hist_stride + mol.mat0;
+  double* eslot = hist_err + slot * hist_stride + mol.mat0;
+  double v[kDiisPart];
+#pragma unroll
+  for (int k = 0; k < kDiisPart; ++k) v[k] = 0.0;
+  for (long long i = lo + tid; i < hi; i += kDiisThreads) {
+    const double p = Pm[i];
+    const double e = p - Po[i];
+    v[0] += e * e;
+    v[1] = fmax(v[1], fabs(e));
+    if (do_diis) {
+      dslot[i] = p;
+      eslot[i] = e;
+#pragma unroll
+      for (int k = 0; k < kMaxDiis; ++k)
+        if (k < count) v[2 + k] += (k == slot ? e : hist_err[k * hist_stride + mol.mat0 + i]) * e;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kDiisPart; ++k) {
+    if (k < 2 + count)
+      for (int o = 16; o > 0; o >>= 1) {
+        const double t = __shfl_xor_sync(0xffffffffu, v[k], o);
+        v[k] = k == 1 ? fmax(v[k], t) : v[k] + t;
+      }
+    if (lane == 0) s_red[warp][k] = v[k];
+  }
+  __syncthreads();
+  double* out = part + (long long)li * kDiisChunksMax * kDiisPart;
+  if (tid < kDiisPart) {
+    double t = s_red[0][tid];
+    for (int w = 1; w < kWarps; ++w) t = tid == 1 ? fmax(t, s_red[w][tid]) : t + s_red[w][tid];
+    out[blockIdx.x * kDiisPart + tid] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(ticket + li, 1) == chunks - 1;
+  __syncthreads();
+  if (!s_last || warp != 0) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < kDiisPart; ++k) {
+    double t = 0.0;
+    if (k < 2 + count) {
+      for (int c = lane; c < chunks; c += 32) {
+        const double x = __ldcg(out + c * kDiisPart + k);
+        t = k == 1 ? fmax(t, x) : t + x;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(0xffffffffu, t, o);
+        t = k == 1 ? fmax(t, x) : t + x;
+      }
+    }
+    if (lane == 0) s_sum[k] = t;
+  }
+  if (lane == 0) ticket[li] = 0;
+  __syncwarp();
+  diis_decide(s, prm, n2, s_sum, trace ? trace + (long long)m * trace_len : nullptr, trace_len, steps + li, s_a, s_f);
 }
 
 __global__ void __launch_bounds__(kDiisThreads)
@@ -359,8 +362,9 @@ diis_apply_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_l
                   ScfParamsDev prm, double* __restrict__ P, const double* __restrict__ Pold,
                   const double* __restrict__ hist_dens, long long hist_stride, const DiisStep* __restrict__ steps) {
   const int li = blockIdx.y;
-  const DiisStep d = steps[li];
-  if (!d.active || (!d.apply && !d.damp)) return;
+  const DiisStep* d = steps + li;
+  const int apply = d->apply, damp = d->damp;
+  if (!d->active || (!apply && !damp)) return;
   const int m = mol_list[li];
   const DevMol mol = mols[m];
   const long long n2 = (long long)mol.nao * mol.nao;
@@ -371,39 +375,48 @@ diis_apply_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_l
   const int M = prm.diis_m;
   double* Pm = P + mol.mat0;
   const double* Po = Pold + mol.mat0;
-  // the newest entry is the one this iteration pushed (diis_head)
+  // the newest entry is the one this iteration pushed (diis_head); oldest first
+  // (MolDS sums the stored densities in slot order through Dgemv)
   const int newest = st[m].diis_head;
-  for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    double v = Pm[i];
-    if (d.apply) {
-      // P = sum_k c_k P_k in chronological order (MolDS sums the stored
-      // densities in slot order through Dgemv)
-      v = 0.0;
-      for (int k = 0; k < M; ++k) {
-        const int rs = (newest + 1 + k) % M;
-        v += d.coef[k] * hist_dens[rs * hist_stride + mol.mat0 + i];
-      }
+  double coef[kMaxDiis];
+  long long off[kMaxDiis];
+#pragma unroll
+  for (int k = 0; k < kMaxDiis; ++k)
+    if (apply && k < M) {
+      coef[k] = d->coef[k];
+      off[k] = ((newest + 1 + k) % M) * hist_stride + mol.mat0;
     }
-    if (d.damp) v = v * (1.0 - prm.damping_weight) + prm.damping_weight * Po[i];
+  for (long long i = lo + threadIdx.x; i < hi; i += kDiisThreads) {
+    double v = Pm[i];
+    if (apply) {
+      v = 0.0;
+#pragma unroll
+      for (int k = 0; k < kMaxDiis; ++k)
+        if (k < M) v += coef[k] * hist_dens[off[k] + i];
+    }
+    if (damp) v = v * (1.0 - prm.damping_weight) + prm.damping_weight * Po[i];
     Pm[i] = v;
   }
 }
 
-void launch_diis(const DevMol* mols, const int* mol_list, int nlist, MolState* st, const ScfParamsDev& prm,
+void launch_diis(const DevMol* mols, const int* mol_list, int nlist, int max_n, MolState* st, const ScfParamsDev& prm,
                  double* P, const double* Pold, double* hist_dens, double* hist_err, long long hist_stride,
-                 TraceEntry* trace, int trace_len, void* scratch, cudaStream_t s) {
+                 TraceEntry* trace, int trace_len, void* scratch, int slots, cudaStream_t s) {
   if (nlist <= 0) return;
   double* part = static_cast<double*>(scratch);
-  DiisStep* steps = reinterpret_cast<DiisStep*>(part + (size_t)nlist * kDiisChunksMax * kDiisPart);
-  diis_partial_kernel<<<dim3(kDiisChunksMax, nlist), kDiisThreads, 0, s>>>(mols, mol_list, st, prm, P, Pold, hist_dens,
-                                                                          hist_err, hist_stride, part);
-  diis_solve_kernel<<<(nlist + 63) / 64, 64, 0, s>>>(mols, mol_list, nlist, st, prm, part, steps, trace, trace_len);
-  diis_apply_kernel<<<dim3(kDiisChunksMax, nlist), kDiisThreads, 0, s>>>(mols, mol_list, st, prm, P, Pold, hist_dens,
-                                                                        hist_stride, steps);
+  DiisStep* steps = reinterpret_cast<DiisStep*>(part + (size_t)slots * kDiisChunksMax * kDiisPart);
+  int* ticket = reinterpret_cast<int*>(steps + slots);
+  const long long n2 = (long long)max_n * max_n;
+  const int chunks = (int)std::max(1LL, std::min<long long>(kDiisChunksMax, (n2 + 2047) / 2048));
+  diis_partial_kernel<<<dim3(chunks, nlist), kDiisThreads, 0, s>>>(mols, mol_list, st, prm, P, Pold, hist_dens, hist_err,
+                                                                  hist_stride, part, steps, ticket, trace, trace_len);
+  diis_apply_kernel<<<dim3(chunks, nlist), kDiisThreads, 0, s>>>(mols, mol_list, st, prm, P, Pold, hist_dens,
+                                                                hist_stride, steps);
 }
 
+// partial sums, decisions and tickets (zero between launches) of `slots` list entries
 size_t diis_scratch_bytes(int slots) {
-  return (size_t)slots * kDiisChunksMax * kDiisPart * sizeof(double) + (size_t)slots * sizeof(DiisStep) + 256;
+  return (size_t)slots * (kDiisChunksMax * kDiisPart * sizeof(double) + sizeof(DiisStep) + sizeof(int)) + 256;
 }
 
 // ---------------------------------------------------------------------------
