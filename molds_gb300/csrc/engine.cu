@@ -343,8 +343,8 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_hh_large_ = dalloc<int>(nm, &bytes_);
   for (int k = 0; k < 3; ++k) d_pur_list_[k] = dalloc<int>(nm, &bytes_);
   d_pur_ = dalloc<PurState>(nm, &bytes_);
-  // 129 basis functions have four tiles; larger bases have fewer per element
-  pur_tile_cap_ = cap.max_n > kPurSmallMaxN ? (size_t)(mat / 4096) + 16 : 1;
+  // 129 basis functions have six tiles; larger bases have fewer per element
+  pur_tile_cap_ = cap.max_n > kPurSmallMaxN ? (size_t)(mat / 2048) + 16 : 1;
   d_pur_tiles_ = dalloc<int4>(pur_tile_cap_, &bytes_);
   cuda_check(cudaHostAlloc(&h_pur_tiles_, sizeof(int4) * pur_tile_cap_, cudaHostAllocDefault), "cudaHostAlloc");
   grid_ctas_ = hh_grid_ctas();
@@ -1076,10 +1076,10 @@ void Batch::hh_reduce(int require) {
 
 bool Batch::purified(const ScfSettings& s) const { return s.eigensolver == 0 && householder(s); }
 
-void Batch::eigen_step(const ScfSettings& s, bool eigen) {
+void Batch::eigen_step(const ScfSettings& s, int effort) {
   if (householder(s)) {
     // the purification gives the density itself; the eigenpairs then only
-    // serve the molecules it could not treat (eigen: launch them as well)
+    // serve the molecules it could not treat (effort 2: launch them as well)
     const int require = purified(s) ? 2 : 1;
     if (purified(s)) {
       const int h = prof_begin(kKPurify, active_work_estimate(kKPurify));
@@ -1090,10 +1090,11 @@ void Batch::eigen_step(const ScfSettings& s, bool eigen) {
       }
       const PurScratch ws{{d_T64, d_S[0], d_S[1], d_S[2], d_S[3], d_S[4], d_S[5]}};
       launches_ += launch_purify_big(d_mols, d_pur_list_[2], (int)pur_list_[2].size(), pur_max_n_[2], d_pur_tiles_,
-                                     (int)pur_tiles_.size(), d_state, d_F, d_P, d_pur_, ws, kPurBigSteps, d_tc_err,
+                                     (int)pur_tiles_.size(), d_state, d_F, d_P, d_pur_, ws,
+                                     effort > 0 ? kPurBigSteps : kPurFewSteps, alone_, d_tc_err,
                                      stream_);
       prof_end(h);
-      if (!eigen) return;
+      if (effort < 2) return;
     }
     int h = prof_begin(kKTridiag, purified(s) ? 0.0 : active_work_estimate(kKTridiag));
     hh_reduce(require);
@@ -1222,7 +1223,7 @@ void Batch::density_step(const ScfSettings& s) {
   cuda_check(cudaGetLastError(), "density step");
 }
 
-void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, bool eigen) {
+void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, int effort) {
   upload_list(which);
   const int nl = (int)which.size();
   launches_ += 3;   // fock + two DIIS kernels
@@ -1231,11 +1232,11 @@ void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, bool ei
                      1, 1, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "fock_kernel");
-  eigen_step(s, eigen);
-  if (eigen || !purified(s)) density_step(s);
+  eigen_step(s, effort);
+  if (effort == 2 || !purified(s)) density_step(s);
   h = prof_begin(kKDiis, active_work_estimate(kKDiis));
   ScfParamsDev prm = to_dev(s);
-  prm.eigen_ran = eigen || !purified(s);
+  prm.eigen_ran = effort == 2 || !purified(s);
   launch_diis(d_mols, d_list, nl, list_max_n_, d_state, prm, d_P, d_Pold, d_hist_dens, d_hist_err, mat_total_,
               s.keep_trace ? d_trace : nullptr, max_iter_alloc_, d_diis_ws, cap_.slots, stream_);
   prof_end(h);
@@ -1257,11 +1258,11 @@ bool same_launches(const ScfSettings& a, const ScfSettings& b) {
 // block Jacobi, which reads a host flag between its sweeps, nor for an iteration
 // with a molecule on the whole-GPU eigensolver (its cooperative launches run long
 // enough that a launch costs nothing, and are not captured).  The iterations
-// with and without the eigensolver launches are two graphs.
-void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which, bool eigen) {
+// of each effort are a graph of their own.
+void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which, int effort) {
   upload_list(which);   // outside any capture: may synchronise when the list changes
-  if (!s.graphs || prof_on_ || !householder(s) || ((eigen || !purified(s)) && !hh_large_.empty())) {
-    iterate(s, which, eigen);
+  if (!s.graphs || prof_on_ || !householder(s) || ((effort == 2 || !purified(s)) && !hh_large_.empty())) {
+    iterate(s, which, effort);
     return;
   }
   if (!same_launches(graph_settings_, s) || graph_layout_ != layout_version_) {
@@ -1270,7 +1271,7 @@ void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which, b
     graph_settings_ = s;
     graph_layout_ = layout_version_;
   }
-  cudaGraphExec_t& exec = graph_exec_[eigen];
+  cudaGraphExec_t& exec = graph_exec_[effort];
   if (!exec) {
     hh_prepare();
     purify_prepare();
@@ -1278,7 +1279,7 @@ void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which, b
     cudaGraph_t g = nullptr;
     cuda_check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
-      iterate(s, which, eigen);
+      iterate(s, which, effort);
     } catch (...) {
       cudaStreamEndCapture(stream_, &g);
       if (g) cudaGraphDestroy(g);
@@ -1288,11 +1289,11 @@ void Batch::iterate_graph(const ScfSettings& s, const std::vector<int>& which, b
     const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     cuda_check(e, "graph instantiate");
-    graph_kernels_[eigen] = launches_ - before;
+    graph_kernels_[effort] = launches_ - before;
     launches_ = before;
   }
   cuda_check(cudaGraphLaunch(exec, stream_), "graph launch");
-  launches_ += graph_kernels_[eigen];
+  launches_ += graph_kernels_[effort];
   ++graph_launches_;
 }
 
@@ -1368,30 +1369,36 @@ void Batch::scf(const ScfSettings& s, bool requires_guess) {
   // so the device never waits for the host.  Every kernel of an iteration
   // skips molecules that are no longer active, so the iterations enqueued past
   // convergence change nothing (and cost only their empty launches).
-  // A molecule that the purification cannot treat waits without advancing until
-  // the host has read that count too and enqueues an iteration with the
-  // eigensolver; from the second such wait on every iteration has it.
+  // A molecule that the purification did not treat waits without advancing until
+  // the host has read that count too and enqueues an iteration of more effort:
+  // 0 few purification steps (18 to 24 are the rule), 1 as many as it has (the
+  // first iterations, whose gaps are small), 2 the eigensolver as well.  From the
+  // second wait for the eigensolver on every iteration has it.
   const int block = all.size() == 1 ? 3 : tuned_check_block();
-  const bool pur = purified(s);
-  int it = 0, nblock = 0, waits = 0;
-  bool eigen = false;
+  const bool pur = purified(s), tiled = pur && !pur_list_[2].empty();   // the one-CTA kernel stops by itself
+  const int early = tiled ? kPurEarly : 0;
+  int it = 0, nblock = 0, waits = 0, effort = 0, since = 0;   // effort used from block `since` on
   for (;;) {
     // past max_iter only molecules that waited are still active
-    for (int b = 0; b < block && (b == 0 || it < s.max_iter); ++b, ++it) iterate_graph(s, all, eigen && (b == 0 || waits > 1));
+    for (int b = 0; b < block && (b == 0 || it < s.max_iter); ++b, ++it)
+      iterate_graph(s, all, std::max(b == 0 || waits > 1 ? effort : 0, it < early ? 1 : 0));
     const bool last = it >= s.max_iter;
     const int slot = nblock & 1;
     count_active_async(all, h_block_count_ + 2 * slot, h_block_active_ + (size_t)slot * cap_.slots, block_ev_[slot]);
     ++nblock;
     if (last && !pur) break;
     if (nblock < 2 && !last) continue;
-    const int seen = last ? slot : slot ^ 1;
-    cuda_check(cudaEventSynchronize(block_ev_[seen]), "block count");
-    if (prof_on_) std::copy(h_block_active_ + (size_t)seen * cap_.slots,
-                            h_block_active_ + (size_t)seen * cap_.slots + h_mols.size(), active_host_.begin());
-    if (h_block_count_[2 * seen] == 0) break;
-    const bool waiting = h_block_count_[2 * seen + 1] > 0;
-    waits += waiting && !eigen;
-    eigen = waiting || waits > 1;
+    const int seen = last ? nblock - 1 : nblock - 2;   // block whose counts are read
+    cuda_check(cudaEventSynchronize(block_ev_[seen & 1]), "block count");
+    if (prof_on_) std::copy(h_block_active_ + (size_t)(seen & 1) * cap_.slots,
+                            h_block_active_ + (size_t)(seen & 1) * cap_.slots + h_mols.size(), active_host_.begin());
+    if (h_block_count_[2 * (seen & 1)] == 0) break;
+    const bool waiting = h_block_count_[2 * (seen & 1) + 1] > 0;
+    if (waits > 1 || seen < since) continue;
+    const int next = !waiting ? 0 : std::min(2, tiled ? effort + 1 : 2);
+    waits += next == 2;
+    if (next > effort) since = nblock;
+    effort = next;
   }
   finish(s, all);
   int tc_err = 0;

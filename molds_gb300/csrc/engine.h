@@ -95,6 +95,8 @@ class Batch {
   Batch& operator=(const Batch&) = delete;
 
   int size() const { return (int)h_mols.size(); }
+  // other streams run beside this batch's (molecule groups, serving lanes)
+  void set_shared() { alone_ = false; }
   int max_n() const { return cap_.max_n; }
   long long epc_capacity() const { return cap_.epcs; }
   cudaStream_t stream() const { return stream_; }
@@ -124,16 +126,17 @@ class Batch {
   void scf(const ScfSettings& s, bool requires_guess);
   // Initialise the SCF state of the listed molecules (serving: admission).
   void begin(const ScfSettings& s, const std::vector<int>& which, bool requires_guess);
-  // One SCF iteration over the listed (active) molecules; eigen: the eigensolver
-  // serves the molecules whose density the purification cannot give
-  void iterate(const ScfSettings& s, const std::vector<int>& which, bool eigen = false);
+  // One SCF iteration over the listed (active) molecules; effort 0: few
+  // purification steps, 1: as many as it has, 2: the eigensolver as well, for the
+  // molecules whose density the purification cannot give
+  void iterate(const ScfSettings& s, const std::vector<int>& which, int effort = 1);
   // Energies / charges of the listed molecules after convergence.
   void finish(const ScfSettings& s, const std::vector<int>& which);
   // Number of still-active molecules among `which` (synchronises).
   int count_active(const std::vector<int>& which);
   // One SCF iteration, replayed from a captured CUDA graph when the settings
   // allow it (iterate() otherwise)
-  void iterate_graph(const ScfSettings& s, const std::vector<int>& which, bool eigen = false);
+  void iterate_graph(const ScfSettings& s, const std::vector<int>& which, int effort = 1);
   long long graph_launches() const { return graph_launches_; }
 
   // results (synchronise and copy out)
@@ -171,7 +174,7 @@ class Batch {
   int list_max_atoms() const;   // largest molecule (atoms) of the current list
   void build_jobs(const std::vector<int>& which);
   void upload_list(const std::vector<int>& which);
-  void eigen_step(const ScfSettings& s, bool eigen);
+  void eigen_step(const ScfSettings& s, int effort);
   // the current list's Householder tridiagonalisations of F (require: see mol_skipped)
   void hh_reduce(int require);
   // density by purification, the eigensolver only for molecules it leaves over
@@ -188,6 +191,7 @@ class Batch {
   cudaStream_t stream_;
   int diis_m_;
   bool pool_ = false;
+  bool alone_ = true;
   BatchCapacity cap_;
   ArenaAlloc a_atoms_, a_pairs_, a_blocks_, a_mat_, a_vec_, a_epc_;
   std::vector<int> free_slots_;
@@ -284,11 +288,11 @@ class Batch {
   void make_jobset(JobSet* js, const std::vector<GemmJob>& jobs);
 
   // captured SCF iteration
-  cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};   // without and with the eigensolver launches
+  cudaGraphExec_t graph_exec_[3] = {nullptr, nullptr, nullptr};   // by effort
   ScfSettings graph_settings_;
   long long graph_layout_ = -1;           // layout_version_ the graph was captured for
   long long layout_version_ = 0;          // bumped whenever the job tables and size buckets are rebuilt
-  long long graph_kernels_[2] = {0, 0};   // kernels in one replay
+  long long graph_kernels_[3] = {0, 0, 0};   // kernels in one replay
   long long graph_launches_ = 0;          // replays so far
   // pipelined convergence checks: pinned counts and their events (two blocks in flight)
   int* h_block_count_ = nullptr;

@@ -46,6 +46,7 @@ GroupedBatch::GroupedBatch(Engine* eng, const std::vector<MoleculeInput>& mols, 
     first_mol_.push_back(mol);
     first_atom_.push_back(atom);
     g_.emplace_back(new Batch(eng, part, diis_m, st));
+    if (groups > 1) g_.back()->set_shared();
     for (const MoleculeInput& m : part) atom += (int)m.Z.size();
     mol += cnt;
   }

@@ -133,6 +133,8 @@ void launch_jacobi_f64(const DevMol* mols, const int* mol_list, int nlist, int m
 // F) of the listed active molecules; sets or clears kNeedEigen in their state.
 constexpr int kPurSmallMaxN = 128;   // one CTA per molecule up to here, tiles of every step above
 constexpr int kPurBigSteps = 56;     // steps launched above kPurSmallMaxN: HOMO-LUMO gaps down to ~3e-4 of the interval
+constexpr int kPurFewSteps = 32;     // and for the later SCF iterations, whose gaps are wide
+constexpr int kPurEarly = 6;         // SCF iterations that get kPurBigSteps from the start
 struct PurState {
   unsigned long long lo, hi;         // Gershgorin interval, order-preserving keys
   long long trace[kPurBigSteps + 1]; // tr X_k
@@ -143,10 +145,11 @@ void purify_prepare();               // one-time kernel attributes (before any s
 int purify_tiles(int mol, int n, int4* out);   // tiles of one molecule (out may be null); returns their number
 void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
                          double* P, int* err, cudaStream_t s);
+// alone: no other stream's work is expected beside this launch sequence
 // returns the number of kernels launched
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
-                      int* err, cudaStream_t s);
+                      bool alone, int* err, cudaStream_t s);
 
 int hh_smem_max_n();     // largest basis whose packed matrix fits one CTA's shared memory
 int hh_back_max_n();     // largest basis the back-transformation kernel serves

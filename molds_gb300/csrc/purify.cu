@@ -578,10 +578,15 @@ __global__ void __launch_bounds__(kPurTileThreads, 1)
 purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ tiles, const MolState* __restrict__ st,
                    PurState* __restrict__ pur, PurScratch ws, int k, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char pu_sm[];
+  // what no step changes is read while the previous step still runs (programmatic
+  // dependent launch); every CTA waits for it before it looks at anything else,
+  // or returns, so that the next step's wait covers all earlier ones
   const int4 tile = tiles[blockIdx.x];
   const int mi = tile.x;
-  if (st[mi].status != kActive) return;
   const DevMol mol = mols[mi];
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  if (st[mi].status != kActive) return;
   const int n = mol.nao, np = pu_np(n);
   const long long occ = (long long)mol.nocc * kTraceOne;
   double lo, hi;
@@ -805,7 +810,7 @@ void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max
 
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
-                      int* err, cudaStream_t s) {
+                      bool alone, int* err, cudaStream_t s) {
   if (nlist <= 0) return 0;
   purify_prepare();
   const int np = (max_n + 31) / 32 * 32;
@@ -813,8 +818,21 @@ int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n,
   purify_reset_kernel<<<nlist, 64, 0, s>>>(list, pur);
   purify_bounds_kernel<<<dim3((max_n + 7) / 8, nlist), 256, 0, s>>>(mols, list, st, F, pur);
   purify_init_kernel<<<dim3(blocks, nlist), 256, 0, s>>>(mols, list, st, F, pur, ws);
-  for (int k = 0; k < steps; ++k)
-    purify_step_kernel<<<ntiles, kPurTileThreads, kPurTileSmem, s>>>(mols, tiles, st, pur, ws, k, err);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ntiles);
+  cfg.blockDim = dim3(kPurTileThreads);
+  cfg.dynamicSmemBytes = kPurTileSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  for (int k = 0; k < steps; ++k) {
+    // CTAs launched ahead hold an SM while they wait: only where no other stream
+    // has work for it (a server's burst took 104 ms without and 119 with them)
+    cfg.numAttrs = alone && k > 0 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, purify_step_kernel, mols, tiles, (const MolState*)st, pur, ws, k, err);
+  }
   purify_store_kernel<<<dim3(blocks, nlist), 256, 0, s>>>(mols, list, st, pur, ws, steps, P);
   return steps + 4;
 }

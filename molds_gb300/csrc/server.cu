@@ -73,6 +73,7 @@ Server::Server(Engine* eng, const ScfSettings& s, size_t hbm_budget, int max_bas
     cuda_check(cudaEventCreateWithFlags(&L->ev, cudaEventDisableTiming), "lane event");
     BatchCapacity c = lane_capacity((size_t)(sp.share * (double)hbm_budget), sp.hi, sp.min_n, m, sp.ws);
     L->b.reset(new Batch(eng_, c, m, L->stream));
+    L->b->set_shared();
     const int slots = c.slots;
     L->slot_ticket.assign(slots, -1);
     L->slot_tsubmit.assign(slots, 0.0);
@@ -279,7 +280,7 @@ bool Server::lane_step(Lane& L) {
   if (L.active.empty()) return false;
   // a molecule the purification cannot treat waits for an iteration with the
   // eigensolver; it waited once, so its next iterations have it as well
-  b.iterate(s_, L.active, L.eigen > 0);
+  b.iterate(s_, L.active, L.eigen > 0 ? 2 : 1);
   b.count_active_async(L.active, L.h_count, L.h_active, L.ev);
   cuda_check(cudaEventSynchronize(L.ev), "lane iteration");
   L.eigen = L.h_count[1] > 0 ? 8 : std::max(0, L.eigen - 1);
