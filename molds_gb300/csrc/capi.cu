@@ -560,7 +560,6 @@ int nddo_batch_scf(nddo_ctx* ctx, int theory, int n_mol, const int* n_atoms, con
     std::vector<nddo::MolResult> r;
     b.results(&r);
     int rc = NDDO_OK;
-    off = 0;
     for (int i = 0; i < n_mol; ++i) {
       results[i].status = r[i].status;
       results[i].iterations = r[i].iterations;
@@ -573,9 +572,8 @@ int nddo_batch_scf(nddo_ctx* ctx, int theory, int n_mol, const int* n_atoms, con
       results[i].vdw_energy = r[i].vdw_energy;
       results[i].core_epc_coulomb = r[i].core_epc;
       if (r[i].status != nddo::kConverged) rc = NDDO_NOT_CONVERGED;
-      if (charges) b.copy_charges(i, charges + off);
-      off += n_atoms[i];
     }
+    if (charges) b.copy_all_charges(charges);
     if (rc != NDDO_OK) ctx->err = "SCF did not met convergence criterion for at least one molecule";
     return rc;
   });
@@ -657,7 +655,6 @@ int nddo_batch_results(nddo_batch* h, nddo_scf_result* results, double* charges)
     std::vector<nddo::MolResult> r;
     h->b->results(&r);
     int rc = NDDO_OK;
-    size_t off = 0;
     for (size_t i = 0; i < r.size(); ++i) {
       results[i].status = r[i].status;
       results[i].iterations = r[i].iterations;
@@ -670,9 +667,8 @@ int nddo_batch_results(nddo_batch* h, nddo_scf_result* results, double* charges)
       results[i].vdw_energy = r[i].vdw_energy;
       results[i].core_epc_coulomb = r[i].core_epc;
       if (r[i].status != nddo::kConverged) rc = NDDO_NOT_CONVERGED;
-      if (charges) h->b->copy_charges((int)i, charges + off);
-      off += h->n_atoms[i];
     }
+    if (charges) h->b->copy_all_charges(charges);
     if (rc != NDDO_OK) h->ctx->err = "SCF did not met convergence criterion for at least one molecule";
     return rc;
   });

@@ -11,6 +11,7 @@
 #include "tuning.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <stdexcept>
@@ -158,6 +159,16 @@ struct MolLayout {
   long long blocks = 0;
 };
 
+// no two of n atoms (3 coordinates each) at the same position: by sorting, not
+// over all pairs, which a batch of 256 x 96 atoms has 1.2 million of
+void check_positions(const double* xyz, int n) {
+  std::vector<std::array<double, 3>> p(n);
+  for (int a = 0; a < n; ++a) p[a] = {xyz[3 * a], xyz[3 * a + 1], xyz[3 * a + 2]};
+  std::sort(p.begin(), p.end());
+  if (std::adjacent_find(p.begin(), p.end()) != p.end())
+    throw std::invalid_argument("two atoms at the same position");
+}
+
 MolLayout layout_molecule(const MoleculeInput& in) {
   MolLayout L;
   const int na = (int)in.Z.size();
@@ -195,12 +206,12 @@ MolLayout layout_molecule(const MoleculeInput& in) {
       if (A.x == in.epc[i] && A.y == in.epc[i + 1] && A.z == in.epc[i + 2])
         throw std::invalid_argument("a point charge at an atom's position");
   }
+  check_positions(in.xyz.data(), na);
+  L.pairs.reserve((size_t)na * (na - 1) / 2);
   for (int a = 0; a < na; ++a)
     for (int b = a + 1; b < na; ++b) {
       const DevAtom& A = L.atoms[a];
       const DevAtom& B = L.atoms[b];
-      const double dx = A.x - B.x, dy = A.y - B.y, dz = A.z - B.z;
-      if (dx == 0.0 && dy == 0.0 && dz == 0.0) throw std::invalid_argument("two atoms at the same position");
       DevPair p;
       p.a = a; p.b = b; p.mol = 0; p.pad = 0;
       p.blk = L.blocks;
@@ -865,11 +876,7 @@ void Batch::set_coordinates(const double* xyz) {
       if (!std::isfinite(xyz[3 * a + k])) throw std::invalid_argument("non-finite coordinate");
     h_atoms[a].x = xyz[3 * a]; h_atoms[a].y = xyz[3 * a + 1]; h_atoms[a].z = xyz[3 * a + 2];
   }
-  for (const DevPair& p : h_pairs) {
-    const DevAtom& A = h_atoms[p.a];
-    const DevAtom& B = h_atoms[p.b];
-    if (A.x == B.x && A.y == B.y && A.z == B.z) throw std::invalid_argument("two atoms at the same position");
-  }
+  for (const DevMol& d : h_mols) check_positions(xyz + 3 * (size_t)d.atom0, d.natoms);
   cuda_check(cudaMemcpyAsync(d_atoms, h_atoms.data(), h_atoms.size() * sizeof(DevAtom), cudaMemcpyHostToDevice, stream_),
              "upload atoms");
 }
@@ -879,12 +886,7 @@ void Batch::set_molecule_coordinates(int m, const double* xyz) {
   const DevMol& d = h_mols[m];
   for (int a = 0; a < 3 * d.natoms; ++a)
     if (!std::isfinite(xyz[a])) throw std::invalid_argument("non-finite coordinate");
-  for (int k = 0; k < d.npairs; ++k) {
-    const DevPair& p = h_pairs[d.pair0 + k];
-    const double* A = xyz + 3 * (p.a - d.atom0);
-    const double* B = xyz + 3 * (p.b - d.atom0);
-    if (A[0] == B[0] && A[1] == B[1] && A[2] == B[2]) throw std::invalid_argument("two atoms at the same position");
-  }
+  check_positions(xyz, d.natoms);
   for (int a = 0; a < d.natoms; ++a) {
     DevAtom& at = h_atoms[d.atom0 + a];
     at.x = xyz[3 * a]; at.y = xyz[3 * a + 1]; at.z = xyz[3 * a + 2];
@@ -902,32 +904,46 @@ void Batch::integrals() {
 void Batch::integrals(const std::vector<int>& which) {
   if (which.empty()) return;
   upload_list(which);
-  // pair index lists of the listed molecules: sp-sp pairs for the warp kernel,
-  // X-H then H-H pairs for the thread-per-pair kernel
-  std::vector<int> heavy, xh, hh;
   double blk = 0.0;
-  for (int m : which) {
-    const DevMol& d = h_mols[m];
-    for (int k = 0; k < d.npairs; ++k) {
-      const int pi = d.pair0 + k;
-      const int na = h_atoms[h_pairs[pi].a].nao, nb = h_atoms[h_pairs[pi].b].nao;
-      blk += (double)((na == 4 ? 10 : 1) * (nb == 4 ? 10 : 1));
-      if (na == 4 && nb == 4) heavy.push_back(pi);
-      else if (na == 4 || nb == 4) xh.push_back(pi);
-      else hh.push_back(pi);
+  if (prof_on_)
+    for (int m : which) {
+      const DevMol& d = h_mols[m];
+      for (int k = 0; k < d.npairs; ++k) {
+        const DevPair& p = h_pairs[d.pair0 + k];
+        blk += (double)((h_atoms[p.a].nao == 4 ? 10 : 1) * (h_atoms[p.b].nao == 4 ? 10 : 1));
+      }
     }
+  // A fixed batch's pairs, and one molecule's, are one range of the arena, over
+  // which each kernel skips the other's pairs; several molecules of a pool get
+  // index lists (sp-sp pairs, then those with a hydrogen).
+  const bool whole = !pool_ && which.size() == h_mols.size();
+  std::vector<int> heavy, light;
+  if (!whole && which.size() > 1) {
+    for (int m : which) {
+      const DevMol& d = h_mols[m];
+      for (int k = 0; k < d.npairs; ++k) {
+        const int pi = d.pair0 + k;
+        const bool hv = h_atoms[h_pairs[pi].a].nao == 4 && h_atoms[h_pairs[pi].b].nao == 4;
+        (hv ? heavy : light).push_back(pi);
+      }
+    }
+    if (!heavy.empty())
+      cuda_check(cudaMemcpyAsync(d_heavy_pairs, heavy.data(), heavy.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload heavy pairs");
+    if (!light.empty())
+      cuda_check(cudaMemcpyAsync(d_light_pairs, light.data(), light.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload light pairs");
   }
-  xh.insert(xh.end(), hh.begin(), hh.end());
-  n_heavy_ = (long long)heavy.size();
-  n_light_ = (long long)xh.size();
-  if (!heavy.empty())
-    cuda_check(cudaMemcpyAsync(d_heavy_pairs, heavy.data(), heavy.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload heavy pairs");
-  if (!xh.empty())
-    cuda_check(cudaMemcpyAsync(d_light_pairs, xh.data(), xh.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload light pairs");
   int h = prof_begin(kKPair, 8.0 * blk);
   launches_ += 2;
-  launch_pair_kernels_split(d_atoms, d_pairs, d_heavy_pairs, n_heavy_, d_light_pairs, n_light_, d_mols, eng_->eri(),
-                            eng_->ovt(), d_blocks, d_H, d_ecore_pair, stream_);
+  if (whole || which.size() == 1) {
+    const long long p0 = whole ? 0 : h_mols[which[0]].pair0;
+    const long long np = whole ? (long long)h_pairs.size() : h_mols[which[0]].npairs;
+    launch_pair_kernel(d_atoms, d_pairs + p0, np, d_mols, eng_->eri(), eng_->ovt(), d_blocks, d_H, d_ecore_pair + p0,
+                       stream_);
+  } else {
+    launch_pair_kernels_split(d_atoms, d_pairs, d_heavy_pairs, (long long)heavy.size(), d_light_pairs,
+                              (long long)light.size(), d_mols, eng_->eri(), eng_->ovt(), d_blocks, d_H, d_ecore_pair,
+                              stream_);
+  }
   prof_end(h);
   cuda_check(cudaGetLastError(), "pair_kernel");
   h = prof_begin(kKHcore, 0.0);
@@ -937,7 +953,7 @@ void Batch::integrals(const std::vector<int>& which) {
   prof_end(h);
   cuda_check(cudaGetLastError(), "hcore_kernel");
   // the pageable index vectors above must outlive their copies
-  cuda_check(cudaStreamSynchronize(stream_), "integrals");
+  if (!heavy.empty() || !light.empty()) cuda_check(cudaStreamSynchronize(stream_), "integrals");
 }
 
 static ScfParamsDev to_dev(const ScfSettings& s) {
@@ -1456,6 +1472,11 @@ void Batch::copy_eps(int m, double* host) const {
 void Batch::copy_charges(int m, double* host) const {
   const DevMol& d = h_mols[m];
   cuda_check(cudaMemcpyAsync(host, d_charges + d.atom0, d.natoms * sizeof(double), cudaMemcpyDeviceToHost, stream_), "copy charges");
+  cuda_check(cudaStreamSynchronize(stream_), "copy charges");
+}
+
+void Batch::copy_all_charges(double* host) const {
+  cuda_check(cudaMemcpyAsync(host, d_charges, h_atoms.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_), "copy charges");
   cuda_check(cudaStreamSynchronize(stream_), "copy charges");
 }
 

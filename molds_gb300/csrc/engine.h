@@ -144,6 +144,7 @@ class Batch {
   void copy_matrix(int which_matrix, int m, double* host) const;   // 0 H, 1 F, 2 P, 3 C
   void copy_eps(int m, double* host) const;
   void copy_charges(int m, double* host) const;
+  void copy_all_charges(double* host) const;   // fixed batch: every atom's, in input order
   // analytic forces (Hartree/bohr, natoms x 3) of molecule m's converged SCF
   void forces(const ScfSettings& s, int m, double* host);
   void copy_blocks(int m, double* host, size_t* count) const;
@@ -215,7 +216,6 @@ class Batch {
   double* d_ecore_pair = nullptr;
   int* d_heavy_pairs = nullptr;   // indices of sp-sp pairs
   int* d_light_pairs = nullptr;   // indices of pairs with a hydrogen (X-H first, then H-H)
-  long long n_heavy_ = 0, n_light_ = 0;
   double *d_H = nullptr, *d_F = nullptr, *d_P = nullptr, *d_Pold = nullptr, *d_C = nullptr, *d_eps = nullptr;
   double *d_hist_dens = nullptr, *d_hist_err = nullptr;
   float *d_G32 = nullptr, *d_T32 = nullptr;
@@ -334,7 +334,7 @@ class GroupedBatch {
   // starts every molecule from its previous density (DoSCF(false))
   void run(const ScfSettings& s, bool requires_guess = true);
   void results(std::vector<MolResult>* out);
-  void copy_charges(int m, double* host) const;
+  void copy_all_charges(double* host) const;
   void copy_matrix(int which_matrix, int m, double* host) const;
   void cartesian_matrix(int m, double* host) const;
   void forces(const ScfSettings& s, int m, double* host);   // analytic forces of molecule m (natoms x 3)

@@ -100,10 +100,8 @@ void GroupedBatch::results(std::vector<MolResult>* out) {
   }
 }
 
-void GroupedBatch::copy_charges(int m, double* host) const {
-  int l = 0;
-  const Batch& b = locate(m, &l);
-  b.copy_charges(l, host);
+void GroupedBatch::copy_all_charges(double* host) const {
+  for (size_t g = 0; g < g_.size(); ++g) g_[g]->copy_all_charges(host + first_atom_[g]);
 }
 
 void GroupedBatch::forces(const ScfSettings& s, int m, double* host) {
