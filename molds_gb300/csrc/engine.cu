@@ -354,8 +354,9 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_hh_large_ = dalloc<int>(nm, &bytes_);
   for (int k = 0; k < 3; ++k) d_pur_list_[k] = dalloc<int>(nm, &bytes_);
   d_pur_ = dalloc<PurState>(nm, &bytes_);
-  // 129 basis functions have six tiles; larger bases have fewer per element
-  pur_tile_cap_ = cap.max_n > kPurSmallMaxN ? (size_t)(mat / 2048) + 16 : 1;
+  // 129 basis functions have four wide tiles; larger bases have fewer per
+  // element; narrow ones are used up to one per SM
+  pur_tile_cap_ = cap.max_n > kPurSmallMaxN ? (size_t)(mat / 4096) + 16 + hh_grid_ctas() : 1;
   d_pur_tiles_ = dalloc<int4>(pur_tile_cap_, &bytes_);
   cuda_check(cudaHostAlloc(&h_pur_tiles_, sizeof(int4) * pur_tile_cap_, cudaHostAllocDefault), "cudaHostAlloc");
   grid_ctas_ = hh_grid_ctas();
@@ -637,16 +638,20 @@ void Batch::build_jobs(const std::vector<int>& which) {
   }
   // purification lists and tiles
   for (int k = 0; k < 3; ++k) { pur_list_[k].clear(); pur_max_n_[k] = 0; }
-  pur_tiles_.clear();
   for (int m : which) {
     const int n = h_mols[m].nao, k = n <= 64 ? 0 : (n <= kPurSmallMaxN ? 1 : 2);
     pur_list_[k].push_back(m);
     pur_max_n_[k] = std::max(pur_max_n_[k], n);
-    if (k == 2) {
+  }
+  // wide tiles, or narrow ones while those still find an SM each
+  for (pur_tn_ = 32; pur_tn_ <= 64; pur_tn_ *= 2) {
+    pur_tiles_.clear();
+    for (int m : pur_list_[2]) {
       const size_t t = pur_tiles_.size();
-      pur_tiles_.resize(t + purify_tiles(m, n, nullptr));
-      purify_tiles(m, n, pur_tiles_.data() + t);
+      pur_tiles_.resize(t + purify_tiles(m, h_mols[m].nao, pur_tn_, nullptr));
+      purify_tiles(m, h_mols[m].nao, pur_tn_, pur_tiles_.data() + t);
     }
+    if ((int)pur_tiles_.size() <= grid_ctas_ || pur_tn_ == 64) break;
   }
   if (pur_tiles_.size() > pur_tile_cap_) throw std::logic_error("purification tile table overflow");
   // chunks of at most grid_ctas_ molecules and their CTA maps
@@ -1106,7 +1111,7 @@ void Batch::eigen_step(const ScfSettings& s, int effort) {
       }
       const PurScratch ws{{d_T64, d_S[0], d_S[1], d_S[2], d_S[3], d_S[4], d_S[5]}};
       launches_ += launch_purify_big(d_mols, d_pur_list_[2], (int)pur_list_[2].size(), pur_max_n_[2], d_pur_tiles_,
-                                     (int)pur_tiles_.size(), d_state, d_F, d_P, d_pur_, ws,
+                                     (int)pur_tiles_.size(), pur_tn_, d_state, d_F, d_P, d_pur_, ws,
                                      effort > 0 ? kPurBigSteps : kPurFewSteps, alone_, d_tc_err,
                                      stream_);
       prof_end(h);

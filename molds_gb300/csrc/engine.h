@@ -238,6 +238,7 @@ class Batch {
   int* d_pur_list_[3] = {};
   int pur_max_n_[3] = {};
   std::vector<int4> pur_tiles_;
+  int pur_tn_ = 64;                      // their columns
   int4* d_pur_tiles_ = nullptr;
   int4* h_pur_tiles_ = nullptr;          // pinned staging of d_pur_tiles_
   size_t pur_tile_cap_ = 0;

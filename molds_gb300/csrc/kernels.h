@@ -97,7 +97,7 @@ void launch_energy_kernel(const DevAtom* atoms, const DevPair* pairs, const DevM
                           MolState* st, double* charges, VdwParams vdw, cudaStream_t s);
 // dipole moment of the listed molecules into MolState::dipole; partial holds
 // nlist * kDipChunks * 4 doubles
-constexpr int kDipChunks = 64;
+constexpr int kDipChunks = 304;   // two CTAs on every SM
 void launch_dipole(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list, int nlist,
                    int max_atoms, const double* P, const double* H, double* partial, MolState* st, cudaStream_t s);
 // STO-6G Cartesian matrix of molecule m: X = 3 x N x N doubles
@@ -142,12 +142,13 @@ struct PurState {
 };
 struct PurScratch { double* m[7]; }; // N x N scratch matrices holding two digit buffers of seven digits each
 void purify_prepare();               // one-time kernel attributes (before any stream capture)
-int purify_tiles(int mol, int n, int4* out);   // tiles of one molecule (out may be null); returns their number
+// tiles of tn columns (64 or 32) of one molecule (out may be null); returns their number
+int purify_tiles(int mol, int n, int tn, int4* out);
 void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
                          double* P, int* err, cudaStream_t s);
 // alone: no other stream's work is expected beside this launch sequence
 // returns the number of kernels launched
-int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
+int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles, int tn,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
                       bool alone, int* err, cudaStream_t s);
 

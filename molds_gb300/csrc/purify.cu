@@ -214,8 +214,20 @@ __device__ __forceinline__ void pu_join8(const uint4* in, long long* x) {
   }
 }
 
+// a double cut to FP32 by integer instructions (0 below 2^-126, huge above 2^127)
+__device__ __forceinline__ float pu_float(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)(b >> 52) & 0x7ff;
+  const uint32_t s = (uint32_t)(b >> 32) & 0x80000000u;
+  if (e < 897) return __uint_as_float(s);
+  if (e > 1150) return __uint_as_float(s | 0x7f000000u);
+  return __uint_as_float(s | ((uint32_t)(e - 896) << 23) | (uint32_t)((b >> 29) & 0x7fffffu));
+}
 __device__ __forceinline__ long long pu_fixed(double v) { return __double2ll_rn(v * 36028797018963968.0); }   // 2^55
-__device__ __forceinline__ double pu_density(long long x) { return (double)x * 5.5511151231257827e-17; }       // 2 * 2^-55
+__device__ __forceinline__ double pu_density(long long x) {   // 2 * 2^-55 x: the exponent by an integer instruction
+  const double v = (double)x;
+  return x ? __hiloint2double(__double2hiint(v) - (54 << 20), __double2loint(v)) : 0.0;
+}
 
 // Where the iteration stands at X_k, with t0, t1 the traces of X_k and X_{k-1}:
 // the step to take (1: X^2, 0: 2 X - X^2), or -1 when X_k is the projector.
@@ -250,7 +262,9 @@ __device__ __forceinline__ bool pu_counted(long long t, long long occ) {
 // recombine the other.
 // Measured (clocks a step, N = 50 / 72 / 120): 18000 / 32000 / 50000 with all
 // levels of 64 columns at a time, conversions by instruction and the trace by
-// shared atomics; see the table in the launcher for what it is now.
+// shared atomics; 11000 / 16000 / 29000 now.  At small N the interval was as dear
+// as the steps: in FP32 with weights it took (H2O)2 from 2.18 to 1.84 ms and
+// C14H30 with 900 external charges from 18.5 to 15.2 ms.
 // ---------------------------------------------------------------------------
 constexpr int kPurSmallWarps = 16;   // recombining; one more issues the MMAs
 
@@ -305,23 +319,79 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   unsigned char* tail = pu_sm + (size_t)(kDigits - 1) * 2 * np_max * np_max + (size_t)256 * np_max;
   const uint32_t bar = pu_smem(tail);                                      // two, one per buffer
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 16);
-  double* red = reinterpret_cast<double*>(tail + 32);                      // 2 x 17
-  long long* diag = reinterpret_cast<long long*>(tail + 32 + 34 * 8);      // 2 x 128
+  long long* diag = reinterpret_cast<long long*>(tail + 32);               // 2 x 128
   const double* Fm = F + mol.mat0;
 
-  // Gershgorin interval
-  double lo = 1e300, hi = -1e300, bad = 0.0;
-  for (int i = warp; i < n; i += kPurSmallWarps + 1) {
-    double s = 0.0;
-    for (int j = lane; j < n; j += 32)
-      if (j != i) s += fabs(Fm[(long long)i * n + j]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const double d = Fm[(long long)i * n + i];
-    if (!(s + fabs(d) < 1e290)) bad = 1.0;
-    lo = fmin(lo, d - s);
-    hi = fmax(hi, d + s);
+  // Interval of the eigenvalues: Gershgorin's circles with positive weights,
+  // F_ii +- sum_j |F_ij| w_j / w_i, bound the spectrum for any w; two rounds of
+  // power iteration bring w towards the best one, for each end its own.  Plain
+  // circles (w = 1) make the interval two to three times as wide as the spectrum,
+  // which costs two of about 22 steps.  In FP32, widened by far more than its
+  // rounding: an FP64 instruction of a warp takes the SM 16 clocks.
+  float flo = -3e37f, fhi = 3e37f;
+  {
+    float* w = reinterpret_cast<float*>(pu_sm);   // two buffers of (upper, lower) weights, where the digits come later
+    float* fred = reinterpret_cast<float*>(diag);
+    for (int i = tid; i < 256; i += kPurSmallThreads) w[i] = 1.0f;
+    float dmin = 0.0f, dmax = 0.0f, eps = 0.0f;
+    for (int pass = 0; pass < 3; ++pass) {
+      __syncthreads();
+      const float* wu = w + (pass & 1) * 256;
+      const float* wl = wu + 128;
+      float* nu = w + ((pass & 1) ^ 1) * 256;
+      float bl = 3e37f, bu = -3e37f, d0 = 3e37f, d1 = -3e37f;
+      for (int i = warp; i < n; i += kPurSmallWarps + 1) {
+        float su = 0.0f, sl = 0.0f, d = 0.0f;
+        bool big = false;
+        for (int j = lane; j < n; j += 32) {
+          const float f = pu_float(Fm[(long long)i * n + j]);
+          big = big || !(fabsf(f) < 1e30f);
+          if (j == i) d = f;
+          else { su += fabsf(f) * wu[j]; sl += fabsf(f) * wl[j]; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+          su += __shfl_xor_sync(0xffffffffu, su, o);
+          sl += __shfl_xor_sync(0xffffffffu, sl, o);
+        }
+        d = __shfl_sync(0xffffffffu, d, i & 31);
+        if (__any_sync(0xffffffffu, big)) bl = -3e38f;
+        d0 = fminf(d0, d);
+        d1 = fmaxf(d1, d);
+        bl = fminf(bl, d - sl / wl[i]);
+        bu = fmaxf(bu, d + su / wu[i]);
+        if (lane == 0) {   // products with dmin and dmax shifting the diagonal, known from pass 1 on
+          nu[i] = su + (pass ? (d - dmin + eps) * wu[i] : 0.0f);
+          nu[128 + i] = sl + (pass ? (dmax - d + eps) * wl[i] : 0.0f);
+          if (!pass) w[512 + i] = d;
+        }
+      }
+      if (lane == 0) { fred[warp] = bl; fred[32 + warp] = bu; fred[64 + warp] = d0; fred[96 + warp] = d1; }
+      __syncthreads();
+      const bool in = lane < kPurSmallWarps + 1;
+      bl = in ? fred[lane] : 3e37f;
+      bu = in ? fred[32 + lane] : -3e37f;
+      d0 = in ? fred[64 + lane] : 3e37f;
+      d1 = in ? fred[96 + lane] : -3e37f;
+      for (int o = 16; o > 0; o >>= 1) {
+        bl = fminf(bl, __shfl_xor_sync(0xffffffffu, bl, o));
+        bu = fmaxf(bu, __shfl_xor_sync(0xffffffffu, bu, o));
+        d0 = fminf(d0, __shfl_xor_sync(0xffffffffu, d0, o));
+        d1 = fmaxf(d1, __shfl_xor_sync(0xffffffffu, d1, o));
+      }
+      flo = pass ? fmaxf(flo, bl) : bl;
+      fhi = pass ? fminf(fhi, bu) : bu;
+      if (pass) continue;
+      if (!(bl > -1e37f && bu > bl)) break;
+      dmin = d0;
+      dmax = d1;
+      eps = 0.02f * (bu - bl);
+      for (int i = tid; i < n; i += kPurSmallThreads) {
+        nu[i] += w[512 + i] - dmin + eps;
+        nu[128 + i] += dmax - w[512 + i] + eps;
+      }
+    }
+    __syncthreads();
   }
-  if (lane == 0) { red[warp] = bad > 0.0 ? -1e300 : lo; red[17 + warp] = hi; }
   for (int i = tid; i < 256; i += kPurSmallThreads) diag[i] = 0;
   int ncols = 32;
   while (ncols < 2 * L * np) ncols <<= 1;
@@ -339,23 +409,26 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  for (int w = 0; w < kPurSmallWarps + 1; ++w) { lo = fmin(lo, red[w]); hi = fmax(hi, red[17 + w]); }
-  const bool usable = lo > -1e299 && hi > lo;
-  const double scale = usable ? 1.0 / (hi - lo) : 0.0;
+  const bool usable = flo > -1e37f && fhi > flo;
+  const float pad = 1e-4f * (fhi - flo) + 1e-5f * (fabsf(flo) + fabsf(fhi));
+  const double scale = usable ? 36028797018963968.0 / ((double)(fhi - flo) + 2.0 * pad) : 0.0;   // 2^55 / width
+  const double top = ((double)fhi + pad) * scale;
 
   long long x[H][16];
 #pragma unroll
-  for (int h = 0; h < H; ++h)
+  for (int h = 0; h < H; ++h) {
+    const int c0 = 64 * h + 16 * g;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const int col = 64 * h + 16 * g + c;
-      long long v = 0;
-      if (r < n && col < n) {
-        const double f = Fm[(long long)max(r, col) * n + min(r, col)];
-        v = pu_fixed(((r == col ? hi : 0.0) - f) * scale);
+    for (int c = 0; c < 16; ++c) x[h][c] = 0;
+    if (q * 32 < n && c0 < n && !issuer) {
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const int col = c0 + c;
+        if (r < n && col < n)
+          x[h][c] = __double2ll_rn(fma(-Fm[(long long)max(r, col) * n + min(r, col)], scale, r == col ? top : 0.0));
       }
-      x[h][c] = v;
     }
+  }
 
   const long long occ = (long long)mol.nocc * kTraceOne;
   const uint32_t slice = 2u * np * np, sbo = 16u * np;
@@ -463,8 +536,12 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
 }
 
 // ---------------------------------------------------------------------------
-// N > 128: one launch per step over the 128 x 64 tiles of every molecule's
-// upper triangle.  The digit matrices live in global memory (L2) in the layout
+// N > 128: one launch per step over the 128 x TN tiles of every molecule's
+// upper triangle, TN = 64, or 32 where the wider tiles would leave half of the
+// SMs without one (a single molecule below N ~ 900): half the work on a CTA's
+// path for twice the CTAs ((H2O)33: 22.0 -> 17.7 ms, (H2O)101: 55.6 -> 43.6 ms; for
+// 256 (H2O)32, where every SM has wide tiles, narrow ones cost 87 -> 95 ms).  The
+// sums are exact, so the choice changes no bit.  The digit matrices live in global memory (L2) in the layout
 // of the MMA operands, [K chunk of 32][8-row group][4 k-blocks][8 rows][8 k], so a
 // tile's rows of one K chunk are one contiguous bulk copy per digit; two
 // buffers alternate between steps.  They share the eigensolver's scratch
@@ -472,12 +549,12 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
 // Np^2 <= 2 N^2 from N = 79 on).
 // ---------------------------------------------------------------------------
 constexpr int kPurTileThreads = 512;
-constexpr int kTileM = 128, kTileN = 64, kChunkK = 32, kStages = 2;
-constexpr uint32_t kStageA = kTileM * kChunkK * 2, kStageB = kTileN * kChunkK * 2;   // bytes per digit
-constexpr uint32_t kStageBytes = kDigits * (kStageA + kStageB);
+constexpr int kTileM = 128, kChunkK = 32, kStages = 2;
+constexpr uint32_t kStageA = kTileM * kChunkK * 2;        // bytes per digit
+constexpr uint32_t stage_bytes(int tn) { return kDigits * (kStageA + (uint32_t)tn * kChunkK * 2); }
 constexpr int kSegChunks = 16;                            // K = 512: the largest sums, of a digit's squares, stay near 0.7 * 2^22
 constexpr int kXPitch = kTileM + 1;                       // transposed tile, 8-byte elements: no bank conflicts either way
-constexpr size_t kPurTileSmem = kStages * kStageBytes + 256;
+constexpr size_t tile_smem(int tn) { return kStages * stage_bytes(tn) + 256; }
 
 __device__ __forceinline__ unsigned char* pu_plane(const PurScratch& ws, const DevMol& mol, int buf, int d) {
   const int s = buf * kDigits + d;
@@ -574,9 +651,13 @@ __device__ __forceinline__ int pu_first(const long long* T, int k) {
 // One step of the molecules that still need one.  tiles: (molecule, row block,
 // column block, 0).  Warp 0 copies, warp 1 issues the MMAs, all eight
 // recombine.
+template <int TN>
 __global__ void __launch_bounds__(kPurTileThreads, 1)
 purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ tiles, const MolState* __restrict__ st,
                    PurState* __restrict__ pur, PurScratch ws, int k, int* __restrict__ err) {
+  constexpr int kCW = TN / 4, kGroups = kCW / 8;   // columns of a warp, groups of eight of them
+  constexpr uint32_t kStageBytes = stage_bytes(TN);
+  constexpr int kTmem = kLevels * TN;
   extern __shared__ __align__(1024) unsigned char pu_sm[];
   // what no step changes is read while the previous step still runs (programmatic
   // dependent launch); every CTA waits for it before it looks at anything else,
@@ -594,15 +675,15 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   const int op = pu_step(pur[mi].trace[k], pur[mi].trace[k > 0 ? k - 1 : 0], k, pu_first(pur[mi].trace, k), occ);   // the same in every CTA of the molecule
   if (op < 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r0 = tile.y * kTileM, c0 = tile.z * kTileN;
-  const int rows = min(kTileM, np - r0), cols = min(kTileN, np - c0);
+  const int r0 = tile.y * kTileM, c0 = tile.z * TN;
+  const int rows = min(kTileM, np - r0), cols = min(TN, np - c0);
   const int chunks = np / kChunkK;
   unsigned char* tail = pu_sm + kStages * kStageBytes;
   const uint32_t full = pu_smem(tail), empty = full + 8 * kStages, last = empty + 8 * kStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 64);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 :: "r"(pu_smem(tmem_slot)), "r"(512));
+                 :: "r"(pu_smem(tmem_slot)), "r"(kTmem));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
@@ -620,12 +701,12 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   const uint32_t sm = pu_smem(pu_sm);
   const int buf = k & 1;
   const int q = warp & 3, r = r0 + q * 32 + lane;
-  const int cw = (warp >> 2) * 16;   // this warp's columns of the tile: cw .. cw + 15
+  const int cw = (warp >> 2) * kCW;   // this warp's first column of the tile
   const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cw;
-  const int groups = q * 32 < rows ? max(0, min(2, (cols - cw) >> 3)) : 0;   // of eight columns
-  long long v[2][8];
+  const int groups = q * 32 < rows ? max(0, min(kGroups, (cols - cw) >> 3)) : 0;   // of eight columns
+  long long v[kGroups][8];
 #pragma unroll
-  for (int s = 0; s < 2; ++s)
+  for (int s = 0; s < kGroups; ++s)
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[s][i] = 0;
   uint32_t range = 0;
@@ -658,7 +739,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t base = pu_desc_lo(sm + s * kStageBytes);
         const uint32_t bb = base + (kDigits * kStageA >> 4), sb = (uint32_t)cols * kChunkK * 2;
-        if (cols == kTileN)
+        if (TN == 64 && cols == TN)
           pu_products<4, 0, kLevels>(tmem, base, kStageA, bb, sb, pu_desc_hi(512), cols, kChunkK / 16, c == cb);
         else
           pu_products<7, 0, kLevels>(tmem, base, kStageA, bb, sb, pu_desc_hi(512), cols, kChunkK / 16, c == cb);
@@ -672,7 +753,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     ok = __syncthreads_and(ok);
     if (ok) {
 #pragma unroll
-      for (int s = 0; s < 2; ++s)
+      for (int s = 0; s < kGroups; ++s)
         if (s < groups) {
           pu_levels8<0, 4>(taddr + 8 * s, cols, 1, v[s], range);
           pu_levels8<4, 4>(taddr + 4 * cols + 8 * s, cols, 1, v[s], range);
@@ -685,13 +766,13 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     if (tid == 0) atomicExch(err, 1);
   } else {
     // X_{k+1}: row r, the digits of eight columns at a time
-    const bool mirror = tile.z >= 2 * tile.y + 2;   // the transposed block is no tile of its own
+    const bool mirror = tile.z >= (kTileM / TN) * (tile.y + 1);   // the transposed block is no tile of its own
     long long* xt = reinterpret_cast<long long*>(pu_sm);   // the operand stages are free now
     // rows past the padded basis are whatever the stage held before
     if (r < np && !pu_in_range(range)) atomicExch(&pur[mi].bad, 1);
     long long tr = 0;
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kGroups; ++s) {
       if (s >= groups) continue;
       const int cl = cw + 8 * s, c = c0 + cl;
       const size_t at = pu_at(np, r, c);
@@ -732,7 +813,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTmem));
 }
 
 // P = 2 X of the molecules whose iteration ended; the others are flagged
@@ -774,7 +855,7 @@ __global__ void purify_reset_kernel(const int* __restrict__ list, PurState* __re
 
 // ---------------------------------------------------------------------------
 static size_t small_smem(int np) {
-  return (size_t)(kDigits - 1) * 2 * np * np + (size_t)256 * np + 32 + 34 * 8 + 2 * 128 * 8;
+  return (size_t)(kDigits - 1) * 2 * np * np + (size_t)256 * np + 32 + 2 * 128 * 8;
 }
 
 void purify_prepare() {
@@ -783,15 +864,16 @@ void purify_prepare() {
     cudaFuncSetAttribute(purify_small_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(64));
     cudaFuncSetAttribute(purify_small_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(80));
     cudaFuncSetAttribute(purify_small_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(128));
-    cudaFuncSetAttribute(purify_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPurTileSmem);
+    cudaFuncSetAttribute(purify_step_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(64));
+    cudaFuncSetAttribute(purify_step_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(32));
   });
 }
 
-int purify_tiles(int mol, int n, int4* out) {
-  const int np = (n + 31) / 32 * 32, nr = (np + kTileM - 1) / kTileM, nc = (np + kTileN - 1) / kTileN;
+int purify_tiles(int mol, int n, int tn, int4* out) {
+  const int np = (n + 31) / 32 * 32, nr = (np + kTileM - 1) / kTileM, nc = (np + tn - 1) / tn;
   int t = 0;
   for (int i = 0; i < nr; ++i)
-    for (int j = 2 * i; j < nc; ++j, ++t)
+    for (int j = kTileM / tn * i; j < nc; ++j, ++t)
       if (out) out[t] = make_int4(mol, i, j, 0);
   return t;
 }
@@ -808,7 +890,7 @@ void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max
   else purify_small_kernel<2, 2><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
 }
 
-int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles,
+int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles, int tn,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
                       bool alone, int* err, cudaStream_t s) {
   if (nlist <= 0) return 0;
@@ -821,7 +903,7 @@ int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n,
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ntiles);
   cfg.blockDim = dim3(kPurTileThreads);
-  cfg.dynamicSmemBytes = kPurTileSmem;
+  cfg.dynamicSmemBytes = tile_smem(tn);
   cfg.stream = s;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -831,7 +913,7 @@ int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n,
     // CTAs launched ahead hold an SM while they wait: only where no other stream
     // has work for it (a server's burst took 104 ms without and 119 with them)
     cfg.numAttrs = alone && k > 0 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, purify_step_kernel, mols, tiles, (const MolState*)st, pur, ws, k, err);
+    cudaLaunchKernelEx(&cfg, tn == 64 ? purify_step_kernel<64> : purify_step_kernel<32>, mols, tiles, (const MolState*)st, pur, ws, k, err);
   }
   purify_store_kernel<<<dim3(blocks, nlist), 256, 0, s>>>(mols, list, st, pur, ws, steps, P);
   return steps + 4;
