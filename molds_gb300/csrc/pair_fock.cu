@@ -592,7 +592,9 @@ constexpr int kFockStage = 256;   // atoms whose densities are staged at a time 
 // Exchange with B > A: a thread per element of the A-B block.
 // What bounds it: latency and the number of loads in flight (the blocks of one
 // molecule are L2-resident).  A warp per atom, with a lane walking whole 10 x 10
-// blocks, left a single molecule on natoms / 8 CTAs.
+// blocks, left a single molecule on natoms / 8 CTAs.  Staging where each partner's
+// block lies takes a dependent load off every one of them: 650 -> 568 us a build
+// for 256 (H2O)32.
 __global__ void __launch_bounds__(kFockAtomThreads)
 fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, const DevMol* __restrict__ mols,
             const int* __restrict__ mol_list, const double* __restrict__ blocks, const double* __restrict__ H,
@@ -601,6 +603,8 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   __shared__ double s_p[kFockStage * 10];
   __shared__ double s_red[kFockAtomThreads];
   __shared__ short s_list[kFockStage];
+  __shared__ int s_ao[kFockStage];          // 2 * first orbital + (sp atom)
+  __shared__ long long s_blk[kFockStage];
   __shared__ int s_n[4];
   const int m = mol_list[blockIdx.y], ia = blockIdx.x;
   const DevMol mol = mols[m];
@@ -629,6 +633,14 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   for (int b0 = 0; b0 < mol.natoms; b0 += kFockStage) {
     const int nb = min(kFockStage, mol.natoms - b0);
     __syncthreads();
+    // where each partner's orbitals and block are: one round of loads here instead
+    // of a dependent one before every block
+    for (int i = tid; i < nb; i += kFockAtomThreads) {
+      const int ib = b0 + i;
+      s_ao[i] = am[ib].ao0 * 2 + (am[ib].nao == 4 ? 1 : 0);
+      if (ib != ia) s_blk[i] = pairs[mol.pair0 + pair_index(min(ia, ib), max(ia, ib), mol.natoms)].blk;
+    }
+    __syncthreads();
     // heavy atoms first in the list, hydrogens from its end: a warp then works
     // on one kind, and the FP64 pipe, which takes 64 clocks a warp instruction,
     // is not spent on lanes that sit out
@@ -636,7 +648,7 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
       int h = 0, l = 0, h0 = 0, l0 = 0;
       for (int base = 0; base < nb; base += 32) {
         const int i = base + tid;
-        const bool in = i < nb, heavy = in && am[b0 + i].nao == 4;
+        const bool in = i < nb, heavy = in && (s_ao[i] & 1);
         const unsigned mh = __ballot_sync(0xffffffffu, heavy), ml = __ballot_sync(0xffffffffu, in && !heavy);
         const unsigned below = (1u << tid) - 1u;
         if (heavy) s_list[h + __popc(mh & below)] = (short)i;
@@ -651,11 +663,11 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
     }
     if (mode == 0)
       for (int e = tid; e < nb * 10; e += kFockAtomThreads) {
-        const DevAtom& B = am[b0 + e / 10];
+        const int ao = s_ao[e / 10], o = ao >> 1;
         int l, sg;
         unpack_index(e % 10, &l, &sg);
         double v = 0.0;
-        if (B.nao == 4 || e % 10 == 0) v = Pm[(B.ao0 + l) * ld + B.ao0 + sg] * (l == sg ? 1.0 : 2.0);
+        if ((ao & 1) || e % 10 == 0) v = Pm[(o + l) * ld + o + sg] * (l == sg ? 1.0 : 2.0);
         s_p[e] = v;
       }
     __syncthreads();
@@ -664,9 +676,8 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
       for (int t = j0; t < nh; t += per) {
         const int i = s_list[t], ib = b0 + i;
         if (ib == ia) continue;
-        bool rows;
-        const double* blk = partner_block(pairs, blocks, mol, ia, ib, &rows);
-        const double* x = rows ? blk + k * 10 : blk + k;
+        const bool rows = ia < ib;
+        const double* x = blocks + s_blk[i] + (rows ? k * 10 : k);
         const int step = rows ? 1 : dA;
         double v = 0.0;
 #pragma unroll
@@ -676,18 +687,17 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
       for (int t = j0; t < nl; t += per) {
         const int i = s_list[kFockStage - 1 - t], ib = b0 + i;
         if (ib == ia) continue;
-        bool rows;
-        acc += partner_block(pairs, blocks, mol, ia, ib, &rows)[k] * s_p[i * 10];
+        acc += blocks[s_blk[i] + k] * s_p[i * 10];
       }
     }
     // two-centre blocks (A, B > A): resonance + exchange -1/2 sum P_nu,si (mu nu|la si);
     // a thread per (B, mu, la)
     const int sh = nA == 4 ? 4 : 2;
     for (int t = h0 + (tid >> sh); t < nh; t += kFockAtomThreads >> sh) {
-      const int ib = b0 + s_list[t], fb = am[ib].ao0, mu = (tid >> 2) & (nA - 1), la = tid & 3;
+      const int i = s_list[t], fb = s_ao[i] >> 1, mu = (tid >> 2) & (nA - 1), la = tid & 3;
       double v = Hm[(fa + mu) * ld + fb + la];
       if (mode == 0) {
-        const double* blk = blocks + pairs[mol.pair0 + pair_index(ia, ib, mol.natoms)].blk;
+        const double* blk = blocks + s_blk[i];
         const double* Pab = Pm + fa * ld + fb;
         double x = 0.0;
         if (nA == 4) {
@@ -708,10 +718,10 @@ fock_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
     }
     const int sl = nA == 4 ? 2 : 0;
     for (int t = l0 + (tid >> sl); t < nl; t += kFockAtomThreads >> sl) {
-      const int ib = b0 + s_list[kFockStage - 1 - t], fb = am[ib].ao0, mu = tid & (nA - 1);
+      const int i = s_list[kFockStage - 1 - t], fb = s_ao[i] >> 1, mu = tid & (nA - 1);
       double v = Hm[(fa + mu) * ld + fb];
       if (mode == 0) {
-        const double* blk = blocks + pairs[mol.pair0 + pair_index(ia, ib, mol.natoms)].blk;
+        const double* blk = blocks + s_blk[i];
         const double* Pab = Pm + fa * ld + fb;
         double x = 0.0;
         for (int n = 0; n < nA; ++n) x += Pab[n * ld] * blk[pack_lut(mu, n)];
@@ -1107,7 +1117,7 @@ __device__ __forceinline__ void shell_contract_warp(const double* ra, const doub
 // molecule's result does not depend on the batch it runs in.
 __host__ __device__ __forceinline__ int dipole_chunks(int natoms) {
   const long long items = (long long)natoms + (long long)natoms * (natoms - 1) / 2;
-  const long long c = (items + 4LL * (kDipThreads / 32) - 1) / (4LL * (kDipThreads / 32));
+  const long long c = (items + 4LL * (kDipThreads / 32) - 1) / (4LL * (kDipThreads / 32));   // four items a warp
   return (int)(c < 1 ? 1 : (c > kDipChunks ? kDipChunks : c));
 }
 
@@ -1207,44 +1217,64 @@ dipole_partial_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restri
   }
 }
 
-// One thread per molecule: chunk sums in a fixed order, the centre of core
+// Sums over a CTA of kFinishThreads, the result in every thread
+constexpr int kFinishThreads = 128;
+__device__ __forceinline__ double finish_sum(double v, double* red) {
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  for (int w = 0; w < kFinishThreads / 32; ++w) t += red[w];
+  return t;
+}
+
+// One CTA per molecule: chunk sums in a fixed order, the centre of core
 // mass (src/base/Molecule.cpp:396-419), the core dipole and the electronic
-// dipole; MolState::dipole = total, electronic, core (x, y, z each).
-__global__ void dipole_finish_kernel(const DevAtom* __restrict__ atoms, const DevMol* __restrict__ mols,
-                                     const int* __restrict__ mol_list, int nlist, int grid_chunks,
-                                     const double* __restrict__ partial, MolState* __restrict__ st) {
-  const int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= nlist) return;
-  const int m = mol_list[li];
+// dipole; MolState::dipole = total, electronic, core (x, y, z each).  (A thread
+// per molecule walked its atoms twice: 270 us for (H2O)180.)
+__global__ void __launch_bounds__(kFinishThreads)
+dipole_finish_kernel(const DevAtom* __restrict__ atoms, const DevMol* __restrict__ mols,
+                     const int* __restrict__ mol_list, int grid_chunks, const double* __restrict__ partial,
+                     MolState* __restrict__ st) {
+  __shared__ double red[kFinishThreads / 32];
+  const int li = blockIdx.x, m = mol_list[li], tid = threadIdx.x;
   const DevMol mol = mols[m];
   const int chunks = dipole_chunks(mol.natoms);
-  double sum[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int c = 0; c < chunks; ++c)
-    for (int q = 0; q < 4; ++q) sum[q] += partial[((long long)li * grid_chunks + c) * 4 + q];
-  double center[3] = {0.0, 0.0, 0.0}, mass = 0.0;
-  for (int a = 0; a < mol.natoms; ++a) {
+  double v[12];
+#pragma unroll
+  for (int q = 0; q < 12; ++q) v[q] = 0.0;
+  for (int c = tid; c < chunks; c += kFinishThreads)
+    for (int q = 0; q < 4; ++q) v[q] += partial[((long long)li * grid_chunks + c) * 4 + q];
+  for (int a = tid; a < mol.natoms; a += kFinishThreads) {
     const DevAtom A = atoms[mol.atom0 + a];
     const double cm = c_params[A.pidx].core_mass;
-    mass += cm;
-    center[0] += A.x * cm;
-    center[1] += A.y * cm;
-    center[2] += A.z * cm;
+    v[4] += cm;
+    v[5] += A.x * cm;
+    v[6] += A.y * cm;
+    v[7] += A.z * cm;
   }
-  for (int k = 0; k < 3; ++k) center[k] /= mass;
-  double core[3] = {0.0, 0.0, 0.0};
-  for (int a = 0; a < mol.natoms; ++a) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = finish_sum(v[q], red);
+  const double center[3] = {v[5] / v[4], v[6] / v[4], v[7] / v[4]};
+  for (int a = tid; a < mol.natoms; a += kFinishThreads) {
     const DevAtom A = atoms[mol.atom0 + a];
     const double z = c_params[A.pidx].core_charge;
-    core[0] += z * (A.x - center[0]);
-    core[1] += z * (A.y - center[1]);
-    core[2] += z * (A.z - center[2]);
+    v[8] += z * (A.x - center[0]);
+    v[9] += z * (A.y - center[1]);
+    v[10] += z * (A.z - center[2]);
   }
-  MolState* s = st + m;
-  for (int k = 0; k < 3; ++k) {
-    const double elec = -sum[k] + center[k] * sum[3];
-    s->dipole[k] = elec + core[k];
-    s->dipole[3 + k] = elec;
-    s->dipole[6 + k] = core[k];
+#pragma unroll
+  for (int q = 8; q < 11; ++q) v[q] = finish_sum(v[q], red);
+  if (tid == 0) {
+    MolState* s = st + m;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double elec = -v[k] + center[k] * v[3];
+      s->dipole[k] = elec + v[8 + k];
+      s->dipole[3 + k] = elec;
+      s->dipole[6 + k] = v[8 + k];
+    }
   }
 }
 
@@ -1253,7 +1283,7 @@ void launch_dipole(const DevAtom* atoms, const DevPair* pairs, const DevMol* mol
   if (nlist <= 0) return;
   const int chunks = dipole_chunks(max_atoms);   // the largest molecule's count sets the grid
   dipole_partial_kernel<<<dim3(chunks, nlist), kDipThreads, 0, s>>>(atoms, pairs, mols, mol_list, P, H, partial);
-  dipole_finish_kernel<<<(nlist + 127) / 128, 128, 0, s>>>(atoms, mols, mol_list, nlist, chunks, partial, st);
+  dipole_finish_kernel<<<nlist, kFinishThreads, 0, s>>>(atoms, mols, mol_list, chunks, partial, st);
 }
 
 // X[k][mu][nu] of molecule m (3 x N x N doubles, row-major), both triangles:

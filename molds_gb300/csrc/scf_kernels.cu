@@ -267,7 +267,7 @@ __device__ void diis_decide(MolState* s, const ScfParamsDev& prm, long long n2, 
   }
 }
 
-__global__ void __launch_bounds__(kDiisThreads)
+__global__ void __launch_bounds__(kDiisThreads, 3)
 diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_list, MolState* __restrict__ st,
                     ScfParamsDev prm, const double* __restrict__ P, const double* __restrict__ Pold,
                     double* __restrict__ hist_dens, double* __restrict__ hist_err, long long hist_stride,
@@ -302,17 +302,39 @@ diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol
   double v[kDiisPart];
 #pragma unroll
   for (int k = 0; k < kDiisPart; ++k) v[k] = 0.0;
-  for (long long i = lo + tid; i < hi; i += kDiisThreads) {
-    const double p = Pm[i];
-    const double e = p - Po[i];
-    v[0] += e * e;
-    v[1] = fmax(v[1], fabs(e));
+  // two elements' loads before the first store: the history is read and written
+  // through one pointer, so the compiler keeps their order
+  constexpr int kU = 2;
+  for (long long i0 = lo + tid; i0 < hi; i0 += kU * kDiisThreads) {
+    double p[kU], e[kU], x[kMaxDiis][kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const long long i = i0 + u * kDiisThreads;
+      p[u] = i < hi ? Pm[i] : 0.0;
+      e[u] = i < hi ? p[u] - Po[i] : 0.0;
+    }
     if (do_diis) {
-      dslot[i] = p;
-      eslot[i] = e;
 #pragma unroll
       for (int k = 0; k < kMaxDiis; ++k)
-        if (k < count) v[2 + k] += (k == slot ? e : hist_err[k * hist_stride + mol.mat0 + i]) * e;
+        if (k < count && k != slot)
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const long long i = i0 + u * kDiisThreads;
+            x[k][u] = i < hi ? hist_err[k * hist_stride + mol.mat0 + i] : 0.0;
+          }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const long long i = i0 + u * kDiisThreads;
+      v[0] += e[u] * e[u];
+      v[1] = fmax(v[1], fabs(e[u]));
+      if (do_diis && i < hi) {
+        dslot[i] = p[u];
+        eslot[i] = e[u];
+#pragma unroll
+        for (int k = 0; k < kMaxDiis; ++k)
+          if (k < count) v[2 + k] += (k == slot ? e[u] : x[k][u]) * e[u];
+      }
     }
   }
 #pragma unroll
