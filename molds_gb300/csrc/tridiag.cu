@@ -23,6 +23,8 @@
 //                       triangle in shared memory (or a global workspace for
 //                       large N); reflector j goes to row j of W, d / e / tau
 //                       to the tridiagonal arena
+//   hh_tridiag_cluster_kernel   the same by eight CTAs, matrix spread over their
+//                       shared memories, for short lists of larger bases
 //   tri_vectors_kernel  one thread per wanted index: the eigenvalue of T by
 //                       bisection on a division-free Sturm sequence, then two
 //                       steps of inverse iteration with a partial-pivoting LU of
@@ -33,6 +35,7 @@
 //   hh_back_kernel      X = Q Z, 32 columns per CTA, reflectors applied in
 //                       reverse order; X written as rows of C (sign-fixed in the
 //                       final pass)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <mutex>
@@ -44,6 +47,10 @@
 namespace nddo {
 
 constexpr int kHhMaxThreads = 1024;   // the CTA size comes from the tuning table (256, 512 or 1024)
+constexpr int kHhCluster = 8, kHhClusterThreads = 512;   // cluster kernel: CTAs per molecule, threads per CTA
+constexpr int kHhClusterMinN = 195;   // its smallest basis, one more than an edge of the engine's size buckets
+constexpr int kHhClusterWaveN = 100;  // basis functions that pay for a wave of clusters, see the launcher
+constexpr int kHhRowShift = 3;        // log2 of the lanes that share a row's product there
 constexpr int kVecThreads = 32;   // one warp: 16 lane pairs, 16 eigenpairs per CTA
 constexpr int kOrthThreads = 256;
 constexpr size_t kOrthStaticSmem = (1024 + kOrthThreads / 32 + 1) * sizeof(double) + 1024;   // and some slack
@@ -80,13 +87,13 @@ template <bool kSmem>
 __global__ void __launch_bounds__(kHhMaxThreads)
 hh_tridiag_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, const MolState* __restrict__ st,
                   int require_active, const double* __restrict__ F, double* __restrict__ W, double* __restrict__ td,
-                  long long vstride, double* __restrict__ Aws, int max_n_served) {
+                  long long vstride, double* __restrict__ Aws, int min_n, int max_n_served) {
   extern __shared__ __align__(16) double hsm[];
   const int mi = list[blockIdx.x];
   if (mol_skipped(st[mi], require_active)) return;
   const DevMol mol = mols[mi];
   const int n = mol.nao;
-  if (n > max_n_served) return;   // served by the whole-GPU kernel (tridiag_grid.cu)
+  if (n < min_n || n > max_n_served) return;   // served by the cluster or the whole-GPU kernel
   const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarps = nth >> 5;
   double* A = kSmem ? hsm : Aws + mol.mat0;
   double* v = kSmem ? hsm + (long long)n * (n + 1) / 2 : hsm;
@@ -137,8 +144,11 @@ hh_tridiag_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list,
     const double tau = sc[k & 1];
     if (tau == 0.0) continue;   // uniform: H = I, nothing to update
     // p = tau A22 v: a group of g lanes per row (g a power of two, g * rows <= threads)
-    int gsh = 0;
-    while (gsh < 5 && (m << (gsh + 1)) <= nth) ++gsh;
+    // or eight for the bases that the cluster kernel may serve: the same sums there
+    // (152 molecules: N = 234 3.34 -> 3.48 ms, 300 7.7 -> 7.3, 396 19.1 -> 16.1)
+    int gsh = n >= kHhClusterMinN ? kHhRowShift : 0;
+    if (n < kHhClusterMinN)
+      while (gsh < 5 && (m << (gsh + 1)) <= nth) ++gsh;
     const int g = 1 << gsh, ngrp = nth >> gsh, grp = tid >> gsh, gl = tid & (g - 1);
     for (int i0 = 0; i0 < m; i0 += ngrp) {
       const int i = i0 + grp;
@@ -188,6 +198,187 @@ hh_tridiag_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list,
     ee[n - 1] = 0.0;
     tt[n - 1] = 0.0;
   }
+}
+
+// ---------------------------------------------------------------------------
+// The same reduction by a cluster of eight CTAs per molecule, for lists of few
+// bases that leave a one-CTA kernel alone on its SM.  The full square matrix is
+// spread over the CTAs' shared memories, row i with CTA i mod 8, and updated as in
+// the whole-GPU kernel (tridiag_grid.cu): one cluster barrier per column; after it
+// every CTA holds p_k, forms w_k, reads the next column from its owner and forms
+// reflector k + 1 itself (four warps; an FP64 instruction of a warp takes the SM 16
+// clocks, so vector work is not given to more), then eight lanes a row update its
+// rows and send their entries of p_{k+1} to all eight.  Both triangles use the
+// lower-triangle formula, so A stays exactly symmetric, and every sum has the terms
+// and the order it has in the one-CTA kernel: the two give the same bits, so the
+// choice may follow the list.
+// Why: one SM's two FMAs per clock bound the one-CTA kernel, (2/3) N^3 of them;
+// eight issue N^3 between them.  ms, one CTA -> cluster: N = 180 1.83 -> 0.99, 234
+// 3.5 -> 1.5, 300 7.3 -> 2.3, 396 16 -> 3.9 (half of it the FP64 pipe, the rest the
+// chain of barriers and reductions of a column).
+// ---------------------------------------------------------------------------
+
+// row pitch = 4 mod 16 doubles: the four rows of a warp lie in different banks
+__host__ __device__ inline int hh_cluster_pitch(int n) { return ((n + 11) & ~15) + 4; }
+size_t hh_cluster_smem_bytes(int n) {
+  return ((size_t)((n + kHhCluster - 1) / kHhCluster) * hh_cluster_pitch(n) + 5 * (size_t)n + 4) * sizeof(double);
+}
+
+__global__ void __cluster_dims__(kHhCluster, 1, 1) __launch_bounds__(kHhClusterThreads, 1)
+hh_tridiag_cluster_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list,
+                          const MolState* __restrict__ st, int require_active, const double* __restrict__ F,
+                          double* __restrict__ W, double* __restrict__ td, long long vstride, int max_n_served) {
+  extern __shared__ __align__(16) double hsm[];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int mi = list[blockIdx.x / kHhCluster];
+  if (mol_skipped(st[mi], require_active)) return;
+  const DevMol mol = mols[mi];
+  const int n = mol.nao;
+  if (n < kHhClusterMinN || n > max_n_served) return;
+  const int rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kVec = 128;                                    // threads that do vector work
+  constexpr int kG = 1 << kHhRowShift, kGroups = kHhClusterThreads >> kHhRowShift;
+  const int grp = tid >> kHhRowShift, gl = tid & (kG - 1);
+  const int ld = hh_cluster_pitch(n);
+  double* A = hsm;                                             // row i of this CTA at (i / 8) ld
+  double* p = A + (size_t)((n + kHhCluster - 1) / kHhCluster) * ld;   // p of two consecutive steps
+  double* v = p + 2 * n;
+  double* w = v + n;
+  double* vn = w + n;
+  double* sc = vn + n;                                         // 0: c, 1: scale, 2: beta, 3: tau
+  const double* Fm = F + mol.mat0;
+  double* Wm = W + mol.mat0;
+  double* dd = td + mol.vec0;
+  double* ee = dd + vstride;
+  double* tt = ee + vstride;
+  auto bar = [] { asm volatile("bar.sync 1, %0;" :: "n"(kVec) : "memory"); };
+  // reflector of x[j0 .. n) (LAPACK dlarfg), x[j0] = 1 on return; by the first
+  // kVec threads, the sum by one warp as in the one-CTA kernel
+  auto house = [&](double* x, int j0) {
+    bar();
+    if (warp == 0) {
+      double s = 0.0;
+      for (int j = j0 + 1 + lane; j < n; j += 32) s = fma(x[j], x[j], s);
+      s = warp_sum_d(s);
+      if (lane == 0) {
+        const double alpha = x[j0];
+        double tau = 0.0, beta = alpha, scal = 0.0;
+        if (s != 0.0) {
+          const double nrm = sqrt(fma(alpha, alpha, s));
+          beta = alpha >= 0.0 ? -nrm : nrm;
+          tau = (beta - alpha) / beta;
+          scal = 1.0 / (alpha - beta);
+        }
+        sc[1] = scal;
+        sc[2] = beta;
+        sc[3] = tau;
+        x[j0] = 1.0;
+      }
+    }
+    bar();
+    const double scal = sc[1];
+    for (int j = j0 + 1 + tid; j < n; j += kVec) x[j] *= scal;
+  };
+  for (int i = rank + kHhCluster * warp; i < n; i += kHhCluster * (kHhClusterThreads / 32))
+    for (int j = lane; j < n; j += 32) A[(size_t)(i / kHhCluster) * ld + j] = Fm[i >= j ? (long long)i * n + j : (long long)j * n + i];
+  if (tid < kVec) {
+    for (int j = 1 + tid; j < n; j += kVec) v[j] = Fm[(long long)j * n];
+    house(v, 1);
+  }
+  cluster.sync();   // also: all eight run before any sends to another
+  double tau = sc[3];
+  if (rank == 0) {
+    if (tid == 0) { dd[0] = Fm[0]; ee[0] = sc[2]; tt[0] = tau; }
+    for (int j = 1 + tid; j < n; j += kHhClusterThreads) Wm[j] = v[j];
+  }
+  // rows of p go to every CTA, lane l of the row's group sending to CTA l
+  static_assert(kG == kHhCluster, "a lane of the group per CTA");
+  for (int i0 = rank; i0 < n; i0 += kHhCluster * kGroups) {
+    const int i = i0 + kHhCluster * grp;
+    double s = 0.0;
+    if (i >= 1 && i < n) {
+      const double* ar = A + (size_t)(i / kHhCluster) * ld;
+      for (int j = 1 + gl; j < n; j += kG) s = fma(ar[j], v[j], s);
+    }
+#pragma unroll
+    for (int o = kG >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (i >= 1 && i < n) cluster.map_shared_rank(p, gl)[i] = tau * s;
+  }
+  cluster.sync();
+  for (int k = 0; k + 2 < n; ++k) {
+    const double* pk = p + (k & 1) * n;
+    double* pn = p + ((k & 1) ^ 1) * n;
+    const int rr = k + 1;
+    const double* arow = cluster.map_shared_rank(A, rr % kHhCluster) + (size_t)(rr / kHhCluster) * ld;
+    if (tid < kVec) {
+      if (warp == 0) {
+        double s = 0.0;
+        for (int j = rr + lane; j < n; j += 32) s = fma(pk[j], v[j], s);
+        s = warp_sum_d(s);
+        if (lane == 0) sc[0] = 0.5 * tau * s;
+      }
+      bar();
+      const double c = sc[0], vr = v[rr], wr = fma(-c, vr, pk[rr]);
+      for (int j = rr + tid; j < n; j += kVec) {
+        const double vj = v[j], wj = fma(-c, vj, pk[j]);
+        w[j] = wj;
+        // column rr after update k: row rr, which its owner leaves alone from now on
+        if (j > rr && k + 3 < n) vn[j] = fma(-vj, wr, fma(-wj, vr, arow[j]));
+      }
+      if (k + 3 < n) house(vn, rr + 1);
+    }
+    __syncthreads();
+    const double vr = v[rr], wr = w[rr];
+    if (k + 3 >= n) {
+      // k = n - 3: the trailing 2 x 2 block after the last update
+      if (rank == 0 && tid == 0) {
+        const int q = n - 1;
+        const double* aq = cluster.map_shared_rank(A, q % kHhCluster) + (size_t)(q / kHhCluster) * ld;
+        const double vq = v[q], wq = w[q];
+        dd[rr] = fma(-vr, wr, fma(-wr, vr, arow[rr]));
+        ee[rr] = fma(-vq, wr, fma(-wq, vr, arow[q]));
+        tt[rr] = 0.0;
+        dd[q] = fma(-vq, wq, fma(-wq, vq, aq[q]));
+        ee[q] = 0.0;
+        tt[q] = 0.0;
+      }
+      break;
+    }
+    const double taun = sc[3];
+    if (rank == 0) {
+      if (tid == 0) { dd[rr] = fma(-vr, wr, fma(-wr, vr, arow[rr])); ee[rr] = sc[2]; tt[rr] = taun; }
+      for (int j = rr + 1 + tid; j < n; j += kHhClusterThreads) Wm[(long long)rr * n + j] = vn[j];
+    }
+    // own rows i >= k + 2: A <- A - v w^T - w v^T, then p_{k+1} = tau A v_{k+1}
+    const int first = k + 2 + ((rank - (k + 2)) & (kHhCluster - 1));
+    for (int i0 = first; i0 < n; i0 += kHhCluster * kGroups) {
+      const int i = i0 + kHhCluster * grp;
+      double s = 0.0;
+      if (i < n) {
+        double* ar = A + (size_t)(i / kHhCluster) * ld;
+        const double vi = v[i], wi = w[i];
+        for (int j = k + 2 + gl; j < n; j += kG) {
+          const double vj = v[j], wj = w[j];
+          const bool low = i >= j;   // (big index, small index) of the lower-triangle formula
+          const double vb = low ? vi : vj, wb = low ? wi : wj, vs = low ? vj : vi, ws = low ? wj : wi;
+          const double a = fma(-vb, ws, fma(-wb, vs, ar[j]));
+          ar[j] = a;
+          s = fma(a, vn[j], s);
+        }
+      }
+#pragma unroll
+      for (int o = kG >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (i < n) cluster.map_shared_rank(pn, gl)[i] = taun * s;
+    }
+    double* t = v;
+    v = vn;
+    vn = t;
+    tau = taun;
+    cluster.sync();
+  }
+  cluster.sync();   // no CTA leaves while another may read its rows
 }
 
 // ---------------------------------------------------------------------------
@@ -982,6 +1173,7 @@ static void hh_set_attributes() {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncSetAttribute(hh_tridiag_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    cudaFuncSetAttribute(hh_tridiag_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     cudaFuncSetAttribute(hh_tridiag_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     cudaFuncSetAttribute(hh_back_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     cudaFuncSetAttribute(hh_back_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -1014,6 +1206,39 @@ size_t hh_back_smem_bytes(int n) {
   return ((size_t)n * (kBackCols + 1) + 2 * kBackWarps * kBackCols + 2 * kBackCols + 3 * n) * sizeof(double);
 }
 
+int hh_cluster_max_n() {
+  static int nmax = 0;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    int n = 8;
+    while (hh_cluster_smem_bytes(n + 1) <= (size_t)hh_optin_smem()) ++n;
+    nmax = n;
+  });
+  return nmax;
+}
+
+// clusters that the GPU holds at once (their CTAs take an SM each)
+static int hh_clusters() {
+  static int count = 1;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kHhCluster * 64);
+    cfg.blockDim = dim3(kHhClusterThreads);
+    cfg.dynamicSmemBytes = hh_cluster_smem_bytes(hh_cluster_max_n());
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kHhCluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int c = 0;
+    if (cudaOccupancyMaxActiveClusters(&c, hh_tridiag_cluster_kernel, &cfg) == cudaSuccess && c > 0) count = c;
+    else (void)cudaGetLastError();
+  });
+  return count;
+}
+
 int hh_back_max_n() {
   static int nmax = 0;
   static std::once_flag once;
@@ -1029,6 +1254,7 @@ void hh_prepare() {
   hh_set_attributes();
   hh_smem_max_n();
   hh_back_max_n();
+  hh_clusters();
 }
 
 void launch_hh_tridiag(const DevMol* mols, const int* list, int nlist, int max_n, const MolState* st,
@@ -1036,15 +1262,27 @@ void launch_hh_tridiag(const DevMol* mols, const int* list, int nlist, int max_n
                        int max_n_served, cudaStream_t s) {
   if (nlist <= 0 || max_n <= 0) return;
   hh_set_attributes();
+  // A cluster has an SM for each CTA, so 15 or so run at a time; a wave of them has
+  // to cost less than its share of the one-CTA kernel, whose time grows as N^3 while
+  // its SMs hold up to 152 molecules: two waves at N = 234 2.9 ms against 3.5, three
+  // at 300 6.8 against 7.3, three at 396 11.7 against 16; two at 180 2.0 against 1.8.
+  int lo_n = 0;
+  const int cap = std::min(max_n, hh_cluster_max_n()), waves = (nlist + hh_clusters() - 1) / hh_clusters();
+  if (max_n >= kHhClusterMinN && waves * kHhClusterWaveN <= cap) {
+    hh_tridiag_cluster_kernel<<<kHhCluster * nlist, kHhClusterThreads, hh_cluster_smem_bytes(cap), s>>>(
+        mols, list, st, require_active, F, W, td, vstride, std::min(cap, max_n_served));
+    if (max_n <= cap) return;
+    lo_n = cap + 1;
+  }
   const bool smem = max_n <= hh_smem_max_n();
   const size_t sh = hh_tridiag_smem_bytes(max_n, smem);
   const int threads = tuned_tridiag_threads(max_n);
   if (smem)
     hh_tridiag_kernel<true><<<nlist, threads, sh, s>>>(mols, list, st, require_active, F, W, td, vstride, Aws,
-                                                       max_n_served);
+                                                       lo_n, max_n_served);
   else
     hh_tridiag_kernel<false><<<nlist, threads, sh, s>>>(mols, list, st, require_active, F, W, td, vstride, Aws,
-                                                        max_n_served);
+                                                        lo_n, max_n_served);
 }
 
 void launch_tri_vectors(const DevMol* mols, const int* list, int nlist, int max_n, int max_k, const MolState* st,
