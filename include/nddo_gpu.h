@@ -35,9 +35,11 @@ enum {
   NDDO_THEORY_PM3PDDG = 5
 };
 enum { NDDO_PRECISION_FP64 = 0, NDDO_PRECISION_MIXED = 1 };
-/* FP64 eigensolver of the SCF (Lapack::Dsyevd's stand-in): AUTO and
- * HOUSEHOLDER = Householder tridiagonalisation + bisection + inverse
- * iteration; JACOBI = the warm-started cyclic Jacobi. */
+/* Eigensolve of the SCF (Lapack::Dsyevd's stand-in): AUTO = the density by
+ * spectral purification in every iteration and the eigenpairs as HOUSEHOLDER
+ * forms them once at the end (and in any iteration whose purification fails);
+ * HOUSEHOLDER = Householder tridiagonalisation + bisection + inverse iteration
+ * in every iteration; JACOBI = the warm-started cyclic Jacobi. */
 enum { NDDO_EIGEN_AUTO = 0, NDDO_EIGEN_JACOBI = 1, NDDO_EIGEN_HOUSEHOLDER = 2 };
 enum {
   NDDO_OK = 0,

@@ -2,7 +2,7 @@
 //
 // (a) pair_kernel -- one warp per atom pair of every molecule in the batch.
 //     Evaluates the distinct diatomic-frame two-centre integrals from the term
-//     table (lane = local integral), rotates the packed 10x10 block to the
+//     table (a lane per term, then a lane per local integral sums its own), rotates the packed 10x10 block to the
 //     molecular frame as T2 L T2^T (T2 = symmetrised product rotation), and
 //     stores it with coalesced lane-strided stores.  The same warp computes the
 //     Slater overlap of the pair (diatomic frame, then rotated), the resonance
@@ -14,11 +14,11 @@
 //     4030-4146), Mndo::GetDiatomCoreRepulsionEnergy (:319-327, :223-240) and
 //     Am1::GetDiatomCoreRepulsionEnergy (src/am1/Am1.cpp:145-170).
 //
-// (b) hcore_kernel / fock_kernel -- one CTA per molecule, one warp per atom.
-//     Coulomb terms of the diagonal block of atom A are gathered from all
-//     partner blocks by the lanes and reduced with a fixed shuffle tree, so the
-//     result does not depend on scheduling (bitwise reproducible, alone or in a
-//     batch).  Exchange blocks are written by the lane that owns the pair.
+// (b) hcore_kernel / fock_kernel -- one CTA per atom.  Coulomb terms of the
+//     diagonal block of atom A are gathered from all partner blocks, a thread per
+//     partner and orbital pair, and summed in a fixed order, so the result does
+//     not depend on scheduling (bitwise reproducible, alone or in a batch).  The
+//     exchange block of a pair is written by the CTA of its first atom.
 //     MolDS: Cndo2::CalcFockMatrix (src/cndo/Cndo2.cpp:1526-1636) with
 //     Mndo::GetFockDiagElement (src/mndo/Mndo.cpp:422-488), GetFockOffDiagElement
 //     (:490-580), GetCoulombInt/GetExchangeInt (:583-639), GetElectronCoreAttraction
