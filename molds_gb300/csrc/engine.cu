@@ -643,15 +643,23 @@ void Batch::build_jobs(const std::vector<int>& which) {
     pur_list_[k].push_back(m);
     pur_max_n_[k] = std::max(pur_max_n_[k], n);
   }
-  // wide tiles, or narrow ones while those still find an SM each
+  // Wide tiles, or narrow ones while those still find an SM each, or one of half
+  // the SMs where other streams run beside this one.  A tile's time goes with its
+  // basis and a step ends with the largest, so tiles count by their share of that:
+  // 16 alike molecules a stream are throughput (64 (H2O)27 in four groups 43 ms with
+  // wide tiles, 52 with narrow), uneven ones the largest's latency (97 molecules
+  // 80 and 77 ms, a burst of 60 requests 86 and 77).
   for (pur_tn_ = 32; pur_tn_ <= 64; pur_tn_ *= 2) {
     pur_tiles_.clear();
+    long long work = 0;
     for (int m : pur_list_[2]) {
       const size_t t = pur_tiles_.size();
       pur_tiles_.resize(t + purify_tiles(m, h_mols[m].nao, pur_tn_, nullptr));
       purify_tiles(m, h_mols[m].nao, pur_tn_, pur_tiles_.data() + t);
+      work += (long long)(pur_tiles_.size() - t) * h_mols[m].nao;
     }
-    if ((int)pur_tiles_.size() <= grid_ctas_ || pur_tn_ == 64) break;
+    if (pur_tn_ == 64 || ((int)pur_tiles_.size() <= grid_ctas_ &&
+                          work * (alone_ ? 1 : 2) <= (long long)grid_ctas_ * pur_max_n_[2])) break;
   }
   if (pur_tiles_.size() > pur_tile_cap_) throw std::logic_error("purification tile table overflow");
   // chunks of at most grid_ctas_ molecules and their CTA maps

@@ -538,10 +538,11 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
 // ---------------------------------------------------------------------------
 // N > 128: one launch per step over the 128 x TN tiles of every molecule's
 // upper triangle, TN = 64, or 32 where the wider tiles would leave half of the
-// SMs without one (a single molecule below N ~ 900): half the work on a CTA's
-// path for twice the CTAs ((H2O)33: 22.0 -> 17.7 ms, (H2O)101: 55.6 -> 43.6 ms; for
-// 256 (H2O)32, where every SM has wide tiles, narrow ones cost 87 -> 95 ms).  The
-// sums are exact, so the choice changes no bit.  The digit matrices live in global memory (L2) in the layout
+// SMs without one (a single molecule below N ~ 900, see Batch::build_jobs): half
+// the work on a CTA's path for twice the CTAs ((H2O)33: 22.0 -> 17.7 ms, (H2O)101:
+// 55.6 -> 43.6 ms; for 256 (H2O)32, where every SM has wide tiles, narrow ones cost
+// 87 -> 95 ms).  The sums are exact, so the choice changes no bit.  The digit
+// matrices live in global memory (L2) in the layout
 // of the MMA operands, [K chunk of 32][8-row group][4 k-blocks][8 rows][8 k], so a
 // tile's rows of one K chunk are one contiguous bulk copy per digit; two
 // buffers alternate between steps.  They share the eigensolver's scratch

@@ -101,3 +101,18 @@ def test_mixed_batch_of_gapped_and_degenerate(ctx):
     assert alone[0]["status"] == M.STATUS_CONVERGED
     assert both[0]["energy"] == alone[0]["energy"] and both[0]["iterations"] == alone[0]["iterations"]
     assert np.array_equal(q0[0], q1[0])
+
+
+@pytest.mark.parametrize("waters", [22, 32, 33, 64])
+def test_narrow_and_wide_tiles_agree(ctx, waters):
+    """Alone a molecule's 128 x 32 tiles find an SM each; 60 of them take 128 x 64
+    tiles.  Bases just above a row tile, at and beside a multiple of both widths, and
+    of three row tiles."""
+    mols = W.water_replicas(W.water_cluster_k(waters, 2), 60)
+    prm = M.SCFParams(damping_weight=0.0, diis_start_error=0.1, diis_end_error=0.0)
+    res, q = M.batch_scf("am1", mols, prm, context=ctx)
+    for i in (0, 59):
+        alone, qa = M.batch_scf("am1", [mols[i]], prm, context=ctx)
+        assert alone[0]["iterations"] == res[i]["iterations"]
+        assert alone[0]["energy"] == res[i]["energy"]
+        assert np.array_equal(qa[0], q[i])
