@@ -668,13 +668,15 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   const DevMol mol = mols[mi];
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();
-  if (st[mi].status != kActive) return;
-  const int n = mol.nao, np = pu_np(n);
-  const long long occ = (long long)mol.nocc * kTraceOne;
+  // every load before the first branch: one trip to L2 instead of three
+  const int status = st[mi].status;
+  const long long t0 = pur[mi].trace[k], t1 = pur[mi].trace[k > 0 ? k - 1 : 0];
   double lo, hi;
-  if (!pu_interval(pur[mi], &lo, &hi)) return;
-  const int op = pu_step(pur[mi].trace[k], pur[mi].trace[k > 0 ? k - 1 : 0], k, pu_first(pur[mi].trace, k), occ);   // the same in every CTA of the molecule
-  if (op < 0) return;
+  const bool usable = pu_interval(pur[mi], &lo, &hi);
+  const int n = mol.nao, np = pu_np(n), first = pu_first(pur[mi].trace, k);
+  const long long occ = (long long)mol.nocc * kTraceOne;
+  const int op = pu_step(t0, t1, k, first, occ);   // the same in every CTA of the molecule
+  if (status != kActive || !usable || op < 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = tile.y * kTileM, c0 = tile.z * TN;
   const int rows = min(kTileM, np - r0), cols = min(TN, np - c0);

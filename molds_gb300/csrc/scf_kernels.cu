@@ -303,7 +303,9 @@ diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol
 #pragma unroll
   for (int k = 0; k < kDiisPart; ++k) v[k] = 0.0;
   // two elements' loads before the first store: the history is read and written
-  // through one pointer, so the compiler keeps their order
+  // through one pointer, so the compiler keeps their order.  A launch takes 24 us for
+  // (H2O)33, 55 for (H2O)180 and 266 for 256 (H2O)32; with one element 27, 69 and 234,
+  // with four (142 registers) 386 for the batch.
   constexpr int kU = 2;
   for (long long i0 = lo + tid; i0 < hi; i0 += kU * kDiisThreads) {
     double p[kU], e[kU], x[kMaxDiis][kU];
