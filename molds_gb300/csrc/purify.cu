@@ -11,9 +11,10 @@
 // tensor cores.  X has its spectrum in [0, 1], so |X_ij| <= 1 and it can be
 // held in fixed point: 64-bit integers with 55 fraction bits.  Each is split
 // into seven signed 8-bit digits, X = sum_i d_i 2^(-7-8i), which FP16 holds
-// exactly.  A product of two digits has 14 bits, a sum of up to K of them stays
-// an integer that FP32 holds exactly, so tcgen05 MMAs with FP32 accumulators
-// multiply the digit matrices without any rounding (the error-free splitting of
+// exactly.  A product of two digits has 14 bits; sums of up to 512 terms (a level
+// of a K segment) stay integers of about 2^22, which FP32 holds exactly and a range
+// check guards, so tcgen05 MMAs with FP32 accumulators multiply the digit matrices
+// without any rounding (the error-free splitting of
 // Ozaki, Ogita, Oishi & Rump, Numer. Algorithms 59, 95 (2012)).  Level l sums
 // the digit products with i + j = l, levels 0 to 7 are kept (34 products) and
 // recombined in 64-bit integers.  What is dropped is below 2^-70 times the
@@ -114,10 +115,15 @@ __device__ __forceinline__ void pu_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
 
-// Accumulators as integers.  They are integers below 2^22 in magnitude, so
-// adding 1.5 * 2^23 leaves them in the low mantissa bits: a full-rate FP32 add
-// where the conversion instruction runs at a quarter of it (5390 -> 1800 clocks
-// for a 128 x 64 tile).  range collects the bits that would show a larger one.
+// Accumulators as integers.  They are integers, so adding 1.375 * 2^23 leaves
+// those from -0.75 * 2^22 up to 1.25 * 2^22 in the low mantissa bits: a full-rate
+// FP32 add where the conversion instruction runs at a quarter of it (5390 -> 1800
+// clocks for a 128 x 64 tile).  range collects the bits that would show one outside.
+// The interval lies off zero because the sums do: a digit's squares on the diagonal
+// have a mean of 0.67 * 2^22 at K = 512 where the digits are spread evenly (a dense
+// X), with a standard deviation of 0.09 * 2^22; everything else has none and 0.08.
+// That leaves 6.4 deviations above; an interval of +-2^22 left 3.8, and from N = 512
+// on a dense molecule went to the eigensolver every few iterations.
 __device__ __forceinline__ void pu_ld8(uint32_t addr, float* v) {
   uint32_t u[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -126,9 +132,9 @@ __device__ __forceinline__ void pu_ld8(uint32_t addr, float* v) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(u[i]);
 }
-constexpr int kMagic = 0x4B400000;
+constexpr int kMagic = 0x4B300000;   // 1.375 * 2^23
 __device__ __forceinline__ int pu_int(float f, uint32_t& range) {
-  const int b = __float_as_int(f + 12582912.0f);
+  const int b = __float_as_int(f + 11534336.0f);
   range |= (uint32_t)(b ^ kMagic);
   return b - kMagic;
 }
@@ -553,7 +559,7 @@ constexpr int kPurTileThreads = 512;
 constexpr int kTileM = 128, kChunkK = 32, kStages = 2;
 constexpr uint32_t kStageA = kTileM * kChunkK * 2;        // bytes per digit
 constexpr uint32_t stage_bytes(int tn) { return kDigits * (kStageA + (uint32_t)tn * kChunkK * 2); }
-constexpr int kSegChunks = 16;                            // K = 512: the largest sums, of a digit's squares, stay near 0.7 * 2^22
+constexpr int kSegChunks = 16;                            // K = 512: see pu_int
 constexpr int kXPitch = kTileM + 1;                       // transposed tile, 8-byte elements: no bank conflicts either way
 constexpr size_t tile_smem(int tn) { return kStages * stage_bytes(tn) + 256; }
 
@@ -714,7 +720,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     for (int i = 0; i < 8; ++i) v[s][i] = 0;
   uint32_t range = 0;
   bool ok = true;
-  // K in segments whose digit sums stay integers below 2^24
+  // K in segments whose digit sums pu_int covers
   for (int seg = 0, cb = 0; cb < chunks && ok; ++seg, cb += kSegChunks) {
     const int ce = min(chunks, cb + kSegChunks);
     if (warp == 0 && lane == 0) {
