@@ -368,7 +368,7 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_charges = dalloc<double>(cap.atoms, &bytes_);
   d_sweeps = dalloc<int>(nm, &bytes_);
   d_count = dalloc<int>(2, &bytes_);
-  d_tc_err = dalloc<int>(1, &bytes_);
+  d_wait_err_ = dalloc<int>(1, &bytes_);
   {
     const size_t b = diis_scratch_bytes(nm);
     cuda_check(cudaMalloc(&d_diis_ws, b), "cudaMalloc DIIS scratch");
@@ -379,7 +379,7 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_active = dalloc<char>(nm, &bytes_);
   cuda_check(cudaMemsetAsync(d_state, 0, nm * sizeof(MolState), stream_), "memset state");
   cuda_check(cudaMemsetAsync(d_sweeps, 0, nm * sizeof(int), stream_), "memset sweeps");
-  cuda_check(cudaMemsetAsync(d_tc_err, 0, sizeof(int), stream_), "memset tc err");
+  cuda_check(cudaMemsetAsync(d_wait_err_, 0, sizeof(int), stream_), "memset wait error");
   cuda_check(cudaMemsetAsync(d_H, 0, mat * sizeof(double), stream_), "memset H");
   cuda_check(cudaMemsetAsync(d_P, 0, mat * sizeof(double), stream_), "memset P");
   cuda_check(cudaMemsetAsync(d_hist_dens, 0, std::max(diis_m_, 1) * mat * sizeof(double), stream_), "memset hist");
@@ -519,7 +519,7 @@ Batch::~Batch() {
   if (d_diis_ws) cudaFree(d_diis_ws);
   void* ptrs[] = {d_atoms, d_epc, d_pairs, d_mols, d_list, d_blocks, d_ecore_pair, d_H, d_F, d_P, d_Pold, d_C, d_eps,
                   d_hist_dens, d_hist_err, d_G32, d_T32, d_Cf, d_Cnf, d_Ff, d_G64, d_T64, d_jA32, d_jV32, d_jA64, d_jV64,
-                  d_state, d_trace, d_charges, d_sweeps, d_count, d_active, d_heavy_pairs, d_light_pairs, d_tc_err, d_dip_ws};
+                  d_state, d_trace, d_charges, d_sweeps, d_count, d_active, d_heavy_pairs, d_light_pairs, d_wait_err_, d_dip_ws};
   for (void* p : ptrs) if (p) cudaFree(p);
   for (int i = 0; i < 6; ++i) if (d_S[i]) cudaFree(d_S[i]);
   if (d_td) cudaFree(d_td);
@@ -1115,13 +1115,13 @@ void Batch::eigen_step(const ScfSettings& s, int effort) {
       for (int k = 0; k < 2; ++k) {
         launches_ += !pur_list_[k].empty();
         launch_purify_small(d_mols, d_pur_list_[k], (int)pur_list_[k].size(), pur_max_n_[k], d_state, d_F, d_P,
-                            d_tc_err, stream_);
+                            d_wait_err_, pur_wait_, stream_);
       }
       const PurScratch ws{{d_T64, d_S[0], d_S[1], d_S[2], d_S[3], d_S[4], d_S[5]}};
       launches_ += launch_purify_big(d_mols, d_pur_list_[2], (int)pur_list_[2].size(), pur_max_n_[2], d_pur_tiles_,
                                      (int)pur_tiles_.size(), pur_tn_, d_state, d_F, d_P, d_pur_, ws,
-                                     effort > 0 ? kPurBigSteps : kPurFewSteps, alone_, d_tc_err,
-                                     stream_);
+                                     effort > 0 ? kPurBigSteps : kPurFewSteps, alone_, d_wait_err_,
+                                     pur_wait_, stream_);
       prof_end(h);
       if (effort < 2) return;
     }
@@ -1159,16 +1159,16 @@ void Batch::eigen_step(const ScfSettings& s, int effort) {
       launches_ += 6;
       int h = prof_begin(kKOrtho, active_work_estimate(kKOrtho));
       launch_tc_shadows(d_mols, d_list, (int)cur_list_.size(), d_state, d_C, d_F, d_Cf, d_Cnf, d_Ff, stream_);
-      launch_tc_gemm(j_ns1_.d, j_ns1_.n, j_ns1_.tc_tiles, d_Cf, d_Cf, d_T32, false, true, d_state, 1, -1, d_tc_err,
+      launch_tc_gemm(j_ns1_.d, j_ns1_.n, j_ns1_.tc_tiles, d_Cf, d_Cf, d_T32, false, true, d_state, 1, -1, d_wait_err_,
                      stream_);
-      launch_tc_gemm(j_ns2_.d, j_ns2_.n, j_ns2_.tc_tiles, d_T32, d_Cf, d_Cnf, false, false, d_state, 1, -1, d_tc_err,
+      launch_tc_gemm(j_ns2_.d, j_ns2_.n, j_ns2_.tc_tiles, d_T32, d_Cf, d_Cnf, false, false, d_state, 1, -1, d_wait_err_,
                      stream_);
       prof_end(h);
       h = prof_begin(kKTransform, active_work_estimate(kKTransform));
       launch_tc_gemm(j_trans1_.d, j_trans1_.n, j_trans1_.tc_tiles, d_Ff, d_Cnf, d_T32, false, true, d_state, 1, -1,
-                     d_tc_err, stream_);
+                     d_wait_err_, stream_);
       launch_tc_gemm(j_trans2_.d, j_trans2_.n, j_trans2_.tc_tiles, d_Cnf, d_T32, d_G32, false, false, d_state, 1, -1,
-                     d_tc_err, stream_);
+                     d_wait_err_, stream_);
       prof_end(h);
       h = prof_begin(kKJacobi, active_work_estimate(kKJacobi));
       run_jacobi(true, s, nullptr, d_Cnf);
@@ -1207,7 +1207,7 @@ void Batch::density_step(const ScfSettings& s) {
                 stream_);
     if (mixed) {
       launches_ += 1;
-      launch_tc_gemm(j_hh_.d, j_hh_.n, j_hh_.tc_tiles, d_Cf, d_Cf, d_P, true, false, d_state, require, 0, d_tc_err,
+      launch_tc_gemm(j_hh_.d, j_hh_.n, j_hh_.tc_tiles, d_Cf, d_Cf, d_P, true, false, d_state, require, 0, d_wait_err_,
                      stream_);
     }
     prof_end(h);
@@ -1221,7 +1221,7 @@ void Batch::density_step(const ScfSettings& s) {
     launches_ += 12;
     int h = prof_begin(kKDensity, active_work_estimate(kKDensity));
     if (s.tensor_cores)
-      launch_tc_gemm(j_dens_.d, j_dens_.n, j_dens_.tc_tiles, d_C, d_C, d_P, true, false, d_state, 1, 0, d_tc_err, stream_);
+      launch_tc_gemm(j_dens_.d, j_dens_.n, j_dens_.tc_tiles, d_C, d_C, d_P, true, false, d_state, 1, 0, d_wait_err_, stream_);
     else
       launch_gemm(j_dens_.d, j_dens_.n, j_dens_.tiles, d_C, d_C, d_P, true, false, 0.0f, d_state, 1, 0, stream_);
     prof_end(h);
@@ -1430,10 +1430,19 @@ void Batch::scf(const ScfSettings& s, bool requires_guess) {
     effort = next;
   }
   finish(s, all);
-  int tc_err = 0;
-  cuda_check(cudaMemcpyAsync(&tc_err, d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, stream_), "tc err");
+  int err = 0;
+  copy_wait_error_async(&err);
   cuda_check(cudaStreamSynchronize(stream_), "scf");
-  if (tc_err) throw std::runtime_error("tensor-core GEMM: an MMA completion wait ran out");
+  if (err) cuda_check(cudaMemsetAsync(d_wait_err_, 0, sizeof(int), stream_), "wait error reset");
+  check_wait_error(err);
+}
+
+void Batch::copy_wait_error_async(int* host) {
+  cuda_check(cudaMemcpyAsync(host, d_wait_err_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "wait error copy");
+}
+
+void check_wait_error(int err) {
+  if (err) throw std::runtime_error("tensor cores: a wait for a copy or an MMA ran out");
 }
 
 void Batch::results(std::vector<MolResult>* out) {

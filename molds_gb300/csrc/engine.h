@@ -115,6 +115,9 @@ class Batch {
   // asynchronous copies into pinned host memory (complete at the next stream sync)
   void copy_states_async(MolState* host);
   void copy_charges_async(int m, double* host);
+  // whether a wait of a tensor-core kernel has run out (scf() checks it itself); for
+  // check_wait_error once the copy is complete
+  void copy_wait_error_async(int* host);
   int nao(int m) const { return h_mols[m].nao; }
   int natoms(int m) const { return h_mols[m].natoms; }
   int nocc(int m) const { return h_mols[m].nocc; }
@@ -266,7 +269,8 @@ class Batch {
   double* d_charges = nullptr;
   int* d_sweeps = nullptr;
   int* d_count = nullptr;
-  int* d_tc_err = nullptr;               // set by a tensor-core GEMM whose MMA wait ran out
+  int* d_wait_err_ = nullptr;            // set by a tensor-core kernel whose wait for a copy or an MMA ran out
+  long long pur_wait_ = kPurWaitCycles;  // clocks that a wait of the purification may take
   void* d_diis_ws = nullptr;             // DIIS partial sums and decisions (diis_scratch_bytes)
   double* d_dip_ws = nullptr;            // dipole partial sums (slots x kDipChunks x 4)
   char* d_active = nullptr;
@@ -377,6 +381,9 @@ class Engine {
 
 // throws std::runtime_error with the CUDA error text
 void cuda_check(cudaError_t e, const char* what);
+
+// throws std::runtime_error when err (Batch::copy_wait_error_async) is set
+void check_wait_error(int err);
 
 // basis functions of a molecule (unknown elements count zero; layout rejects them)
 int molecule_nao(const MoleculeInput& in);

@@ -135,22 +135,26 @@ constexpr int kPurSmallMaxN = 128;   // one CTA per molecule up to here, tiles o
 constexpr int kPurBigSteps = 56;     // steps launched above kPurSmallMaxN: HOMO-LUMO gaps down to ~3e-4 of the interval
 constexpr int kPurFewSteps = 32;     // and for the later SCF iterations, whose gaps are wide
 constexpr int kPurEarly = 6;         // SCF iterations that get kPurBigSteps from the start
+constexpr long long kPurWaitCycles = 2000000000LL;   // ~1 s: a copy or an MMA that has not completed by then never will
 struct PurState {
   unsigned long long lo, hi;         // Gershgorin interval, order-preserving keys
+  int bad;                           // 1 + the step in which a digit sum left the range its recombination covers
+                                     // or a wait ran out; 0: none
   long long trace[kPurBigSteps + 1]; // tr X_k
-  int bad;                           // a digit sum left the range its recombination covers
 };
 struct PurScratch { double* m[7]; }; // N x N scratch matrices holding two digit buffers of seven digits each
 void purify_prepare();               // one-time kernel attributes (before any stream capture)
 // tiles of tn columns (64 or 32) of one molecule (out may be null); returns their number
 int purify_tiles(int mol, int n, int tn, int4* out);
+// limit: clocks after which a wait for a copy or an MMA counts as run out; the
+// molecule is then flagged and *err set
 void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
-                         double* P, int* err, cudaStream_t s);
+                         double* P, int* err, long long limit, cudaStream_t s);
 // alone: no other stream's work is expected beside this launch sequence
 // returns the number of kernels launched
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles, int tn,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
-                      bool alone, int* err, cudaStream_t s);
+                      bool alone, int* err, long long limit, cudaStream_t s);
 
 int hh_smem_max_n();     // largest basis whose packed matrix fits one CTA's shared memory
 int hh_back_max_n();     // largest basis the back-transformation kernel serves

@@ -44,7 +44,6 @@ namespace nddo {
 constexpr int kDigits = 7, kLevels = 8;
 constexpr int kPurSmallThreads = 17 * 32;
 constexpr int kPurSmallSteps = 100;                // the one-CTA kernel stops by itself; its steps are cheap
-constexpr long long kPurWaitCycles = 2000000000LL; // ~1 s: a copy or an MMA that has not completed by then never will
 constexpr int kTraceShift = 12;                    // traces are summed in units of 2^-43
 constexpr long long kTraceOne = 1LL << (55 - kTraceShift);
 constexpr long long kTraceTol = kTraceOne >> 30;   // tr(X - X^2) that two more steps square away
@@ -102,14 +101,18 @@ __device__ __forceinline__ void pu_products(uint32_t tmem, uint32_t a, uint32_t 
   }
 }
 
-__device__ __forceinline__ bool pu_wait(uint32_t bar, uint32_t parity) {
+// whether a phase came within `limit` clocks
+__device__ __forceinline__ bool pu_wait(uint32_t bar, uint32_t parity, long long limit) {
   uint32_t done = 0;
   const long long t0 = clock64();
-  while (!done && clock64() - t0 < kPurWaitCycles)
+  while (!done && clock64() - t0 < limit)
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
+// After a wait that ran out: no copy and no MMA that a CTA has set going may outlive
+// it, so what was waited for is waited for once more, with the usual limit.
+__device__ __noinline__ void pu_drain(uint32_t bar, uint32_t parity) { pu_wait(bar, parity, kPurWaitCycles); }
 
 __device__ __forceinline__ void pu_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
@@ -311,7 +314,8 @@ __device__ __forceinline__ void pu_drained(int j, bool issuer) {
 template <int H, int L>
 __global__ void __launch_bounds__(kPurSmallThreads, 1)
 purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, MolState* __restrict__ st,
-                    const double* __restrict__ F, double* __restrict__ P, int np_max, int* __restrict__ err) {
+                    const double* __restrict__ F, double* __restrict__ P, int np_max, long long limit,
+                    int* __restrict__ err) {
   constexpr int G = (kLevels + L - 1) / L;   // level groups
   extern __shared__ __align__(1024) unsigned char pu_sm[];
   const int mi = list[blockIdx.x];
@@ -501,7 +505,10 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
         for (int c = 0; c < 16; ++c) x[h][c] = op ? 0 : 2 * x[h][c];
 #pragma unroll
       for (int j = 0; j < G; ++j) {
-        ok = pu_wait(bar + 8 * (j & 1), parity[j & 1]) && ok;
+        if (!pu_wait(bar + 8 * (j & 1), parity[j & 1], limit)) {
+          ok = false;
+          pu_drain(bar + 8 * (j & 1), parity[j & 1]);
+        }
         parity[j & 1] ^= 1;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (work) {
@@ -661,7 +668,7 @@ __device__ __forceinline__ int pu_first(const long long* T, int k) {
 template <int TN>
 __global__ void __launch_bounds__(kPurTileThreads, 1)
 purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ tiles, const MolState* __restrict__ st,
-                   PurState* __restrict__ pur, PurScratch ws, int k, int* __restrict__ err) {
+                   PurState* __restrict__ pur, PurScratch ws, int k, long long limit, int* __restrict__ err) {
   constexpr int kCW = TN / 4, kGroups = kCW / 8;   // columns of a warp, groups of eight of them
   constexpr uint32_t kStageBytes = stage_bytes(TN);
   constexpr int kTmem = kLevels * TN;
@@ -675,14 +682,16 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();
   // every load before the first branch: one trip to L2 instead of three
-  const int status = st[mi].status;
+  const int status = st[mi].status, bad = pur[mi].bad;
   const long long t0 = pur[mi].trace[k], t1 = pur[mi].trace[k > 0 ? k - 1 : 0];
   double lo, hi;
   const bool usable = pu_interval(pur[mi], &lo, &hi);
   const int n = mol.nao, np = pu_np(n), first = pu_first(pur[mi].trace, k);
   const long long occ = (long long)mol.nocc * kTraceOne;
   const int op = pu_step(t0, t1, k, first, occ);   // the same in every CTA of the molecule
-  if (status != kActive || !usable || op < 0) return;
+  // bad: an earlier step's tile failed; those of this one write k + 1, so that all
+  // threads of a CTA decide alike whichever value they read
+  if (status != kActive || !usable || (bad > 0 && bad <= k) || op < 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = tile.y * kTileM, c0 = tile.z * TN;
   const int rows = min(kTileM, np - r0), cols = min(TN, np - c0);
@@ -720,6 +729,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     for (int i = 0; i < 8; ++i) v[s][i] = 0;
   uint32_t range = 0;
   bool ok = true;
+  int issued = 0;   // K chunks whose copies (thread 0) or MMAs (thread 32) this thread has issued
   // K in segments whose digit sums pu_int covers
   for (int seg = 0, cb = 0; cb < chunks && ok; ++seg, cb += kSegChunks) {
     const int ce = min(chunks, cb + kSegChunks);
@@ -727,7 +737,8 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
       const uint32_t ba = (uint32_t)rows * kChunkK * 2, bb = (uint32_t)cols * kChunkK * 2;
       for (int c = cb; c < ce; ++c) {
         const int s = c % kStages;
-        if (c >= kStages && !pu_wait(empty + 8 * s, ((c / kStages) - 1) & 1)) { ok = false; break; }
+        if (c >= kStages && !pu_wait(empty + 8 * s, ((c / kStages) - 1) & 1, limit)) { ok = false; break; }
+        issued = c + 1;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                      :: "r"(full + 8 * s), "r"((ba + bb) * kDigits) : "memory");
         for (int d = 0; d < kDigits; ++d) {
@@ -744,7 +755,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
       asm volatile("tcgen05.fence::after_thread_sync;");
       for (int c = cb; c < ce; ++c) {
         const int s = c % kStages;
-        if (!pu_wait(full + 8 * s, (c / kStages) & 1)) { ok = false; break; }
+        if (!pu_wait(full + 8 * s, (c / kStages) & 1, limit)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t base = pu_desc_lo(sm + s * kStageBytes);
         const uint32_t bb = base + (kDigits * kStageA >> 4), sb = (uint32_t)cols * kChunkK * 2;
@@ -753,11 +764,12 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
         else
           pu_products<7, 0, kLevels>(tmem, base, kStageA, bb, sb, pu_desc_hi(512), cols, kChunkK / 16, c == cb);
         pu_commit(empty + 8 * s);
+        issued = c + 1;
       }
       if (ok) pu_commit(last);
     }
     __syncwarp();
-    ok = pu_wait(last, seg & 1) && ok;
+    ok = pu_wait(last, seg & 1, limit) && ok;
     asm volatile("tcgen05.fence::after_thread_sync;");
     ok = __syncthreads_and(ok);
     if (ok) {
@@ -772,13 +784,20 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     __syncthreads();
   }
   if (!ok) {
-    if (tid == 0) atomicExch(err, 1);
+    // a wait ran out: this tile of X_{k+1} is missing, the molecule goes to the
+    // eigensolver
+    for (int c = max(0, issued - kStages); c < issued; ++c)
+      pu_drain((warp == 0 ? full : empty) + 8 * (c % kStages), (c / kStages) & 1);
+    if (tid == 0) {
+      atomicExch(&pur[mi].bad, k + 1);
+      atomicExch(err, 1);
+    }
   } else {
     // X_{k+1}: row r, the digits of eight columns at a time
     const bool mirror = tile.z >= (kTileM / TN) * (tile.y + 1);   // the transposed block is no tile of its own
     long long* xt = reinterpret_cast<long long*>(pu_sm);   // the operand stages are free now
     // rows past the padded basis are whatever the stage held before
-    if (r < np && !pu_in_range(range)) atomicExch(&pur[mi].bad, 1);
+    if (r < np && !pu_in_range(range)) atomicExch(&pur[mi].bad, k + 1);
     long long tr = 0;
 #pragma unroll
     for (int s = 0; s < kGroups; ++s) {
@@ -888,20 +907,20 @@ int purify_tiles(int mol, int n, int tn, int4* out) {
 }
 
 void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
-                         double* P, int* err, cudaStream_t s) {
+                         double* P, int* err, long long limit, cudaStream_t s) {
   if (nlist <= 0) return;
   purify_prepare();
   const int np = (max_n + 15) / 16 * 16;
   const size_t sm = small_smem(np);
   // levels per group: two buffers of L x np of the 512 columns of tensor memory
-  if (np <= 64) purify_small_kernel<1, 4><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
-  else if (np <= 80) purify_small_kernel<2, 3><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
-  else purify_small_kernel<2, 2><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, err);
+  if (np <= 64) purify_small_kernel<1, 4><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, err);
+  else if (np <= 80) purify_small_kernel<2, 3><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, err);
+  else purify_small_kernel<2, 2><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, err);
 }
 
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles, int tn,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
-                      bool alone, int* err, cudaStream_t s) {
+                      bool alone, int* err, long long limit, cudaStream_t s) {
   if (nlist <= 0) return 0;
   purify_prepare();
   const int np = (max_n + 31) / 32 * 32;
@@ -922,7 +941,8 @@ int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n,
     // CTAs launched ahead hold an SM while they wait: only where no other stream
     // has work for it (a server's burst took 104 ms without and 119 with them)
     cfg.numAttrs = alone && k > 0 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, tn == 64 ? purify_step_kernel<64> : purify_step_kernel<32>, mols, tiles, (const MolState*)st, pur, ws, k, err);
+    cudaLaunchKernelEx(&cfg, tn == 64 ? purify_step_kernel<64> : purify_step_kernel<32>, mols, tiles,
+                       (const MolState*)st, pur, ws, k, limit, err);
   }
   purify_store_kernel<<<dim3(blocks, nlist), 256, 0, s>>>(mols, list, st, pur, ws, steps, P);
   return steps + 4;

@@ -78,7 +78,7 @@ Server::Server(Engine* eng, const ScfSettings& s, size_t hbm_budget, int max_bas
     L->slot_ticket.assign(slots, -1);
     L->slot_tsubmit.assign(slots, 0.0);
     L->slot_tadmit.assign(slots, 0.0);
-    cuda_check(cudaHostAlloc(&L->h_count, 2 * sizeof(int), cudaHostAllocDefault), "pinned");
+    cuda_check(cudaHostAlloc(&L->h_count, 3 * sizeof(int), cudaHostAllocDefault), "pinned");
     cuda_check(cudaHostAlloc(&L->h_active, slots, cudaHostAllocDefault), "pinned");
     cuda_check(cudaHostAlloc(&L->h_states, slots * sizeof(MolState), cudaHostAllocDefault), "pinned");
     cuda_check(cudaHostAlloc(&L->h_charges, c.atoms * sizeof(double), cudaHostAllocDefault), "pinned");
@@ -289,8 +289,10 @@ bool Server::lane_step(Lane& L) {
   if (!fin.empty()) {
     b.finish(s_, fin);
     b.copy_states_async(L.h_states);
+    b.copy_wait_error_async(L.h_count + 2);
     for (int m : fin) b.copy_charges_async(m, L.h_charges + b.mol_table()[m].atom0);
     cuda_check(cudaStreamSynchronize(L.stream), "lane results");
+    check_wait_error(L.h_count[2]);
     const double t = now();
     for (int m : fin) {
       const MolState& st = L.h_states[m];

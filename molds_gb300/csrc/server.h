@@ -70,7 +70,7 @@ class Server {
     std::vector<long long> slot_ticket;
     std::vector<double> slot_tsubmit, slot_tadmit;
     int eigen = 0;                            // iterations still to run with the eigensolver launches
-    int* h_count = nullptr;                   // active molecules, those waiting for the eigensolver
+    int* h_count = nullptr;                   // active molecules, those waiting for the eigensolver, wait error
     char* h_active = nullptr;
     MolState* h_states = nullptr;
     double* h_charges = nullptr;

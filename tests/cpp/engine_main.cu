@@ -2,10 +2,16 @@
 // not show.  Usage: engine_main MODE ARGUMENTS; exit code 3 when the engine throws.
 //   purify IN OUT   IN: int n, int nocc, n x n doubles F; OUT: int flags, int
 //                   error word, n x n doubles P
+//   waits MOLECULE  an iteration whose purification waits run out at once, the same
+//                   again with the usual limit, a whole SCF of either kind; prints
+//                   flags, iteration, error word and the energies
+//   server MOLECULE a served request after a lane's wait error was set
+// MOLECULE: the theory number, then "Z x y z" per line (bohr).
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <exception>
+#include <fstream>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -53,7 +59,7 @@ static int purify(const char* in, const char* out) {
   double* d_F = device(F);
   double* d_P = device(std::vector<double>(F.size(), 0.0));
   if (n <= kPurSmallMaxN) {
-    launch_purify_small(d_mol, d_list, 1, n, d_st, d_F, d_P, d_err, nullptr);
+    launch_purify_small(d_mol, d_list, 1, n, d_st, d_F, d_P, d_err, kPurWaitCycles, nullptr);
   } else {
     std::vector<int4> tiles(purify_tiles(0, n, 64, nullptr));
     purify_tiles(0, n, 64, tiles.data());
@@ -62,7 +68,7 @@ static int purify(const char* in, const char* out) {
     PurScratch ws;
     for (double*& m : ws.m) m = device(std::vector<double>((F.size() + 31) / 32 * 32, 0.0));
     launch_purify_big(d_mol, d_list, 1, n, d_tiles, (int)tiles.size(), 64, d_st, d_F, d_P, d_pur, ws, kPurBigSteps, true,
-                      d_err, nullptr);
+                      d_err, kPurWaitCycles, nullptr);
   }
   cuda_check(cudaGetLastError(), "launch");
   cuda_check(cudaDeviceSynchronize(), "purify");
@@ -79,10 +85,100 @@ static int purify(const char* in, const char* out) {
   return 0;
 }
 
+static MoleculeInput molecule(const char* file) {
+  std::ifstream in(file);
+  MoleculeInput m;
+  in >> m.theory;
+  int z;
+  double x, y, w;
+  while (in >> z >> x >> y >> w) {
+    m.Z.push_back(z);
+    m.xyz.insert(m.xyz.end(), {x, y, w});
+  }
+  return m;
+}
+
+static ScfSettings settings() {
+  ScfSettings s;
+  s.max_iter = 60;
+  s.damping_weight = 0.0;
+  s.diis_start_error = 0.1;
+  s.diis_end_error = 0.0;
+  return s;
+}
+
+static int waits(const char* file) {
+  const ScfSettings s = settings();
+  Engine eng(0);
+  std::vector<double> P[2];
+  for (int limited = 1; limited >= 0; --limited) {
+    Batch b(&eng, {molecule(file)}, s.diis_num_error_vect);
+    b.integrals();
+    b.begin(s, {0}, true);
+    const int n = b.nao(0);
+    for (int pass = 1 - limited; pass < 2; ++pass) {   // without and with time for the waits
+      b.pur_wait_ = pass == 0 ? 0 : kPurWaitCycles;
+      b.iterate(s, {0}, 1);
+      MolState st;
+      int err = 0;
+      b.copy_states_async(&st);
+      b.copy_wait_error_async(&err);
+      cuda_check(cudaMemsetAsync(b.d_wait_err_, 0, sizeof(int), b.stream()), "reset");
+      cuda_check(cudaStreamSynchronize(b.stream()), "iteration");
+      if (limited) std::printf("pass %d flags %d iter %d error %d\n", pass, st.flags, st.iter, err);
+    }
+    P[limited].resize((size_t)n * n);
+    b.copy_matrix(2, 0, P[limited].data());
+  }
+  std::printf("same_density %d\n", (int)(P[0] == P[1]));
+  for (int limited = 1; limited >= 0; --limited) {
+    Batch b(&eng, {molecule(file)}, s.diis_num_error_vect);
+    if (limited) b.pur_wait_ = 0;
+    b.integrals();
+    for (int again = 0; again <= limited; ++again) {
+      if (again) b.pur_wait_ = kPurWaitCycles, ++b.layout_version_;   // a graph holds the limit it was captured with
+      try {
+        b.scf(s, true);
+        std::printf("scf_ok 1\n");
+      } catch (const std::exception& e) {
+        std::printf("scf_error %s\n", e.what());
+      }
+      std::vector<MolResult> r;
+      b.results(&r);
+      std::printf("energy %.15e status %d iterations %d\n", r[0].energy, r[0].status, r[0].iterations);
+    }
+  }
+  return 0;
+}
+
+static int server(const char* file) {
+  Engine eng(0);
+  Server srv(&eng, settings(), (size_t)1 << 30, 300);
+  for (int k = 0; k < 2; ++k) {
+    if (k) {
+      const int one = 1;
+      for (auto& L : srv.lanes_)
+        cuda_check(cudaMemcpy(L->b->d_wait_err_, &one, sizeof(int), cudaMemcpyHostToDevice), "copy");
+    }
+    srv.submit(molecule(file));
+    int got = 0;
+    try {
+      for (int t = 0; t < 100 && !got; ++t) got = srv.poll(100000);
+    } catch (const std::exception& e) {
+      std::printf("poll_error %s\n", e.what());
+    }
+    ServeResult r;
+    if (got && srv.take(&r)) std::printf("served status %d energy %.15e\n", r.status, r.energy);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   try {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "purify" && argc == 4) return purify(argv[2], argv[3]);
+    if (mode == "waits" && argc == 3) return waits(argv[2]);
+    if (mode == "server" && argc == 3) return server(argv[2]);
     std::fprintf(stderr, "unknown mode\n");
     return 2;
   } catch (const std::exception& e) {

@@ -19,3 +19,11 @@ def build_engine_program(directory):
 
 def run_engine_program(exe, *args):
     return subprocess.run([exe] + [str(a) for a in args], capture_output=True, text=True, timeout=300)
+
+
+def write_molecule(directory, theory, mol):
+    """theory: its number in the C ABI; mol: atomic numbers Z and xyz in bohr"""
+    p = directory / "molecule.txt"
+    p.write_text("\n".join([str(theory)] + [f"{int(z)} {x:.17g} {y:.17g} {w:.17g}" for z, (x, y, w) in
+                                            zip(mol.Z, mol.xyz.reshape(-1, 3).tolist())]) + "\n")
+    return str(p)
