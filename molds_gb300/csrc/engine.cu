@@ -416,9 +416,9 @@ void Batch::allocate(const BatchCapacity& cap) {
   JobSet* all[] = {&j_trans1_, &j_trans2_, &j_dens_, &j_w_, &j_kt_, &j_yt_, &j_m_, &j_d2_, &j_z_, &j_p_, &j_ns1_, &j_ns2_, &j_ov_, &j_hh_};
   for (JobSet* j : all) { j->d = dalloc<GemmJob>(job_cap_, &bytes_); j->cap = job_cap_; }
   cuda_check(cudaHostAlloc(&h_jobs_, sizeof(GemmJob) * (size_t)job_cap_ * 14, cudaHostAllocDefault), "cudaHostAlloc jobs");
-  cuda_check(cudaHostAlloc(&h_lists_, sizeof(int) * (size_t)nm * (kJacobiBuckets + 6), cudaHostAllocDefault),
+  cuda_check(cudaHostAlloc(&h_lists_, sizeof(int) * (size_t)nm * (kSizeBuckets + 6), cudaHostAllocDefault),
              "cudaHostAlloc lists");
-  for (int b = 0; b < kJacobiBuckets; ++b) d_bucket_lists_.push_back(dalloc<int>(nm, &bytes_));
+  for (int b = 0; b < kSizeBuckets; ++b) d_bucket_lists_.push_back(dalloc<int>(nm, &bytes_));
   cuda_check(cudaStreamSynchronize(stream_), "allocate");
 }
 
@@ -699,7 +699,7 @@ void Batch::upload_list(const std::vector<int>& which) {
   build_jobs(which);
   {
     // the Householder path's two lists (staged behind the bucket lists)
-    int* stage = h_lists_ + (size_t)(kJacobiBuckets + 1) * nm;
+    int* stage = h_lists_ + (size_t)(kSizeBuckets + 1) * nm;
     std::copy(hh_small_.begin(), hh_small_.end(), stage);
     std::copy(hh_large_.begin(), hh_large_.end(), stage + nm);
     for (int k = 0; k < 3; ++k) {
@@ -727,34 +727,29 @@ void Batch::upload_list(const std::vector<int>& which) {
                  "upload grid map");
     }
   }
-  // Jacobi size buckets: smaller molecules get a smaller shared-memory
-  // footprint; the first edge keeps bases below the cluster Jacobi's minimum
-  // apart from the ones it serves, so a molecule's kernel follows its own size
   buckets_.clear();
+  bucket_slot_.clear();
   bucket_max_n_.clear();
   bucket_hh_max_n_.clear();
   bucket_dev_.clear();
-  const int edges[kJacobiBuckets] = {kClusterJacobiMinN - 1, 64, 96, 128, 160, 194, 256, 338, 1 << 30};
-  int lo = 0, bi = 0;
-  for (int hi : edges) {
+  for (int slot = 0; slot < kSizeBuckets; ++slot) {
     std::vector<int> b;
     int mx = 0, mx_hh = 0;
     for (int m : which) {
       const int n = h_mols[m].nao;
-      if (n > lo && n <= hi) {
+      if (size_bucket(n) == slot) {
         b.push_back(m);
         mx = std::max(mx, n);
         if (n <= hh_served_max_n_) mx_hh = std::max(mx_hh, n);
       }
     }
-    lo = hi;
-    const int slot = bi++;
     if (b.empty()) continue;
     int* stage = h_lists_ + (size_t)(slot + 1) * nm;
     std::copy(b.begin(), b.end(), stage);
     cuda_check(cudaMemcpyAsync(d_bucket_lists_[slot], stage, b.size() * sizeof(int), cudaMemcpyHostToDevice, stream_),
                "upload bucket");
     buckets_.push_back(b);
+    bucket_slot_.push_back(slot);
     bucket_max_n_.push_back(mx);
     bucket_hh_max_n_.push_back(mx_hh);
     bucket_dev_.push_back(d_bucket_lists_[slot]);
@@ -1087,13 +1082,17 @@ void Batch::hh_vectors(const ScfSettings& s, int final_pass, int require_active)
 }
 
 // FP64 Householder tridiagonalisation (one launch per size bucket, each with
-// its own shared-memory footprint)
+// its own shared-memory footprint).  Groups that reduce in every iteration do so at
+// the same time; the final pass, or that of a few flagged molecules, comes when a
+// group gets there, and counts its own list alone (64 (H2O)66 in four groups, final
+// pass only: 118 ms a batch, 130 with the groups counted together).
 void Batch::hh_reduce(int require) {
   for (size_t b = 0; b < buckets_.size(); ++b) {
     if (bucket_hh_max_n_[b] == 0) continue;
     launches_ += 1;
     launch_hh_tridiag(d_mols, bucket_dev_[b], (int)buckets_[b].size(), bucket_hh_max_n_[b], d_state, require, d_F, d_G64,
-                      d_td, vec_total_, d_S[4], hh_served_max_n_, stream_);
+                      d_td, vec_total_, d_S[4], hh_served_max_n_,
+                      require == 1 ? peers_[bucket_slot_[b]] : 0, stream_);
   }
   // the whole-GPU path: each chunk's molecules share one cooperative launch
   for (const GridChunk& c : grid_chunks_) {

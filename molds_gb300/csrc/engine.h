@@ -2,6 +2,7 @@
 // molecule batches, and drives the batched SCF state machine.
 #pragma once
 #include <cuda_runtime.h>
+#include <array>
 #include <map>
 #include <memory>
 #include <string>
@@ -95,8 +96,9 @@ class Batch {
   Batch& operator=(const Batch&) = delete;
 
   int size() const { return (int)h_mols.size(); }
-  // other streams run beside this batch's (molecule groups, serving lanes)
-  void set_shared() { alone_ = false; }
+  // other streams run beside this batch's (molecule groups, serving lanes); peers:
+  // molecules of all groups by size bucket, where the groups run the same launches
+  void set_shared(const std::array<int, kSizeBuckets>& peers = {}) { alone_ = false; peers_ = peers; }
   int max_n() const { return cap_.max_n; }
   long long epc_capacity() const { return cap_.epcs; }
   cudaStream_t stream() const { return stream_; }
@@ -196,6 +198,7 @@ class Batch {
   int diis_m_;
   bool pool_ = false;
   bool alone_ = true;
+  std::array<int, kSizeBuckets> peers_{};
   BatchCapacity cap_;
   ArenaAlloc a_atoms_, a_pairs_, a_blocks_, a_mat_, a_vec_, a_epc_;
   std::vector<int> free_slots_;
@@ -246,6 +249,7 @@ class Batch {
   int4* h_pur_tiles_ = nullptr;          // pinned staging of d_pur_tiles_
   size_t pur_tile_cap_ = 0;
   PurState* d_pur_ = nullptr;
+  std::vector<int> bucket_slot_;         // size bucket of each entry of buckets_
   std::vector<int> bucket_hh_max_n_;     // per size bucket: largest basis on the per-molecule kernels
   int hh_served_max_n_ = 0;              // the per-molecule kernels serve bases up to this; larger: whole-GPU kernels
   // whole-GPU path: the large molecules in chunks of at most one per SM, each

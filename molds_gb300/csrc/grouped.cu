@@ -32,6 +32,8 @@ GroupedBatch::GroupedBatch(Engine* eng, const std::vector<MoleculeInput>& mols, 
   for (const MoleculeInput& m : mols)
     if (molecule_nao(m) >= kGridShareMinN) { groups = 1; break; }
   // contiguous groups of near-equal molecule count, in input order
+  std::array<int, kSizeBuckets> peers{};
+  for (const MoleculeInput& m : mols) ++peers[size_bucket(molecule_nao(m))];
   int atom = 0, mol = 0;
   for (int g = 0; g < groups; ++g) {
     const int cnt = n_ / groups + (g < n_ % groups ? 1 : 0);
@@ -46,7 +48,7 @@ GroupedBatch::GroupedBatch(Engine* eng, const std::vector<MoleculeInput>& mols, 
     first_mol_.push_back(mol);
     first_atom_.push_back(atom);
     g_.emplace_back(new Batch(eng, part, diis_m, st));
-    if (groups > 1) g_.back()->set_shared();
+    if (groups > 1) g_.back()->set_shared(peers);
     for (const MoleculeInput& m : part) atom += (int)m.Z.size();
     mol += cnt;
   }

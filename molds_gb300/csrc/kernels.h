@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "nddo_batch.cuh"
+#include "schedule.h"
 
 namespace nddo {
 
@@ -44,8 +45,7 @@ constexpr int kSmallJacobiMaxN = 194;
 // FP64 lists of at most this many molecules with a basis of at least
 // kClusterJacobiMinN use the cluster Jacobi (one 8-CTA cluster per molecule)
 constexpr int kClusterJacobiMaxMols = 8;
-constexpr int kClusterJacobiMinN = 32;
-constexpr int kJacobiBuckets = 9;   // size buckets of a molecule list (edges in Batch::upload_list)
+constexpr int kClusterJacobiMinN = kSizeBucketEdges[0] + 1;
 size_t block_jacobi_workspace(int max_n, int nslots, int elem, long long* stride, long long* qstride);
 int launch_block_jacobi_f32(const DevMol* mols, const int* list, int nlist, int max_n, const MolState* st,
                             const float* G, const double* Cin, double* Cout, double* eps, void* ws, int max_sweeps,
@@ -159,10 +159,12 @@ int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n,
 int hh_smem_max_n();     // largest basis whose packed matrix fits one CTA's shared memory
 int hh_back_max_n();     // largest basis the back-transformation kernel serves
 void hh_prepare();       // one-time kernel attributes and device limits (before any stream capture)
-// molecules above max_n_served are skipped (the whole-GPU path serves them)
+// molecules above max_n_served are skipped (the whole-GPU path serves them);
+// peers: molecules like the list's, itself included, that are tridiagonalised at
+// about the same time on other streams as well (0: this list's alone)
 void launch_hh_tridiag(const DevMol* mols, const int* list, int nlist, int max_n, const MolState* st,
                        int require_active, const double* F, double* W, double* td, long long vstride, double* Aws,
-                       int max_n_served, cudaStream_t s);
+                       int max_n_served, int peers, cudaStream_t s);
 // eigenvalues (bisection + Laguerre) and inverse-iteration vectors of T into
 // eps and the columns of Z (N x k per molecule)
 void launch_tri_vectors(const DevMol* mols, const int* list, int nlist, int max_n, int max_k, const MolState* st,

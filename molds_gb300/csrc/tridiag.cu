@@ -48,8 +48,6 @@ namespace nddo {
 
 constexpr int kHhMaxThreads = 1024;   // the CTA size comes from the tuning table (256, 512 or 1024)
 constexpr int kHhCluster = 8, kHhClusterThreads = 512;   // cluster kernel: CTAs per molecule, threads per CTA
-constexpr int kHhClusterMinN = 195;   // its smallest basis, one more than an edge of the engine's size buckets
-constexpr int kHhClusterWaveN = 100;  // basis functions that pay for a wave of clusters, see the launcher
 constexpr int kHhRowShift = 3;        // log2 of the lanes that share a row's product there
 constexpr int kVecThreads = 32;   // one warp: 16 lane pairs, 16 eigenpairs per CTA
 constexpr int kOrthThreads = 256;
@@ -1259,16 +1257,12 @@ void hh_prepare() {
 
 void launch_hh_tridiag(const DevMol* mols, const int* list, int nlist, int max_n, const MolState* st,
                        int require_active, const double* F, double* W, double* td, long long vstride, double* Aws,
-                       int max_n_served, cudaStream_t s) {
+                       int max_n_served, int peers, cudaStream_t s) {
   if (nlist <= 0 || max_n <= 0) return;
   hh_set_attributes();
-  // A cluster has an SM for each CTA, so 15 or so run at a time; a wave of them has
-  // to cost less than its share of the one-CTA kernel, whose time grows as N^3 while
-  // its SMs hold up to 152 molecules: two waves at N = 234 2.9 ms against 3.5, three
-  // at 300 6.8 against 7.3, three at 396 11.7 against 16; two at 180 2.0 against 1.8.
   int lo_n = 0;
-  const int cap = std::min(max_n, hh_cluster_max_n()), waves = (nlist + hh_clusters() - 1) / hh_clusters();
-  if (max_n >= kHhClusterMinN && waves * kHhClusterWaveN <= cap) {
+  const int cap = std::min(max_n, hh_cluster_max_n());
+  if (hh_cluster_pays(std::max(nlist, peers), cap, hh_clusters())) {
     hh_tridiag_cluster_kernel<<<kHhCluster * nlist, kHhClusterThreads, hh_cluster_smem_bytes(cap), s>>>(
         mols, list, st, require_active, F, W, td, vstride, std::min(cap, max_n_served));
     if (max_n <= cap) return;
