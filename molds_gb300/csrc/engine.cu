@@ -1397,37 +1397,20 @@ void Batch::scf(const ScfSettings& s, bool requires_guess) {
   // so the device never waits for the host.  Every kernel of an iteration
   // skips molecules that are no longer active, so the iterations enqueued past
   // convergence change nothing (and cost only their empty launches).
-  // A molecule that the purification did not treat waits without advancing until
-  // the host has read that count too and enqueues an iteration of more effort:
-  // 0 few purification steps (18 to 24 are the rule), 1 as many as it has (the
-  // first iterations, whose gaps are small), 2 the eigensolver as well.  From the
-  // second wait for the eigensolver on every iteration has it.
   const int block = all.size() == 1 ? 3 : tuned_check_block();
-  const bool pur = purified(s), tiled = pur && !pur_list_[2].empty();   // the one-CTA kernel stops by itself
-  const int early = tiled ? kPurEarly : 0;
-  int it = 0, nblock = 0, waits = 0, effort = 0, since = 0;   // effort used from block `since` on
-  for (;;) {
-    // past max_iter only molecules that waited are still active
-    for (int b = 0; b < block && (b == 0 || it < s.max_iter); ++b, ++it)
-      iterate_graph(s, all, std::max(b == 0 || waits > 1 ? effort : 0, it < early ? 1 : 0));
-    const bool last = it >= s.max_iter;
-    const int slot = nblock & 1;
-    count_active_async(all, h_block_count_ + 2 * slot, h_block_active_ + (size_t)slot * cap_.slots, block_ev_[slot]);
-    ++nblock;
-    if (last && !pur) break;
-    if (nblock < 2 && !last) continue;
-    const int seen = last ? nblock - 1 : nblock - 2;   // block whose counts are read
-    cuda_check(cudaEventSynchronize(block_ev_[seen & 1]), "block count");
-    if (prof_on_) std::copy(h_block_active_ + (size_t)(seen & 1) * cap_.slots,
-                            h_block_active_ + (size_t)(seen & 1) * cap_.slots + h_mols.size(), active_host_.begin());
-    if (h_block_count_[2 * (seen & 1)] == 0) break;
-    const bool waiting = h_block_count_[2 * (seen & 1) + 1] > 0;
-    if (waits > 1 || seen < since) continue;
-    const int next = !waiting ? 0 : std::min(2, tiled ? effort + 1 : 2);
-    waits += next == 2;
-    if (next > effort) since = nblock;
-    effort = next;
-  }
+  const bool pur = purified(s);
+  run_blocks(
+      block, s.max_iter, pur, EffortPlan(pur && !pur_list_[2].empty(), kPurEarly),
+      [&](int effort) { iterate_graph(s, all, effort); },
+      [&](int slot) {
+        count_active_async(all, h_block_count_ + 2 * slot, h_block_active_ + (size_t)slot * cap_.slots, block_ev_[slot]);
+      },
+      [&](int slot) {
+        cuda_check(cudaEventSynchronize(block_ev_[slot]), "block count");
+        if (prof_on_) std::copy(h_block_active_ + (size_t)slot * cap_.slots,
+                                h_block_active_ + (size_t)slot * cap_.slots + h_mols.size(), active_host_.begin());
+        return BlockCounts{h_block_count_[2 * slot], h_block_count_[2 * slot + 1]};
+      });
   finish(s, all);
   int err = 0;
   copy_wait_error_async(&err);

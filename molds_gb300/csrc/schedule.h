@@ -28,4 +28,79 @@ inline bool hh_cluster_pays(int count, int n, int clusters) {
   return n >= kHhClusterMinN && (count + clusters - 1) / clusters * kHhClusterWaveN <= n;
 }
 
+// The effort of each SCF iteration of a batch whose density comes from the
+// purification.  Effort 0: few purification steps (18 to 24 are the rule), 1: as many
+// as it has, 2: the eigensolver as well.  A molecule that the purification did not
+// treat waits without advancing until the host has read the counts of its block and
+// enqueues an iteration of more effort.  The first `early` iterations, whose gaps are
+// small, have effort 1 from the start.  A wait after few steps asks for all of them in
+// the next blocks, and for good at the second time; a wait although a block had all of
+// them asks for the eigensolver in the first iteration of the next blocks, and in
+// every iteration from the second time on.  tiled: some molecule is on the tile kernel;
+// the one-CTA kernel takes the steps it needs at any effort.
+// Raised only for a block's first iteration, effort 1 could not settle a molecule that
+// keeps needing more than the few steps: it was counted as waiting again at the
+// block's end and the whole batch went over to the eigensolver.
+class EffortPlan {
+ public:
+  EffortPlan(bool tiled, int early) : tiled_(tiled), early_(tiled ? early : 0) {}
+  // effort of the b-th iteration of block `block`, the it-th of all
+  int next(int block, int b, int it) {
+    const int e = std::max(b == 0 ? first_ : rest_, it < early_ ? 1 : 0);
+    int& low = low_[block & 1];
+    low = b == 0 ? e : std::min(low, e);
+    return e;
+  }
+  // whether a molecule was waiting at the end of block `block`; `upcoming` is the
+  // next one to be enqueued
+  void seen(int block, bool waiting, int upcoming) {
+    if (rest_ == 2 || block < since_) return;   // nothing more to raise, or enqueued before the last raise
+    if (!waiting) {
+      first_ = rest_ = step_waits_ > 1 ? 1 : 0;
+      return;
+    }
+    if (tiled_ && low_[block & 1] == 0) {
+      ++step_waits_;
+      first_ = rest_ = 1;
+    } else {
+      ++eigen_waits_;
+      first_ = 2;
+      rest_ = eigen_waits_ > 1 ? 2 : tiled_ ? 1 : 0;
+    }
+    since_ = upcoming;
+  }
+
+ private:
+  bool tiled_;
+  int early_;
+  int first_ = 0, rest_ = 0;                // effort of a block's first iteration and of its others
+  int step_waits_ = 0, eigen_waits_ = 0;
+  int since_ = 0;                           // first block enqueued with the efforts of the last raise
+  int low_[2] = {0, 0};                     // lowest effort of the last two blocks
+};
+
+// molecules still active after a block, and those of them that wait
+struct BlockCounts { int active, waiting; };
+
+// The SCF loop: blocks of iterations, enqueued one ahead of the counts that are read.
+// iterate(effort) enqueues an iteration, count(slot) the counts after a block, read(slot)
+// waits for them (slot 0 or 1, alternately).  Past max_iter only molecules that waited
+// are still active.
+template <typename Iterate, typename Count, typename Read>
+void run_blocks(int block, int max_iter, bool purified, EffortPlan plan, Iterate iterate, Count count, Read read) {
+  int it = 0, nblock = 0;
+  for (;;) {
+    for (int b = 0; b < block && (b == 0 || it < max_iter); ++b, ++it) iterate(plan.next(nblock, b, it));
+    const bool last = it >= max_iter;
+    count(nblock & 1);
+    ++nblock;
+    if (last && !purified) break;
+    if (nblock < 2 && !last) continue;
+    const int seen = last ? nblock - 1 : nblock - 2;
+    const BlockCounts c = read(seen & 1);
+    if (c.active == 0) break;
+    plan.seen(seen, c.waiting > 0, nblock);
+  }
+}
+
 }  // namespace nddo

@@ -32,3 +32,56 @@ def test_size_buckets(rule):
     for k, e in enumerate(edges):
         assert int(rule("bucket", e)) == k and int(rule("bucket", e + 1)) == k + 1
     assert int(rule("bucket", 1)) == 0 and int(rule("bucket", 100000)) == len(edges)
+
+
+NEVER = 1000   # steps that no iteration has
+
+
+def _scf(rule, mols, tiled=1, block=3, max_iter=100):
+    """iterations of each effort; (status, waits) of each molecule (converged, from, steps)"""
+    out = [int(x) for x in rule("scf", tiled, 6, block, max_iter, 32, 56, *[v for m in mols for v in m]).split()]
+    return out[:3], list(zip(out[3::2], out[4::2]))
+
+
+@pytest.mark.parametrize("block", [1, 2, 3])
+def test_effort_without_waits(rule, block):
+    used, mols = _scf(rule, [(20, 0, 24), (31, 0, 32)], block=block)
+    assert mols == [(1, 0), (1, 0)]
+    assert used[1:] == [6, 0] and used[0] <= 25 + 2 * block
+
+
+@pytest.mark.parametrize("block", [1, 2, 3])
+@pytest.mark.parametrize("steps", [33, 56])
+def test_more_steps_settle_without_the_eigensolver(rule, block, steps):
+    """A molecule that goes on needing more than the few steps: it waits twice at
+    most, once for each raise, and the eigensolver is never launched."""
+    used, mols = _scf(rule, [(20, 0, 24), (60, 8, steps)], block=block)
+    assert mols[0] == (1, 0) and mols[1][0] == 1
+    assert used[2] == 0
+    assert mols[1][1] <= 4 * block
+    assert sum(used) <= 60 + 7 * block
+
+
+@pytest.mark.parametrize("block", [1, 2, 3])
+@pytest.mark.parametrize("tiled", [0, 1])
+def test_no_gap_takes_the_eigensolver(rule, block, tiled):
+    used, mols = _scf(rule, [(20, 0, 24), (40, 0, NEVER)], tiled=tiled, block=block)
+    assert mols[0] == (1, 0) and mols[1][0] == 1
+    assert used[2] >= 38 and mols[1][1] <= 4 * block
+    assert sum(used) <= 40 + 7 * block
+
+
+@pytest.mark.parametrize("block", [1, 2, 3])
+@pytest.mark.parametrize("tiled", [0, 1])
+def test_single_iteration_without_a_gap(rule, block, tiled):
+    """One iteration that needs the eigensolver, and one later that needs all steps."""
+    used, mols = _scf(rule, [(40, 12, 24), (41, 40, NEVER)], tiled=tiled, block=block)
+    assert mols[0] == (1, 0) and mols[1][0] == 1 and used[2] >= 1
+
+
+@pytest.mark.parametrize("max_iter", [1, 2, 7])
+@pytest.mark.parametrize("mol", [(50, 0, 24), (50, 0, 40), (50, 0, NEVER), (50, 6, NEVER)])
+def test_max_iter_ends_the_loop(rule, max_iter, mol):
+    """Molecules that waited are carried past max_iter until they have had it."""
+    used, mols = _scf(rule, [mol, (50, 0, 24)], max_iter=max_iter)
+    assert [m[0] for m in mols] == [2, 2]
