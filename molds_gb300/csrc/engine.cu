@@ -49,6 +49,7 @@ __global__ void init_state_kernel(const DevMol* __restrict__ mols, const int* __
     memset(&s, 0, sizeof(s));
     s.status = kActive;
     s.requires_guess = requires_guess;
+    s.flags = mol.natoms == 1 ? kNeedEigen : 0;
     s.ecore = st[m].ecore;   // computed by the integral pass
     s.ecore_epc = st[m].ecore_epc;
     st[m] = s;
@@ -638,7 +639,9 @@ void Batch::build_jobs(const std::vector<int>& which) {
   }
   // purification lists and tiles
   for (int k = 0; k < 3; ++k) { pur_list_[k].clear(); pur_max_n_[k] = 0; }
+  lone_atom_ = false;
   for (int m : which) {
+    if (h_mols[m].natoms == 1) { lone_atom_ = true; continue; }
     const int n = h_mols[m].nao, k = n <= 64 ? 0 : (n <= kPurSmallMaxN ? 1 : 2);
     pur_list_[k].push_back(m);
     pur_max_n_[k] = std::max(pur_max_n_[k], n);
@@ -1400,7 +1403,7 @@ void Batch::scf(const ScfSettings& s, bool requires_guess) {
   const int block = all.size() == 1 ? 3 : tuned_check_block();
   const bool pur = purified(s);
   run_blocks(
-      block, s.max_iter, pur, EffortPlan(pur && !pur_list_[2].empty(), kPurEarly),
+      block, s.max_iter, pur, EffortPlan(pur && !pur_list_[2].empty(), kPurEarly, pur && lone_atom_),
       [&](int effort) { iterate_graph(s, all, effort); },
       [&](int slot) {
         count_active_async(all, h_block_count_ + 2 * slot, h_block_active_ + (size_t)slot * cap_.slots, block_ev_[slot]);

@@ -243,6 +243,7 @@ class Batch {
   std::vector<int> pur_list_[3];
   int* d_pur_list_[3] = {};
   int pur_max_n_[3] = {};
+  bool lone_atom_ = false;               // the list holds one (see kNeedEigen)
   std::vector<int4> pur_tiles_;
   int pur_tn_ = 64;                      // their columns
   int4* d_pur_tiles_ = nullptr;

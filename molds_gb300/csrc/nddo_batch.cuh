@@ -43,7 +43,9 @@ struct DevMol {
 enum MolStatus { kActive = 0, kConverged = 1, kNotConverged = 2, kFailed = 3 };
 
 // MolState::flags: the purification gave no density.  The molecule then waits,
-// its state untouched, for an iteration that runs the eigensolver as well.
+// its state untouched, for an iteration that runs the eigensolver as well.  A lone
+// atom has the flag throughout and is not purified: its p shell is partly filled, so
+// it has no gap (a lone hydrogen has an odd electron and is refused).
 constexpr int kNeedEigen = 1;
 
 struct MolState {

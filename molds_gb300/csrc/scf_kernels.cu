@@ -183,7 +183,6 @@ __device__ void diis_decide(MolState* s, const ScfParamsDev& prm, long long n2, 
                      (count == M);
   __syncwarp();
   if (lane == 0) {
-    s->flags &= ~kNeedEigen;
     if (trace && iter < trace_len) {
       TraceEntry te;
       te.rms = rms; te.diis_err = s->diis_err; te.diis_on = s->diis_on; te.damp_on = s->damp_on;
@@ -376,7 +375,10 @@ diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol
     }
     if (lane == 0) s_sum[k] = t;
   }
-  if (lane == 0) ticket[li] = 0;
+  if (lane == 0) {
+    ticket[li] = 0;
+    if (mol.natoms > 1) s->flags &= ~kNeedEigen;
+  }
   __syncwarp();
   diis_decide(s, prm, n2, s_sum, trace ? trace + (long long)m * trace_len : nullptr, trace_len, steps + li, s_a, s_f);
 }

@@ -270,6 +270,7 @@ bool Server::lane_step(Lane& L) {
     L.slot_tsubmit[slot] = tq;
     L.slot_tadmit[slot] = now();
     fresh.push_back(slot);
+    if (b.natoms(slot) == 1) L.eigen = 8;   // a lone atom has no gap
   }
   if (!fresh.empty()) {
     b.integrals(fresh);

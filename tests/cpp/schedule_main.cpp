@@ -1,7 +1,7 @@
 // Prints the rules of schedule.h.  Usage:
 //   schedule_main cluster COUNT N CLUSTERS   whether the cluster tridiagonalisation pays
 //   schedule_main bucket N                   size bucket
-//   schedule_main scf TILED EARLY BLOCK MAX_ITER FEW ALL (CONVERGED FROM STEPS)...
+//   schedule_main scf TILED EARLY GAPLESS BLOCK MAX_ITER FEW ALL (CONVERGED FROM STEPS)...
 //                                            the SCF loop over molecules that converge
 //                                            in iteration CONVERGED and need STEPS
 //                                            purification steps from iteration FROM on,
@@ -16,11 +16,11 @@
 
 struct Mol { int converged, from, steps, iter = 0, status = 0, waits = 0; bool flag = false; };
 
-static void scf(bool tiled, int early, int block, int max_iter, int few, int all, std::vector<Mol> mols) {
+static void scf(bool tiled, int early, bool gapless, int block, int max_iter, int few, int all, std::vector<Mol> mols) {
   int used[3] = {0, 0, 0};
   nddo::BlockCounts slots[2] = {};
   nddo::run_blocks(
-      block, max_iter, true, nddo::EffortPlan(tiled, early),
+      block, max_iter, true, nddo::EffortPlan(tiled, early, gapless),
       [&](int effort) {
         ++used[effort];
         for (Mol& m : mols) {
@@ -47,10 +47,10 @@ int main(int argc, char** argv) {
   auto arg = [&](int k) { return std::atoi(argv[k]); };
   if (mode == "cluster" && argc == 5) std::printf("%d\n", (int)nddo::hh_cluster_pays(arg(2), arg(3), arg(4)));
   else if (mode == "bucket" && argc == 3) std::printf("%d\n", nddo::size_bucket(arg(2)));
-  else if (mode == "scf" && argc >= 11 && (argc - 8) % 3 == 0) {
+  else if (mode == "scf" && argc >= 12 && (argc - 9) % 3 == 0) {
     std::vector<Mol> mols;
-    for (int k = 8; k < argc; k += 3) mols.push_back({arg(k), arg(k + 1), arg(k + 2)});
-    scf(arg(2), arg(3), arg(4), arg(5), arg(6), arg(7), mols);
+    for (int k = 9; k < argc; k += 3) mols.push_back({arg(k), arg(k + 1), arg(k + 2)});
+    scf(arg(2), arg(3), arg(4), arg(5), arg(6), arg(7), arg(8), mols);
   } else return 2;
   return 0;
 }

@@ -37,9 +37,9 @@ def test_size_buckets(rule):
 NEVER = 1000   # steps that no iteration has
 
 
-def _scf(rule, mols, tiled=1, block=3, max_iter=100):
+def _scf(rule, mols, tiled=1, block=3, max_iter=100, gapless=0):
     """iterations of each effort; (status, waits) of each molecule (converged, from, steps)"""
-    out = [int(x) for x in rule("scf", tiled, 6, block, max_iter, 32, 56, *[v for m in mols for v in m]).split()]
+    out = [int(x) for x in rule("scf", tiled, 6, gapless, block, max_iter, 32, 56, *[v for m in mols for v in m]).split()]
     return out[:3], list(zip(out[3::2], out[4::2]))
 
 
@@ -85,3 +85,11 @@ def test_max_iter_ends_the_loop(rule, max_iter, mol):
     """Molecules that waited are carried past max_iter until they have had it."""
     used, mols = _scf(rule, [mol, (50, 0, 24)], max_iter=max_iter)
     assert [m[0] for m in mols] == [2, 2]
+
+
+@pytest.mark.parametrize("block", [1, 2, 3])
+@pytest.mark.parametrize("tiled", [0, 1])
+def test_known_gapless_never_waits(rule, block, tiled):
+    used, mols = _scf(rule, [(20, 0, 24), (2, 0, NEVER)], tiled=tiled, block=block, gapless=1)
+    assert mols == [(1, 0), (1, 0)]
+    assert used[:2] == [0, 0] and used[2] <= 20 + 2 * block
