@@ -959,8 +959,9 @@ void Batch::integrals(const std::vector<int>& which) {
   cuda_check(cudaGetLastError(), "pair_kernel");
   h = prof_begin(kKHcore, 0.0);
   launches_ += 2;
+  // the eigensolver's d, e, tau are not in use yet (an atom has a basis function at least)
   launch_hcore_kernel(d_atoms, d_pairs, d_mols, d_list, (int)which.size(), list_max_atoms(), d_blocks, d_ecore_pair,
-                      eng_->eri(), d_epc, d_H, d_state, stream_);
+                      d_td, eng_->eri(), d_epc, d_H, d_state, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "hcore_kernel");
   // the pageable index vectors above must outlive their copies

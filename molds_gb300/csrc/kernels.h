@@ -74,9 +74,10 @@ void launch_pair_kernels_split(const DevAtom* atoms, const DevPair* pairs, const
                                const int* light_list, long long n_light, const DevMol* mols, const EriTable* eri,
                                const OverlapTable* ovt, double* blocks, double* H, double* ecore_pair,
                                cudaStream_t s);
+// ecore_row: scratch, a double per atom from each molecule's vec0 on
 void launch_hcore_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
-                         int nlist, int max_atoms, const double* blocks, double* ecore_pair, const EriTable* eri,
-                         const double* epc, double* H, MolState* st, cudaStream_t s);
+                         int nlist, int max_atoms, const double* blocks, const double* ecore_pair, double* ecore_row,
+                         const EriTable* eri, const double* epc, double* H, MolState* st, cudaStream_t s);
 void launch_fock_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
                         int nlist, int max_atoms, const double* blocks, const double* H, const double* P, double* F,
                         double* Pold, const MolState* st, int mode_override, int copy_old, int require_active,

@@ -46,7 +46,8 @@ constexpr size_t kOffMol = align256(kOffPairs + sizeof(DevPair) * kNoAllocMaxPai
 constexpr size_t kOffList = align256(kOffMol + sizeof(DevMol));
 constexpr size_t kOffState = align256(kOffList + sizeof(int));
 constexpr size_t kOffEcore = align256(kOffState + sizeof(MolState));
-constexpr size_t kOffRowOff = align256(kOffEcore + sizeof(double) * kNoAllocMaxPairs);
+constexpr size_t kOffEcoreRow = align256(kOffEcore + sizeof(double) * kNoAllocMaxPairs);
+constexpr size_t kOffRowOff = align256(kOffEcoreRow + sizeof(double) * kNoAllocMaxAtoms);
 constexpr size_t kOffEri = align256(kOffRowOff + sizeof(long long) * kNoAllocMaxAtoms);
 constexpr size_t kOffOvt = align256(kOffEri + sizeof(EriTable));
 constexpr size_t kScratchBytes = align256(kOffOvt + sizeof(OverlapTable));
@@ -242,8 +243,8 @@ extern "C" int nddo_pair_integrals_noalloc(int device, int theory, int n_atoms, 
       }
     }
     if (ce == cudaSuccess) {
-      launch_hcore_kernel(d_atoms, d_pairs, d_mol, d_list, 1, n_atoms, d_pair_blocks, d_ecore, d_eri, nullptr,
-                          d_core_hamiltonian, d_state, s);
+      launch_hcore_kernel(d_atoms, d_pairs, d_mol, d_list, 1, n_atoms, d_pair_blocks, d_ecore,
+                          reinterpret_cast<double*>(base + kOffEcoreRow), d_eri, nullptr, d_core_hamiltonian, d_state, s);
       ce = cudaGetLastError();
     }
     double ecore = 0.0;

@@ -463,7 +463,7 @@ __device__ __forceinline__ double epc_slot_value(const EriTable* __restrict__ er
 __global__ void __launch_bounds__(kFockThreads)
 hcore_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, const DevMol* __restrict__ mols,
              const int* __restrict__ mol_list, const double* __restrict__ blocks,
-             double* __restrict__ ecore_pair, const EriTable* __restrict__ eri,
+             const double* __restrict__ ecore_pair, double* __restrict__ ecore_row, const EriTable* __restrict__ eri,
              const double* __restrict__ epc, double* __restrict__ H) {
   const int m = mol_list[blockIdx.y];
   const DevMol mol = mols[m];
@@ -471,13 +471,13 @@ hcore_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pair
   const long long ld = mol.nao;
   // a warp per atom
   for (int ia = blockIdx.x * nwarps + warp; ia < mol.natoms; ia += gridDim.x * nwarps) {
-    // the row's core-core energies, sum over B > A, in the place of its first one
+    // the row's core-core energies, sum over B > A
     if (ia + 1 < mol.natoms) {
-      double* row = ecore_pair + mol.pair0 + pair_index(ia, ia + 1, mol.natoms);
+      const double* row = ecore_pair + mol.pair0 + pair_index(ia, ia + 1, mol.natoms);
       double e = 0.0;
       for (int k = lane; k < mol.natoms - 1 - ia; k += 32) e += row[k];
       e = warp_sum(e);
-      if (lane == 0) row[0] = e;
+      if (lane == 0) ecore_row[mol.vec0 + ia] = e;
     }
     const DevAtom A = atoms[mol.atom0 + ia];
     const int dA = A.nao == 4 ? 10 : 1;
@@ -538,14 +538,14 @@ hcore_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pair
 // in the field of the point charges
 __global__ void __launch_bounds__(kFockThreads)
 ecore_kernel(const DevAtom* __restrict__ atoms, const DevMol* __restrict__ mols, const int* __restrict__ mol_list,
-             const double* __restrict__ ecore_pair, const double* __restrict__ epc, MolState* __restrict__ st) {
+             const double* __restrict__ ecore_row, const double* __restrict__ epc, MolState* __restrict__ st) {
   __shared__ double red[2][kFockThreads / 32];
   const int m = mol_list[blockIdx.x];
   const DevMol mol = mols[m];
   const int tid = threadIdx.x;
   double e = 0.0, q = 0.0;
   for (int ia = tid; ia + 1 < mol.natoms; ia += kFockThreads)
-    e += ecore_pair[mol.pair0 + pair_index(ia, ia + 1, mol.natoms)];
+    e += ecore_row[mol.vec0 + ia];
   for (long long t = tid; t < (long long)mol.natoms * mol.nepc; t += kFockThreads) {
     const DevAtom& A = atoms[mol.atom0 + t / mol.nepc];
     const double* pc = epc + 4 * (mol.epc0 + t % mol.nepc);
@@ -790,13 +790,14 @@ void launch_pair_kernels_split(const DevAtom* atoms, const DevPair* pairs, const
 }
 
 void launch_hcore_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
-                         int nlist, int max_atoms, const double* blocks, double* ecore_pair, const EriTable* eri,
-                         const double* epc, double* H, MolState* st, cudaStream_t s) {
+                         int nlist, int max_atoms, const double* blocks, const double* ecore_pair,
+                         double* ecore_row, const EriTable* eri, const double* epc, double* H, MolState* st,
+                         cudaStream_t s) {
   if (nlist <= 0) return;
   constexpr int kWarps = kFockThreads / 32;
   hcore_kernel<<<dim3((max_atoms + kWarps - 1) / kWarps, nlist), kFockThreads, 0, s>>>(
-      atoms, pairs, mols, mol_list, blocks, ecore_pair, eri, epc, H);
-  ecore_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, mols, mol_list, ecore_pair, epc, st);
+      atoms, pairs, mols, mol_list, blocks, ecore_pair, ecore_row, eri, epc, H);
+  ecore_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, mols, mol_list, ecore_row, epc, st);
 }
 
 void launch_fock_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,

@@ -6,6 +6,8 @@
 //                   again with the usual limit, a whole SCF of either kind; prints
 //                   flags, iteration, error word and the energies
 //   server MOLECULE a served request after a lane's wait error was set
+//   hcore MOLECULE  the core-core energy after the integrals and after the core
+//                   Hamiltonian was formed from them once more
 // MOLECULE: the theory number, then "Z x y z" per line (bohr).
 #include <cstdio>
 #include <cstdlib>
@@ -173,11 +175,28 @@ static int server(const char* file) {
   return 0;
 }
 
+static int hcore(const char* file) {
+  Engine eng(0);
+  Batch b(&eng, {molecule(file)}, 5);
+  for (int k = 0; k < 2; ++k) {
+    if (k == 0) b.integrals();
+    else
+      launch_hcore_kernel(b.d_atoms, b.d_pairs, b.d_mols, b.d_list, 1, b.natoms(0), b.d_blocks, b.d_ecore_pair, b.d_td,
+                          eng.eri(), b.d_epc, b.d_H, b.d_state, b.stream());
+    MolState st;
+    b.copy_states_async(&st);
+    cuda_check(cudaStreamSynchronize(b.stream()), "hcore");
+    std::printf("ecore %.17e\n", st.ecore);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   try {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "purify" && argc == 4) return purify(argv[2], argv[3]);
     if (mode == "waits" && argc == 3) return waits(argv[2]);
+    if (mode == "hcore" && argc == 3) return hcore(argv[2]);
     if (mode == "server" && argc == 3) return server(argv[2]);
     std::fprintf(stderr, "unknown mode\n");
     return 2;
