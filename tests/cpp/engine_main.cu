@@ -6,6 +6,8 @@
 //                   again with the usual limit, a whole SCF of either kind; prints
 //                   flags, iteration, error word and the energies
 //   server MOLECULE a served request after a lane's wait error was set
+//   guess MOLECULE  flags, iteration and error word after an iteration from the guess
+//                   that has every purification step but not the eigensolver
 //   hcore MOLECULE  the core-core energy after the integrals and after the core
 //                   Hamiltonian was formed from them once more
 // MOLECULE: the theory number, then "Z x y z" per line (bohr).
@@ -175,6 +177,22 @@ static int server(const char* file) {
   return 0;
 }
 
+static int guess(const char* file) {
+  const ScfSettings s = settings();
+  Engine eng(0);
+  Batch b(&eng, {molecule(file)}, s.diis_num_error_vect);
+  b.integrals();
+  b.begin(s, {0}, true);
+  b.iterate(s, {0}, 1);
+  MolState st;
+  int err = 0;
+  b.copy_states_async(&st);
+  b.copy_wait_error_async(&err);
+  cuda_check(cudaStreamSynchronize(b.stream()), "iteration");
+  std::printf("n %d flags %d iter %d error %d\n", b.nao(0), st.flags, st.iter, err);
+  return 0;
+}
+
 static int hcore(const char* file) {
   Engine eng(0);
   Batch b(&eng, {molecule(file)}, 5);
@@ -196,6 +214,7 @@ int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "purify" && argc == 4) return purify(argv[2], argv[3]);
     if (mode == "waits" && argc == 3) return waits(argv[2]);
+    if (mode == "guess" && argc == 3) return guess(argv[2]);
     if (mode == "hcore" && argc == 3) return hcore(argv[2]);
     if (mode == "server" && argc == 3) return server(argv[2]);
     std::fprintf(stderr, "unknown mode\n");
