@@ -38,9 +38,9 @@ struct EriTable {
   EriTerm terms[kNumSlots][kMaxTermsPerSlot];
   // local packed 10x10 entry (mu<=nu on A, la<=si on B) -> slot (or -1 = zero)
   signed char slot_of[10][10];
-  // the terms of all slots behind one another, those a pair with a hydrogen can
-  // need first (flat_light of flat_heavy): slot s has nterms[s] from flat_first[s] on
-  int flat_light, flat_heavy;
+  // the terms of all slots behind one another, nflat in all: slot s has nterms[s] from
+  // flat_first[s] on
+  int nflat;
   int flat_first[kNumSlots];
   EriTerm flat[kMaxFlatTerms];
 };
@@ -73,18 +73,6 @@ __host__ __device__ inline void unpack_index(int k, int* m, int* n) {
   *m = mm[k]; *n = nn[k];
 }
 
-template <typename T>
-__host__ __device__ inline T eval_term(const EriTerm& t, T R, const T* dA, const T* dB,
-                                       const T* rA, const T* rB) {
-  T da = dA[t.la], db = dB[t.lb];
-  T l = R + (T)t.c1 * da + (T)t.c2 * db;
-  T u = (T)t.c3 * da + (T)t.c4 * db;
-  T v = (T)t.c5 * da + (T)t.c6 * db;
-  T a = rA[t.la] + rB[t.lb];
-  T arg = l * l + u * u + v * v + a * a;
-  return t.coef * ((T)1 / sqrt(arg));
-}
-
 // rotation: rows = space-frame orbital (s, py, pz, px), columns = local
 // orbital, local z along A->B and gamma = 0 (MolDS Cndo2.cpp:5498-5527 with
 // EularAngle.cpp:38-64, written without trigonometric round trips).
@@ -102,53 +90,7 @@ __host__ __device__ inline void rotation_matrix(T x, T y, T z, T Rm[4][4]) {
   Rm[3][1] = -sa; Rm[3][2] = ca * sb; Rm[3][3] = ca * cb;
 }
 
-// T2[(mu nu)][(i j)] for packed pairs: the rotation of a product of two
-// orbitals, symmetrised over the local pair so that a symmetric local block
-// L[(ij)][(kl)] (stored once per unordered pair) rotates as T2 L T2^T.
-template <typename T>
-__host__ __device__ inline T pair_rotation(const T Rm[4][4], int P, int Q) {
-  int m, n, i, j;
-  unpack_index(P, &m, &n);
-  unpack_index(Q, &i, &j);
-  if (i == j) return Rm[m][i] * Rm[n][i];
-  return Rm[m][i] * Rm[n][j] + Rm[m][j] * Rm[n][i];
-}
-
-// A_k(p) = int_1^inf xi^k e^{-p xi}: closed sum, every k independent
-template <typename T>
-__host__ __device__ inline T aux_a(int k, T p) {
-  // e^{-p} * sum_{m=0}^{k} k!/m! / p^{k-m+1}
-  T s = 0, term = (T)1 / p;        // m = k term: 1/p
-  for (int m = k; m >= 0; --m) {
-    s += term;
-    term *= (T)m / p;              // next: k!/(m-1)! / p^{k-m+2}
-  }
-  return exp(-p) * s;
-}
-
-// B_k(q) = int_-1^1 eta^k e^{-q eta}: series for |q| < 3, closed sums otherwise
-template <typename T>
-__host__ __device__ inline T aux_b(int k, T q) {
-  if (fabs(q) < (T)3) {
-    T term = 1, sum = 0;
-    for (int m = 0; m < 80; ++m) {
-      if (((k + m) & 1) == 0) sum += term * (T)2 / (T)(k + m + 1);
-      term *= -q / (T)(m + 1);
-    }
-    return sum;
-  }
-  // B_k = [-e^{-q} sum_m k!/(k-m)! q^{-(m+1)}] + [(-1)^k e^{q} sum_m (-1)^m k!/(k-m)! q^{-(m+1)}]
-  T s1 = 0, s2 = 0, f = (T)1 / q;
-  for (int m = 0; m <= k; ++m) {
-    s1 += f;
-    s2 += (m & 1) ? -f : f;
-    f *= (T)(k - m) / q;
-  }
-  T sgn = (k & 1) ? (T)-1 : (T)1;
-  return -exp(-q) * s1 + sgn * exp(q) * s2;
-}
-
-// All A_k(p), k = 0..kmax, by the upward recurrence A_k = (e^-p + k A_{k-1}) / p
+// All A_k(p) = int_1^inf xi^k e^{-p xi}, k = 0..kmax, by the upward recurrence A_k = (e^-p + k A_{k-1}) / p
 // (stable for p > 0: every term is positive).
 template <typename T>
 __host__ __device__ inline void aux_a_all(T p, int kmax, T* a) {
@@ -158,7 +100,7 @@ __host__ __device__ inline void aux_a_all(T p, int kmax, T* a) {
   for (int k = 1; k <= kmax; ++k) { v = (e + (T)k * v) * ip; a[k] = v; }
 }
 
-// All B_k(q), k = 0..kmax.  For |q| <= 4: B_kmax from its power series, then
+// All B_k(q) = int_-1^1 eta^k e^{-q eta}, k = 0..kmax.  For |q| <= 4: B_kmax from its power series, then
 // the downward recurrence B_{k-1} = (q B_k - (-1)^k e^q + e^-q) / k, which
 // damps errors by |q|/k per step.  For |q| > 4: the upward recurrence
 // B_k = (k B_{k-1} + (-1)^k e^q - e^-q) / q from B_0 = (e^q - e^-q) / q, whose

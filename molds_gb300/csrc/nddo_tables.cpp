@@ -204,19 +204,16 @@ void build_eri_table(EriTable* t) {
   set(8, 3, 19); set(5, 1, 19);
   set(8, 8, 20); set(5, 5, 20);
   set(6, 6, 21);
-  // flat list: (ss|ss), the X-H slots of either atom order, then the others
-  static const int order[21] = {0, 3, 4, 10, 1, 2, 13, 5, 6, 7, 8, 9, 11, 12, 14, 15, 16, 17, 18, 19, 20};
   int n = 0;
   t->flat_first[21] = 0;   // slot 21 is a combination of two others
   for (int k = 0; k < 21; ++k) {
-    if (k == 7) t->flat_light = n;
-    t->flat_first[order[k]] = n;
-    for (int q = 0; q < t->nterms[order[k]]; ++q) {
+    t->flat_first[k] = n;
+    for (int q = 0; q < t->nterms[k]; ++q) {
       if (n == kMaxFlatTerms) throw std::logic_error("two-centre term table overflow");
-      t->flat[n++] = t->terms[order[k]][q];
+      t->flat[n++] = t->terms[k][q];
     }
   }
-  t->flat_heavy = n;
+  t->nflat = n;
 }
 
 void build_overlap_table(OverlapTable* t) {

@@ -240,6 +240,7 @@ pair_light_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__
   ecore_pair[p] = core_core(px, py, R, s0, mol.theory);
 }
 
+// Pairs of two atoms with s and p orbitals, one warp per pair.
 __global__ void __launch_bounds__(kPairWarps * 32)
 pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs, const int* __restrict__ list,
             long long npairs, const DevMol* __restrict__ mols, const EriTable* __restrict__ eri,
@@ -249,7 +250,7 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   __shared__ double s_T2[kPairWarps][100];
   __shared__ double s_L[kPairWarps][100];
   __shared__ double s_M[kPairWarps][100];
-  __shared__ double s_ab[kPairWarps][4][24];
+  __shared__ double s_ab[kPairWarps][4][2][7];
   __shared__ double s_ov[kPairWarps][8];
   __shared__ double s_R[kPairWarps][16];
   __shared__ double s_term[kPairWarps][kMaxFlatTerms];
@@ -267,8 +268,6 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   const nddo_atom_params& pb = c_params[B.pidx];
   const double dx = B.x - A.x, dy = B.y - A.y, dz = B.z - A.z;
   const double R = sqrt(dx * dx + dy * dy + dz * dz);
-  const int nA = A.nao, nB = B.nao;
-  const int dA = nA == 4 ? 10 : 1, dB = nB == 4 ? 10 : 1;
 
   // ---- rotation matrix (lane 0) ------------------------------------------
   if (lane == 0) {
@@ -280,8 +279,7 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   // ---- local two-centre integrals: lane = point-charge term, then lane = slot.
   // A warp instruction takes the FP64 pipe 64 clocks however few lanes it has:
   // by slot, 21 lanes walked up to 24 terms each.
-  const bool heavy = nA == 4 && nB == 4;
-  const int nterm = heavy ? eri->flat_heavy : eri->flat_light;
+  const int nterm = eri->nflat;
   for (int t = lane; t < nterm; t += 32) {
     const EriTerm e = eri->flat[t];
     const double da = sel3(e.la, pa.d[0], pa.d[1], pa.d[2]);
@@ -298,38 +296,25 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
   __syncwarp();
   double val = 0.0;
   if (lane < 21) {
-    bool need;
-    if (heavy) need = true;
-    else if (nA == 4) need = (lane == 0 || lane == 3 || lane == 4 || lane == 10);
-    else if (nB == 4) need = (lane == 0 || lane == 1 || lane == 2 || lane == 13);
-    else need = (lane == 0);
-    if (need) {
-      const int first = eri->flat_first[lane], nt = eri->nterms[lane];
-      for (int t = 0; t < nt; ++t) val += s_term[warp][first + t];
-    }
+    const int first = eri->flat_first[lane], nt = eri->nterms[lane];
+    for (int t = 0; t < nt; ++t) val += s_term[warp][first + t];
   }
   const double s5 = __shfl_sync(full, val, 5), s6 = __shfl_sync(full, val, 6);
-  if (lane == 21) val = heavy ? 0.5 * (s5 - s6) : 0.0;
+  if (lane == 21) val = 0.5 * (s5 - s6);
   if (lane < 22) s_val[warp][lane] = val;
 
-  // ---- overlap auxiliary integrals: lane zc computes A_0..11 of zeta combination
-  //      zc, lane 4 + zc its B_0..11 (zc: ss, s-p, p-s, p-p exponents) --------
+  // ---- overlap auxiliary integrals: lane zc computes A_0..6 of zeta combination
+  //      zc, lane 4 + zc its B_0..6 (zc: ss, s-p, p-s, p-p exponents) ----------
   const int na = pa.principal_n, nb = pb.principal_n;
   if (lane < 8) {
     const int zc = lane & 3;
-    const bool need = (zc == 0) || (zc == 1 && nB == 4) || (zc == 2 && nA == 4) || (zc == 3 && nA == 4 && nB == 4);
-    double v[12];
-    if (need) {
-      const double za = (zc >= 2) ? pa.zeta[1] : pa.zeta[0];
-      const double zb = (zc & 1) ? pb.zeta[1] : pb.zeta[0];
-      if (lane < 4) aux_a_all(0.5 * R * (za + zb), 6, v);
-      else aux_b_all(0.5 * R * (za - zb), 6, v, c_inv);
-    } else {
+    const double za = (zc >= 2) ? pa.zeta[1] : pa.zeta[0];
+    const double zb = (zc & 1) ? pb.zeta[1] : pb.zeta[0];
+    double v[7];
+    if (lane < 4) aux_a_all(0.5 * R * (za + zb), 6, v);
+    else aux_b_all(0.5 * R * (za - zb), 6, v, c_inv);
 #pragma unroll
-      for (int k = 0; k < 12; ++k) v[k] = 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < 12; ++k) s_ab[warp][zc][(lane < 4 ? 0 : 12) + k] = v[k];
+    for (int k = 0; k < 7; ++k) s_ab[warp][zc][lane >> 2][k] = v[k];
   }
   __syncwarp();
 
@@ -342,71 +327,59 @@ pair_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restrict__ pairs
     const double* Rm = s_R[warp];
     s_T2[warp][e] = (i == j) ? Rm[m * 4 + i] * Rm[n * 4 + i]
                              : Rm[m * 4 + i] * Rm[n * 4 + j] + Rm[m * 4 + j] * Rm[n * 4 + i];
-    double l = 0.0;
-    if (P < dA && Q < dB) {
-      const int sl = eri->slot_of[P][Q];
-      if (sl >= 0) l = s_val[warp][sl];
-    }
-    s_L[warp][e] = l;
+    const int sl = eri->slot_of[P][Q];
+    s_L[warp][e] = sl >= 0 ? s_val[warp][sl] : 0.0;
   }
   // overlap sums, lane = combination (ss, s-sigma, sigma-s, sigma-sigma, pi-pi)
   if (lane < 5) {
-    const int c = lane;
-    const bool need = (c == 0) || (c == 1 && nB == 4) || (c == 2 && nA == 4) || (c >= 3 && nA == 4 && nB == 4);
+    const int c = lane, zc = (c == 4) ? 3 : c;
+    const int nt = ovt->nterms[na - 1][nb - 1][c];
     double s = 0.0;
-    if (need) {
-      const int zc = (c == 4) ? 3 : c;
-      const int nt = ovt->nterms[na - 1][nb - 1][c];
-      for (int t = 0; t < nt; ++t)
-        s += ovt->tc[na - 1][nb - 1][c][t] * s_ab[warp][zc][ovt->ti[na - 1][nb - 1][c][t]] *
-             s_ab[warp][zc][12 + ovt->tj[na - 1][nb - 1][c][t]];
-      const double norm = pa.sto_norm[c >= 2 ? 1 : 0] * pb.sto_norm[(c == 1 || c >= 3) ? 1 : 0];
-      double rp = 1.0;
-      for (int i = 0; i < na + nb + 1; ++i) rp *= 0.5 * R;
-      s *= norm * ovt->ang[c] * rp;
-    }
-    s_ov[warp][c] = s;
+    for (int t = 0; t < nt; ++t)
+      s += ovt->tc[na - 1][nb - 1][c][t] * s_ab[warp][zc][0][ovt->ti[na - 1][nb - 1][c][t]] *
+           s_ab[warp][zc][1][ovt->tj[na - 1][nb - 1][c][t]];
+    const double norm = pa.sto_norm[c >= 2 ? 1 : 0] * pb.sto_norm[(c == 1 || c >= 3) ? 1 : 0];
+    double rp = 1.0;
+    for (int i = 0; i < na + nb + 1; ++i) rp *= 0.5 * R;
+    s_ov[warp][c] = s * (norm * ovt->ang[c] * rp);
   }
   __syncwarp();
 
   // ---- M = L T2^T,  W = T2 M ----------------------------------------------
-  for (int e = lane; e < dA * 10; e += 32) {
+  for (int e = lane; e < 100; e += 32) {
     const int P = e / 10, Qp = e % 10;
     double s = 0.0;
-    if (Qp < dB)
-      for (int Q = 0; Q < dB; ++Q) s += s_L[warp][P * 10 + Q] * s_T2[warp][Qp * 10 + Q];
+    for (int Q = 0; Q < 10; ++Q) s += s_L[warp][P * 10 + Q] * s_T2[warp][Qp * 10 + Q];
     s_M[warp][e] = s;
   }
   __syncwarp();
   double* out = blocks + pr.blk;
-  for (int e = lane; e < dA * dB; e += 32) {
-    const int Pp = e / dB, Qp = e % dB;
+  for (int e = lane; e < 100; e += 32) {
+    const int Pp = e / 10, Qp = e % 10;
     double s = 0.0;
-    for (int P = 0; P < dA; ++P) s += s_T2[warp][Pp * 10 + P] * s_M[warp][P * 10 + Qp];
+    for (int P = 0; P < 10; ++P) s += s_T2[warp][Pp * 10 + P] * s_M[warp][P * 10 + Qp];
     out[e] = s;
   }
 
   // ---- resonance block of H:  1/2 (beta_mu + beta_nu) S_mu,nu --------------
   if (lane < 16) {
     const int mu = lane >> 2, nu = lane & 3;
-    if (mu < nA && nu < nB) {
-      double Ls[4][4] = {};
-      Ls[0][0] = s_ov[warp][0];
-      Ls[0][2] = s_ov[warp][1];
-      Ls[2][0] = s_ov[warp][2];
-      Ls[2][2] = s_ov[warp][3];
-      Ls[1][1] = s_ov[warp][4];
-      Ls[3][3] = s_ov[warp][4];
-      const double* Rm = s_R[warp];
-      double s = 0.0;
-      for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) s += Rm[mu * 4 + i] * Ls[i][j] * Rm[nu * 4 + j];
-      const double h = 0.5 * (pa.beta[mu == 0 ? 0 : 1] + pb.beta[nu == 0 ? 0 : 1]) * s;
-      const long long ld = mol.nao;
-      const long long r0 = A.ao0 + mu, c0 = B.ao0 + nu;
-      H[mol.mat0 + r0 * ld + c0] = h;
-      H[mol.mat0 + c0 * ld + r0] = h;
-    }
+    double Ls[4][4] = {};
+    Ls[0][0] = s_ov[warp][0];
+    Ls[0][2] = s_ov[warp][1];
+    Ls[2][0] = s_ov[warp][2];
+    Ls[2][2] = s_ov[warp][3];
+    Ls[1][1] = s_ov[warp][4];
+    Ls[3][3] = s_ov[warp][4];
+    const double* Rm = s_R[warp];
+    double s = 0.0;
+    for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j) s += Rm[mu * 4 + i] * Ls[i][j] * Rm[nu * 4 + j];
+    const double h = 0.5 * (pa.beta[mu == 0 ? 0 : 1] + pb.beta[nu == 0 ? 0 : 1]) * s;
+    const long long ld = mol.nao;
+    const long long r0 = A.ao0 + mu, c0 = B.ao0 + nu;
+    H[mol.mat0 + r0 * ld + c0] = h;
+    H[mol.mat0 + c0 * ld + r0] = h;
   }
 
   // ---- core-core repulsion --------------------------------------------------
