@@ -10,9 +10,10 @@ Mulliken charges of all 256 molecules.
   python bench.py [--gpus N] [--steps K] [--warmup W] [--precision fp64|mixed]
   python bench.py --impl reference ...      # the CPU restatement on the host cores
 
-The headline line is the FP64 path (every eigensolve, Fock build, density,
-DIIS and energy in FP64), as the workload specifies; the mixed-precision
-path is measured on the same molecules and reported under the "mixed" key.
+The headline line is the FP64 path (every Fock build, eigensolve, DIIS and energy in
+FP64, the densities by purification in fixed point with 55 fraction bits), as the
+workload specifies; precision = mixed is measured on the same molecules and reported
+under the "mixed" key.
 
 Prints one JSON line.  Under torchrun (N > 1) each rank solves its own 256
 replicas (weak scaling) and rank 0 reports the max-over-ranks time.
@@ -47,6 +48,9 @@ def parse():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--precision", default=None, choices=["fp64", "mixed"],
                     help="default: mixed for the uneven alkanes (their precision ramp), fp64 otherwise")
+    ap.add_argument("--eigensolver", default="auto", choices=["auto", "householder", "jacobi"],
+                    help="auto: densities by purification, whose products are exact in either precision; "
+                         "householder, jacobi: an eigensolve in every iteration")
     ap.add_argument("--no-mixed", action="store_true", help="skip the mixed-precision measurement")
     ap.add_argument("--nmol", type=int, default=N_MOL)
     ap.add_argument("--dipole", default="on", choices=["on", "off"],
@@ -72,6 +76,25 @@ def parse():
     if a.precision is None:
         a.precision = "mixed" if a.workload == "alkanes" else "fp64"
     return a
+
+
+def compute_dtype(args, precision=None):
+    """The mixed path has an FP32 phase only with an eigensolver; the purification is
+    FP64-exact (fixed point, 55 fraction bits) in either precision."""
+    return "fp32+fp64" if (precision or args.precision) == "mixed" and args.eigensolver != "auto" else "f64"
+
+
+def mixed_note(args):
+    if args.eigensolver == "auto":
+        return ("default eigensolver: both phases form the density by the FP64-exact purification, so this repeats "
+                "the FP64 path; an FP32 phase needs --eigensolver householder or jacobi")
+    if args.eigensolver == "jacobi":
+        return ("FP32 phase (Jacobi eigensolver and density in FP32 and 3xTF32) until the DIIS error is below 1e-4, "
+                "then FP64; integrals, Fock build, DIIS, core-core and energies always FP64")
+    return ("FP32 phase (back-transformation of the density's eigenvectors on the CUDA cores in FP32, "
+            "density on the tensor cores, 3xTF32) until the DIIS error is below 1e-4, then FP64; "
+            "integrals, Fock build, eigensolve (tridiagonalisation, bisection, inverse iteration), DIIS, "
+            "core-core and energies always FP64")
 
 
 def workload(rank: int, nmol: int):
@@ -278,7 +301,7 @@ def run_ours(args):
     torch.cuda.set_device(local)
     ctx = M.Context(local)
     mols = workload(rank, args.nmol)
-    params = M.SCFParams(**SCF, precision=args.precision, dipole=args.dipole == "on")
+    params = M.SCFParams(**SCF, precision=args.precision, eigensolver=args.eigensolver, dipole=args.dipole == "on")
     batch = M.ResidentBatch("am1", mols, context=ctx)
 
     batch.profile(True)            # the per-class event pool is created during the warm-up
@@ -348,7 +371,7 @@ def run_ours(args):
     if not args.no_mixed and args.precision == "fp64":
         nP = min(32, args.nmol)
         P64 = [batch.density(i, 192) for i in range(nP)]
-        pm = M.SCFParams(**SCF, precision="mixed", dipole=args.dipole == "on")
+        pm = M.SCFParams(**SCF, precision="mixed", eigensolver=args.eigensolver, dipole=args.dipole == "on")
         for _ in range(args.warmup):
             batch.run(pm)
         barrier_sync(dist)
@@ -364,11 +387,7 @@ def run_ours(args):
         dP = [float(np.max(np.abs(batch.density(i, 192) - P64[i]))) for i in range(nP)]
         its_m = [r["iterations"] for r in res_m]
         mixed = {"value": aggregate_throughput(world, args.nmol, ms_mixed), "unit": "solves/s",
-                 "ms_per_step": ms_mixed, "dtype": "fp32+fp64",
-                 "what": "FP32 phase (back-transformation of the density's eigenvectors on the CUDA cores in FP32, "
-                         "density on the tensor cores, 3xTF32) until the DIIS error is below 1e-4, then FP64; "
-                         "integrals, Fock build, eigensolve (tridiagonalisation, bisection, inverse iteration), DIIS, "
-                         "core-core and energies always FP64",
+                 "ms_per_step": ms_mixed, "dtype": compute_dtype(args, "mixed"), "what": mixed_note(args),
                  "max_abs_dE_vs_fp64_gpu_Eh": float(de.max()),
                  "p50_abs_dE_vs_fp64_gpu_Eh": float(np.percentile(de, 50)),
                  "p99_abs_dE_vs_fp64_gpu_Eh": float(np.percentile(de, 99)),
@@ -381,8 +400,8 @@ def run_ours(args):
     # ---- plain path: one molecule at a time, FP64, ElectronicStructure ------
     plain = None
     if rank == 0 and args.plain_sample > 0:
-        es = M.ElectronicStructure("am1", M.SCFParams(**SCF, precision="fp64", dipole=args.dipole == "on"),
-                                   context=ctx)
+        es = M.ElectronicStructure("am1", M.SCFParams(**SCF, precision="fp64", eigensolver=args.eigensolver,
+                                                      dipole=args.dipole == "on"), context=ctx)
         lat = []
         for i, m in enumerate(mols[:args.plain_sample] * 2):
             t0 = time.perf_counter()
@@ -408,22 +427,33 @@ def run_ours(args):
             dom = name
             break
     d = kt[dom]
-    compute_bound = dom in ("purification", "jacobi_eigensolver", "warm_start_transform", "basis_orthonormalise", "density",
+    compute_bound = dom in ("jacobi_eigensolver", "warm_start_transform", "basis_orthonormalise", "density",
                             "fp64_refinement", "tridiagonalisation", "tridiagonal_eigenvectors")
     roof = None
     if rank == 0 and d["launches"] > 0 and d["ms"] > 0:
         avg_ms = d["ms"] / d["launches"]
         per_launch = d["work"] / d["launches"]
-        if compute_bound:
-            prec = "fp64" if (dom in ("purification", "fp64_refinement", "tridiagonalisation", "tridiagonal_eigenvectors")
+        if dom == "purification":
+            peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
+                os.path.join(ROOT, "MEASURED_PEAKS.json")) else {"bf16_tflops_sustained": 1700.0}
+            peak = peaks["bf16_tflops_sustained"]
+            achieved = d["work"] / args.steps / (per_step_ms * 1e-3) / 1e12
+            roof = {"bound": "tensor (tcgen05 kind::f16)", "kernel": dom, "achieved": achieved, "peak": peak,
+                    "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None, "traffic_source": None,
+                    "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained (FP16 has bf16's rate)",
+                    "work_per_launch": per_launch, "avg_launch_ms": avg_ms, "launches": d["launches"],
+                    "note": "executed FP16 flops of the digit products (34 a purification step, over the tiles' 128 "
+                            "rows, by the steps that the molecules took) over the whole benchmark step, other kernels "
+                            "included, so achieved is a lower bound.  A launch here is a molecule group's purification "
+                            "of one SCF iteration, empty steps included; its CUDA events span the other groups' kernels "
+                            "as well"}
+        elif compute_bound:
+            prec = "fp64" if (dom in ("fp64_refinement", "tridiagonalisation", "tridiagonal_eigenvectors")
                               or args.precision == "fp64") else "fp32"
             peak = ctx.fma_peak_tflops(prec)
             achieved = per_launch / (avg_ms * 1e-3) / 1e12
             traffic, tsrc = profiled_traffic(dom)
-            work_note = {"purification": "work = (4/3) N^3 + 3 N^2 k flops per molecule, the eigensolve and density it "
-                                         "stands in for (its products run on the tensor cores in exact digit slices, "
-                                         "so this rate may exceed the FP64 pipe's)",
-                         "tridiagonalisation": "work = (4/3) N^3 flops per molecule, the tridiagonalisation share "
+            work_note = {"tridiagonalisation": "work = (4/3) N^3 flops per molecule, the tridiagonalisation share "
                                                "of the (10/3) N^3 eigensolver convention",
                          "jacobi_eigensolver": "work by the (10/3) N^3 eigensolver convention"}.get(dom, "algorithmic flops")
             roof = {"bound": f"{prec}-cuda-core", "kernel": dom, "achieved": achieved, "peak": peak,
@@ -458,11 +488,11 @@ def run_ours(args):
         line = {"metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": per_step_ms, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None,
-                "dtype": "fp32+fp64" if args.precision == "mixed" else "f64",
+                "dtype": compute_dtype(args),
                 "data": "synthetic: seeded (H2O)32 replicas (no public dataset is named for this path)",
                 "config": {"workload": f"{args.nmol} replicas of (H2O)32 per GPU, AM1, batched SCF to RMS 1e-8",
                            "molecules_per_gpu": args.nmol, "atoms": 96, "basis_functions": 192, "occupied": 128,
-                           "precision": args.precision, "scf": SCF, "dipole": args.dipole == "on",
+                           "precision": args.precision, "eigensolver": args.eigensolver, "scf": SCF, "dipole": args.dipole == "on",
                            "l2": f"inputs larger than L2: {batch.device_bytes() / 1e9:.2f} GB resident per GPU",
                            "parallelism": f"replicas x{world} (molecules sharded, no collective)"},
                 "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
@@ -512,9 +542,10 @@ def _cpu_worker_pm3(args):
 def run_alkanes(args):
     """All molecules of this rank in one device-resident batch; a step =
     integrals + SCF + energies of all of them.  The uneven workload's precision
-    ramp is `--precision mixed` (FP32 back-transformation and density until the
-    DIIS error drops below 1e-4, FP64 eigensolve throughout); each molecule's
-    |dE| and max|dP| against the FP64 GPU path of the same batch.  Under
+    ramp is `--precision mixed`, which the default eigensolver's exact purification
+    does not need (with `--eigensolver householder`: FP32 back-transformation and
+    density until the DIIS error drops below 1e-4, FP64 eigensolve throughout); each
+    molecule's |dE| and max|dP| against the FP64 GPU path of the same batch.  Under
     torchrun the molecules are split over the ranks by predicted cost
     (molds_gb300/sharding.py)."""
     import numpy as np
@@ -544,7 +575,7 @@ def run_alkanes(args):
     nao = np.array([int(sum(4 if z > 1 else 1 for z in m.Z)) for m in mols])
     steps = args.steps if args.steps != 10 else 2
     warm = args.warmup if args.warmup != 3 else 1
-    params = M.SCFParams(**SCF, precision=args.precision, dipole=args.dipole == "on")
+    params = M.SCFParams(**SCF, precision=args.precision, eigensolver=args.eigensolver, dipole=args.dipole == "on")
     batch = M.ResidentBatch("pm3", mols, context=ctx)
     batch.profile(True)
     for _ in range(warm):
@@ -566,7 +597,7 @@ def run_alkanes(args):
     batch.profile(False)
     res, q = batch.results()
     ref = M.ResidentBatch("pm3", mols, context=ctx)
-    ref.run(M.SCFParams(**SCF, precision="fp64"))
+    ref.run(M.SCFParams(**SCF, precision="fp64", eigensolver=args.eigensolver))
     res64, q64 = ref.results()
     conv = np.array([r["status"] == M.STATUS_CONVERGED for r in res])
     conv64 = np.array([r["status"] == M.STATUS_CONVERGED for r in res64])
@@ -600,11 +631,11 @@ def run_alkanes(args):
     line = {"metric": "converged SCF solves/s, uneven batch of random alkanes with the precision ramp",
             "value": value, "unit": "solves/s", "n_gpus": world, "steps": steps, "warmup": warm, "ms_per_step": ms,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "fp32+fp64" if args.precision == "mixed" else "f64",
+            "dtype": compute_dtype(args),
             "data": f"synthetic: {args.alkanes} seeded random alkanes (seed 3e6 + j), generated in {t_gen:.1f} s",
             "config": {"workload": f"{args.alkanes} alkanes CnH2n+2, n uniform 3..60, PM3, one batch",
                        "basis_min_median_max": [int(nao.min()), int(np.median(nao)), int(nao.max())],
-                       "precision": args.precision, "scf": SCF, "dipole": args.dipole == "on",
+                       "precision": args.precision, "eigensolver": args.eigensolver, "scf": SCF, "dipole": args.dipole == "on",
                        "l2": f"inputs larger than L2: {batch.device_bytes() / 1e9:.2f} GB resident"},
             "gpu_launches": launches, "kernels_ms": {k: round(v["ms"] / steps, 3) for k, v in kt.items()},
             "convergence": {"converged": int(conv.sum()), "fp64_converged": int(conv64.sum()),
@@ -642,7 +673,7 @@ def run_octane(args):
     build.build()
     ctx = M.Context(0)
     mol = W.octane()
-    es = M.ElectronicStructure("pm3", M.SCFParams(**SCF, precision="fp64"), context=ctx)
+    es = M.ElectronicStructure("pm3", M.SCFParams(**SCF, precision="fp64", eigensolver=args.eigensolver), context=ctx)
     for _ in range(5):
         es.SetMolecule(mol)
         es.DoSCF()
@@ -697,7 +728,7 @@ def run_md(args):
     build.build()
     ctx = M.Context(0)
     mols = workload(0, args.nmol)
-    params = M.SCFParams(**SCF, precision=args.precision, dipole=args.dipole == "on")
+    params = M.SCFParams(**SCF, precision=args.precision, eigensolver=args.eigensolver, dipole=args.dipole == "on")
     b = M.ResidentBatch("am1", mols, context=ctx)
     rng = np.random.default_rng(7)
     x = np.concatenate([m.xyz for m in mols])
@@ -730,10 +761,10 @@ def run_md(args):
     line = {"metric": "warm-started SCF solves/s (MD / RPMD steps of resident molecules)", "value": value,
             "unit": "solves/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": 1e3 * wall / args.steps, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "fp32+fp64" if args.precision == "mixed" else "f64",
+            "vs_baseline": None, "dtype": compute_dtype(args),
             "data": "synthetic: seeded (H2O)32 replicas on a random walk",
             "config": {"workload": f"{args.nmol} replicas of (H2O)32, AM1, 0.01 A random-walk step, "
-                                   "SCF from the previous density", "precision": args.precision,
+                                   "SCF from the previous density", "precision": args.precision, "eigensolver": args.eigensolver,
                        "scf": SCF, "dipole": args.dipole == "on"},
             "e2e": {"value": value, "unit": "solves/s",
                     "h2d_bytes_per_step": int(x.size * 8), "d2h_bytes_per_step": int(args.nmol * ctypes.sizeof(M.ScfResultC)),
@@ -751,8 +782,8 @@ def run_md(args):
 # ---------------------------------------------------------------------------
 def run_water512(args):
     """One SCF of a 512-water cluster (8x8x8 jittered lattice, seed 4) under
-    MNDO through the plain ElectronicStructure path (N = 3072: the whole-GPU
-    Householder eigensolver), FP64 and then mixed precision, with the RMS /
+    MNDO through the plain ElectronicStructure path (N = 3072: densities by
+    purification, final eigenpairs by the whole-GPU Householder eigensolver), FP64 and then mixed precision, with the RMS /
     DIIS-error trace.  The reference's algorithm does not converge on this
     cluster with the benchmark's SCF block (density DIIS falls into an
     occupation-swapping 2-cycle, in the oracle as here), so the line reports
@@ -769,7 +800,7 @@ def run_water512(args):
     clocks.start()
     precs = [args.precision] + (["mixed"] if args.precision == "fp64" and not args.no_mixed else [])
     for prec in precs:
-        es = M.ElectronicStructure("mndo", M.SCFParams(**scf, precision=prec), context=ctx)
+        es = M.ElectronicStructure("mndo", M.SCFParams(**scf, precision=prec, eigensolver=args.eigensolver), context=ctx)
         t0 = time.perf_counter()
         es.SetMolecule(mol)
         t1 = time.perf_counter()
@@ -790,7 +821,7 @@ def run_water512(args):
     line = {"metric": "large single SCF: (H2O)512 MNDO, seconds per SCF iteration", "value": first["s_per_iteration"],
             "unit": "s/iteration", "n_gpus": 1, "steps": 1, "warmup": 0, "ms_per_step": 1e3 * first["scf_s"],
             "higher_is_better": False, "scaling": "replicas only", "vs_baseline": None,
-            "dtype": "f64" if precs[0] == "fp64" else "fp32+fp64",
+            "dtype": compute_dtype(args, precs[0]),
             "data": "synthetic: (H2O)512 on a jittered 8x8x8 lattice, seed 4",
             "config": {"workload": "(H2O)512 MNDO, 1536 atoms, 3072 basis functions, 2048 occupied", "scf": scf},
             "runs": out, "clocks": clk}
@@ -814,7 +845,7 @@ def run_serving(args):
     mols = [m for _, m in stream]
     nao = [int(sum(4 if z > 1 else 1 for z in m.Z)) for m in mols]
     ctx = M.Context(0)
-    params = M.SCFParams(**SCF, precision=args.precision, dipole=args.dipole == "on")
+    params = M.SCFParams(**SCF, precision=args.precision, eigensolver=args.eigensolver, dipole=args.dipole == "on")
     srv = M.Server(params, hbm_budget_bytes=int(args.hbm_gb * (1 << 30)), max_basis=args.max_basis, context=ctx)
     # warm-up: one small and one large request
     srv.submit("pm3", W.water_cluster_k(8, 1))
@@ -867,11 +898,11 @@ def run_serving(args):
         print(json.dumps({"rate": rate, **per_rate[-1]}), file=sys.stderr, flush=True)
     clk = clocks.stop()
     srv.close()
-    # accuracy of the served (mixed-precision) energies against the FP64 path
+    # accuracy of the served energies against the FP64 path
     acc = None
     sample = list(range(0, len(mols), max(1, len(mols) // 48)))[:48]
     sample = [k for k in sample if k in energies]
-    ref, _ = M.batch_scf("pm3", [mols[k] for k in sample], M.SCFParams(**SCF, precision="fp64"), context=ctx)
+    ref, _ = M.batch_scf("pm3", [mols[k] for k in sample], M.SCFParams(**SCF, precision="fp64", eigensolver=args.eigensolver), context=ctx)
     both = [(k, r) for k, r in zip(sample, ref) if r["status"] == M.STATUS_CONVERGED]
     acc = {"sample": len(sample), "both_converged": len(both),
            "max_abs_dE_vs_fp64_gpu_Eh": max((abs(energies[k] - r["energy"]) for k, r in both), default=None)}
@@ -880,7 +911,7 @@ def run_serving(args):
                       "requests",
             "value": best["converged_solves_s"], "unit": "solves/s", "n_gpus": 1, "steps": len(rates), "warmup": 1,
             "ms_per_step": None, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "fp32+fp64" if args.precision == "mixed" else "f64",
+            "dtype": compute_dtype(args),
             "data": "synthetic: seeded serving stream (sizes log-uniform 5..500 atoms; alkanes n <= 60, "
                     "water clusters)",
             "config": {"workload": f"{len(mols)} PM3 requests per rate, Poisson arrivals, rates {rates}",

@@ -232,7 +232,8 @@ void nddo_batch_destroy(nddo_batch* b);
 /* Per-kernel-class CUDA-event timing on the launching stream: after enabling,
  * nddo_batch_kernel_times returns, per class, the accumulated milliseconds,
  * the number of timed launches and the algorithmic work of those launches
- * (FLOPs for contractions and the eigensolver, bytes for memory-bound steps).
+ * (FLOPs for contractions and the eigensolver, bytes for memory-bound steps; for
+ * the purification the FP16 flops of the steps that its molecules took).
  * Returns the number of classes. */
 int nddo_batch_profile(nddo_batch* b, int enable);
 int nddo_batch_kernel_times(nddo_batch* b, int max_classes, double* ms, long long* launches, double* work);

@@ -355,6 +355,7 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_hh_large_ = dalloc<int>(nm, &bytes_);
   for (int k = 0; k < 3; ++k) d_pur_list_[k] = dalloc<int>(nm, &bytes_);
   d_pur_ = dalloc<PurState>(nm, &bytes_);
+  cuda_check(cudaMemsetAsync(d_pur_, 0, sizeof(PurState) * (size_t)nm, stream_), "memset purification state");
   // 129 basis functions have four wide tiles; larger bases have fewer per
   // element; narrow ones are used up to one per SM
   pur_tile_cap_ = cap.max_n > kPurSmallMaxN ? (size_t)(mat / 4096) + 16 + hh_grid_ctas() : 1;
@@ -821,6 +822,16 @@ void Batch::profile_collect(double* ms, long long* launches, double* work) {
   }
   recs_.clear();
   ev_used_ = 0;
+  // the purification's executed flops, from the steps the molecules took
+  if (prof_launches_[kKPurify] > 0) {
+    std::vector<unsigned long long> steps(h_mols.size());
+    cuda_check(cudaMemcpy2DAsync(steps.data(), sizeof(steps[0]), &d_pur_->steps, sizeof(PurState), sizeof(steps[0]),
+                                 steps.size(), cudaMemcpyDeviceToHost, stream_), "profile steps");
+    cuda_check(cudaStreamSynchronize(stream_), "profile steps");
+    prof_work_[kKPurify] = 0.0;
+    for (size_t m = 0; m < steps.size(); ++m)
+      if (h_mols[m].nao > 0) prof_work_[kKPurify] += (double)steps[m] * purify_step_flops(h_mols[m].nao, pur_tn_);
+  }
   for (int k = 0; k < kKNumClasses; ++k) {
     if (ms) ms[k] = prof_ms_[k];
     if (launches) launches[k] = prof_launches_[k];
@@ -833,11 +844,14 @@ void Batch::profile_reset() {
   recs_.clear();
   ev_used_ = 0;
   for (int k = 0; k < kKNumClasses; ++k) { prof_ms_[k] = 0; prof_launches_[k] = 0; prof_work_[k] = 0; }
+  cuda_check(cudaMemset2DAsync(&d_pur_->steps, sizeof(PurState), 0, sizeof(unsigned long long), cap_.slots, stream_),
+             "profile steps");
 }
 
 // Algorithmic work of one launch over the molecules that are still active:
 // FLOPs for the contractions and the eigensolver (eigensolve counted as
-// 10/3 N^3 whatever the method), bytes for the memory-bound steps.
+// 10/3 N^3 whatever the method), bytes for the memory-bound steps.  (The
+// purification's is counted, not estimated: profile_collect.)
 double Batch::active_work_estimate(int cls) const {
   double w = 0.0;
   for (int m : cur_list_) {
@@ -850,8 +864,6 @@ double Batch::active_work_estimate(int cls) const {
       case kKTridiag: w += 4.0 / 3.0 * n * n * n; break;
       // back-transformation of the k = min(o, v) density vectors (2 N^2 k flops)
       case kKEigvec: w += 2.0 * n * n * std::min(o, v); break;
-      // P from F: the same count as the eigensolve and density it stands in for
-      case kKPurify: w += 4.0 / 3.0 * n * n * n + 3.0 * n * n * std::min(o, v); break;
       case kKTransform: w += 4.0 * n * n * n; break;
       case kKOrtho: w += 4.0 * n * n * n; break;
       case kKDensity: w += 2.0 * n * n * o; break;
@@ -1114,11 +1126,11 @@ void Batch::eigen_step(const ScfSettings& s, int effort) {
     // serve the molecules it could not treat (effort 2: launch them as well)
     const int require = purified(s) ? 2 : 1;
     if (purified(s)) {
-      const int h = prof_begin(kKPurify, active_work_estimate(kKPurify));
+      const int h = prof_begin(kKPurify, 0.0);   // its work: profile_collect
       for (int k = 0; k < 2; ++k) {
         launches_ += !pur_list_[k].empty();
         launch_purify_small(d_mols, d_pur_list_[k], (int)pur_list_[k].size(), pur_max_n_[k], d_state, d_F, d_P,
-                            d_wait_err_, pur_wait_, stream_);
+                            d_pur_, d_wait_err_, pur_wait_, stream_);
       }
       const PurScratch ws{{d_T64, d_S[0], d_S[1], d_S[2], d_S[3], d_S[4], d_S[5]}};
       launches_ += launch_purify_big(d_mols, d_pur_list_[2], (int)pur_list_[2].size(), pur_max_n_[2], d_pur_tiles_,

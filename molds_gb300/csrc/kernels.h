@@ -142,15 +142,17 @@ struct PurState {
   int bad;                           // 1 + the step in which a digit sum left the range its recombination covers
                                      // or a wait ran out; 0: none
   long long trace[kPurBigSteps + 1]; // tr X_k
+  unsigned long long steps;          // steps taken since Batch::profile_reset
 };
 struct PurScratch { double* m[7]; }; // N x N scratch matrices holding two digit buffers of seven digits each
 void purify_prepare();               // one-time kernel attributes (before any stream capture)
 // tiles of tn columns (64 or 32) of one molecule (out may be null); returns their number
 int purify_tiles(int mol, int n, int tn, int4* out);
+double purify_step_flops(int n, int tn);   // FP16 flops that one step of one molecule executes
 // limit: clocks after which a wait for a copy or an MMA counts as run out; the
 // molecule is then flagged and *err set
 void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
-                         double* P, int* err, long long limit, cudaStream_t s);
+                         double* P, PurState* pur, int* err, long long limit, cudaStream_t s);
 // alone: no other stream's work is expected beside this launch sequence
 // returns the number of kernels launched
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles, int tn,

@@ -315,7 +315,7 @@ template <int H, int L>
 __global__ void __launch_bounds__(kPurSmallThreads, 1)
 purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, MolState* __restrict__ st,
                     const double* __restrict__ F, double* __restrict__ P, int np_max, long long limit,
-                    int* __restrict__ err) {
+                    PurState* __restrict__ pur, int* __restrict__ err) {
   constexpr int G = (kLevels + L - 1) / L;   // level groups
   extern __shared__ __align__(1024) unsigned char pu_sm[];
   const int mi = list[blockIdx.x];
@@ -448,7 +448,8 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   bool ok = true, done = false;
   int first = -1;
   long long t0 = 0, t1 = 0;   // traces of X_k and X_{k-1}
-  for (int k = 0; usable; ++k) {
+  int k = 0;
+  for (; usable; ++k) {
     // digits of X_k into shared memory, its diagonal
 #pragma unroll
     for (int h = 0; h < H; ++h) {
@@ -544,6 +545,7 @@ purify_small_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   if (tid == 0) {
     if (!ok) atomicExch(err, 1);
     st[mi].flags = done ? 0 : kNeedEigen;
+    atomicAdd(&pur[mi].steps, (unsigned long long)k);
   }
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols));
 }
@@ -847,7 +849,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
 // P = 2 X of the molecules whose iteration ended; the others are flagged
 __global__ void __launch_bounds__(256)
 purify_store_kernel(const DevMol* __restrict__ mols, const int* __restrict__ list, MolState* __restrict__ st,
-                    const PurState* __restrict__ pur, PurScratch ws, int steps, double* __restrict__ P) {
+                    PurState* __restrict__ pur, PurScratch ws, int steps, double* __restrict__ P) {
   const int mi = list[blockIdx.y];
   if (st[mi].status != kActive) return;
   const DevMol mol = mols[mi];
@@ -856,7 +858,10 @@ purify_store_kernel(const DevMol* __restrict__ mols, const int* __restrict__ lis
   const int first = pu_first(pur[mi].trace, steps);
   const bool done = !pur[mi].bad && pu_interval(pur[mi], &lo, &hi) && first >= 0 && first + 3 <= steps &&
                     pu_counted(pur[mi].trace[first + 3], (long long)mol.nocc * kTraceOne);
-  if (blockIdx.x == 0 && threadIdx.x == 0) st[mi].flags = done ? 0 : kNeedEigen;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st[mi].flags = done ? 0 : kNeedEigen;
+    atomicAdd(&pur[mi].steps, (unsigned long long)(first >= 0 && first + 3 < steps ? first + 3 : steps));
+  }
   if (!done) return;
   const int buf = (first + 3) & 1;
   double* Pm = P + mol.mat0;
@@ -906,16 +911,29 @@ int purify_tiles(int mol, int n, int tn, int4* out) {
   return t;
 }
 
+// 34 digit products, M = 128 rows whatever the basis
+double purify_step_flops(int n, int tn) {
+  if (n <= kPurSmallMaxN) {
+    const double np = (n + 15) / 16 * 16;
+    return 34.0 * 2.0 * kTileM * np * np;
+  }
+  const int np = (n + 31) / 32 * 32;
+  double cols = 0.0;
+  for (int i = 0; i * kTileM < np; ++i)
+    for (int j = kTileM / tn * i; j * tn < np; ++j) cols += std::min(tn, np - j * tn);
+  return 34.0 * 2.0 * kTileM * cols * np;
+}
+
 void launch_purify_small(const DevMol* mols, const int* list, int nlist, int max_n, MolState* st, const double* F,
-                         double* P, int* err, long long limit, cudaStream_t s) {
+                         double* P, PurState* pur, int* err, long long limit, cudaStream_t s) {
   if (nlist <= 0) return;
   purify_prepare();
   const int np = (max_n + 15) / 16 * 16;
   const size_t sm = small_smem(np);
   // levels per group: two buffers of L x np of the 512 columns of tensor memory
-  if (np <= 64) purify_small_kernel<1, 4><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, err);
-  else if (np <= 80) purify_small_kernel<2, 3><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, err);
-  else purify_small_kernel<2, 2><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, err);
+  if (np <= 64) purify_small_kernel<1, 4><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, pur, err);
+  else if (np <= 80) purify_small_kernel<2, 3><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, pur, err);
+  else purify_small_kernel<2, 2><<<nlist, kPurSmallThreads, sm, s>>>(mols, list, st, F, P, np, limit, pur, err);
 }
 
 int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n, const int4* tiles, int ntiles, int tn,

@@ -62,13 +62,13 @@ static int purify(const char* in, const char* out) {
   int* d_err = device(std::vector<int>{0});
   double* d_F = device(F);
   double* d_P = device(std::vector<double>(F.size(), 0.0));
+  PurState* d_pur = device(std::vector<PurState>(1));
   if (n <= kPurSmallMaxN) {
-    launch_purify_small(d_mol, d_list, 1, n, d_st, d_F, d_P, d_err, kPurWaitCycles, nullptr);
+    launch_purify_small(d_mol, d_list, 1, n, d_st, d_F, d_P, d_pur, d_err, kPurWaitCycles, nullptr);
   } else {
     std::vector<int4> tiles(purify_tiles(0, n, 64, nullptr));
     purify_tiles(0, n, 64, tiles.data());
     int4* d_tiles = device(tiles);
-    PurState* d_pur = device(std::vector<PurState>(1));
     PurScratch ws;
     for (double*& m : ws.m) m = device(std::vector<double>((F.size() + 31) / 32 * 32, 0.0));
     launch_purify_big(d_mol, d_list, 1, n, d_tiles, (int)tiles.size(), 64, d_st, d_F, d_P, d_pur, ws, kPurBigSteps, true,

@@ -30,3 +30,27 @@ def test_gapped_molecule_is_purified(exe, tmp_path, n):
 def test_small_gaps(exe, tmp_path, waters, flag):
     r = run_engine_program(exe, "guess", write_molecule(tmp_path, 0, _degenerate(waters)))
     assert r.stdout == f"n {6 * waters + 4} flags {flag} iter {1 - flag} error 0\n", (r.stdout, r.stderr)
+
+
+@pytest.mark.parametrize("waters", [8, 32])
+def test_executed_flops_count_the_steps(waters):
+    """kernel_times()'s work: 34 digit products a step over 128-row tiles, by the steps taken."""
+    import molds_gb300 as M
+    from molds_gb300 import workloads as W
+    ctx = M.Context(0)
+    b = M.ResidentBatch("am1", [W.water_cluster_k(waters, 3)], context=ctx)
+    p = M.SCFParams(damping_weight=0.0, diis_start_error=0.1, diis_end_error=0.0)
+    b.run(p)
+    b.profile(True)
+    b.run(p)
+    work = b.kernel_times()["purification"]["work"]
+    iterations = b.results()[0][0]["iterations"]
+    b.close()
+    ctx.close()
+    n = 6 * waters
+    if n <= 128:
+        step = 34 * 2 * 128 * 48 * 48
+    else:                                   # 192: row tiles 0 (192 columns) and 1 (64 columns)
+        step = 34 * 2 * 128 * (192 + 64) * 192
+    steps = work / step
+    assert steps == int(steps) and 12 * iterations <= steps <= 56 * iterations
