@@ -36,9 +36,9 @@ struct ScfSettings {
   int dipole = 1;               // dipole moment after convergence (MolDS DoSCF always computes it)
   int vdw = 0;                  // empirical dispersion energy (SCF block "vdW yes"; always on for AM1-D / PM3-D)
   double vdw_s6 = 1.40, vdw_d = 23.0;
-  int eigensolver = 0;          // FP64 eigensolves: 0 auto (Householder), 1 Jacobi, 2 Householder
-  int graphs = 1;               // replay each SCF iteration from a captured CUDA graph (Householder path,
-                                // profiling off)
+  int eigensolver = 0;          // 0 auto (purification, then Householder), 1 Jacobi, 2 Householder
+  int graphs = 1;               // replay each SCF iteration from a captured CUDA graph (not on the Jacobi path,
+                                // nor while profiling)
 };
 
 // settings that change the launches of an SCF iteration (a captured graph is
@@ -221,7 +221,7 @@ class Batch {
   double* d_blocks = nullptr;
   double* d_ecore_pair = nullptr;
   int* d_heavy_pairs = nullptr;   // indices of sp-sp pairs
-  int* d_light_pairs = nullptr;   // indices of pairs with a hydrogen (X-H first, then H-H)
+  int* d_light_pairs = nullptr;   // indices of pairs with a hydrogen
   double *d_H = nullptr, *d_F = nullptr, *d_P = nullptr, *d_Pold = nullptr, *d_C = nullptr, *d_eps = nullptr;
   double *d_hist_dens = nullptr, *d_hist_err = nullptr;
   float *d_G32 = nullptr, *d_T32 = nullptr;

@@ -127,9 +127,6 @@ void launch_jacobi_f64(const DevMol* mols, const int* mol_list, int nlist, int m
                        double* eps, double* Aws, double* Vws, long long ws_stride, int max_sweeps,
                        int* sweeps_out, cudaStream_t s);
 
-// tridiag.cu: FP64 Householder tridiagonalisation + bisection + inverse
-// iteration + back-transformation.  td holds d, e, tau of every molecule at
-// vec0, vec0 + vstride, vec0 + 2 vstride; W (N x N arena) the reflectors.
 // Purification (purify.cu): P = 2 (projector on the nocc lowest eigenvectors of
 // F) of the listed active molecules; sets or clears kNeedEigen in their state.
 constexpr int kPurSmallMaxN = 128;   // one CTA per molecule up to here, tiles of every step above
@@ -159,6 +156,9 @@ int launch_purify_big(const DevMol* mols, const int* list, int nlist, int max_n,
                       MolState* st, const double* F, double* P, PurState* pur, const PurScratch& ws, int steps,
                       bool alone, int* err, long long limit, cudaStream_t s);
 
+// tridiag.cu: FP64 Householder tridiagonalisation + bisection + inverse
+// iteration + back-transformation.  td holds d, e, tau of every molecule at
+// vec0, vec0 + vstride, vec0 + 2 vstride; W (N x N arena) the reflectors.
 int hh_smem_max_n();     // largest basis whose packed matrix fits one CTA's shared memory
 int hh_back_max_n();     // largest basis the back-transformation kernel serves
 void hh_prepare();       // one-time kernel attributes and device limits (before any stream capture)
@@ -230,8 +230,8 @@ void launch_gemm(const GemmJob* jobs, int njobs, int ntiles, const double* A, co
 void launch_gemm(const GemmJob* jobs, int njobs, int ntiles, const float* A, const double* B, double* C,
                  bool ta, bool tb, float acc_tag, const MolState* st, int require_active, int require_phase,
                  cudaStream_t s);
-// DIIS in three launches (partial sums, per-molecule solve, apply); scratch
-// holds diis_scratch_bytes(nlist) bytes
+// DIIS in two launches (partial sums with the per-molecule solve, apply); scratch
+// holds diis_scratch_bytes(slots) bytes, zero before the first launch
 size_t diis_scratch_bytes(int slots);
 void launch_diis(const DevMol* mols, const int* mol_list, int nlist, int max_n, MolState* st, const ScfParamsDev& prm,
                  double* P, const double* Pold, double* hist_dens, double* hist_err, long long hist_stride,

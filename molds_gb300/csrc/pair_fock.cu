@@ -14,11 +14,11 @@
 //     4030-4146), Mndo::GetDiatomCoreRepulsionEnergy (:319-327, :223-240) and
 //     Am1::GetDiatomCoreRepulsionEnergy (src/am1/Am1.cpp:145-170).
 //
-// (b) hcore_kernel / fock_kernel -- one CTA per atom.  Coulomb terms of the
-//     diagonal block of atom A are gathered from all partner blocks, a thread per
-//     partner and orbital pair, and summed in a fixed order, so the result does
-//     not depend on scheduling (bitwise reproducible, alone or in a batch).  The
-//     exchange block of a pair is written by the CTA of its first atom.
+// (b) hcore_kernel, a warp per atom, and fock_kernel, one CTA per atom.  Coulomb
+//     terms of the diagonal block of atom A are gathered from all partner blocks
+//     (Fock: a thread per partner and orbital pair) and summed in a fixed order, so
+//     the result does not depend on scheduling (bitwise reproducible, alone or in a
+//     batch).  The exchange block of a pair is written by the CTA of its first atom.
 //     MolDS: Cndo2::CalcFockMatrix (src/cndo/Cndo2.cpp:1526-1636) with
 //     Mndo::GetFockDiagElement (src/mndo/Mndo.cpp:422-488), GetFockOffDiagElement
 //     (:490-580), GetCoulombInt/GetExchangeInt (:583-639), GetElectronCoreAttraction

@@ -17,11 +17,13 @@
 // without any rounding (the error-free splitting of
 // Ozaki, Ogita, Oishi & Rump, Numer. Algorithms 59, 95 (2012)).  Level l sums
 // the digit products with i + j = l, levels 0 to 7 are kept (34 products) and
-// recombined in 64-bit integers.  What is dropped is below 2^-70 times the
-// number of terms, and each step's result is rounded once, at 2^-56 absolute:
-// finer than FP64's rounding of entries of order one.  Integer sums do not
-// depend on their order, so X stays exactly symmetric and a molecule's result
-// does not depend on its batch.
+// recombined in 64-bit integers, rounded to 2^-55 (half a step is 2^-56): finer than
+// FP64's rounding of entries of order one.  What is dropped, levels 8 to 12, is at
+// most 2^-64 a term of a level-8 product.  For a dense X it sums to 2^-57 at N = 256;
+// on the diagonal the squares of digit 4 make it a positive bias of about N 2^-65.6,
+// half a rounding step at N = 770 and two at 3072.  Integer sums do not depend on
+// their order, so X stays exactly symmetric and a molecule's result does not depend
+// on its batch.
 //
 // The error of the last step is known from the traces: tr X_{k+1} - tr X_k is
 // +- tr(X_k - X_k^2), the sum of lambda (1 - lambda).  Once that is below 2^-30
@@ -665,7 +667,7 @@ __device__ __forceinline__ int pu_first(const long long* T, int k) {
 }
 
 // One step of the molecules that still need one.  tiles: (molecule, row block,
-// column block, 0).  Warp 0 copies, warp 1 issues the MMAs, all eight
+// column block, 0).  Warp 0 copies, warp 1 issues the MMAs, all sixteen
 // recombine.
 template <int TN>
 __global__ void __launch_bounds__(kPurTileThreads, 1)
