@@ -372,12 +372,12 @@ void Batch::allocate(const BatchCapacity& cap) {
   d_count = dalloc<int>(2, &bytes_);
   d_wait_err_ = dalloc<int>(1, &bytes_);
   {
-    const size_t b = diis_scratch_bytes(nm);
+    const size_t b = diis_scratch_bytes(nm, cap.max_n);
     cuda_check(cudaMalloc(&d_diis_ws, b), "cudaMalloc DIIS scratch");
     cuda_check(cudaMemsetAsync(d_diis_ws, 0, b, stream_), "memset DIIS scratch");
     bytes_ += b;
   }
-  d_dip_ws = dalloc<double>((size_t)nm * kDipChunks * 4, &bytes_);
+  d_dip_ws = dalloc<double>(reduce_scratch_doubles(nm, cap.max_n), &bytes_);
   d_active = dalloc<char>(nm, &bytes_);
   cuda_check(cudaMemsetAsync(d_state, 0, nm * sizeof(MolState), stream_), "memset state");
   cuda_check(cudaMemsetAsync(d_sweeps, 0, nm * sizeof(int), stream_), "memset sweeps");
@@ -1282,7 +1282,7 @@ void Batch::iterate(const ScfSettings& s, const std::vector<int>& which, int eff
   ScfParamsDev prm = to_dev(s);
   prm.eigen_ran = effort == 2 || !purified(s);
   launch_diis(d_mols, d_list, nl, list_max_n_, d_state, prm, d_P, d_Pold, d_hist_dens, d_hist_err, mat_total_,
-              s.keep_trace ? d_trace : nullptr, max_iter_alloc_, d_diis_ws, cap_.slots, stream_);
+              s.keep_trace ? d_trace : nullptr, max_iter_alloc_, d_diis_ws, cap_.slots, cap_.max_n, stream_);
   prof_end(h);
   cuda_check(cudaGetLastError(), "diis_kernel");
 }

@@ -277,7 +277,7 @@ class Batch {
   int* d_wait_err_ = nullptr;            // set by a tensor-core kernel whose wait for a copy or an MMA ran out
   long long pur_wait_ = kPurWaitCycles;  // clocks that a wait of the purification may take
   void* d_diis_ws = nullptr;             // DIIS partial sums and decisions (diis_scratch_bytes)
-  double* d_dip_ws = nullptr;            // dipole partial sums (slots x kDipChunks x 4)
+  double* d_dip_ws = nullptr;            // energy and dipole partial sums (reduce_scratch_doubles)
   char* d_active = nullptr;
 
   // current molecule list and its GEMM job tables

@@ -92,13 +92,13 @@ struct VdwParams {
 void launch_forces(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, int m, long long pair0,
                    long long npairs, int natoms, const EriTable* eri, const OverlapTable* ovt, const double* P,
                    VdwParams vdw, double* grad, double* forces, cudaStream_t s);
-// partial: scratch of nlist x kDipChunks x 2 doubles
+// partial: reduce_scratch_doubles(nlist, max_n) doubles, as for launch_dipole
+size_t reduce_scratch_doubles(int slots, int cap_n);
 void launch_energy_kernel(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list,
                           int nlist, int max_n, const double* P, const double* F, const double* H, double* partial,
                           MolState* st, double* charges, VdwParams vdw, cudaStream_t s);
-// dipole moment of the listed molecules into MolState::dipole; partial holds
-// nlist * kDipChunks * 4 doubles
-constexpr int kDipChunks = 304;   // two CTAs on every SM
+// dipole moment of the listed molecules into MolState::dipole
+constexpr int kDipChunks = 304;   // CTAs of a molecule at most: two on every SM
 void launch_dipole(const DevAtom* atoms, const DevPair* pairs, const DevMol* mols, const int* mol_list, int nlist,
                    int max_atoms, const double* P, const double* H, double* partial, MolState* st, cudaStream_t s);
 // STO-6G Cartesian matrix of molecule m: X = 3 x N x N doubles
@@ -231,11 +231,12 @@ void launch_gemm(const GemmJob* jobs, int njobs, int ntiles, const float* A, con
                  bool ta, bool tb, float acc_tag, const MolState* st, int require_active, int require_phase,
                  cudaStream_t s);
 // DIIS in two launches (partial sums with the per-molecule solve, apply); scratch
-// holds diis_scratch_bytes(slots) bytes, zero before the first launch
-size_t diis_scratch_bytes(int slots);
+// holds diis_scratch_bytes(slots, cap_n) bytes, zero before the first launch, for
+// lists of up to `slots` molecules of up to cap_n basis functions
+size_t diis_scratch_bytes(int slots, int cap_n);
 void launch_diis(const DevMol* mols, const int* mol_list, int nlist, int max_n, MolState* st, const ScfParamsDev& prm,
                  double* P, const double* Pold, double* hist_dens, double* hist_err, long long hist_stride,
-                 TraceEntry* trace, int trace_len, void* scratch, int slots, cudaStream_t s);
+                 TraceEntry* trace, int trace_len, void* scratch, int slots, int cap_n, cudaStream_t s);
 
 void launch_newton_scale(const DevMol* mols, const int* mol_list, int nlist, const MolState* st, int require_phase,
                          double* K, const double* O, const double* eps, cudaStream_t s);

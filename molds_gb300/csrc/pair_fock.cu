@@ -834,22 +834,22 @@ energy_partial_kernel(const DevAtom* __restrict__ atoms, const DevPair* __restri
   if (threadIdx.x < 2) {
     double v = 0.0;
     for (int w = 0; w < kFockThreads / 32; ++w) v += red[threadIdx.x][w];
-    partial[((long long)blockIdx.y * kDipChunks + blockIdx.x) * 2 + threadIdx.x] = v;
+    partial[((long long)blockIdx.y * gridDim.x + blockIdx.x) * 2 + threadIdx.x] = v;
   }
 }
 
 __global__ void __launch_bounds__(kFockThreads)
 energy_kernel(const DevAtom* __restrict__ atoms, const DevMol* __restrict__ mols, const int* __restrict__ mol_list,
-              const double* __restrict__ P, const double* __restrict__ partial, MolState* __restrict__ st,
-              double* __restrict__ charges) {
+              int grid_chunks, const double* __restrict__ P, const double* __restrict__ partial,
+              MolState* __restrict__ st, double* __restrict__ charges) {
   __shared__ double red[3][kFockThreads / 32];
   const int m = mol_list[blockIdx.x], tid = threadIdx.x;
   const DevMol mol = mols[m];
   const int chunks = energy_chunks((long long)mol.nao * mol.nao);
   double e = 0.0, v = 0.0, f = 0.0;
   for (int c = tid; c < chunks; c += kFockThreads) {
-    e += partial[((long long)blockIdx.x * kDipChunks + c) * 2];
-    v += partial[((long long)blockIdx.x * kDipChunks + c) * 2 + 1];
+    e += partial[((long long)blockIdx.x * grid_chunks + c) * 2];
+    v += partial[((long long)blockIdx.x * grid_chunks + c) * 2 + 1];
   }
   for (int a = tid; a < mol.natoms; a += kFockThreads) {
     const DevAtom A = atoms[mol.atom0 + a];
@@ -880,9 +880,10 @@ void launch_energy_kernel(const DevAtom* atoms, const DevPair* pairs, const DevM
                           int nlist, int max_n, const double* P, const double* F, const double* H, double* partial,
                           MolState* st, double* charges, VdwParams vdw, cudaStream_t s) {
   if (nlist <= 0) return;
-  energy_partial_kernel<<<dim3(energy_chunks((long long)max_n * max_n), nlist), kFockThreads, 0, s>>>(
-      atoms, pairs, mols, mol_list, P, F, H, partial, vdw);
-  energy_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, mols, mol_list, P, partial, st, charges);
+  const int chunks = energy_chunks((long long)max_n * max_n);   // the largest molecule's count sets the grid
+  energy_partial_kernel<<<dim3(chunks, nlist), kFockThreads, 0, s>>>(atoms, pairs, mols, mol_list, P, F, H, partial,
+                                                                     vdw);
+  energy_kernel<<<nlist, kFockThreads, 0, s>>>(atoms, mols, mol_list, chunks, P, partial, st, charges);
 }
 
 // ---------------------------------------------------------------------------
@@ -1093,6 +1094,10 @@ __host__ __device__ __forceinline__ int dipole_chunks(int natoms) {
   const long long items = (long long)natoms + (long long)natoms * (natoms - 1) / 2;
   const long long c = (items + 4LL * (kDipThreads / 32) - 1) / (4LL * (kDipThreads / 32));   // four items a warp
   return (int)(c < 1 ? 1 : (c > kDipChunks ? kDipChunks : c));
+}
+
+size_t reduce_scratch_doubles(int slots, int cap_n) {
+  return (size_t)slots * std::max(2 * energy_chunks((long long)cap_n * cap_n), 4 * dipole_chunks(cap_n));
 }
 
 // One work item: atom t of the molecule (t < natoms, the same-atom block) or

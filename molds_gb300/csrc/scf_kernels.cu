@@ -156,7 +156,7 @@ constexpr int kDiisThreads = 256;
 constexpr int kDiisChunksMax = 128;
 constexpr int kDiisPart = 2 + kMaxDiis;     // sum e^2, max |e|, dots
 
-__device__ __forceinline__ int diis_chunks(long long n2) {
+__host__ __device__ __forceinline__ int diis_chunks(long long n2) {
   const long long c = (n2 + 2047) / 2048;
   return (int)(c < kDiisChunksMax ? (c < 1 ? 1 : c) : kDiisChunksMax);
 }
@@ -348,7 +348,7 @@ diis_partial_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol
     if (lane == 0) s_red[warp][k] = v[k];
   }
   __syncthreads();
-  double* out = part + (long long)li * kDiisChunksMax * kDiisPart;
+  double* out = part + (long long)li * gridDim.x * kDiisPart;
   if (tid < kDiisPart) {
     double t = s_red[0][tid];
     for (int w = 1; w < kWarps; ++w) t = tid == 1 ? fmax(t, s_red[w][tid]) : t + s_red[w][tid];
@@ -427,13 +427,12 @@ diis_apply_kernel(const DevMol* __restrict__ mols, const int* __restrict__ mol_l
 
 void launch_diis(const DevMol* mols, const int* mol_list, int nlist, int max_n, MolState* st, const ScfParamsDev& prm,
                  double* P, const double* Pold, double* hist_dens, double* hist_err, long long hist_stride,
-                 TraceEntry* trace, int trace_len, void* scratch, int slots, cudaStream_t s) {
+                 TraceEntry* trace, int trace_len, void* scratch, int slots, int cap_n, cudaStream_t s) {
   if (nlist <= 0) return;
   double* part = static_cast<double*>(scratch);
-  DiisStep* steps = reinterpret_cast<DiisStep*>(part + (size_t)slots * kDiisChunksMax * kDiisPart);
+  DiisStep* steps = reinterpret_cast<DiisStep*>(part + (size_t)slots * diis_chunks((long long)cap_n * cap_n) * kDiisPart);
   int* ticket = reinterpret_cast<int*>(steps + slots);
-  const long long n2 = (long long)max_n * max_n;
-  const int chunks = (int)std::max(1LL, std::min<long long>(kDiisChunksMax, (n2 + 2047) / 2048));
+  const int chunks = diis_chunks((long long)max_n * max_n);
   diis_partial_kernel<<<dim3(chunks, nlist), kDiisThreads, 0, s>>>(mols, mol_list, st, prm, P, Pold, hist_dens, hist_err,
                                                                   hist_stride, part, steps, ticket, trace, trace_len);
   diis_apply_kernel<<<dim3(chunks, nlist), kDiisThreads, 0, s>>>(mols, mol_list, st, prm, P, Pold, hist_dens,
@@ -441,8 +440,10 @@ void launch_diis(const DevMol* mols, const int* mol_list, int nlist, int max_n, 
 }
 
 // partial sums, decisions and tickets (zero between launches) of `slots` list entries
-size_t diis_scratch_bytes(int slots) {
-  return (size_t)slots * (kDiisChunksMax * kDiisPart * sizeof(double) + sizeof(DiisStep) + sizeof(int)) + 256;
+// of up to cap_n basis functions
+size_t diis_scratch_bytes(int slots, int cap_n) {
+  const size_t part = (size_t)diis_chunks((long long)cap_n * cap_n) * kDiisPart * sizeof(double);
+  return (size_t)slots * (part + sizeof(DiisStep) + sizeof(int)) + 256;
 }
 
 // ---------------------------------------------------------------------------
