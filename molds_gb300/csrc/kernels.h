@@ -136,8 +136,7 @@ constexpr int kPurEarly = 6;         // SCF iterations that get kPurBigSteps fro
 constexpr long long kPurWaitCycles = 2000000000LL;   // ~1 s: a copy or an MMA that has not completed by then never will
 struct PurState {
   unsigned long long lo, hi;         // Gershgorin interval, order-preserving keys
-  int bad;                           // 1 + the step in which a digit sum left the range its recombination covers
-                                     // or a wait ran out; 0: none
+  int bad;                           // a digit sum left the range its recombination covers, or a wait ran out
   long long trace[kPurBigSteps + 1]; // tr X_k
   unsigned long long steps;          // steps taken since Batch::profile_reset
 };

@@ -666,6 +666,15 @@ __device__ __forceinline__ int pu_first(const long long* T, int k) {
   return a ? __ffs(a) - 1 : (b ? __ffs(b) + 31 : -1);
 }
 
+// A tile of step k failed: the molecule's X is lost.  The steps after k learn it from
+// the trace that they read anyway (a flag of its own cost them 0.3 %; written during
+// the step, it would also let the threads of one CTA decide differently).
+constexpr long long kTraceFailed = 1LL << 60;   // traces are below N 2^43
+__device__ __forceinline__ void pu_failed(PurState& s, int k) {
+  atomicExch(&s.bad, 1);
+  atomicExch(reinterpret_cast<unsigned long long*>(&s.trace[k + 1]), (unsigned long long)(2 * kTraceFailed));
+}
+
 // One step of the molecules that still need one.  tiles: (molecule, row block,
 // column block, 0).  Warp 0 copies, warp 1 issues the MMAs, all sixteen
 // recombine.
@@ -686,16 +695,18 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();
   // every load before the first branch: one trip to L2 instead of three
-  const int status = st[mi].status, bad = pur[mi].bad;
+  const int status = st[mi].status;
   const long long t0 = pur[mi].trace[k], t1 = pur[mi].trace[k > 0 ? k - 1 : 0];
   double lo, hi;
   const bool usable = pu_interval(pur[mi], &lo, &hi);
   const int n = mol.nao, np = pu_np(n), first = pu_first(pur[mi].trace, k);
   const long long occ = (long long)mol.nocc * kTraceOne;
   const int op = pu_step(t0, t1, k, first, occ);   // the same in every CTA of the molecule
-  // bad: an earlier step's tile failed; those of this one write k + 1, so that all
-  // threads of a CTA decide alike whichever value they read
-  if (status != kActive || !usable || (bad > 0 && bad <= k) || op < 0) return;
+  const bool failed = t0 >= kTraceFailed;
+  if (status != kActive || !usable || op < 0 || failed) {
+    if (failed && threadIdx.x == 0) pur[mi].trace[k + 1] = 2 * kTraceFailed;
+    return;
+  }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = tile.y * kTileM, c0 = tile.z * TN;
   const int rows = min(kTileM, np - r0), cols = min(TN, np - c0);
@@ -793,7 +804,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     for (int c = max(0, issued - kStages); c < issued; ++c)
       pu_drain((warp == 0 ? full : empty) + 8 * (c % kStages), (c / kStages) & 1);
     if (tid == 0) {
-      atomicExch(&pur[mi].bad, k + 1);
+      pu_failed(pur[mi], k);
       atomicExch(err, 1);
     }
   } else {
@@ -801,7 +812,7 @@ purify_step_kernel(const DevMol* __restrict__ mols, const int4* __restrict__ til
     const bool mirror = tile.z >= (kTileM / TN) * (tile.y + 1);   // the transposed block is no tile of its own
     long long* xt = reinterpret_cast<long long*>(pu_sm);   // the operand stages are free now
     // rows past the padded basis are whatever the stage held before
-    if (r < np && !pu_in_range(range)) atomicExch(&pur[mi].bad, k + 1);
+    if (r < np && !pu_in_range(range)) pu_failed(pur[mi], k);
     long long tr = 0;
 #pragma unroll
     for (int s = 0; s < kGroups; ++s) {
