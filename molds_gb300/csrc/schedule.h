@@ -104,7 +104,7 @@ void run_blocks(int block, int max_iter, bool purified, EffortPlan plan, Iterate
     const int seen = last ? nblock - 1 : nblock - 2;
     const BlockCounts c = read(seen & 1);
     if (c.active == 0) break;
-    plan.seen(seen, c.waiting > 0, nblock);
+    if (purified) plan.seen(seen, c.waiting > 0, nblock);
   }
 }
 

@@ -33,6 +33,19 @@ def test_atom_needs_no_more_iterations_than_with_the_eigensolver(ctx, z):
     assert out[0][0] == M.STATUS_CONVERGED
 
 
+def test_repeated_runs_replay_one_graph_per_iteration(ctx):
+    """A second run with the same settings replays as many iterations as the first, for either solver."""
+    for solver in ("auto", "householder"):
+        b = M.ResidentBatch("pm3", [_atom(8), _atom(16)], context=ctx)
+        counts = []
+        for _ in range(2):
+            before = b.graph_launch_count()
+            b.run(M.SCFParams(eigensolver=solver))
+            counts.append(b.graph_launch_count() - before)
+        b.close()
+        assert counts[0] == counts[1]
+
+
 def test_atom_beside_molecules(ctx):
     """The same bits as alone, for the atom and for its neighbours of either kernel."""
     prm = M.SCFParams(damping_weight=0.0, diis_start_error=0.1, diis_end_error=0.0)
